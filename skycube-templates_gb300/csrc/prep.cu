@@ -182,11 +182,78 @@ __global__ void k_scatter(const uint32_t* __restrict__ keys,
 // quantiles only make the cells informative.
 constexpr int kPivotSample = 4096;
 
+// One compare-exchange stage of the bitonic sort below on a thread's four
+// consecutive elements e, e + 1, e + 2, e + 3 (e = 4 * thread): stride 1 and
+// 2 stay in the thread, strides 4 .. 64 meet lane ^ (stride / 4).
+template <int STRIDE>
+__device__ __forceinline__ void sort_stage(float (&v)[4], int e, int size) {
+  const bool up = (e & size) == 0;  // size >= 4: the same for all four
+  if constexpr (STRIDE >= 4) {
+    const bool take_min = ((e & STRIDE) == 0) == up;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float o = __shfl_xor_sync(0xffffffffu, v[j], STRIDE / 4);
+      v[j] = take_min ? fminf(v[j], o) : fmaxf(v[j], o);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j & STRIDE) continue;
+      const float lo = fminf(v[j], v[j | STRIDE]), hi = fmaxf(v[j], v[j | STRIDE]);
+      v[j] = up ? lo : hi;
+      v[j | STRIDE] = up ? hi : lo;
+    }
+  }
+}
+
+// Ascending bitonic sort of s[0 .. 4096) by 1,024 threads; s[cnt ..) holds
+// FLT_MAX, so only the smallest power of two >= cnt is sorted. A thread owns
+// four consecutive elements: strides up to 64 are exchanged in registers and
+// by shuffles inside the warp's 128 elements, only strides of 128 and more go
+// through shared memory (15 exchanges of the 78 stages, which a barrier per
+// stage made a chain of 78 barriers). k_pivots on one GB300: 26 -> 8.5 us.
+__device__ __forceinline__ void sort_sample(float* s, uint32_t cnt) {
+  const int e = 4 * threadIdx.x;
+  float v[4];
+  const float4 in = *reinterpret_cast<const float4*>(s + e);
+  v[0] = in.x; v[1] = in.y; v[2] = in.z; v[3] = in.w;
+  // size 2: pairs (0, 1) ascending, (2, 3) descending
+  {
+    const float a = fminf(v[0], v[1]), b = fmaxf(v[0], v[1]);
+    const float c = fmaxf(v[2], v[3]), d = fminf(v[2], v[3]);
+    v[0] = a; v[1] = b; v[2] = c; v[3] = d;
+  }
+  for (int size = 4; size <= kPivotSample && (uint32_t)(size >> 1) < cnt; size <<= 1) {
+    if (size > 128) {
+      for (int stride = size >> 1; stride >= 128; stride >>= 1) {
+        *reinterpret_cast<float4*>(s + e) = make_float4(v[0], v[1], v[2], v[3]);
+        __syncthreads();
+        const float4 o = *reinterpret_cast<const float4*>(s + (e ^ stride));
+        const bool take_min = ((e & stride) == 0) == ((e & size) == 0);
+        v[0] = take_min ? fminf(v[0], o.x) : fmaxf(v[0], o.x);
+        v[1] = take_min ? fminf(v[1], o.y) : fmaxf(v[1], o.y);
+        v[2] = take_min ? fminf(v[2], o.z) : fmaxf(v[2], o.z);
+        v[3] = take_min ? fminf(v[3], o.w) : fmaxf(v[3], o.w);
+        __syncthreads();
+      }
+    }
+    if (size >= 128) sort_stage<64>(v, e, size);
+    if (size >= 64) sort_stage<32>(v, e, size);
+    if (size >= 32) sort_stage<16>(v, e, size);
+    if (size >= 16) sort_stage<8>(v, e, size);
+    if (size >= 8) sort_stage<4>(v, e, size);
+    sort_stage<2>(v, e, size);
+    sort_stage<1>(v, e, size);
+  }
+  *reinterpret_cast<float4*>(s + e) = make_float4(v[0], v[1], v[2], v[3]);
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(1024) k_pivots(
     const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, int depth, float* __restrict__ pivots,
     unsigned long long* __restrict__ spread) {
-  __shared__ float s[kPivotSample];
+  __shared__ __align__(16) float s[kPivotSample];
   const int k = blockIdx.x;
   if (spread && k == 0 && threadIdx.x < 3) spread[threadIdx.x] = 0;  // k_cells adds to it
   const uint32_t m = *m_ptr;
@@ -201,22 +268,7 @@ __global__ void __launch_bounds__(1024) k_pivots(
     s[t] = v;
   }
   __syncthreads();
-  // bitonic sort, ascending
-  for (int size = 2; size <= kPivotSample; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < kPivotSample / 2; t += blockDim.x) {
-        const int lo = 2 * t - (t & (stride - 1));
-        const int hi = lo + stride;
-        const bool up = (lo & size) == 0;
-        const float a = s[lo], b = s[hi];
-        if ((a > b) == up) {
-          s[lo] = b;
-          s[hi] = a;
-        }
-      }
-      __syncthreads();
-    }
-  }
+  sort_sample(s, cnt);
   const int P = (1 << depth) - 1;
   for (int r = threadIdx.x; r < kMaxPivots; r += blockDim.x) {
     float v = FLT_MAX;
