@@ -272,12 +272,30 @@ constexpr int kDefaultChunk = 1;
 // Device-side result of the full-space step.
 struct FullSpace {
   uint4* cells = nullptr;    // by point id (depth of the call)
+  uint32_t* amin = nullptr;  // per attribute: ordered-uint minimum over all points
   uint32_t* sky = nullptr;   // full-space skyline ids, ascending
   uint32_t* ext = nullptr;   // full-space extended skyline ids, ascending
   uint32_t* cand = nullptr;  // union, ascending
   uint32_t* counts = nullptr;  // device [0]=|sky| [1]=|ext| [2]=|cand|
   uint32_t h_counts[3] = {0, 0, 0};
 };
+
+// Scratch of launch_partition_skyline for lists of up to mmax entries.
+static int part_scratch(Arena& A, uint64_t mmax, PartScratch* ps) {
+  const uint32_t Kmax = 1u << kMaxPartitionDims;
+  const uint64_t blocks = (mmax + 31) / 32;
+  SKC_TRY(A.alloc(&ps->keys, mmax));
+  SKC_TRY(A.alloc(&ps->sorted, mmax));
+  SKC_TRY(A.alloc(&ps->ccells, blocks * 32));
+  SKC_TRY(A.alloc(&ps->bmin, blocks));
+  SKC_TRY(A.alloc(&ps->smin, blocks * 4));
+  SKC_TRY(A.alloc(&ps->hmin, blocks * 8));
+  SKC_TRY(A.alloc(&ps->counts, Kmax + 1));
+  SKC_TRY(A.alloc(&ps->fine, kMaxSortBuckets + 1));
+  SKC_TRY(A.alloc(&ps->sums, kMaxScanSums));
+  SKC_TRY(A.alloc(&ps->splits, Kmax));
+  return A.alloc(&ps->item_off, Kmax + 1);
+}
 
 static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A,
                           FullSpace& F, Tracer& T) {
@@ -293,12 +311,9 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   float* pivots;
   SKC_TRY(A.alloc(&pivots, (uint64_t)kMaxDims * kMaxPivots));
   SKC_TRY(A.alloc(&F.cells, n));
-  // The cells kernel also sums the points' cell sums and their squares: the
-  // spread that picks the skyline kernel's order (partition.cu, gray_order).
-  unsigned long long* spread;
-  SKC_TRY(A.alloc(&spread, 3));
+  SKC_TRY(A.alloc(&F.amin, kMaxDims));
   SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, nullptr, d_n, n, depth, pivots, F.cells,
-                              spread));
+                              F.amin));
   T.mark("full: pivots+cells");
 
   // Pruner prefilter: the skyline kernel then runs over the survivors only
@@ -332,34 +347,12 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
 
   LevelTables LT;
   SKC_TRY(level_tables(ctx, partition_dims(full), &LT));
-  const uint32_t K = 1u << LT.B;
   PartScratch ps;
-  SKC_TRY(A.alloc(&ps.keys, n));
-  SKC_TRY(A.alloc(&ps.sorted, n));
-  SKC_TRY(A.alloc(&ps.ccells, n));
-  SKC_TRY(A.alloc(&ps.cx, (uint64_t)d * round_up(n, 128)));
-  if (n >= kConfirmedMinPoints) {
-    SKC_TRY(A.alloc(&ps.conf_cells, n));
-    SKC_TRY(A.alloc(&ps.conf_x, (uint64_t)d * round_up(n, 128)));
-    SKC_TRY(A.alloc(&ps.ccount, K));
-    SKC_TRY(A.alloc(&ps.pdone, K));
-  }
-  SKC_TRY(A.alloc(&ps.counts, K + 1));
-  SKC_TRY(A.alloc(&ps.cursor, kMaxSortBuckets + 1));
-  SKC_TRY(A.alloc(&ps.fine, kMaxSortBuckets + 1));
-  SKC_TRY(A.alloc(&ps.items, K + 1));
-  ps.spread = spread;
+  SKC_TRY(part_scratch(A, n, &ps));
   uint8_t* status;
   SKC_TRY(A.alloc(&status, round_up(n, 4)));
-  PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_list, n, full, status};
-  // Slices pay on candidate-dense lists (the survivors); on lists full of
-  // dominated points the slices after the strongest partitions would run to
-  // their end for points the first slice already settles.
-  if (list) {
-    pa.split_target = (uint32_t)ctx->num_sms * kSplitCtasPerSm;
-    pa.spread_ready = true;  // the spread of all n points picks the order
-  }
-  SKC_TRY(launch_partition_skyline(s, d, depth, LT, pa, ps));
+  PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_list, n, full, status, F.amin};
+  SKC_TRY(launch_partition_skyline(s, ctx->num_sms, d, depth, LT, pa, ps));
   T.mark("full: skyline kernel");
 
   const uint64_t nblk = (n + 1023) / 1024 + 1;
@@ -453,24 +446,23 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   // anticorrelated, bitmap kernel 29.6 -> 23.2 ms (binary pattern order)
   // -> 21.6 ms (Gray order).
   const uint32_t K = 1u << LT.B;
-  int sub_bits = 0;
-  while (sub_bits < 8 && ((uint64_t)K << (sub_bits + 1)) <= kMaxSortBuckets) ++sub_bits;
+  const int sub_bits = sort_sub_bits(m, K, std::min(8, d * (depth - 1)));
   const uint32_t KB = K << sub_bits;
   BucketScratch b;
-  uint32_t* boff;
+  uint32_t *boff, *sums;
   SKC_TRY(A.alloc(&b.keys, m));
-  SKC_TRY(A.alloc(&b.counts, KB + 1));
-  SKC_TRY(A.alloc(&b.cursor, KB + 1));
+  SKC_TRY(A.alloc(&b.counts, KB));
+  SKC_TRY(A.alloc(&sums, kMaxScanSums));
   SKC_TRY(A.alloc(&boff, K + 1));
   uint32_t *qperm, *qidx, *qids;
   SKC_TRY(A.alloc(&qperm, m));
   SKC_TRY(A.alloc(&qidx, m));
   SKC_TRY(A.alloc(&qids, m));
-  SKC_TRY(launch_mask_keys(s, cc, qpos, mq_ptr, m, nsub - 1, d, LT.B, depth, sub_bits,
-                           depth >= 2 ? 1 : 0,
-                           LT.rank, b.keys));
-  SKC_TRY(launch_counting_sort(s, b.keys, mq_ptr, m, KB, b, qperm, nullptr));
-  SKC_TRY(launch_partition_offsets(s, b.counts, K, sub_bits, boff));
+  SKC_CUDA(cudaMemsetAsync(b.counts, 0, KB * sizeof(uint32_t), s));
+  SKC_TRY(launch_mask_keys(s, cc, qpos, mq_ptr, m, nsub - 1, d, LT.B, depth, sub_bits, LT.rank,
+                           b.keys, b.counts));
+  SKC_TRY(launch_bucket_scan(s, b.counts, KB, sums, sub_bits, boff));
+  SKC_TRY(launch_scatter(s, b.keys, mq_ptr, m, b.counts, qperm));
   SKC_TRY(launch_gather_u32(s, qpos, qperm, mq_ptr, m, qidx));  // q order -> candidate position
   SKC_TRY(launch_gather_u32(s, F.cand, qidx, mq_ptr, m, qids));
   SKC_TRY(launch_gather_soa(s, ds->x, ds->n_pad, d, qids, mq_ptr, m, m_pad, xq));
@@ -592,22 +584,8 @@ struct CuboidScratch {
 };
 
 static int cuboid_scratch(Arena& A, int d, uint64_t mmax, CuboidScratch* cs) {
-  PartScratch& ps = cs->ps;
-  const uint32_t Kmax = 1u << kMaxPartitionDims;
-  SKC_TRY(A.alloc(&ps.keys, mmax));
-  SKC_TRY(A.alloc(&ps.sorted, mmax));
-  SKC_TRY(A.alloc(&ps.ccells, mmax));
-  SKC_TRY(A.alloc(&ps.cx, (uint64_t)d * round_up(mmax, 128)));
-  if (mmax >= kConfirmedMinPoints) {
-    SKC_TRY(A.alloc(&ps.conf_cells, mmax));
-    SKC_TRY(A.alloc(&ps.conf_x, (uint64_t)d * round_up(mmax, 128)));
-    SKC_TRY(A.alloc(&ps.ccount, Kmax));
-    SKC_TRY(A.alloc(&ps.pdone, Kmax));
-  }
-  SKC_TRY(A.alloc(&ps.counts, Kmax + 1));
-  SKC_TRY(A.alloc(&ps.cursor, kMaxSortBuckets + 1));
-  SKC_TRY(A.alloc(&ps.fine, kMaxSortBuckets + 1));
-  SKC_TRY(A.alloc(&ps.items, Kmax + 1));
+  (void)d;
+  SKC_TRY(part_scratch(A, mmax, &cs->ps));
   SKC_TRY(A.alloc(&cs->cand, mmax));
   SKC_TRY(A.alloc(&cs->status, round_up(mmax, 4)));
   SKC_TRY(A.alloc(&cs->d_m, 1));
@@ -628,8 +606,8 @@ static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Arena
   SKC_TRY(launch_set_u32(s, cs.d_m, (uint32_t)mc));
   LevelTables LT;
   SKC_TRY(level_tables(E.ctx, partition_dims(c), &LT));
-  PartitionSkylineArgs pa{cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status};
-  SKC_TRY(launch_partition_skyline(s, ds->d, depth, LT, pa, cs.ps));
+  PartitionSkylineArgs pa{cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status, F.amin};
+  SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, depth, LT, pa, cs.ps));
   SKC_TRY(A.alloc(osky, mc));
   SKC_TRY(A.alloc(oext, mc));
   SKC_TRY(launch_status_compact(s, cs.status, cand, cs.d_m, mc, 0, cs.blk0, cs.blk1, *osky,
@@ -1462,23 +1440,8 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
     const uint64_t m = F.h_counts[2];
     LevelTables LT;
     SKC_TRY(level_tables(E.ctx, partition_dims(S), &LT));
-    const uint32_t K = 1u << LT.B;
     PartScratch ps;
-    SKC_TRY(A.alloc(&ps.keys, m));
-    SKC_TRY(A.alloc(&ps.sorted, m));
-    SKC_TRY(A.alloc(&ps.ccells, m));
-    SKC_TRY(A.alloc(&ps.cx, (uint64_t)d * round_up(m, 128)));
-    SKC_TRY(A.alloc(&ps.counts, K + 1));
-    SKC_TRY(A.alloc(&ps.cursor, kMaxSortBuckets + 1));
-    SKC_TRY(A.alloc(&ps.fine, kMaxSortBuckets + 1));
-    SKC_TRY(A.alloc(&ps.items, K + 1));
-    SKC_TRY(A.alloc(&ps.spread, 3));
-    if (m >= kConfirmedMinPoints) {
-      SKC_TRY(A.alloc(&ps.conf_cells, m));
-      SKC_TRY(A.alloc(&ps.conf_x, (uint64_t)d * round_up(m, 128)));
-      SKC_TRY(A.alloc(&ps.ccount, K));
-      SKC_TRY(A.alloc(&ps.pdone, K));
-    }
+    SKC_TRY(part_scratch(A, m, &ps));
     uint8_t* status;
     uint32_t *blk0, *blk1, *cnt;
     SKC_TRY(A.alloc(&status, round_up(m, 4)));
@@ -1515,13 +1478,8 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
       list = surv;
       m_ptr = d_ns;
     }
-    PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_ptr, m, S, status};
-    if (filter) {
-      pa.split_target = (uint32_t)E.ctx->num_sms * kSplitCtasPerSm;
-      pa.spread_ids = F.cand;  // the spread of the candidates on S picks the order
-      pa.spread_m = F.counts + 2;
-    }
-    SKC_TRY(launch_partition_skyline(s, d, depth, LT, pa, ps));
+    PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_ptr, m, S, status, F.amin};
+    SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, d, depth, LT, pa, ps));
     SKC_TRY(launch_status_compact(s, status, list, m_ptr, m, 0, blk0, blk1, sky, ext, cnt, cnt + 1));
     uint32_t h[2] = {0, 0};
     SKC_TRY(copy_d2h(h, cnt, sizeof(h), s));

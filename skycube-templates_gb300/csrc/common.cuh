@@ -81,6 +81,14 @@ __host__ __device__ __forceinline__ uint32_t guard_mask(uint32_t S, int w) {
   return m;
 }
 
+#ifdef __CUDACC__
+// Order-preserving map of a float to uint32 (for integer minima and maxima).
+__device__ __forceinline__ uint32_t ordered_u32(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+#endif
+
 __host__ __device__ __forceinline__ uint32_t word_of(const uint4& v, int w) {
   return w == 0 ? v.x : (w == 1 ? v.y : (w == 2 ? v.z : v.w));
 }

@@ -28,10 +28,12 @@ int launch_bucket_order(cudaStream_t s, const float* x, uint64_t n_pad, int d,
 int launch_counting_sort(cudaStream_t s, const uint32_t* keys,
                          const uint32_t* m_ptr, uint64_t m_max, uint32_t K,
                          const BucketScratch& b, uint32_t* sorted, uint32_t* hi);
+int launch_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* m_ptr, uint64_t m_max,
+                   uint32_t* cursor, uint32_t* sorted);
 int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
                         uint64_t m_max, int depth, float* pivots, uint4* cells,
-                        unsigned long long* spread = nullptr);
+                        uint32_t* amin = nullptr);
 int launch_status_compact(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
                           const uint32_t* m_ptr, uint64_t m_max, int merge01,
                           uint32_t* blk0, uint32_t* blk1, uint32_t* out0,
@@ -88,7 +90,6 @@ int launch_skyline(cudaStream_t s, int d, const SkylineArgs& a);
 // value), its inverse, and for every mask the ranks of its submasks in
 // level order.
 constexpr int kMaxPartitionDims = 10;
-constexpr uint64_t kConfirmedMinPoints = 32768;
 constexpr uint64_t kMaxSortBuckets = 1u << 18;  // partition x strength buckets
 struct LevelTables {
   int B = 0;
@@ -98,25 +99,17 @@ struct LevelTables {
   const uint32_t* sub_list = nullptr;  // [3^B]
 };
 struct PartScratch {
-  uint32_t* keys;    // [m_max]
-  uint32_t* sorted;  // [m_max]
-  uint4* ccells;     // [m_max] compact cells in partition order
-  float* cx;         // [|S| * round_up(m_max, 128)] compact floats
-  // Confirmed lists (partition.cu), used for lists of at least
-  // kConfirmedMinPoints points; nullptr disables them.
-  uint4* conf_cells = nullptr;  // [m_max]
-  float* conf_x = nullptr;      // [|S| * round_up(m_max, 128)]
-  uint32_t* ccount = nullptr;   // [2^B]
-  uint32_t* pdone = nullptr;    // [2^B]
-  uint32_t* counts;  // [2^B + 1] partition offsets after the sort
-  uint32_t* fine;    // [kMaxSortBuckets + 1] counting-sort offsets
-  uint32_t* cursor;  // [kMaxSortBuckets + 1]
-  uint32_t* items;   // [2^B + 1]
-  // Spread of the cell sums of the list before the prefilter (sum, sum of
-  // squares, count), for sliced lists; nullptr: strength order, no tile box.
-  // Zeroed by k_pivots and filled by k_cells when launch_pivots_cells is
-  // given it.
-  unsigned long long* spread = nullptr;  // [3]
+  uint32_t* keys;      // [m_max]
+  uint32_t* sorted;    // [m_max]
+  uint4* ccells;       // [m_max, rounded up to 32] compact cells in partition order
+  uint4* bmin;         // [m_max / 32 + 1] minimum cells per 32-point block,
+  uint4* smin;         // [(m_max / 32 + 1) * 4] 8-point quarter
+  uint4* hmin;         // [(m_max / 32 + 1) * 8] and 4-point half
+  uint32_t* counts;    // [2^B + 1] partition offsets after the sort
+  uint32_t* fine;      // [kMaxSortBuckets + 1] counting-sort offsets, work counter
+  uint32_t* sums;      // [kMaxScanSums]
+  uint32_t* splits;    // [2^B]
+  uint32_t* item_off;  // [2^B + 1]
 };
 struct PartitionSkylineArgs {
   const uint32_t* ids;  // list position -> point id (nullptr: identity)
@@ -127,22 +120,23 @@ struct PartitionSkylineArgs {
   uint64_t m_max;
   uint32_t S;
   uint8_t* status;      // list position -> status; m_max rounded up to 4 bytes
-  uint32_t split_target = 0;  // CTAs the skyline kernel's work is cut into (0: no slicing)
-  // Sliced lists: the list whose cell-sum spread picks the order inside the
-  // partitions (point ids, nullptr: 0 .. count - 1; count on the device).
-  const uint32_t* spread_ids = nullptr;
-  const uint32_t* spread_m = nullptr;
-  bool spread_ready = false;  // PartScratch::spread already holds the spread
+  const uint32_t* amin; // [d] ordered-uint minima over a superset of the list
 };
-// Skyline kernel: CTAs per SM the work is balanced over (split_target).
-constexpr uint32_t kSplitCtasPerSm = 32;
+constexpr uint32_t kMaxScanSums = 64;  // kMaxSortBuckets / 4096
+// Skyline kernel: work items per SM the plan aims at (48 warps are resident).
+constexpr uint32_t kItemsPerSm = 256;
+constexpr int kMaxSubBits = 15;  // sub-key bits inside a partition
+int sort_sub_bits(uint64_t m_max, uint32_t K, int most);
 int launch_mask_keys(cudaStream_t s, const uint4* cells, const uint32_t* ids,
                      const uint32_t* m_ptr, uint64_t m_max, uint32_t S, int d,
-                     int B, int depth, int sub_bits, int sub_mode, const uint32_t* rank,
-                     uint32_t* keys);
-int launch_partition_offsets(cudaStream_t s, const uint32_t* fine, uint32_t K, int sub_bits,
-                             uint32_t* boff);
-int launch_partition_skyline(cudaStream_t s, int d, int depth,
+                     int B, int depth, int sub_bits, const uint32_t* rank,
+                     uint32_t* keys, uint32_t* counts);
+// Exclusive scan of counts[0 .. len) in place (len a power of two, at most
+// kMaxSortBuckets); boff[b] = offset of bucket b << sub_bits, boff[len >>
+// sub_bits] = the total.
+int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t* sums,
+                       int sub_bits, uint32_t* boff);
+int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth,
                              const LevelTables& T, const PartitionSkylineArgs& a,
                              const PartScratch& ps);
 

@@ -1,278 +1,274 @@
 // Median-partition skyline of a point list on one subspace S.
 //
-// Points are grouped by their median mask over the first B = min(|S|, 10)
-// attributes of S (bit j set when the point is worse than the median on that
-// attribute: the top bit of its grid cell). A point q can only dominate p
-// when q's mask is a subset of p's: on an attribute where q is above the
-// median and p is not, q is strictly worse. This is the partition test of
-// the suite's SkyAlign and Hybrid skylines (distribute_pitch_two_level_median,
+// Points are grouped by their median mask over the first B <= 10 attributes
+// of S (bit j set when the point is worse than the median on that attribute:
+// the top bit of its grid cell). A point q can only dominate p when q's mask
+// is a subset of p's: on an attribute where q is above the median and p is
+// not, q is strictly worse. This is the partition test of the suite's
+// SkyAlign and Hybrid skylines (distribute_pitch_two_level_median,
 // src/utilities/kernels.cu:99-125; canskip_partition, src/utilities/
 // SubTuple.h:69-73), applied here to whole partitions at once.
 //
 // Layout. A counting sort groups the list by the lattice-level rank of the
-// mask (popcount, then value), so partitions of stronger points come first.
-// One CTA owns up to 256 points of ONE partition (a work item); it visits
-// only the partitions whose mask is a subset of its own, in level order, and
-// streams their points through shared memory 256 at a time. Each thread
-// tests its point against every staged point with the grid-cell SWAR test
-// and, when cells tie, exact float32 comparisons (see skyline.cu). A
-// strictly dominated point stops; the CTA stops when all its points have.
+// mask (popcount, then value), so partitions of stronger points come first;
+// inside a partition points follow a Gray order of their quartile (then
+// finer) cell bits, so any run of them shares its quartile on most
+// attributes. The byte-wise minimum cells of every 32-point block, 8-point
+// quarter and 4-point half form a box tree over the sorted list.
+//
+// k_skyline_tree gives a warp up to 32 points of ONE partition (a work item)
+// and walks the tree under the submask partitions: a box whose minimum lies
+// above p's cell on some attribute holds no q that dominates p. See there.
 #include <algorithm>
 
 #include "kernels.cuh"
 
 namespace skc {
 
-// Order inside the partitions of a sliced skyline list. The strength order
-// (cell sum) lets a dominated point meet a dominator early; the Gray order
-// keeps q tiles' minimum-cell boxes tight, so whole tiles are skipped. Which
-// wins follows the spread of the points' cell sums: where they are
-// concentrated (anticorrelated data, points near a hyperplane) the strength
-// order carries little and the Gray order wins; where they spread as much
-// as independent attributes would, or more, the strength order wins.
-// Measured (skyline kernel, strength -> Gray + tile boxes): anticorrelated
-// 1M x 10 7.03 -> 5.99 ms, 400k x 12 3.77 -> 3.48 ms, 200k x 8 0.50 -> 0.44
-// ms (spread 0.51-0.62 of the independent value); uniform 1M x 10 1.74 ->
-// 1.80 ms, 500k x 16 6.38 -> 6.57 ms (1.01); correlated 1M x 10 2.47 ->
-// 3.61 ms, quantised 566k x 15 1.31 -> 1.93 ms (3.1-3.8). Only the
-// partition part of the key matters for correctness. With the choice made
-// on the device (both skyline instantiations launched, one returning at
-// once): anticorrelated 1M x 10 6.90 -> 5.93 ms, 400k x 12 3.74 -> 3.47 ms,
-// 500k x 16 8.48 -> 8.14 ms; the others within 1 %.
-constexpr double kGraySpread = 0.8;  // limit, as a fraction of the independent spread
-// Below this many points the choice is not made (strength order): the
-// second skyline launch it needs costs about 13 us, more than the Gray
-// order gains on such lists.
-constexpr uint64_t kSpreadMinPoints = 1u << 17;
-
-// spread[0] += sum over list entries of the cell sum over S, spread[1] += its
-// square, spread[2] = the count. Cell sums are at most 16 * 127, so both
-// sums fit 64 bits for any list of 32-bit length.
-__global__ void k_cell_spread(const uint4* __restrict__ cells, const uint32_t* __restrict__ ids,
-                              const uint32_t* __restrict__ m_ptr, uint32_t S, int d,
-                              unsigned long long* __restrict__ spread) {
-  const uint32_t m = *m_ptr;
-  unsigned long long s1 = 0, s2 = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += gridDim.x * blockDim.x) {
-    const uint4 c = cells[ids ? ids[i] : i];
-    uint32_t sum = 0;
-    for (int k = 0; k < d; ++k)
-      if (S & (1u << k)) sum += (word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu;
-    s1 += sum;
-    s2 += (unsigned long long)sum * sum;
-  }
-  for (int o = 16; o; o >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  if ((threadIdx.x & 31) == 0 && s1) {
-    atomicAdd(&spread[0], s1);
-    atomicAdd(&spread[1], s2);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) spread[2] = m;
-}
-
-// Gray order when the variance of the cell sums is below `limit`
-// (kGraySpread^2 times the variance of a sum of |S| independent uniform
-// cells). Every thread of the sort and skyline kernels evaluates it, so it
-// is single precision (FP64 is a slow pipe here: in double it cost 80 us on
-// 100k points); the variance is in the thousands and its rounding error
-// below 0.1.
-__device__ __forceinline__ bool gray_order(const unsigned long long* spread, float limit) {
-  const unsigned long long n = spread[2];
-  if (n < 2) return false;
-  const float inv = 1.0f / (float)n;
-  const float mean = (float)spread[0] * inv;
-  const float var = (float)spread[1] * inv - mean * mean;
-  return var < limit;
+static inline unsigned blocks_for(uint64_t items, int threads, int cap) {
+  uint64_t b = (items + threads - 1) / threads;
+  if (b < 1) b = 1;
+  if (b > (uint64_t)cap) b = cap;
+  return (unsigned)b;
 }
 
 // key[i] = rank of the median mask of list entry i over the first B
-// attributes of S, times 2^sub_bits, plus (when sub_bits > 0) the sum of its
-// grid cells over S scaled to sub_bits bits. Sorting by the key groups
-// points by partition and, inside a partition, from strong to weak, so
-// points that survive long share warps. With sub_mode 1 the sub-key orders
-// points by the quartile-cell bits (the cell bit below the median bit) of
-// the first sub_bits attributes of S, as a Gray code: a point's pattern is
-// ranked by its position in the reflected binary sequence (the prefix XOR of
-// its bits, attribute 0 most significant), so consecutive patterns differ in
-// one attribute and any run of them varies in few. Consecutive points then
-// share their quartile on most attributes, which keeps the minimum-cell
-// boxes of 32-point blocks tight. Only the partition part matters for
-// correctness. Sub_mode 2 takes the Gray order when the list's cell sums
-// are concentrated (gray_order below) and the strength order otherwise.
+// attributes of S, times 2^sub_bits, plus a sub-key: the cell bits below the
+// median bit, quartile bits of S's attributes first, then the next finer
+// ones, sub_bits in all, as a Gray code (a point's pattern is ranked by its
+// position in the reflected binary sequence, the prefix XOR of its bits, the
+// first bit most significant, so consecutive patterns differ in one bit and
+// any run of them varies in few). Consecutive points then share their
+// quartile on most attributes, which keeps the minimum-cell boxes of the
+// blocks tight. Only the partition part matters for correctness.
+// With `counts`, also the histogram of the keys (zeroed by the caller); with
+// `status`, zeroes the list's statuses.
 __global__ void k_mask_keys(const uint4* __restrict__ cells,
                             const uint32_t* __restrict__ ids,
                             const uint32_t* __restrict__ m_ptr, uint32_t S,
-                            int d, int B, int depth, int sub_bits, int sub_mode,
+                            int d, int B, int depth, int sub_bits,
                             const uint32_t* __restrict__ rank,
-                            uint32_t* __restrict__ keys,
-                            const unsigned long long* __restrict__ spread,
-                            float spread_limit) {
+                            uint32_t* __restrict__ keys, uint32_t* __restrict__ counts,
+                            uint8_t* __restrict__ status) {
   const uint32_t m = *m_ptr;
-  if (sub_mode == 2) sub_mode = gray_order(spread, spread_limit) ? 1 : 0;
   const int sh = depth - 1;
-  const uint32_t cmax = (1u << depth) - 1;
-  const uint32_t span = cmax * (uint32_t)__popc(S);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += gridDim.x * blockDim.x) {
     const uint32_t id = ids ? ids[i] : i;
     const uint4 c = cells[id];
-    uint32_t cm = 0, csum = 0, qpat = 0;
+    uint32_t cm = 0, g = 0;
     int j = 0;
-    for (int k = 0; k < d; ++k) {
+    for (int k = 0; k < d && j < B; ++k) {
       if (!(S & (1u << k))) continue;
       const uint32_t cell = (word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu;
-      if (j < B) cm |= ((cell >> sh) & 1u) << j;
-      if (j < sub_bits && sh >= 1) qpat |= ((cell >> (sh - 1)) & 1u) << (sub_bits - 1 - j);
-      csum += cell;
+      cm |= ((cell >> sh) & 1u) << j;
       ++j;
     }
-    uint32_t key = rank[cm] << sub_bits;
-    if (sub_mode == 1) {
-      uint32_t g = qpat;  // rank of qpat in the Gray sequence
-      for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;
-      key |= g;
+    int t = sub_bits;
+    for (int lv = sh - 1; lv >= 0 && t > 0; --lv) {
+      for (int k = 0; k < d && t > 0; ++k) {
+        if (!(S & (1u << k))) continue;
+        --t;
+        g |= ((word_of(c, k >> 2) >> (8 * (k & 3) + lv)) & 1u) << t;
+      }
     }
-    else if (sub_bits && span) key |= (csum * ((1u << sub_bits) - 1)) / span;
+    for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;  // rank in the Gray sequence
+    const uint32_t key = (rank[cm] << sub_bits) | g;
     keys[i] = key;
+    if (counts) atomicAdd(&counts[key], 1u);
+    if (status) status[i] = 0;
   }
 }
 
-// boff[b] = offsets[b << sub_bits] for b in [0, K]: partition offsets out of
-// the finer counting-sort offsets.
-__global__ void k_partition_offsets(const uint32_t* __restrict__ offsets, uint32_t K,
-                                    int sub_bits, uint32_t* __restrict__ boff) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= K;
-       b += gridDim.x * blockDim.x)
-    boff[b] = offsets[(uint64_t)b << sub_bits];
+// Exclusive scan of the bucket counts in two launches: a CTA per 4,096
+// buckets adds them up, then every CTA adds the sums before it (at most 64)
+// and scans its own 4,096 in place. The former single-CTA scan walked 2^18
+// buckets in 64 dependent tiles: 115 us on one GB300; these two: 5.
+// boff[b] = offset of bucket b << sub_bits, boff[K] = the total.
+constexpr uint32_t kScanTile = 4096;
+
+__global__ void __launch_bounds__(1024) k_bucket_sums(const uint32_t* __restrict__ counts,
+                                                      uint32_t* __restrict__ sums) {
+  __shared__ uint32_t red[32];
+  const uint4 v = reinterpret_cast<const uint4*>(counts)[(size_t)blockIdx.x * 1024 + threadIdx.x];
+  const uint32_t s = __reduce_add_sync(0xffffffffu, v.x + v.y + v.z + v.w);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const uint32_t t = __reduce_add_sync(0xffffffffu, red[threadIdx.x]);
+    if (threadIdx.x == 0) sums[blockIdx.x] = t;
+  }
 }
 
-// items[b] = number of 256-point work items of partition b.
-__global__ void k_chunk_counts(const uint32_t* __restrict__ boff, uint32_t K,
-                               uint32_t* __restrict__ items) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < K;
-       b += gridDim.x * blockDim.x)
-    items[b] = (boff[b + 1] - boff[b] + 255) / 256;
+__global__ void __launch_bounds__(1024) k_bucket_scan(uint32_t* __restrict__ counts, uint32_t len,
+                                                      const uint32_t* __restrict__ sums,
+                                                      int sub_bits, uint32_t* __restrict__ boff) {
+  __shared__ uint32_t wsum[32];
+  __shared__ uint32_t s_base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (wid == 0) {  // the CTAs before this one: at most kMaxSortBuckets / kScanTile = 64
+    uint32_t b = 0;
+    for (uint32_t j = lane; j < blockIdx.x; j += 32) b += sums[j];
+    b = __reduce_add_sync(0xffffffffu, b);
+    if (lane == 0) s_base = b;
+  }
+  const uint32_t base = blockIdx.x * kScanTile + 4 * threadIdx.x;
+  uint32_t v[4], local = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = base + j < len ? counts[base + j] : 0u;
+    local += v[j];
+  }
+  uint32_t incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) wsum[wid] = incl;
+  __syncthreads();
+  if (wid == 0) {
+    const uint32_t w = wsum[lane];
+    uint32_t sw = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, sw, o);
+      if (lane >= o) sw += u;
+    }
+    wsum[lane] = sw - w;
+  }
+  __syncthreads();
+  uint32_t run = s_base + wsum[wid] + incl - local;
+  const uint32_t smask = (1u << sub_bits) - 1u;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t i = base + j;
+    if (i < len) {
+      counts[i] = run;
+      if ((i & smask) == 0u) boff[i >> sub_bits] = run;
+      run += v[j];
+      if (i == len - 1) boff[len >> sub_bits] = run;
+    }
+  }
 }
 
-// Compact copy of a list in partition order, restricted to the k attributes
-// of S: cells repacked so attribute t of S sits in byte t % 4 of word t / 4,
-// and attribute-major floats xs[t * pitch + j].
-__global__ void k_gather_compact(const uint4* __restrict__ cells,
-                                 const float* __restrict__ x, uint64_t n_pad,
-                                 const uint32_t* __restrict__ ids,
-                                 const uint32_t* __restrict__ sorted,
-                                 const uint32_t* __restrict__ m_ptr, uint32_t S,
-                                 int d, uint64_t pitch,
-                                 uint4* __restrict__ out_cells,
-                                 float* __restrict__ out_x) {
+int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t* sums,
+                       int sub_bits, uint32_t* boff) {
+  const uint32_t g = (len + kScanTile - 1) / kScanTile;
+  if (g > 1) {  // then len is a multiple of the tile (both are powers of two)
+    k_bucket_sums<<<g, 1024, 0, s>>>(counts, sums);
+    SKC_LAUNCH_CHECK();
+  }
+  k_bucket_scan<<<g, 1024, 0, s>>>(counts, len, sums, sub_bits, boff);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
+// Places list entry i in its bucket (the scanned offsets are the cursors):
+// sorted[pos] = i and its cells restricted to S's attributes, attribute t of
+// S in byte t % 4 of word t / 4. The order inside a bucket is unspecified;
+// nothing depends on it. The last block is filled up with cells of 127.
+__global__ void k_part_scatter(const uint32_t* __restrict__ keys,
+                               const uint32_t* __restrict__ m_ptr,
+                               uint32_t* __restrict__ cursor, const uint4* __restrict__ cells,
+                               const uint32_t* __restrict__ ids, uint32_t S, int d,
+                               uint32_t* __restrict__ sorted, uint4* __restrict__ out_cells) {
   const uint32_t m = *m_ptr;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m;
-       j += gridDim.x * blockDim.x) {
-    const uint32_t pos = sorted[j];
-    const uint32_t id = ids ? ids[pos] : pos;
-    const uint4 c = cells[id];
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    const uint32_t i = m + threadIdx.x;
+    if (i < ((m + 31) & ~31u))
+      out_cells[i] = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
+  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
+       i += gridDim.x * blockDim.x) {
+    const uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);
+    const uint4 c = cells[ids ? ids[i] : i];
     uint32_t w[4] = {0, 0, 0, 0};
     int t = 0;
     for (int k = 0; k < d; ++k) {
       if (!(S & (1u << k))) continue;
       const uint32_t cell = (word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu;
-      w[t >> 2] |= cell << (8 * (t & 3));
-      out_x[(uint64_t)t * pitch + j] = x[(uint64_t)k * n_pad + id];
+      const uint32_t sv = cell << (8 * (t & 3));
+#pragma unroll
+      for (int j = 0; j < 4; ++j)  // constant indexes: w stays in registers
+        if ((t >> 2) == j) w[j] |= sv;
       ++t;
     }
-    out_cells[j] = make_uint4(w[0], w[1], w[2], w[3]);
+    sorted[pos] = i;
+    out_cells[pos] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
-struct PartKernelArgs {
-  // Confirmed lists (optional, see k_skyline_part): the points of partition b
-  // that are not strictly dominated, conf_*[boff[b] + k] for k < ccount[b],
-  // complete once pdone[b] equals b's number of work items.
-  uint4* conf_cells;
-  float* conf_x;
-  uint32_t* ccount;
-  uint32_t* pdone;
-  const uint32_t* sorted;   // sorted index -> list position (for the output)
-  const uint4* cells;       // compact cells in sorted order
-  const float* xs;          // compact floats in sorted order, pitch `pitch`
-  uint64_t pitch;
-  const uint32_t* boff;     // partition offsets in sorted order [K + 1]
-  const uint32_t* items;    // work item prefix per partition [K + 1]
-  const uint32_t* unrank;   // rank -> mask
-  const uint32_t* sub_off;  // mask -> range in sub_list
-  const uint32_t* sub_list; // ranks of submasks, level order
-  uint32_t K;
-  uint8_t* status;          // list position -> status (zeroed, 4-byte padded)
-  const uint32_t* splits;   // slices per work item of partition b [K]
-  const uint32_t* cta_off;  // first CTA of partition b [K + 1]
-  uint32_t lvl_mul;         // strength level = cell sum * lvl_mul / lvl_span
-  uint32_t lvl_span;        //   (the sort's sub-key, k_mask_keys); 0: no cut
-  // Sliced lists: the cell-sum spread and its limit (gray_order); when the
-  // partitions are in Gray order, q tiles are box-tested (nullptr: never).
-  const unsigned long long* spread;
-  float spread_limit;
-};
+constexpr uint32_t kMaxSplits = 255;
+constexpr uint64_t kMinSliceWork = 2048;  // q's: below this a slice is not worth an item
 
-// Cell sum of compact cells over NA attributes (the sort's strength level
-// is sum * lvl_mul / lvl_span, k_mask_keys).
-template <int NA>
-__device__ __forceinline__ uint32_t cell_sum_na(const uint4& c) {
-  uint32_t sum = 0;
+// CTA 0: the work items of the skyline kernel. An item of partition b is 32
+// of its points; its cost is the number of points in the partitions under
+// b's mask, work[b], the same for all of b's items and spread over orders of
+// magnitude. With W = max(total work / target, kMinSliceWork) every item of
+// b gets ceil(work[b] / W) slices (at most kMaxSplits); item_off is the
+// exclusive prefix of items * slices. The sums over the submask partitions
+// are one subset-sum transform over the B mask bits in shared memory (a
+// loop over each partition's submask list took 75 us at B = 10; 4 here).
+// The other CTAs: byte-wise minimum cells of the 32-q blocks, 8-q quarters
+// and 4-q halves of the sorted list (padded to whole blocks).
+__global__ void __launch_bounds__(1024) k_boxes_and_plan(
+    const uint4* __restrict__ cells, const uint32_t* __restrict__ m_ptr,
+    uint4* __restrict__ bmin, uint4* __restrict__ smin, uint4* __restrict__ hmin,
+    const uint32_t* __restrict__ boff, const uint32_t* __restrict__ rank,
+    const uint32_t* __restrict__ unrank, uint32_t K, int B, uint32_t target,
+    uint32_t* __restrict__ splits, uint32_t* __restrict__ item_off) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (blockIdx.x > 0) {
+    const uint32_t nblk = (*m_ptr + 31) / 32;
+    for (uint32_t b = (blockIdx.x - 1) * 32 + wid; b < nblk; b += (gridDim.x - 1) * 32) {
+      uint4 c = cells[(uint64_t)b * 32 + lane];
 #pragma unroll
-  for (int k = 0; k < NA; ++k) sum += (word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu;
-  return sum;
-}
-
-constexpr uint32_t kMaxSplits = 64;
-constexpr uint64_t kMinSliceWork = 256;  // q's (one tile): below this a slice is not worth a CTA
-
-// Work-proportional slicing of the skyline kernel's items (one CTA of 1024
-// threads, thread b = partition rank b). An item of partition b scans the
-// points of every partition under b's mask, so its cost is work[b] = their
-// count, the same for all of b's items. With W = max(total work / target,
-// kMinSliceWork), each item of b gets ceil(work[b] / W) slices (at most
-// kMaxSplits), so the heavy items of high-mask partitions no longer set the
-// kernel's duration. cta_off is the exclusive prefix of CTAs per partition.
-__global__ void __launch_bounds__(1024) k_split_plan(const uint32_t* __restrict__ boff,
-                                                     const uint32_t* __restrict__ items,
-                                                     const uint32_t* __restrict__ unrank,
-                                                     const uint32_t* __restrict__ sub_off,
-                                                     const uint32_t* __restrict__ sub_list,
-                                                     uint32_t K, uint32_t target,
-                                                     uint32_t* __restrict__ splits,
-                                                     uint32_t* __restrict__ cta_off) {
+      for (int o = 1; o < 32; o <<= 1) {
+        c.x = __vminu4(c.x, __shfl_xor_sync(0xffffffffu, c.x, o));
+        c.y = __vminu4(c.y, __shfl_xor_sync(0xffffffffu, c.y, o));
+        c.z = __vminu4(c.z, __shfl_xor_sync(0xffffffffu, c.z, o));
+        c.w = __vminu4(c.w, __shfl_xor_sync(0xffffffffu, c.w, o));
+        if (o == 2 && (lane & 3) == 0) hmin[(uint64_t)b * 8 + (lane >> 2)] = c;
+        if (o == 4 && (lane & 7) == 0) smin[(uint64_t)b * 4 + (lane >> 3)] = c;
+      }
+      if (lane == 0) bmin[b] = c;
+    }
+    return;
+  }
+  __shared__ uint32_t s_work[1024];
   __shared__ unsigned long long s_total;
   __shared__ uint32_t wsum[32];
-  const uint32_t b = threadIdx.x;
-  const int lane = b & 31, wid = b >> 5;
-  if (b == 0) s_total = 0;
+  const uint32_t t = threadIdx.x;
+  if (t == 0) s_total = 0;
+  if (t < K) {  // by mask
+    const uint32_t r = rank[t];
+    s_work[t] = boff[r + 1] - boff[r];
+  }
   __syncthreads();
+  for (int j = 0; j < B; ++j) {
+    if (t < K && (t & (1u << j))) s_work[t] += s_work[t ^ (1u << j)];
+    __syncthreads();
+  }
   unsigned long long work = 0;
   uint32_t chunks = 0;
-  if (b < K) {
-    const uint32_t mb = unrank[b];
-    for (uint32_t si = sub_off[mb]; si < sub_off[mb + 1]; ++si) {
-      const uint32_t qb = sub_list[si];
-      work += boff[qb + 1] - boff[qb];
-    }
-    chunks = items[b + 1] - items[b];
+  if (t < K) {  // by rank
+    work = s_work[unrank[t]];
+    chunks = (boff[t + 1] - boff[t] + 31) / 32;
     if (chunks) atomicAdd(&s_total, work * chunks);
   }
   __syncthreads();
-  const unsigned long long total = s_total;
-  unsigned long long W = target ? (total + target - 1) / target : ~0ull;
+  unsigned long long W = (s_total + target - 1) / target;
   if (W < kMinSliceWork) W = kMinSliceWork;
   uint32_t sb = 1;
-  if (b < K && target) {
+  if (t < K) {
     const unsigned long long q = (work + W - 1) / W;
     sb = (uint32_t)(q < 1 ? 1 : (q > kMaxSplits ? kMaxSplits : q));
+    splits[t] = sb;
   }
-  if (b < K) splits[b] = sb;
-  const uint32_t c = b < K ? chunks * sb : 0u;
+  const uint32_t c = chunks * sb;
   uint32_t inc = c;
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += u;
@@ -282,6 +278,7 @@ __global__ void __launch_bounds__(1024) k_split_plan(const uint32_t* __restrict_
   if (wid == 0) {
     const uint32_t v = wsum[lane];
     uint32_t vi = v;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t u = __shfl_up_sync(0xffffffffu, vi, o);
       if (lane >= o) vi += u;
@@ -290,535 +287,406 @@ __global__ void __launch_bounds__(1024) k_split_plan(const uint32_t* __restrict_
   }
   __syncthreads();
   const uint32_t excl = wsum[wid] + inc - c;
-  if (b < K) cta_off[b] = excl;
-  if (b == K - 1) cta_off[K] = excl + c;
+  if (t < K) item_off[t] = excl;
+  if (t == K - 1) item_off[K] = excl + c;
 }
 
-// NA = number of attributes of the subspace (all of them are compared).
-//
-// Confirmed lists. Work items start in lattice-level order, so the lower
-// partitions under a CTA's mask have often finished by the time it reaches
-// them. A finished partition is read through its confirmed list (its points
-// that are not strictly dominated) instead of all its points. That is exact:
-// if a strictly dominated q dominates p, the confirmed point that strictly
-// dominates q lies in a partition under p's mask as well and strictly
-// dominates p. Nothing waits: an unfinished partition is read in full. A CTA
-// publishes its confirmed points, fences, then counts itself in pdone.
-//
-// Slices (k_split_plan). An item of partition b is cut into splits[b] CTAs,
-// each taking an equal slice of the concatenated submask partitions; the
-// slices' statuses combine by a byte-wise atomic OR of bit flags (1
-// dominated, 2 strictly dominated; 3 reads as strictly dominated). A sliced
-// partition neither publishes nor uses confirmed lists (no CTA knows its
-// points' final status); the others still do.
-//
-// LV (level cutoffs, used on unsliced lists): a thread stops scanning a
-// sorted partition at the first q above its own strength level.
-constexpr uint32_t kFullMask = 0xffffffffu;
+struct TreeArgs {
+  const uint32_t* sorted;    // sorted index -> list position
+  const uint32_t* ids;       // list position -> point id (nullptr: identity)
+  const uint4* cells;        // compact cells in sorted order, padded to whole blocks
+  const uint4* bmin;         // per 32-q block: byte-wise minimum cells
+  const uint4* smin;         // per 8-q quarter
+  const uint4* hmin;         // per 4-q half
+  const float* x;            // attribute-major points
+  uint64_t n_pad;
+  unsigned long long attrs;  // attribute t of S in bits 4t .. 4t + 3
+  const uint32_t* amin;      // per attribute: ordered-uint minimum of a superset of the list
+  const uint32_t* boff;      // partition offsets in sorted order [K + 1]
+  const uint32_t* unrank;    // rank -> mask
+  const uint32_t* sub_off;   // mask -> range in sub_list
+  const uint32_t* sub_list;  // ranks of submasks, level order
+  uint32_t K;
+  const uint32_t* splits;    // slices per work item of partition b [K]
+  const uint32_t* item_off;  // first item of partition b [K + 1]
+  uint32_t* work;            // work counter, zero
+  uint8_t* status;           // list position -> status (zeroed, 4-byte padded)
+};
 
-// Up to 10 attributes the sliced variant holds 6 CTAs per SM (40 registers,
-// no spill; it had taken 48 and 5 CTAs): 1M x 10 anticorrelated full
-// skycube 28.4 -> 27.7 ms. Above 10 attributes the bound would spill, and
-// the unsliced level-cutoff variant (LV) keeps the free register budget.
-// BOX (sliced lists only): q tiles are box-tested. Both instantiations are
-// launched for a sliced list whose order follows the spread, and the one
-// that does not match the device's choice (gray_order) returns at once: a
-// runtime switch kept both paths' registers live and spilled at 40.
-template <int NA, bool LV, bool BOX>
-__global__ void __launch_bounds__(256, (!LV && NA <= 10) ? 6 : 1) k_skyline_part(PartKernelArgs a) {
+constexpr uint32_t kAll = 0xffffffffu;
+constexpr int kTreeWarps = 8;
+constexpr uint32_t kBlkQ = 40, kQuarQ = 48, kHalfQ = 40;  // per-warp stacks, entries
+
+// Guard bits where every cell of q is <= p's (pH: p's cells with the guard
+// bits set): kGuard when q may dominate p. Bytes beyond NA are 0 in both.
+template <int NW>
+__device__ __forceinline__ bool cells_le(const uint32_t (&pH)[NW], const uint4& q) {
+  uint32_t a = pH[0] - q.x;
+  if constexpr (NW > 1) a &= pH[1] - q.y;
+  if constexpr (NW > 2) a &= pH[2] - q.z;
+  if constexpr (NW > 3) a &= pH[3] - q.w;
+  return (a & kGuard) == kGuard;
+}
+
+// Skyline status of the list's points on S (NA attributes, all compared): a
+// warp takes a work item (32 points of one partition, or a slice of their
+// q's) from a device counter, heavy partitions first.
+//
+//  1. Blocks. The submask partitions' blocks form one list; 32 blocks per
+//     step, a lane each, are tested against the GROUP's byte-wise maximum
+//     cells. Open ones wait in a stack.
+//  2. Quarters. 8 waiting blocks' 32 quarters are tested against the group
+//     maximum, a lane each; for each open quarter all 32 points test its
+//     minimum with their own cells, a lane each. (point, quarter) pairs wait.
+//  3. Halves. 16 waiting pairs' halves, a lane each: (point, half) pairs wait.
+//  4. Walk. 8 waiting pairs, a lane per q: cells, and where cells tie the
+//     exact floats (read by point id: 1 to 2 q's per point get here on
+//     continuous data).
+//
+// The tests shared by the group and the pair stacks keep the 32 lanes busy
+// with tests that are open so far, where the form before (each thread its own
+// point against every q of a 32-q tile staged in shared memory) visited every
+// tile of the submask partitions: per point of 1M x 10 anticorrelated data
+// 561 blocks lie under its mask, 75 of their quarters are open, 34 halves,
+// and 2 q's pass the cell test. Bound by instruction issue. Full skyline
+// step (sort, boxes, kernel) on one GB300, before -> after: 1M x 10
+// anticorrelated 5.62 -> 1.25 ms, 500k x 16 anticorrelated 8.07 -> 1.52,
+// 1M x 12 uniform 4.08 -> 0.91, 581k x 10 ties 2.10 -> 0.27.
+//
+// A point that holds the list's minimum on some attribute of S cannot be
+// strictly dominated, so its first dominator settles it (status 1); one that
+// holds it on every attribute of S is not dominated at all. On tied data
+// nearly every remaining point is of the first kind (values clipped at the
+// range's end: 24,600 of 24,600 at 581k x 10 ties), and the walk over all
+// its weak dominators was the skyline kernel's whole time there; quantised
+// data has thousands of equal points of the second kind. amin may belong to
+// a superset of the list: a point of the list equal to it is its minimum.
+//
+// Slices of one item combine their statuses with a byte-wise atomic OR of
+// flags (1 dominated, 2 strictly dominated; 3 reads as strictly dominated).
+template <int NA>
+__global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a) {
   constexpr int NW = (NA + 3) / 4;
-  if (a.spread != nullptr && gray_order(a.spread, a.spread_limit) != BOX) return;
-  constexpr int TQ = 256;
-  __shared__ uint4 q_cells[TQ];
-  __shared__ float q_x[NA][TQ];
-  __shared__ uint16_t q_sum[LV ? TQ : 1];
+  __shared__ uint4 s_p[kTreeWarps][32];
+  __shared__ uint32_t s_bq[kTreeWarps][kBlkQ];
+  __shared__ uint2 s_sq[kTreeWarps][kQuarQ];  // (box id, point of the group)
+  __shared__ uint2 s_hq[kTreeWarps][kHalfQ];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  uint4* ps = s_p[wid];
+  uint32_t* bq = s_bq[wid];
+  uint2* sq = s_sq[wid];
+  uint2* hq = s_hq[wid];
+  const uint32_t n_items = a.item_off[a.K];
+  const uint32_t m = a.boff[a.K];
 
-  __shared__ uint32_t s_conf_end;
-  __shared__ unsigned long long s_total;
-  // CTAs go in partition rank order (lattice level: lower partitions first).
-  if (blockIdx.x >= a.cta_off[a.K]) return;
-  uint32_t lo = 0, hi = a.K;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a.cta_off[mid] <= blockIdx.x) lo = mid; else hi = mid;
-  }
-  const uint32_t b = lo;
-  const uint32_t splits = a.splits[b];
-  const uint32_t local = blockIdx.x - a.cta_off[b];
-  const uint32_t chunk = local / splits;
-  const uint32_t sp = local - chunk * splits;
-  const bool use_conf = a.conf_cells != nullptr && splits == 1;
-  const uint32_t pbeg = a.boff[b] + chunk * TQ;
-  const uint32_t pend = min(a.boff[b + 1], pbeg + TQ);
-  const uint32_t i = pbeg + threadIdx.x;
-  const bool valid = i < pend;
-
-  uint32_t hS[NW];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) hS[w] = guard_mask((1u << NA) - 1, w);
-  uint32_t pc[NW], pH[NW];
-  float pv[NA];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) pc[w] = pH[w] = 0;
-#pragma unroll
-  for (int k = 0; k < NA; ++k) pv[k] = 0.f;
-  uint4 my_cells = make_uint4(0, 0, 0, 0);
-  if (valid) {
-    my_cells = a.cells[i];
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(a.work, 1u);
+    it = __shfl_sync(kAll, it, 0);
+    if (it >= n_items) return;
+    it = n_items - 1 - it;  // the partitions with the most work first
+    uint32_t b = 0;
+    {
+      uint32_t hi = a.K;
+      while (hi - b > 1) {
+        const uint32_t mid = (b + hi) >> 1;
+        if (a.item_off[mid] <= it) b = mid; else hi = mid;
+      }
+    }
+    const uint32_t splits = a.splits[b];
+    const uint32_t local = it - a.item_off[b];
+    const uint32_t chunk = local / splits, sp = local - chunk * splits;
+    const uint32_t i = a.boff[b] + chunk * 32 + lane;
+    const bool valid = i < a.boff[b + 1];
+    uint4 pc = make_uint4(0, 0, 0, 0);
+    uint32_t pos = 0, id = 0;
+    if (valid) {
+      pc = a.cells[i];
+      pos = a.sorted[i];
+      id = a.ids ? a.ids[pos] : pos;
+    }
+    uint32_t pH[NW], gH[NW];  // own cells and the group's maximum, with guard bits
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
-      pc[w] = word_of(my_cells, w);
-      pH[w] = pc[w] | kGuard;
-    }
+      uint32_t g = word_of(pc, w);
+      pH[w] = g | kGuard;
 #pragma unroll
-    for (int k = 0; k < NA; ++k) pv[k] = a.xs[(uint64_t)k * a.pitch + i];
-  }
+      for (int o = 1; o < 32; o <<= 1) g = __vmaxu4(g, __shfl_xor_sync(kAll, g, o));
+      gH[w] = g | kGuard;
+    }
+    __syncwarp();  // the previous item's readers of ps are done
+    ps[lane] = pc;
+    // Attributes on which the point holds the list's minimum (its cell is then 0).
+    int n_min = 0;
+    if (valid) {
+#pragma unroll
+      for (int t = 0; t < NA; ++t) {
+        if (((word_of(pc, t >> 2) >> (8 * (t & 3))) & 0x7fu) == 0u) {
+          const uint32_t k = (uint32_t)(a.attrs >> (4 * t)) & 15u;
+          n_min += ordered_u32(a.x[(uint64_t)k * a.n_pad + id]) == a.amin[k];
+        }
+      }
+    }
+    const uint32_t no_strict = __ballot_sync(kAll, n_min > 0);
+    uint32_t dom = 0, strict = 0;  // per point of the group
+    uint32_t done = __ballot_sync(kAll, !valid || n_min == NA);
+    if (splits > 1) {  // settled by another slice already?
+      const uint32_t st = valid ? *(volatile const uint8_t*)(a.status + pos) : 0u;
+      done |= __ballot_sync(kAll, st >= 2u || (st && n_min));
+    }
+    __syncwarp();
 
-  uint8_t st = 0;
-  bool done = !valid;
-  // Sort-filter bound: a q that dominates p, even weakly, has every cell
-  // <= p's, so its cell sum and strength level are <= p's. Inside a
-  // partition q's ascend in level, so a thread is finished with the
-  // partition at the first q above its own level. level(q) > level(p)
-  // exactly when cellsum(q) >= sum_cut, the smallest sum of a higher level.
-  uint32_t sum_cut = 0xffffffffu;  // no cut without strength levels
-  if (LV && a.lvl_mul) {
-    const uint32_t plv = cell_sum_na<NA>(my_cells) * a.lvl_mul / a.lvl_span;
-    sum_cut = ((plv + 1) * a.lvl_span + a.lvl_mul - 1) / a.lvl_mul;
-  }
-  const uint32_t mb = a.unrank[b];
-  const uint32_t s0 = a.sub_off[mb], s1 = a.sub_off[mb + 1];
-  // This CTA's slice [s_lo, s_hi) of the concatenated submask partitions.
-  uint64_t s_lo = 0, s_hi = ~0ull;
-  if (splits > 1) {
-    if (threadIdx.x == 0) s_total = 0;
-    __syncthreads();
-    unsigned long long part = 0;
-    for (uint32_t si = s0 + threadIdx.x; si < s1; si += blockDim.x) {
-      const uint32_t qb = a.sub_list[si];
-      part += a.boff[qb + 1] - a.boff[qb];
-    }
-    if (part) atomicAdd(&s_total, part);
-    __syncthreads();
-    const uint64_t total = s_total;
-    s_lo = total * sp / splits;
-    s_hi = total * (sp + 1) / splits;
-  }
-  // Unsliced lists with level cutoffs stream q tiles per CTA (a thread stops
-  // at its level, so the CTA's tiles stay short); sliced lists stream them
-  // per warp. Measured both ways: the per-warp loop cost the per-cuboid
-  // form 800 -> 954 ms on 1M x 10, the per-CTA loop cost sliced lists up to
-  // 34 % (581k x 10 ties).
-  if constexpr (LV) {
-  bool all_done = false;
-  uint64_t acc = 0;  // q's of the partitions before si (uniform over the CTA)
-  for (uint32_t si = s0; si < s1 && !all_done && acc < s_hi; ++si) {
-    const uint32_t qb = a.sub_list[si];
-    uint32_t qbeg = a.boff[qb];
-    uint32_t qend = a.boff[qb + 1];
-    if (splits > 1) {
-      const uint64_t start = acc, sz = qend - qbeg;
-      acc += sz;
-      const uint64_t c0 = max(s_lo, start), c1 = min(s_hi, start + sz);
-      if (c0 >= c1) continue;
-      qend = qbeg + (uint32_t)(c1 - start);
-      qbeg = qbeg + (uint32_t)(c0 - start);
-    }
-    bool beyond = false;  // past this thread's level in this partition
-    bool conf = false;
-    if (use_conf && qb != b) {
-      if (threadIdx.x == 0) {
-        uint32_t e = 0xffffffffu;
-        const uint32_t need = a.items[qb + 1] - a.items[qb];
-        if (atomicAdd(&a.pdone[qb], 0u) == need) {
-          __threadfence();
-          e = qbeg + atomicAdd(&a.ccount[qb], 0u);
-        }
-        s_conf_end = e;
-      }
-      __syncthreads();
-      if (s_conf_end != 0xffffffffu) {
-        conf = true;
-        qend = s_conf_end;
-      }
-    }
-    const uint4* qc = conf ? a.conf_cells : a.cells;
-    const float* qxs = conf ? a.conf_x : a.xs;
-    bool first = true;
-    for (uint32_t base = qbeg; base < qend; base += TQ) {
-      // Without level cutoffs, or on a partition's first tile (nobody is
-      // beyond yet), the vote is "every point of the CTA is strictly
-      // dominated": the CTA is finished.
-      if (__syncthreads_and(done || (LV && beyond))) {
-        if (!LV || first) all_done = true;
-        break;
-      }
-      first = false;
-      const uint32_t j = base + threadIdx.x;
-      if (j < qend) {
-        // Confirmed lists are written during this launch by other SMs: read
-        // them through L2 (ld.cg), never from a possibly stale L1 line.
-        uint4 qcl;
-        if (conf) {
-          qcl = __ldcg(qc + j);
+    uint32_t bq_n = 0, sq_n = 0, hq_n = 0;
+    // Walk step over the top c (<= 8) waiting (point, half) pairs.
+    auto walk = [&](uint32_t c) {
+      const uint32_t slot = lane >> 2;
+      const uint2 e = hq[hq_n - c + min(slot, c - 1)];
+      hq_n -= c;
+      const uint32_t pi = e.y;
+      const uint32_t q = e.x * 4 + (lane & 3);
+      bool live = slot < c && !((done >> pi) & 1u) && q < m;
+      uint32_t Z = 0;  // equal cells (attribute bits)
+      bool any_lt = false, all_lt = true;
+      const uint4 q4 = a.cells[q];  // the cells are padded to whole blocks
+      const uint4 p4 = ps[pi];
+      uint32_t wH[NW];
 #pragma unroll
-          for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = __ldcg(qxs + (uint64_t)k * a.pitch + j);
-        } else {
-          qcl = qc[j];
+      for (int w = 0; w < NW; ++w) wH[w] = word_of(p4, w) | kGuard;
+      live = live && cells_le<NW>(wH, q4);
+      const uint32_t pid = __shfl_sync(kAll, id, pi);
+      if (live) {
 #pragma unroll
-          for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = qxs[(uint64_t)k * a.pitch + j];
-        }
-        q_cells[threadIdx.x] = qcl;
-        if constexpr (LV) q_sum[threadIdx.x] = (uint16_t)cell_sum_na<NA>(qcl);
-      }
-      __syncthreads();
-      if (!done && !(LV && beyond)) {
-        uint32_t lim = min((uint32_t)TQ, qend - base);
-        if (LV && !conf && sum_cut != 0xffffffffu) {
-          // First q of the tile above p's level (levels ascend in a sorted
-          // partition; confirmed lists are unordered and fully scanned).
-          uint32_t lo = 0, hi = lim;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (q_sum[mid] >= sum_cut) hi = mid; else lo = mid + 1;
-          }
-          if (lo < lim) {
-            lim = lo;
-            beyond = true;
-          }
-        }
-        for (uint32_t t = 0; t < lim; ++t) {
-          const uint4 q = q_cells[t];
-          uint32_t worse = 0;  // guard bits where cell(q) > cell(p)
-#pragma unroll
-          for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
-          if (worse) continue;
-          uint32_t not_less = 0;  // guard bits where cell(q) >= cell(p)
-#pragma unroll
-          for (int w = 0; w < NW; ++w)
-            not_less |= ge_bytes(word_of(q, w) | kGuard, pc[w]) & hS[w];
-          if (!not_less) {  // a smaller cell on every attribute: strict
-            st = 2;
-            done = true;
-            break;
-          }
-          bool le = true, lt_any = false, lt_all = true;
-#pragma unroll
-          for (int k = 0; k < NA; ++k) {
-            const float v = q_x[k][t];
-            le &= (v <= pv[k]);
-            lt_any |= (v < pv[k]);
-            lt_all &= (v < pv[k]);
-          }
-          if (le && lt_any) {
-            if (lt_all) {
-              st = 2;
-              done = true;
-              break;
-            }
-            st = 1;
+        for (int w = 0; w < NW; ++w)
+          Z |= pack_guards(ge_bytes(word_of(q4, w) | kGuard, word_of(p4, w))) << (4 * w);
+        Z &= (1u << NA) - 1u;
+        any_lt = Z != (1u << NA) - 1u;
+        if (Z) {
+          const uint32_t qpos = a.sorted[q];
+          const uint32_t qid = a.ids ? a.ids[qpos] : qpos;
+          for (uint32_t z = Z; z && live; z &= z - 1) {
+            const int t = __ffs(z) - 1;
+            const uint64_t row = ((a.attrs >> (4 * t)) & 15u) * a.n_pad;
+            const float qv = a.x[row + qid], pv = a.x[row + pid];
+            live = qv <= pv;
+            if (qv < pv) any_lt = true; else all_lt = false;
           }
         }
       }
-      __syncthreads();
-    }
-  }
-  } else {
-  uint64_t acc = 0;  // q's of the partitions before si
-  // Each warp streams the q's through its own 32-entry slice of the tile
-  // arrays and stops on its own: no CTA barrier inside the loop, so a warp
-  // whose points are all settled does not wait for the slowest warp.
-  const int lane = threadIdx.x & 31;
-  // In Gray order a tile's q's share their quartile on most attributes, so
-  // its byte-wise minimum cells often lie above a point's cell somewhere;
-  // a point below the minimum on some attribute is dominated by no q of the
-  // tile, and a tile no point of the warp can be dominated by is skipped.
-  // In strength order the boxes are loose and the test only costs
-  // (1M x 10 anticorrelated: 6.9 -> 8.3 ms).
-  constexpr bool box = BOX;
-  // With tile boxes a tile's floats are fetched only when some lane of the
-  // warp walks it (after the box test, so a tile every lane's box rejects is
-  // never read past its cells). Measured on anticorrelated data, full-space
-  // skyline, before -> after: 1M x 6 0.81 -> 0.77 ms, x 8 2.67 -> 2.48, x 9
-  // 4.60 -> 4.39, x 10 5.95 -> 5.83, 600k x 11 4.87 -> 4.37, 400k x 14
-  // 5.18 -> 4.80; slower at 400k x 12 (3.57 -> 3.63) and 300k x 16 (3.85
-  // -> 3.91), which load the floats with the cells as before.
-  constexpr bool defer_x = box && NA != 12 && NA != 16;
-  const uint32_t wbase = threadIdx.x & ~31u;  // this warp's slice
-  bool wdone = false;  // every point of the warp is settled
-  for (uint32_t si = s0; si < s1 && !wdone && acc < s_hi; ++si) {
-    const uint32_t qb = a.sub_list[si];
-    uint32_t qbeg = a.boff[qb];
-    uint32_t qend = a.boff[qb + 1];
-    if (splits > 1) {
-      const uint64_t start = acc, sz = qend - qbeg;
-      acc += sz;
-      const uint64_t c0 = max(s_lo, start), c1 = min(s_hi, start + sz);
-      if (c0 >= c1) continue;
-      qend = qbeg + (uint32_t)(c1 - start);
-      qbeg = qbeg + (uint32_t)(c0 - start);
-    }
-    bool beyond = false;  // past this thread's level in this partition
-    bool conf = false;
-    if (use_conf && qb != b) {
-      uint32_t e = 0xffffffffu;
-      if (lane == 0) {
-        const uint32_t need = a.items[qb + 1] - a.items[qb];
-        if (atomicAdd(&a.pdone[qb], 0u) == need) {
-          __threadfence();
-          e = qbeg + atomicAdd(&a.ccount[qb], 0u);
-        }
+      const bool d = live && any_lt;
+      if (__any_sync(kAll, d)) {
+        dom |= __reduce_or_sync(kAll, d ? 1u << pi : 0u);
+        strict |= __reduce_or_sync(kAll, (d && all_lt) ? 1u << pi : 0u);
+        done |= strict | (dom & no_strict);
       }
-      e = __shfl_sync(kFullMask, e, 0);
-      if (e != 0xffffffffu) {
-        __threadfence();  // the list's entries are read after its count
-        conf = true;
-        qend = e;
-      }
-    }
-    const uint4* qc = conf ? a.conf_cells : a.cells;
-    const float* qxs = conf ? a.conf_x : a.xs;
-    bool first = true;
-    for (uint32_t base = qbeg; base < qend; base += 32) {
-      // Without level cutoffs, or on a partition's first tile (nobody is
-      // beyond yet), the vote is "every point of the warp is strictly
-      // dominated": the warp is finished.
-      if (__all_sync(kFullMask, done || (LV && beyond))) {
-        if (!LV || first) wdone = true;
-        break;
-      }
-      first = false;
-      const uint32_t j = base + lane;
-      uint4 qcl = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
-      if (j < qend) {
-        // Confirmed lists are written during this launch by other SMs: read
-        // them through L2 (ld.cg), never from a possibly stale L1 line.
-        if constexpr (defer_x) {
-          qcl = conf ? __ldcg(qc + j) : qc[j];
-        } else if (conf) {
-          qcl = __ldcg(qc + j);
+      __syncwarp();  // read before a later push overwrites the entries
+    };
+    // Half step over the top c (<= 16) waiting (point, quarter) pairs.
+    auto half_step = [&](uint32_t c) {
+      const uint32_t slot = lane >> 1;
+      const uint2 e = sq[sq_n - c + min(slot, c - 1)];
+      sq_n -= c;
+      const uint32_t pi = e.y;
+      const uint32_t hid = e.x * 2 + (lane & 1);
+      const uint4 hm = a.hmin[hid];
+      const uint4 p4 = ps[pi];
+      uint32_t wH[NW];
 #pragma unroll
-          for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = __ldcg(qxs + (uint64_t)k * a.pitch + j);
-        } else {
-          qcl = qc[j];
-#pragma unroll
-          for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = qxs[(uint64_t)k * a.pitch + j];
-        }
-        q_cells[threadIdx.x] = qcl;
-        if constexpr (LV) q_sum[threadIdx.x] = (uint16_t)cell_sum_na<NA>(qcl);
-      }
-      bool box_out = false;  // no q of the tile dominates this point
-      if constexpr (box) {
-        uint32_t worse = 0;  // guard bits where the minimum cell is above p's
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {  // one word at a time: few live registers
-          uint32_t mn = word_of(qcl, w);
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) mn = __vminu4(mn, __shfl_xor_sync(kFullMask, mn, o));
-          worse |= ~(pH[w] - mn) & hS[w];
-        }
-        box_out = worse != 0;
-      }
-      const bool walk = !done && !(LV && beyond) && !box_out;
-      if constexpr (defer_x) {
-        if (__any_sync(kFullMask, walk) && j < qend) {
-          if (conf) {
-#pragma unroll
-            for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = __ldcg(qxs + (uint64_t)k * a.pitch + j);
-          } else {
-#pragma unroll
-            for (int k = 0; k < NA; ++k) q_x[k][threadIdx.x] = qxs[(uint64_t)k * a.pitch + j];
-          }
-        }
-      }
+      for (int w = 0; w < NW; ++w) wH[w] = word_of(p4, w) | kGuard;
+      const bool open = slot < c && !((done >> pi) & 1u) && cells_le<NW>(wH, hm);
+      const uint32_t om = __ballot_sync(kAll, open);
+      if (open) hq[hq_n + __popc(om & lt_mask)] = make_uint2(hid, pi);
+      hq_n += __popc(om);
       __syncwarp();
-      if (walk) {
-        uint32_t lim = min(32u, qend - base);
-        if (LV && !conf && sum_cut != 0xffffffffu) {
-          // First q of the tile above p's level (levels ascend in a sorted
-          // partition; confirmed lists are unordered and fully scanned).
-          uint32_t lo = 0, hi = lim;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (q_sum[wbase + mid] >= sum_cut) hi = mid; else lo = mid + 1;
-          }
-          if (lo < lim) {
-            lim = lo;
-            beyond = true;
-          }
-        }
-        for (uint32_t t = 0; t < lim; ++t) {
-          const uint4 q = q_cells[wbase + t];
-          uint32_t worse = 0;  // guard bits where cell(q) > cell(p)
-#pragma unroll
-          for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
-          if (worse) continue;
-          uint32_t not_less = 0;  // guard bits where cell(q) >= cell(p)
-#pragma unroll
-          for (int w = 0; w < NW; ++w)
-            not_less |= ge_bytes(word_of(q, w) | kGuard, pc[w]) & hS[w];
-          if (!not_less) {  // a smaller cell on every attribute: strict
-            st = 2;
-            done = true;
-            break;
-          }
-          bool le = true, lt_any = false, lt_all = true;
-#pragma unroll
-          for (int k = 0; k < NA; ++k) {
-            const float v = q_x[k][wbase + t];
-            le &= (v <= pv[k]);
-            lt_any |= (v < pv[k]);
-            lt_all &= (v < pv[k]);
-          }
-          if (le && lt_any) {
-            if (lt_all) {
-              st = 2;
-              done = true;
-              break;
-            }
-            st = 1;
-          }
-        }
-      }
+      while (hq_n >= 8) walk(8);
+    };
+    // Quarter step over the top c (<= 8) waiting blocks.
+    auto quarter_step = [&](uint32_t c) {
+      const uint32_t slot = lane >> 2;
+      const uint32_t sid = bq[bq_n - c + min(slot, c - 1)] * 4 + (lane & 3);
+      bq_n -= c;
+      const uint4 sm = a.smin[sid];
+      uint32_t qm = __ballot_sync(kAll, slot < c && cells_le<NW>(gH, sm));
       __syncwarp();
+      for (; qm; qm &= qm - 1) {
+        const int src = __ffs(qm) - 1;
+        uint4 q4;
+        q4.x = __shfl_sync(kAll, sm.x, src);
+        if constexpr (NW > 1) q4.y = __shfl_sync(kAll, sm.y, src);
+        if constexpr (NW > 2) q4.z = __shfl_sync(kAll, sm.z, src);
+        if constexpr (NW > 3) q4.w = __shfl_sync(kAll, sm.w, src);
+        const bool open = !((done >> lane) & 1u) && cells_le<NW>(pH, q4);
+        const uint32_t om = __ballot_sync(kAll, open);
+        if (!om) continue;
+        const uint32_t s = __shfl_sync(kAll, sid, src);
+        if (open) sq[sq_n + __popc(om & lt_mask)] = make_uint2(s, (uint32_t)lane);
+        sq_n += __popc(om);
+        __syncwarp();
+        while (sq_n >= 16) half_step(16);
+      }
+    };
+
+    const uint32_t mb = a.unrank[b];
+    const uint32_t s0 = a.sub_off[mb], s1 = a.sub_off[mb + 1];
+    // This slice's range [s_lo, s_hi) of the concatenated submask partitions.
+    uint32_t s_lo = 0, s_hi = kAll;
+    if (splits > 1) {
+      uint32_t part = 0;
+      for (uint32_t si = s0 + lane; si < s1; si += 32) {
+        const uint32_t qb = a.sub_list[si];
+        part += a.boff[qb + 1] - a.boff[qb];
+      }
+      const uint64_t total = __reduce_add_sync(kAll, part);
+      s_lo = (uint32_t)(total * sp / splits);
+      s_hi = (uint32_t)(total * (sp + 1) / splits);
     }
-  }
-  }
-  if (valid) {
-    const uint32_t pos = a.sorted[i];
-    if (splits == 1)
-      a.status[pos] = st;
-    else if (st)
-      atomicOr(reinterpret_cast<unsigned int*>(a.status + (pos & ~3u)),
-               (unsigned int)st << (8 * (pos & 3u)));
-  }
-  if (use_conf) {
-    if (valid && st != 2) {
-      const uint32_t slot = a.boff[b] + atomicAdd(&a.ccount[b], 1u);
-      a.conf_cells[slot] = my_cells;
+    uint32_t acc = 0;       // q's of the partitions before this step's
+    uint32_t next_blk = 0;  // blocks below this one were listed already
+    for (uint32_t si = s0; si < s1 && done != kAll && acc < s_hi; si += 32) {
+      uint32_t beg = 0, end = 0;
+      if (si + lane < s1) {
+        const uint32_t qb = a.sub_list[si + lane];
+        beg = a.boff[qb];
+        end = a.boff[qb + 1];
+      }
+      if (splits > 1) {  // cut to the slice
+        const uint32_t sz = end - beg;
+        uint32_t incl = sz;
 #pragma unroll
-      for (int k = 0; k < NA; ++k) a.conf_x[(uint64_t)k * a.pitch + slot] = pv[k];
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(kAll, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const uint32_t start = acc + incl - sz;
+        const uint32_t c0 = max(s_lo, start), c1 = min(s_hi, start + sz);
+        acc += __shfl_sync(kAll, incl, 31);
+        end = c0 < c1 ? beg + (c1 - start) : 0u;
+        beg = c0 < c1 ? beg + (c0 - start) : 0u;
+      }
+      // The partitions' blocks laid end to end; a block shared with the
+      // partition before is listed once (ranks, and so offsets, ascend).
+      const bool sel = beg < end;
+      const uint32_t be = (end + 31) / 32;
+      const uint32_t parts = __ballot_sync(kAll, sel);
+      if (!parts) continue;
+      const uint32_t lower = parts & lt_mask;
+      const uint32_t prev_be = __shfl_sync(kAll, be, lower ? 31 - __clz(lower) : 0);
+      const uint32_t bf = max(beg / 32, lower ? prev_be : next_blk);
+      const uint32_t cnt = (sel && be > bf) ? be - bf : 0u;
+      uint32_t incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kAll, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const uint32_t total = __shfl_sync(kAll, incl, 31);
+      next_blk = max(next_blk, __shfl_sync(kAll, be, 31 - __clz(parts)));
+      const uint32_t base = bf - (incl - cnt);  // list entry g of this lane is block g + base
+      for (uint32_t t0 = 0; t0 < total && done != kAll; t0 += 32) {
+        const uint32_t g = t0 + lane;
+        int j = 0;  // owner of list entry g: the first lane whose inclusive sum is > g
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+          const uint32_t v = __shfl_sync(kAll, incl, j + step - 1);
+          if (v <= g) j += step;
+        }
+        const uint32_t kb = g + __shfl_sync(kAll, base, j);
+        bool open = false;
+        if (g < total) open = cells_le<NW>(gH, a.bmin[kb]);
+        const uint32_t om = __ballot_sync(kAll, open);
+        if (open) bq[bq_n + __popc(om & lt_mask)] = kb;
+        bq_n += __popc(om);
+        __syncwarp();
+        while (bq_n >= 8) quarter_step(8);
+      }
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) atomicAdd(&a.pdone[b], 1u);
+    if (done != kAll) {  // what still waits: one short step of each kind
+      if (bq_n) quarter_step(bq_n);
+      if (sq_n) half_step(sq_n);
+      if (hq_n) walk(hq_n);
+    }
+    const uint32_t st = ((dom >> lane) & 1u) | (((strict >> lane) & 1u) << 1);
+    if (valid && st) {
+      if (splits == 1)
+        a.status[pos] = (uint8_t)(st & 2u ? 2u : 1u);
+      else
+        atomicOr(reinterpret_cast<unsigned int*>(a.status + (pos & ~3u)), st << (8 * (pos & 3u)));
+    }
   }
 }
-
-static inline unsigned blocks_for(uint64_t items, int threads, int cap);
 
 int launch_mask_keys(cudaStream_t s, const uint4* cells, const uint32_t* ids,
                      const uint32_t* m_ptr, uint64_t m_max, uint32_t S, int d,
-                     int B, int depth, int sub_bits, int sub_mode, const uint32_t* rank,
-                     uint32_t* keys) {
+                     int B, int depth, int sub_bits, const uint32_t* rank,
+                     uint32_t* keys, uint32_t* counts) {
   k_mask_keys<<<blocks_for(m_max, 256, 152 * 8), 256, 0, s>>>(cells, ids, m_ptr, S, d, B, depth,
-                                                               sub_bits, sub_mode, rank, keys,
-                                                               nullptr, 0.0f);
+                                                               sub_bits, rank, keys, counts,
+                                                               nullptr);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
-int launch_partition_offsets(cudaStream_t s, const uint32_t* fine, uint32_t K, int sub_bits,
-                             uint32_t* boff) {
-  k_partition_offsets<<<blocks_for(K + 1, 256, 64), 256, 0, s>>>(fine, K, sub_bits, boff);
+// Sub-key bits of a sort of up to m_max entries in K partitions: as many as
+// `most`, while the buckets stay within kMaxSortBuckets and about two per
+// entry (more only cost the scan).
+int sort_sub_bits(uint64_t m_max, uint32_t K, int most) {
+  int b = 0;
+  while (b < most && ((uint64_t)K << (b + 1)) <= kMaxSortBuckets &&
+         ((uint64_t)K << b) < m_max)
+    ++b;
+  return b;
+}
+
+template <int NA>
+static int launch_tree(cudaStream_t s, int num_sms, const TreeArgs& a) {
+  static_assert(NA >= 1 && NA <= kMaxDims, "attributes");
+  int per_sm = 0;
+  SKC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_skyline_tree<NA>,
+                                                         32 * kTreeWarps, 0));
+  k_skyline_tree<NA><<<std::max(1, per_sm) * num_sms, 32 * kTreeWarps, 0, s>>>(a);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
-static inline unsigned blocks_for(uint64_t items, int threads, int cap) {
-  uint64_t b = (items + threads - 1) / threads;
-  if (b < 1) b = 1;
-  if (b > (uint64_t)cap) b = cap;
-  return (unsigned)b;
-}
-
-int launch_partition_skyline(cudaStream_t s, int d, int depth,
-                             const LevelTables& T, const PartitionSkylineArgs& a,
-                             const PartScratch& ps) {
+int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, const LevelTables& T,
+                             const PartitionSkylineArgs& a, const PartScratch& ps) {
   const uint32_t K = 1u << T.B;
   const int na = __builtin_popcount(a.S);
-  // Strength order inside partitions: as many cell-sum levels as keep the
-  // counting sort at <= kMaxSortBuckets buckets.
-  int sub_bits = 0;
-  while (sub_bits < 8 && ((uint64_t)K << (sub_bits + 1)) <= kMaxSortBuckets) ++sub_bits;
+  const int sub_bits = sort_sub_bits(a.m_max, K, std::min(kMaxSubBits, na * (depth - 1)));
   const uint32_t KB = K << sub_bits;
-  BucketScratch bs;
-  bs.keys = ps.keys;
-  bs.counts = ps.fine;
-  bs.cursor = ps.cursor;
-  // Sliced lists: the order inside the partitions by the spread of the
-  // cell sums over the list before the prefilter (gray_order).
-  const bool by_spread = a.split_target && depth >= 2 && ps.spread &&
-                         (a.spread_m || a.spread_ready) && a.m_max >= kSpreadMinPoints;
-  const uint32_t c1 = 1u << depth;  // cells per attribute
-  const float spread_limit =
-      (float)(kGraySpread * kGraySpread * (double)na * ((double)c1 * c1 - 1.0) / 12.0);
-  if (by_spread && !a.spread_ready) {
-    SKC_CUDA(cudaMemsetAsync(ps.spread, 0, 3 * sizeof(unsigned long long), s));
-    k_cell_spread<<<blocks_for(a.m_max, 256, 152 * 4), 256, 0, s>>>(
-        a.cells, a.spread_ids, a.spread_m, a.S, d, ps.spread);
-    SKC_LAUNCH_CHECK();
-  }
-  k_mask_keys<<<blocks_for(a.m_max, 256, 152 * 8), 256, 0, s>>>(
-      a.cells, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits, by_spread ? 2 : 0, T.rank, ps.keys,
-      ps.spread, spread_limit);
+  uint32_t* work = ps.fine + KB;  // the skyline kernel's work counter, behind the buckets
+  SKC_CUDA(cudaMemsetAsync(ps.fine, 0, (KB + 1) * sizeof(uint32_t), s));
+  const unsigned grid = blocks_for(a.m_max, 256, 152 * 8);
+  k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits, T.rank,
+                                   ps.keys, ps.fine, a.status);
   SKC_LAUNCH_CHECK();
-  SKC_TRY(launch_counting_sort(s, ps.keys, a.m_ptr, a.m_max, KB, bs, ps.sorted, nullptr));
-  k_partition_offsets<<<blocks_for(K + 1, 256, 64), 256, 0, s>>>(ps.fine, K, sub_bits, ps.counts);
+  SKC_TRY(launch_bucket_scan(s, ps.fine, KB, ps.sums, sub_bits, ps.counts));
+  k_part_scatter<<<grid, 256, 0, s>>>(ps.keys, a.m_ptr, ps.fine, a.cells, a.ids, a.S, d,
+                                      ps.sorted, ps.ccells);
   SKC_LAUNCH_CHECK();
-  const uint64_t pitch = (a.m_max + 127) / 128 * 128;
-  k_gather_compact<<<blocks_for(a.m_max, 256, 152 * 8), 256, 0, s>>>(
-      a.cells, a.x, a.n_pad, a.ids, ps.sorted, a.m_ptr, a.S, d, pitch, ps.ccells, ps.cx);
+  // Items: enough slices that a warp takes several and the last ones are
+  // short (kItemsPerSm per SM, 48 warps resident).
+  k_boxes_and_plan<<<1 + blocks_for(a.m_max, 1024, 152 * 2), 1024, 0, s>>>(
+      ps.ccells, a.m_ptr, ps.bmin, ps.smin, ps.hmin, ps.counts, T.rank, T.unrank, K, T.B,
+      (uint32_t)num_sms * kItemsPerSm, ps.splits, ps.item_off);
   SKC_LAUNCH_CHECK();
-  k_chunk_counts<<<blocks_for(K, 256, 64), 256, 0, s>>>(ps.counts, K, ps.items);
-  SKC_LAUNCH_CHECK();
-  SKC_TRY(launch_scan_single_u32(s, ps.items, K));
-  // Slices per item and CTA offsets, in the counting sort's cursor scratch
-  // (free once the partition offsets are extracted): [0, K) and [K, 2K + 1).
-  uint32_t* splits = ps.cursor;
-  uint32_t* cta_off = ps.cursor + K;
-  k_split_plan<<<1, 1024, 0, s>>>(ps.counts, ps.items, T.unrank, T.sub_off, T.sub_list, K,
-                                  a.split_target, splits, cta_off);
-  SKC_LAUNCH_CHECK();
-  PartKernelArgs k{ps.conf_cells, ps.conf_x, ps.ccount, ps.pdone, ps.sorted, ps.ccells, ps.cx,
-                   pitch, ps.counts, ps.items, T.unrank, T.sub_off, T.sub_list, K, a.status,
-                   splits, cta_off,
-                   // Level cutoffs pay on lists full of dominated points (no
-                   // prefilter); on candidate-dense, sliced lists they only
-                   // cost (581k x 10 ties survivors: 3.05 -> 3.43 ms).
-                   a.split_target ? 0u : (1u << sub_bits) - 1u,
-                   ((1u << depth) - 1u) * (uint32_t)na,
-                   by_spread ? ps.spread : nullptr, spread_limit};
-  // Split CTAs OR their statuses in: start from zero (the buffer is padded
-  // to a multiple of 4 bytes).
-  SKC_CUDA(cudaMemsetAsync(a.status, 0, (a.m_max + 3) & ~3ull, s));
-  if (ps.conf_cells) {
-    SKC_CUDA(cudaMemsetAsync(ps.ccount, 0, K * sizeof(uint32_t), s));
-    SKC_CUDA(cudaMemsetAsync(ps.pdone, 0, K * sizeof(uint32_t), s));
-  }
-  // Upper bound of the CTAs k_split_plan hands out: sum over items of
-  // ceil(work / W) <= target + items.
-  const unsigned grid = (unsigned)((a.m_max + 255) / 256 + K + a.split_target);
-#define SKC_PART_CASE(N)                                           \
-  case N:                                                          \
-    if (k.lvl_mul) {                                               \
-      k_skyline_part<N, true, false><<<grid, 256, 0, s>>>(k);      \
-    } else {                                                       \
-      if (by_spread) k_skyline_part<N, false, true><<<grid, 256, 0, s>>>(k); \
-      k_skyline_part<N, false, false><<<grid, 256, 0, s>>>(k);     \
-    }                                                              \
-    break;
+  unsigned long long attrs = 0;
+  for (int k = 0, t = 0; k < d; ++k)
+    if (a.S & (1u << k)) attrs |= (unsigned long long)k << (4 * t++);
+  const TreeArgs k{ps.sorted, a.ids, ps.ccells, ps.bmin, ps.smin, ps.hmin, a.x, a.n_pad, attrs,
+                   a.amin, ps.counts, T.unrank, T.sub_off, T.sub_list, K, ps.splits, ps.item_off,
+                   work, a.status};
+#define SKC_TREE_CASE(N) \
+  case N: return launch_tree<N>(s, num_sms, k);
   switch (na) {
-    SKC_PART_CASE(1) SKC_PART_CASE(2) SKC_PART_CASE(3) SKC_PART_CASE(4)
-    SKC_PART_CASE(5) SKC_PART_CASE(6) SKC_PART_CASE(7) SKC_PART_CASE(8)
-    SKC_PART_CASE(9) SKC_PART_CASE(10) SKC_PART_CASE(11) SKC_PART_CASE(12)
-    SKC_PART_CASE(13) SKC_PART_CASE(14) SKC_PART_CASE(15) SKC_PART_CASE(16)
+    SKC_TREE_CASE(1) SKC_TREE_CASE(2) SKC_TREE_CASE(3) SKC_TREE_CASE(4)
+    SKC_TREE_CASE(5) SKC_TREE_CASE(6) SKC_TREE_CASE(7) SKC_TREE_CASE(8)
+    SKC_TREE_CASE(9) SKC_TREE_CASE(10) SKC_TREE_CASE(11) SKC_TREE_CASE(12)
+    SKC_TREE_CASE(13) SKC_TREE_CASE(14) SKC_TREE_CASE(15) SKC_TREE_CASE(16)
     default:
       return set_error(SKC_ERR_INVALID, "subspace with %d attributes", na);
   }
-#undef SKC_PART_CASE
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
+#undef SKC_TREE_CASE
 }
 
 }  // namespace skc

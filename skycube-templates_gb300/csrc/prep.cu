@@ -37,11 +37,6 @@ __global__ void k_iota(uint32_t* __restrict__ out, uint64_t n) {
     out[i] = (uint32_t)i;
 }
 
-// Order-preserving map of a float to uint32 (for atomic min/max).
-__device__ __forceinline__ uint32_t f2u_ordered(float f) {
-  uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 __device__ __forceinline__ float u2f_ordered(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
@@ -63,7 +58,7 @@ __global__ void k_score(const float* __restrict__ x, uint64_t n_pad,
     for (int k = 0; k < d; ++k)
       if (S & (1u << k)) s += x[(uint64_t)k * n_pad + id];
     f[i] = s;
-    const uint32_t u = f2u_ordered(s);
+    const uint32_t u = ordered_u32(s);
     lo = min(lo, u);
     hi = max(hi, u);
   }
@@ -175,6 +170,16 @@ __global__ void k_scatter(const uint32_t* __restrict__ keys,
   }
 }
 
+__global__ void k_scatter_cursor(const uint32_t* __restrict__ keys,
+                                 const uint32_t* __restrict__ m_ptr,
+                                 uint32_t* __restrict__ cursor,
+                                 uint32_t* __restrict__ sorted) {
+  const uint32_t m = *m_ptr;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
+       i += gridDim.x * blockDim.x)
+    sorted[atomicAdd(&cursor[keys[i]], 1u)] = i;
+}
+
 // --------------------------------------------------------------------------
 // Pivots: one CTA per attribute samples up to kPivotSample values of the
 // list (evenly strided), sorts them in shared memory and keeps
@@ -252,10 +257,10 @@ __device__ __forceinline__ void sort_sample(float* s, uint32_t cnt) {
 __global__ void __launch_bounds__(1024) k_pivots(
     const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, int depth, float* __restrict__ pivots,
-    unsigned long long* __restrict__ spread) {
+    uint32_t* __restrict__ amin) {
   __shared__ __align__(16) float s[kPivotSample];
   const int k = blockIdx.x;
-  if (spread && k == 0 && threadIdx.x < 3) spread[threadIdx.x] = 0;  // k_cells adds to it
+  if (amin && threadIdx.x == 0) amin[k] = 0xffffffffu;  // k_cells lowers it
   const uint32_t m = *m_ptr;
   const uint32_t cnt = m < kPivotSample ? m : kPivotSample;
   for (int t = threadIdx.x; t < kPivotSample; t += blockDim.x) {
@@ -277,52 +282,56 @@ __global__ void __launch_bounds__(1024) k_pivots(
   }
 }
 
-// cells[i] = grid cells of point ids[i] (see common.cuh).
-// With `spread`, also the sum and the sum of squares of the points' cell
-// sums and their count (k_cell_spread's layout, every attribute).
-__global__ void k_cells(const float* __restrict__ x, uint64_t n_pad,
-                        const uint32_t* __restrict__ ids,
-                        const uint32_t* __restrict__ m_ptr, int d, int depth,
-                        const float* __restrict__ pivots,
-                        uint4* __restrict__ cells,
-                        unsigned long long* __restrict__ spread) {
-  __shared__ float piv[kMaxDims * kMaxPivots];
-  for (int t = threadIdx.x; t < d * kMaxPivots; t += blockDim.x) piv[t] = pivots[t];
+// cells[i] = grid cells of point ids[i] (see common.cuh). With `amin`, also
+// lowers amin[k] to the ordered-uint minimum of attribute k over the list.
+// The D values are loaded before any search, and a search is `depth`
+// branch-free steps, so a thread has D independent chains in flight (the
+// runtime-d loop with a data-dependent search took 46 us on 1M x 10).
+template <int D>
+__global__ void __launch_bounds__(256) k_cells(
+    const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
+    const uint32_t* __restrict__ m_ptr, int depth, const float* __restrict__ pivots,
+    uint4* __restrict__ cells, uint32_t* __restrict__ amin) {
+  __shared__ float piv[D * kMaxPivots];
+  __shared__ uint32_t s_min[D];
+  for (int t = threadIdx.x; t < D * kMaxPivots; t += blockDim.x) piv[t] = pivots[t];
+  if (threadIdx.x < D) s_min[threadIdx.x] = 0xffffffffu;
   __syncthreads();
   const uint32_t m = *m_ptr;
-  const int P = (1 << depth) - 1;
-  unsigned long long s1 = 0, s2 = 0;
+  float mn[D];
+#pragma unroll
+  for (int k = 0; k < D; ++k) mn[k] = FLT_MAX;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += gridDim.x * blockDim.x) {
     const uint32_t id = ids ? ids[i] : i;
+    float v[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) v[k] = x[(uint64_t)k * n_pad + id];
+    uint32_t lo[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      lo[k] = 0;
+      mn[k] = fminf(mn[k], v[k]);
+    }
+    // The number of pivots below v, its bits from the highest down.
+    for (uint32_t step = 1u << (depth - 1); step; step >>= 1) {
+#pragma unroll
+      for (int k = 0; k < D; ++k)
+        if (piv[k * kMaxPivots + lo[k] + step - 1] < v[k]) lo[k] += step;
+    }
     uint32_t w[4] = {0, 0, 0, 0};
-    uint32_t sum = 0;
-    for (int k = 0; k < d; ++k) {
-      const float v = x[(uint64_t)k * n_pad + id];
-      const float* pk = piv + k * kMaxPivots;
-      int lo = 0, hi = P;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (pk[mid] < v) lo = mid + 1; else hi = mid;
-      }
-      w[k >> 2] |= (uint32_t)lo << (8 * (k & 3));
-      sum += (uint32_t)lo;
-    }
+#pragma unroll
+    for (int k = 0; k < D; ++k) w[k >> 2] |= lo[k] << (8 * (k & 3));
     cells[i] = make_uint4(w[0], w[1], w[2], w[3]);
-    s1 += sum;
-    s2 += (unsigned long long)sum * sum;
   }
-  if (spread) {
-    for (int o = 16; o; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    }
-    if ((threadIdx.x & 31) == 0 && s1) {
-      atomicAdd(&spread[0], s1);
-      atomicAdd(&spread[1], s2);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) spread[2] = m;
+  if (!amin) return;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const uint32_t u = __reduce_min_sync(0xffffffffu, ordered_u32(mn[k]));
+    if ((threadIdx.x & 31) == 0) atomicMin(&s_min[k], u);
   }
+  __syncthreads();
+  if (threadIdx.x < D) atomicMin(&amin[threadIdx.x], s_min[threadIdx.x]);
 }
 
 // --------------------------------------------------------------------------
@@ -621,16 +630,40 @@ int launch_counting_sort(cudaStream_t s, const uint32_t* keys,
   return SKC_OK;
 }
 
-int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
-                        const uint32_t* ids, const uint32_t* m_ptr,
-                        uint64_t m_max, int depth, float* pivots, uint4* cells,
-                        unsigned long long* spread) {
-  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, spread);
-  SKC_LAUNCH_CHECK();
-  k_cells<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(x, n_pad, ids, m_ptr, d, depth, pivots,
-                                                         cells, spread);
+template <int D>
+static int launch_cells(cudaStream_t s, const float* x, uint64_t n_pad, const uint32_t* ids,
+                        const uint32_t* m_ptr, uint64_t m_max, int depth, const float* pivots,
+                        uint4* cells, uint32_t* amin) {
+  k_cells<D><<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots,
+                                                            cells, amin);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
+}
+
+// Scatter whose scanned offsets are the cursors themselves (launch_bucket_scan).
+int launch_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* m_ptr, uint64_t m_max,
+                   uint32_t* cursor, uint32_t* sorted) {
+  k_scatter_cursor<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(keys, m_ptr, cursor, sorted);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
+int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
+                        const uint32_t* ids, const uint32_t* m_ptr,
+                        uint64_t m_max, int depth, float* pivots, uint4* cells, uint32_t* amin) {
+  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, amin);
+  SKC_LAUNCH_CHECK();
+  switch (d) {
+#define SKC_CELLS_CASE(D) \
+  case D: return launch_cells<D>(s, x, n_pad, ids, m_ptr, m_max, depth, pivots, cells, amin);
+    SKC_CELLS_CASE(2) SKC_CELLS_CASE(3) SKC_CELLS_CASE(4) SKC_CELLS_CASE(5) SKC_CELLS_CASE(6)
+    SKC_CELLS_CASE(7) SKC_CELLS_CASE(8) SKC_CELLS_CASE(9) SKC_CELLS_CASE(10) SKC_CELLS_CASE(11)
+    SKC_CELLS_CASE(12) SKC_CELLS_CASE(13) SKC_CELLS_CASE(14) SKC_CELLS_CASE(15)
+    SKC_CELLS_CASE(16)
+#undef SKC_CELLS_CASE
+    default:
+      return set_error(SKC_ERR_INVALID, "unsupported d=%d", d);
+  }
 }
 
 int launch_status_compact(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
