@@ -90,7 +90,8 @@ typedef struct skc_options {
                         skyline (-q; Config::pq_size, src/utilities/config.h:20):
                         > 0 that many, applied when n > 2 * pq_size as the
                         suite does (src/mdmc/MDMC.cu:251); < 0 off; 0 auto
-                        (default 512 when n >= 32768). Applied in two
+                        (default 128 from 32,768 points, 512
+                        from 700,000). Applied in two
                         passes: the strongest pq_size / 16 on every point,
                         the rest on the survivors when at least a quarter
                         of the points survive */

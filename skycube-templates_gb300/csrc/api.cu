@@ -276,9 +276,24 @@ struct FullSpace {
   uint32_t* sky = nullptr;   // full-space skyline ids, ascending
   uint32_t* ext = nullptr;   // full-space extended skyline ids, ascending
   uint32_t* cand = nullptr;  // union, ascending
+  uint8_t* cand_st = nullptr;   // per candidate: 0 full-space skyline, 2 dominated there
+  uint32_t* sky_pos = nullptr;  // positions of the skyline points among the candidates
   uint32_t* counts = nullptr;  // device [0]=|sky| [1]=|ext| [2]=|cand|
   uint32_t h_counts[3] = {0, 0, 0};
 };
+
+// Scratch of launch_prefilter for lists of up to mmax entries and Kq pruners.
+static int prefilter_scratch(Arena& A, int d, uint64_t mmax, uint32_t Kq, PrefilterScratch* pf) {
+  if (!pf->hist) SKC_TRY(A.alloc(&pf->hist, kSumBins + 8));
+  SKC_TRY(A.alloc(&pf->pr_ids, Kq));
+  SKC_TRY(A.alloc(&pf->pr_key, Kq));
+  SKC_TRY(A.alloc(&pf->pr_cells, Kq));
+  SKC_TRY(A.alloc(&pf->pr_x, (uint64_t)d * Kq));
+  SKC_TRY(A.alloc(&pf->blk0, (mmax + 1023) / 1024 + 2));
+  SKC_TRY(A.alloc(&pf->blk1, (mmax + 1023) / 1024 + 2));
+  SKC_TRY(A.alloc(&pf->mid, mmax));
+  return A.alloc(&pf->mid_count, 1);
+}
 
 // Scratch of launch_partition_skyline for lists of up to mmax entries.
 static int part_scratch(Arena& A, uint64_t mmax, PartScratch* ps) {
@@ -286,6 +301,7 @@ static int part_scratch(Arena& A, uint64_t mmax, PartScratch* ps) {
   const uint64_t blocks = (mmax + 31) / 32;
   SKC_TRY(A.alloc(&ps->keys, mmax));
   SKC_TRY(A.alloc(&ps->sorted, mmax));
+  SKC_TRY(A.alloc(&ps->sorted_id, mmax));
   SKC_TRY(A.alloc(&ps->ccells, blocks * 32));
   SKC_TRY(A.alloc(&ps->bmin, blocks));
   SKC_TRY(A.alloc(&ps->smin, blocks * 4));
@@ -312,36 +328,28 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(A.alloc(&pivots, (uint64_t)kMaxDims * kMaxPivots));
   SKC_TRY(A.alloc(&F.cells, n));
   SKC_TRY(A.alloc(&F.amin, kMaxDims));
+  PrefilterScratch pf{};
+  if (P.pq_size > 0) SKC_TRY(A.alloc(&pf.hist, kSumBins + 8));
   SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, nullptr, d_n, n, depth, pivots, F.cells,
-                              F.amin));
+                              F.amin, pf.hist));
   T.mark("full: pivots+cells");
 
-  // Pruner prefilter: the skyline kernel then runs over the survivors only
-  // (as point ids, ascending; their count stays on the device).
-  const uint32_t* list = nullptr;
-  const uint32_t* m_list = d_n;
+  // Pruner prefilter: the skyline kernel then runs over the points it leaves
+  // open only (ascending; their count stays on the device).
+  uint8_t* status;
+  SKC_TRY(A.alloc(&status, round_up(n, 4)));
+  const uint32_t* open = nullptr;
+  const uint32_t* m_open = d_n;
   if (P.pq_size > 0) {
     const uint32_t Kq = (uint32_t)P.pq_size;
-    const uint64_t nb = (n + 1023) / 1024 + 1;
-    PrefilterScratch pf;
-    SKC_TRY(A.alloc(&pf.hist, prefilter_sum_bins()));
-    SKC_TRY(A.alloc(&pf.sel, 8));
-    SKC_TRY(A.alloc(&pf.pr_ids, Kq));
-    SKC_TRY(A.alloc(&pf.pr_key, Kq));
-    SKC_TRY(A.alloc(&pf.pr_cells, Kq));
-    SKC_TRY(A.alloc(&pf.pr_x, (uint64_t)d * Kq));
-    SKC_TRY(A.alloc(&pf.st, n));
-    SKC_TRY(A.alloc(&pf.blk0, nb));
-    SKC_TRY(A.alloc(&pf.blk1, nb));
-    SKC_TRY(A.alloc(&pf.mid_ids, n));
-    SKC_TRY(A.alloc(&pf.mid_count, 1));
+    SKC_TRY(prefilter_scratch(A, d, n, Kq, &pf));
     uint32_t *surv, *d_ns;
     SKC_TRY(A.alloc(&surv, n));
     SKC_TRY(A.alloc(&d_ns, 1));
-    PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, nullptr, d_n, n, full, Kq, pf};
+    PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, nullptr, d_n, n, full, Kq, depth, F.amin, pf, status, true};
     SKC_TRY(launch_prefilter(s, d, ctx->num_sms, pfa, surv, d_ns));
-    list = surv;
-    m_list = d_ns;
+    open = surv;
+    m_open = d_ns;
     T.mark("full: prefilter");
   }
 
@@ -349,13 +357,12 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(level_tables(ctx, partition_dims(full), &LT));
   PartScratch ps;
   SKC_TRY(part_scratch(A, n, &ps));
-  uint8_t* status;
-  SKC_TRY(A.alloc(&status, round_up(n, 4)));
-  PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_list, n, full, status, F.amin};
+  PartitionSkylineArgs pa{open, nullptr, F.cells, ds->x, ds->n_pad, m_open, n, full, status,
+                          F.amin};
   SKC_TRY(launch_partition_skyline(s, ctx->num_sms, d, depth, LT, pa, ps));
   T.mark("full: skyline kernel");
 
-  const uint64_t nblk = (n + 1023) / 1024 + 1;
+  const uint64_t nblk = (n + 1023) / 1024 + 2;
   uint32_t *blk0, *blk1;
   SKC_TRY(A.alloc(&blk0, nblk));
   SKC_TRY(A.alloc(&blk1, nblk));
@@ -363,14 +370,14 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(A.alloc(&F.sky, n));
   SKC_TRY(A.alloc(&F.ext, n));
   SKC_TRY(A.alloc(&F.cand, n));
-  SKC_TRY(launch_status_compact(s, status, list, m_list, n, 0, blk0, blk1, F.sky, F.ext,
-                                F.counts + 0, F.counts + 1));
-  SKC_TRY(launch_status_compact(s, status, list, m_list, n, 1, blk0, blk1, F.cand, nullptr,
-                                F.counts + 2, nullptr));
+  SKC_TRY(A.alloc(&F.cand_st, n));
+  SKC_TRY(A.alloc(&F.sky_pos, n));
+  SKC_TRY(launch_status_split(s, status, nullptr, d_n, n, blk0, blk1, F.sky, F.ext, F.counts,
+                              F.cand, F.cand_st, F.sky_pos));
   if (E.plan) {
     // Plan mode: candidates sized by the plan's capacity (no read-back).
     const uint64_t cap = std::min<uint64_t>(E.plan->m_cap, n);
-    SKC_TRY(launch_cap_count(s, F.counts + 2, (uint32_t)cap, E.plan->stats, 0));
+    SKC_TRY(launch_cap_count(s, F.counts + 2, F.counts, (uint32_t)cap, E.plan->stats, 0));
     F.h_counts[0] = F.h_counts[1] = 0;
     F.h_counts[2] = (uint32_t)cap;
     return SKC_OK;
@@ -398,16 +405,16 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   float *xc, *xq;
   SKC_TRY(A.alloc(&xc, (uint64_t)d * m_pad));
   SKC_TRY(A.alloc(&xq, (uint64_t)d * m_pad));
-  SKC_TRY(launch_gather_soa(s, ds->x, ds->n_pad, d, F.cand, m_ptr, m, m_pad, xc));
   float* pivots;
   uint4 *cc, *qc, *bmin, *smin, *hmin;
   SKC_TRY(A.alloc(&pivots, (uint64_t)kMaxDims * kMaxPivots));
   SKC_TRY(A.alloc(&cc, m));
-  SKC_TRY(A.alloc(&qc, round_up(m, 32)));  // padded to whole blocks (k_pad_q)
+  SKC_TRY(A.alloc(&qc, round_up(m, 32)));  // padded to whole blocks (k_q_scatter)
   SKC_TRY(A.alloc(&bmin, (m + 31) / 32));
   SKC_TRY(A.alloc(&smin, (m + 31) / 32 * 4));
   SKC_TRY(A.alloc(&hmin, (m + 31) / 32 * 8));
-  SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, F.cand, m_ptr, m, depth, pivots, cc));
+  SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, F.cand, m_ptr, m, depth, pivots, cc,
+                              nullptr, nullptr, xc, m_pad));
 
   // q list: the full-space skyline only. If a point q' weakly dominates q
   // (q' <= q on every attribute), then for every p, LT(q, p) and LE(q, p)
@@ -417,20 +424,8 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   // they are nearly all candidates: 581k x 10 ties has 9 skyline points
   // among 24,446 candidates). q's are kept as positions in candidate order;
   // their count stays on the device.
-  uint32_t *qpos, *mq_ptr;
-  SKC_TRY(A.alloc(&qpos, m));
-  SKC_TRY(A.alloc(&mq_ptr, 1));
-  uint8_t* qst;  // per candidate: 0 full-space skyline, 2 dominated there
-  SKC_TRY(A.alloc(&qst, m));
-  {
-    const uint64_t nb = (m + 1023) / 1024 + 1;
-    uint32_t *b0, *b1;
-    SKC_TRY(A.alloc(&b0, nb));
-    SKC_TRY(A.alloc(&b1, nb));
-    SKC_TRY(launch_member_flags(s, F.cand, m_ptr, m, F.sky, F.counts + 0, qst));
-    SKC_TRY(launch_status_compact(s, qst, nullptr, m_ptr, m, 1, b0, b1, qpos, nullptr, mq_ptr,
-                                  nullptr));
-  }
+  const uint32_t* qpos = F.sky_pos;
+  const uint32_t* mq_ptr = F.counts + 0;
   // Host-side size of the q list (plans know only the candidate capacity).
   const uint64_t mq_host = E.plan ? m : F.h_counts[0];
 
@@ -448,33 +443,22 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   const uint32_t K = 1u << LT.B;
   const int sub_bits = sort_sub_bits(m, K, std::min(8, d * (depth - 1)));
   const uint32_t KB = K << sub_bits;
-  BucketScratch b;
-  uint32_t *boff, *sums;
-  SKC_TRY(A.alloc(&b.keys, m));
-  SKC_TRY(A.alloc(&b.counts, KB));
+  uint32_t *keys, *buckets, *boff, *sums;  // buckets[KB]: the bitmap kernel's work counter
+  SKC_TRY(A.alloc(&keys, m));
+  SKC_TRY(A.alloc(&buckets, KB + 1));
   SKC_TRY(A.alloc(&sums, kMaxScanSums));
   SKC_TRY(A.alloc(&boff, K + 1));
-  uint32_t *qperm, *qidx, *qids;
-  SKC_TRY(A.alloc(&qperm, m));
-  SKC_TRY(A.alloc(&qidx, m));
-  SKC_TRY(A.alloc(&qids, m));
-  SKC_CUDA(cudaMemsetAsync(b.counts, 0, KB * sizeof(uint32_t), s));
+  SKC_CUDA(cudaMemsetAsync(buckets, 0, (KB + 1) * sizeof(uint32_t), s));
   SKC_TRY(launch_mask_keys(s, cc, qpos, mq_ptr, m, nsub - 1, d, LT.B, depth, sub_bits, LT.rank,
-                           b.keys, b.counts));
-  SKC_TRY(launch_bucket_scan(s, b.counts, KB, sums, sub_bits, boff));
-  SKC_TRY(launch_scatter(s, b.keys, mq_ptr, m, b.counts, qperm));
-  SKC_TRY(launch_gather_u32(s, qpos, qperm, mq_ptr, m, qidx));  // q order -> candidate position
-  SKC_TRY(launch_gather_u32(s, F.cand, qidx, mq_ptr, m, qids));
-  SKC_TRY(launch_gather_soa(s, ds->x, ds->n_pad, d, qids, mq_ptr, m, m_pad, xq));
-  SKC_TRY(launch_gather_u4(s, cc, qidx, mq_ptr, m, qc));
-  SKC_TRY(launch_pad_q(s, mq_ptr, d, qc, xq, m_pad));
+                           keys, buckets));
+  SKC_TRY(launch_bucket_scan(s, buckets, KB, sums, sub_bits, boff));
+  SKC_TRY(launch_q_scatter(s, keys, mq_ptr, m, buckets, qpos, cc, xc, m_pad, d, qc, xq));
   SKC_TRY(launch_block_min(s, qc, mq_ptr, m, bmin, smin, hmin));
 
   T.mark("cand: cells+q order");
-  uint32_t *dom, *ext = nullptr, *work;
+  uint32_t *dom, *ext = nullptr, *work = buckets + KB;
   SKC_TRY(A.alloc(&dom, m * W));
   if (want_ext) SKC_TRY(A.alloc(&ext, m * W));
-  SKC_TRY(A.alloc(&work, 1));
 
   uint64_t slab_words = 0;
   uint32_t* slab = nullptr;
@@ -488,10 +472,9 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   // (want_bitmaps) keep the full computation.
   if (max_d <= d - 2 && !o.want_bitmaps) {
     ba.cap = max_d;
-    ba.full_dom = qst;
+    ba.full_dom = F.cand_st;
   }
   if (o.mode == SKC_MODE_BATCHED) {
-    SKC_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), s));
     SKC_TRY(launch_bitmaps(s, d, ctx->num_sms, ba));
   } else {
     // One launch per batch of points with a host round trip after each
@@ -589,10 +572,10 @@ static int cuboid_scratch(Arena& A, int d, uint64_t mmax, CuboidScratch* cs) {
   SKC_TRY(A.alloc(&cs->cand, mmax));
   SKC_TRY(A.alloc(&cs->status, round_up(mmax, 4)));
   SKC_TRY(A.alloc(&cs->d_m, 1));
-  const uint64_t nblk = (mmax + 1023) / 1024 + 1;
+  const uint64_t nblk = (mmax + 1023) / 1024 + 2;
   SKC_TRY(A.alloc(&cs->blk0, nblk));
   SKC_TRY(A.alloc(&cs->blk1, nblk));
-  SKC_TRY(A.alloc(&cs->cnt, 2));
+  SKC_TRY(A.alloc(&cs->cnt, 3));
   return SKC_OK;
 }
 
@@ -606,12 +589,12 @@ static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Arena
   SKC_TRY(launch_set_u32(s, cs.d_m, (uint32_t)mc));
   LevelTables LT;
   SKC_TRY(level_tables(E.ctx, partition_dims(c), &LT));
-  PartitionSkylineArgs pa{cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status, F.amin};
+  PartitionSkylineArgs pa{nullptr, cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status, F.amin};
   SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, depth, LT, pa, cs.ps));
   SKC_TRY(A.alloc(osky, mc));
   SKC_TRY(A.alloc(oext, mc));
-  SKC_TRY(launch_status_compact(s, cs.status, cand, cs.d_m, mc, 0, cs.blk0, cs.blk1, *osky,
-                                *oext, cs.cnt, cs.cnt + 1));
+  SKC_TRY(launch_status_split(s, cs.status, cand, cs.d_m, mc, cs.blk0, cs.blk1, *osky, *oext,
+                              cs.cnt));
   SKC_TRY(copy_d2h(cs.h_cnt, cs.cnt, 2 * sizeof(uint32_t), s));
   *nsky = cs.h_cnt[0];
   *next = cs.h_cnt[1];
@@ -1029,10 +1012,16 @@ static int auto_depth(uint64_t n, int d) {
 
 // Defaults of the work parameters (used when neither the options nor a
 // stored tuning set them).
-// Pruners: 512 in two passes (32 on every point, the rest on the survivors
-// when at least a quarter survive; prefilter.cu). The suite's -q default is
-// 128 (one pass).
-constexpr int kDefaultPruners = 512;
+// Pruners, in two passes (a 16th of them on every point, the rest on the
+// points left open when those are at least a quarter; prefilter.cu): 128, the
+// suite's -q default, up to 700,000 points, 512 above, where each further
+// pruner meets more dominated points. Prefilter + skyline kernel with 128 /
+// 512 pruners, ms on one GB300: 1M points: anticorrelated x 10 1.71 / 1.66, x
+// 6 0.52 / 0.47, uniform x 12 1.33 / 1.19; below: ties 581k x 10 0.09 / 0.11,
+// anticorrelated 500k x 16 1.67 / 1.81, uniform 200k x 9 0.20 / 0.24, 100k x 6
+// 0.12 / 0.15.
+constexpr uint64_t kManyPrunersMinPoints = 700000;
+static int default_pruners(uint64_t n) { return n >= kManyPrunersMinPoints ? 512 : 128; }
 constexpr uint64_t kPrefilterMinPoints = 32768;  // below: launch-bound anyway
 constexpr int kDefaultTilePoints = 256;
 
@@ -1136,7 +1125,7 @@ static int resolve_params(skc_dataset* ds, cudaStream_t s, const skc_options& o,
   P.depth = o.depth ? o.depth : have ? tv.depth : auto_depth(n, ds->d);
   int pq = 0;
   if (o.pq_size > 0) pq = o.pq_size;
-  else if (o.pq_size == 0) pq = have ? tv.pq_size : (n >= kPrefilterMinPoints ? kDefaultPruners : 0);
+  else if (o.pq_size == 0) pq = have ? tv.pq_size : (n >= kPrefilterMinPoints ? default_pruners(n) : 0);
   P.pq_size = (pq > 0 && n > 2ull * (uint64_t)pq) ? pq : 0;
   P.tile_points = o.tile_points ? o.tile_points : have ? tv.tile_points : kDefaultTilePoints;
   P.chunk = o.chunk ? o.chunk : have ? tv.chunk : kDefaultChunk;
@@ -1445,42 +1434,33 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
     uint8_t* status;
     uint32_t *blk0, *blk1, *cnt;
     SKC_TRY(A.alloc(&status, round_up(m, 4)));
-    const uint64_t nblk = (m + 1023) / 1024 + 1;
+    const uint64_t nblk = (m + 1023) / 1024 + 2;
     SKC_TRY(A.alloc(&blk0, nblk));
     SKC_TRY(A.alloc(&blk1, nblk));
-    SKC_TRY(A.alloc(&cnt, 2));
+    SKC_TRY(A.alloc(&cnt, 3));
     SKC_TRY(A.alloc(&sky, m));
     SKC_TRY(A.alloc(&ext, m));
-    const uint32_t* list = F.cand;
+    const uint32_t* open = nullptr;
     const uint32_t* m_ptr = F.counts + 2;
+    const uint32_t* m_open = m_ptr;
     const bool filter = P.pq_size > 0 && m > 2ull * (uint64_t)P.pq_size;
     if (filter) {
       // The prefilter on S over the full-space candidates (same argument as
       // in the full space: every dominator of a survivor on S survives).
       const uint32_t Kq = (uint32_t)P.pq_size;
-      PrefilterScratch pf;
-      SKC_TRY(A.alloc(&pf.hist, prefilter_sum_bins()));
-      SKC_TRY(A.alloc(&pf.sel, 8));
-      SKC_TRY(A.alloc(&pf.pr_ids, Kq));
-      SKC_TRY(A.alloc(&pf.pr_key, Kq));
-      SKC_TRY(A.alloc(&pf.pr_cells, Kq));
-      SKC_TRY(A.alloc(&pf.pr_x, (uint64_t)d * Kq));
-      SKC_TRY(A.alloc(&pf.st, m));
-      SKC_TRY(A.alloc(&pf.blk0, nblk));
-      SKC_TRY(A.alloc(&pf.blk1, nblk));
-      SKC_TRY(A.alloc(&pf.mid_ids, m));
-      SKC_TRY(A.alloc(&pf.mid_count, 1));
+      PrefilterScratch pf{};
+      SKC_TRY(prefilter_scratch(A, d, m, Kq, &pf));
       uint32_t *surv, *d_ns;
       SKC_TRY(A.alloc(&surv, m));
       SKC_TRY(A.alloc(&d_ns, 1));
-      PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, F.cand, m_ptr, m, S, Kq, pf};
+      PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, F.cand, m_ptr, m, S, Kq, depth, F.amin, pf, status, false};
       SKC_TRY(launch_prefilter(s, d, E.ctx->num_sms, pfa, surv, d_ns));
-      list = surv;
-      m_ptr = d_ns;
+      open = surv;
+      m_open = d_ns;
     }
-    PartitionSkylineArgs pa{list, F.cells, ds->x, ds->n_pad, m_ptr, m, S, status, F.amin};
+    PartitionSkylineArgs pa{open, F.cand, F.cells, ds->x, ds->n_pad, m_open, m, S, status, F.amin};
     SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, d, depth, LT, pa, ps));
-    SKC_TRY(launch_status_compact(s, status, list, m_ptr, m, 0, blk0, blk1, sky, ext, cnt, cnt + 1));
+    SKC_TRY(launch_status_split(s, status, F.cand, m_ptr, m, blk0, blk1, sky, ext, cnt));
     uint32_t h[2] = {0, 0};
     SKC_TRY(copy_d2h(h, cnt, sizeof(h), s));
     nsky = h[0];
@@ -2000,7 +1980,7 @@ int skc_autotune(skc_context* ctx, skc_dataset* ds, const skc_options* base, int
   cur.depth = o.depth ? o.depth : auto_depth(n, d);
   const int pq0 = o.pq_size > 0 ? o.pq_size
                   : o.pq_size < 0 ? 0
-                                  : (n >= kPrefilterMinPoints ? kDefaultPruners : 0);
+                                  : (n >= kPrefilterMinPoints ? default_pruners(n) : 0);
   cur.pq_size = (pq0 > 0 && n > 2ull * (uint64_t)pq0) ? pq0 : 0;
   cur.tile_points = o.tile_points ? o.tile_points : kDefaultTilePoints;
   cur.chunk = o.chunk ? o.chunk : kDefaultChunk;

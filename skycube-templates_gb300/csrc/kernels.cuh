@@ -20,7 +20,6 @@ struct BucketScratch {
 // prep.cu
 int launch_rows_to_soa(cudaStream_t s, const float* rows, uint64_t n, int d,
                        uint64_t n_pad, float* x, uint32_t* bad);
-int launch_iota(cudaStream_t s, uint32_t* out, uint64_t n);
 int launch_bucket_order(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
                         uint64_t m_max, uint32_t S, uint32_t K,
@@ -28,25 +27,28 @@ int launch_bucket_order(cudaStream_t s, const float* x, uint64_t n_pad, int d,
 int launch_counting_sort(cudaStream_t s, const uint32_t* keys,
                          const uint32_t* m_ptr, uint64_t m_max, uint32_t K,
                          const BucketScratch& b, uint32_t* sorted, uint32_t* hi);
-int launch_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* m_ptr, uint64_t m_max,
-                   uint32_t* cursor, uint32_t* sorted);
+constexpr uint32_t kSumBins = 2048;  // cell sums: 127 * 16 < 2048
 int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
                         uint64_t m_max, int depth, float* pivots, uint4* cells,
-                        uint32_t* amin = nullptr);
-int launch_status_compact(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
-                          const uint32_t* m_ptr, uint64_t m_max, int merge01,
-                          uint32_t* blk0, uint32_t* blk1, uint32_t* out0,
-                          uint32_t* out1, uint32_t* n0, uint32_t* n1);
-int launch_scan_single_u32(cudaStream_t s, uint32_t* a, uint32_t len);
+                        uint32_t* amin = nullptr, uint32_t* hist = nullptr,
+                        float* xout = nullptr, uint64_t out_pad = 0);
+// Entries of status 0 / 1 into sky / ext (ids in list order), n[0] / n[1]
+// their counts, n[2] the sum; with `both`, also their union in list order,
+// its entries' flags (0 for status 0, else 2) and the union positions of the
+// status-0 entries. blk0, blk1: [m_max / 1024 + 2].
+int launch_status_split(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
+                        const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* blk1,
+                        uint32_t* sky, uint32_t* ext, uint32_t* n, uint32_t* both = nullptr,
+                        uint8_t* both_st = nullptr, uint32_t* pos0 = nullptr);
+// List entries sub[i] (sub nullptr: i) of status 0 into out, *n their count;
+// blk0[b] holds the count over i in [1024 b, 1024 b + 1024) (zero past the list).
+int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
+                       const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* out,
+                       uint32_t* n);
 int launch_scan_u32_to_u64(cudaStream_t s, const uint32_t* in, uint64_t len,
                            uint64_t* bsum, uint64_t* out);
 uint64_t scan_bsum_entries(uint64_t len);
-int launch_gather_soa(cudaStream_t s, const float* x, uint64_t n_pad, int d,
-                      const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max,
-                      uint64_t out_pad, float* out);
-int launch_gather_u4(cudaStream_t s, const uint4* in, const uint32_t* perm,
-                     const uint32_t* m_ptr, uint64_t m_max, uint4* out);
 int launch_block_min(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr,
                      uint64_t m_max, uint4* bmin, uint4* smin, uint4* hmin);
 int launch_csr_gather(cudaStream_t s, const uint32_t* const* srcs,
@@ -54,20 +56,11 @@ int launch_csr_gather(cudaStream_t s, const uint32_t* const* srcs,
 int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v);
 int launch_merge_disjoint(cudaStream_t s, const uint32_t* a, uint32_t na,
                           const uint32_t* b, uint32_t nb, uint32_t* out);
-int launch_gather_u32(cudaStream_t s, const uint32_t* in, const uint32_t* perm,
-                      const uint32_t* m_ptr, uint64_t m_max, uint32_t* out);
-int launch_member_flags(cudaStream_t s, const uint32_t* list, const uint32_t* m_ptr,
-                        uint64_t m_max, const uint32_t* sorted_set, const uint32_t* nset_ptr,
-                        uint8_t* st);
-int launch_pad_q(cudaStream_t s, const uint32_t* mq_ptr, int d, uint4* qc, float* qx,
-                 uint64_t pitch);
 int launch_sample_signature(cudaStream_t s, const float* x, uint64_t n_pad, uint64_t n, int d,
                             uint32_t* out);
-int launch_cap_count(cudaStream_t s, uint32_t* m_ptr, uint32_t cap, uint64_t* stats, int slot);
+int launch_cap_count(cudaStream_t s, uint32_t* m_ptr, uint32_t* nsky_ptr, uint32_t cap,
+                     uint64_t* stats, int slot);
 int launch_stat_u64(cudaStream_t s, const uint64_t* src, uint64_t* stats, int slot);
-int launch_csr_assemble(cudaStream_t s, const uint32_t* src,
-                        const uint64_t* src_off, const uint64_t* dst_off,
-                        uint32_t ncub, uint32_t* dst);
 
 // skyline.cu: status of every list entry on subspace S (0 skyline,
 // 1 extended skyline, 2 strictly dominated).
@@ -100,7 +93,8 @@ struct LevelTables {
 };
 struct PartScratch {
   uint32_t* keys;      // [m_max]
-  uint32_t* sorted;    // [m_max]
+  uint32_t* sorted;    // [m_max] list positions in partition order
+  uint32_t* sorted_id; // [m_max] their point ids
   uint4* ccells;       // [m_max, rounded up to 32] compact cells in partition order
   uint4* bmin;         // [m_max / 32 + 1] minimum cells per 32-point block,
   uint4* smin;         // [(m_max / 32 + 1) * 4] 8-point quarter
@@ -112,14 +106,16 @@ struct PartScratch {
   uint32_t* item_off;  // [2^B + 1]
 };
 struct PartitionSkylineArgs {
+  const uint32_t* sub;  // the list's positions to settle, ascending (the prefilter's
+                        // survivors, whose statuses are 0 already); nullptr: all
   const uint32_t* ids;  // list position -> point id (nullptr: identity)
   const uint4* cells;   // point id -> grid cells
   const float* x;
   uint64_t n_pad;
-  const uint32_t* m_ptr;
+  const uint32_t* m_ptr;  // entries of `sub`, or of the list
   uint64_t m_max;
   uint32_t S;
-  uint8_t* status;      // list position -> status; m_max rounded up to 4 bytes
+  uint8_t* status;      // list position -> status; rounded up to 4 bytes
   const uint32_t* amin; // [d] ordered-uint minima over a superset of the list
 };
 constexpr uint32_t kMaxScanSums = 64;  // kMaxSortBuckets / 4096
@@ -136,24 +132,27 @@ int launch_mask_keys(cudaStream_t s, const uint4* cells, const uint32_t* ids,
 // sub_bits] = the total.
 int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t* sums,
                        int sub_bits, uint32_t* boff);
+int launch_q_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* mq_ptr, uint64_t m_max,
+                     uint32_t* cursor, const uint32_t* qpos, const uint4* pcells, const float* px,
+                     uint64_t pitch, int d, uint4* qcells, float* qx);
 int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth,
                              const LevelTables& T, const PartitionSkylineArgs& a,
                              const PartScratch& ps);
 
-// prefilter.cu: pruner prefilter of a list on subspace S. Survivors (the
-// entries no pruner strictly dominates) come out as point ids in list order.
+// prefilter.cu: pruner prefilter of a list on subspace S. Every list position
+// gets a status: 2 strictly dominated by a pruner, 1 dominated by one and
+// never strictly (it holds an attribute's minimum), 0 open. The open ones
+// come out as list positions, ascending.
 constexpr int kMaxPruners = 1024;
 struct PrefilterScratch {
-  uint32_t* hist;      // [prefilter_sum_bins()]
-  uint32_t* sel;       // [8]
+  uint32_t* hist;      // [kSumBins + 8] cell sums over S (see hist_ready), then counters
   uint32_t* pr_ids;    // [K]
   uint32_t* pr_key;    // [K]
   uint4* pr_cells;     // [K] pruner cells, rank order
   float* pr_x;         // [d * K] pruner floats, rank order
-  uint8_t* st;         // [m_max]
-  uint32_t* blk0;      // [m_max / 1024 + 1]
-  uint32_t* blk1;      // [m_max / 1024 + 1]
-  uint32_t* mid_ids;   // [m_max] survivors of the first pass
+  uint32_t* blk0;      // [m_max / 1024 + 2] kept entries per 1024, first pass
+  uint32_t* blk1;      // [m_max / 1024 + 2] and second pass
+  uint32_t* mid;       // [m_max] open positions after the first pass
   uint32_t* mid_count; // [1]
 };
 struct PrefilterArgs {
@@ -165,11 +164,14 @@ struct PrefilterArgs {
   uint64_t m_max;
   uint32_t S;
   uint32_t K;            // pruners, 1 .. kMaxPruners
+  int depth;             // grid depth of the cells
+  const uint32_t* amin;  // [d] ordered-uint minima over a superset of the list
   PrefilterScratch ps;
+  uint8_t* status;       // [m_max] by list position
+  bool hist_ready;       // ps.hist already holds the list's cell sums, its counters are 0
 };
 int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
-                     uint32_t* out_ids, uint32_t* out_count);
-uint32_t prefilter_sum_bins();
+                     uint32_t* out, uint32_t* out_count);
 size_t prefilter_smem(int d, uint32_t K);
 
 // mdmc.cu: per-point dominated-subspace bitmaps over the candidate set.

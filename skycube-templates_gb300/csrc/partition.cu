@@ -32,7 +32,7 @@ static inline unsigned blocks_for(uint64_t items, int threads, int cap) {
   return (unsigned)b;
 }
 
-// key[i] = rank of the median mask of list entry i over the first B
+// key[i] = rank of the median mask of list entry sub[i] (sub nullptr: i) over the first B
 // attributes of S, times 2^sub_bits, plus a sub-key: the cell bits below the
 // median bit, quartile bits of S's attributes first, then the next finer
 // ones, sub_bits in all, as a Gray code (a point's pattern is ranked by its
@@ -44,6 +44,7 @@ static inline unsigned blocks_for(uint64_t items, int threads, int cap) {
 // With `counts`, also the histogram of the keys (zeroed by the caller); with
 // `status`, zeroes the list's statuses.
 __global__ void k_mask_keys(const uint4* __restrict__ cells,
+                            const uint32_t* __restrict__ sub,
                             const uint32_t* __restrict__ ids,
                             const uint32_t* __restrict__ m_ptr, uint32_t S,
                             int d, int B, int depth, int sub_bits,
@@ -54,8 +55,8 @@ __global__ void k_mask_keys(const uint4* __restrict__ cells,
   const int sh = depth - 1;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += gridDim.x * blockDim.x) {
-    const uint32_t id = ids ? ids[i] : i;
-    const uint4 c = cells[id];
+    const uint32_t at = sub ? sub[i] : i;
+    const uint4 c = cells[ids ? ids[at] : at];
     uint32_t cm = 0, g = 0;
     int j = 0;
     for (int k = 0; k < d && j < B; ++k) {
@@ -164,15 +165,18 @@ int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t*
   return SKC_OK;
 }
 
-// Places list entry i in its bucket (the scanned offsets are the cursors):
-// sorted[pos] = i and its cells restricted to S's attributes, attribute t of
-// S in byte t % 4 of word t / 4. The order inside a bucket is unspecified;
-// nothing depends on it. The last block is filled up with cells of 127.
+// Places list entry sub[i] (sub nullptr: i) in its bucket (the scanned offsets
+// are the cursors): its list position, its point id and its cells restricted
+// to S's attributes, attribute t of S in byte t % 4 of word t / 4. The order
+// inside a bucket is unspecified; nothing depends on it. The last block is
+// filled up with cells of 127.
 __global__ void k_part_scatter(const uint32_t* __restrict__ keys,
                                const uint32_t* __restrict__ m_ptr,
                                uint32_t* __restrict__ cursor, const uint4* __restrict__ cells,
+                               const uint32_t* __restrict__ sub,
                                const uint32_t* __restrict__ ids, uint32_t S, int d,
-                               uint32_t* __restrict__ sorted, uint4* __restrict__ out_cells) {
+                               uint32_t* __restrict__ sorted, uint32_t* __restrict__ sorted_id,
+                               uint4* __restrict__ out_cells) {
   const uint32_t m = *m_ptr;
   if (blockIdx.x == 0 && threadIdx.x < 32) {
     const uint32_t i = m + threadIdx.x;
@@ -182,7 +186,9 @@ __global__ void k_part_scatter(const uint32_t* __restrict__ keys,
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += gridDim.x * blockDim.x) {
     const uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);
-    const uint4 c = cells[ids ? ids[i] : i];
+    const uint32_t at = sub ? sub[i] : i;
+    const uint32_t id = ids ? ids[at] : at;
+    const uint4 c = cells[id];
     uint32_t w[4] = {0, 0, 0, 0};
     int t = 0;
     for (int k = 0; k < d; ++k) {
@@ -194,13 +200,42 @@ __global__ void k_part_scatter(const uint32_t* __restrict__ keys,
         if ((t >> 2) == j) w[j] |= sv;
       ++t;
     }
-    sorted[pos] = i;
+    sorted[pos] = at;
+    sorted_id[pos] = id;
     out_cells[pos] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
+// The bitmap kernel's q's in their order: entry i of qpos (positions in
+// candidate order) goes to the next place of its bucket with its cells and
+// its floats. The last 32-q block is filled up with entries that add
+// nothing, so the kernel tests every lane of a block without a bounds check:
+// cells 127 and floats +inf. Such a q is worse than p on every attribute
+// where p's cell is below 127, and where p's cell is 127 too the float test
+// +inf <= p fails (inputs are finite), so LE = LT = {} for every p.
+__global__ void k_q_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ mq_ptr,
+                            uint32_t* __restrict__ cursor, const uint32_t* __restrict__ qpos,
+                            const uint4* __restrict__ pcells, const float* __restrict__ px,
+                            uint64_t pitch, int d, uint4* __restrict__ qcells,
+                            float* __restrict__ qx) {
+  const uint32_t mq = *mq_ptr;
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    const uint32_t i = mq + threadIdx.x;
+    if (i < ((mq + 31) & ~31u)) {
+      qcells[i] = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
+      for (int k = 0; k < d; ++k) qx[(uint64_t)k * pitch + i] = __int_as_float(0x7f800000);
+    }
+  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < mq; i += gridDim.x * blockDim.x) {
+    const uint32_t p = qpos[i];
+    const uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);
+    qcells[pos] = pcells[p];
+    for (int k = 0; k < d; ++k) qx[(uint64_t)k * pitch + pos] = px[(uint64_t)k * pitch + p];
+  }
+}
+
 constexpr uint32_t kMaxSplits = 255;
-constexpr uint64_t kMinSliceWork = 2048;  // q's: below this a slice is not worth an item
+constexpr uint64_t kMinSliceWork = 512;  // q's: below this a slice is not worth an item
 
 // CTA 0: the work items of the skyline kernel. An item of partition b is 32
 // of its points; its cost is the number of points in the partitions under
@@ -293,7 +328,7 @@ __global__ void __launch_bounds__(1024) k_boxes_and_plan(
 
 struct TreeArgs {
   const uint32_t* sorted;    // sorted index -> list position
-  const uint32_t* ids;       // list position -> point id (nullptr: identity)
+  const uint32_t* sorted_id; // sorted index -> point id
   const uint4* cells;        // compact cells in sorted order, padded to whole blocks
   const uint4* bmin;         // per 32-q block: byte-wise minimum cells
   const uint4* smin;         // per 8-q quarter
@@ -404,7 +439,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a)
     if (valid) {
       pc = a.cells[i];
       pos = a.sorted[i];
-      id = a.ids ? a.ids[pos] : pos;
+      id = a.sorted_id[i];
     }
     uint32_t pH[NW], gH[NW];  // own cells and the group's maximum, with guard bits
 #pragma unroll
@@ -462,8 +497,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a)
         Z &= (1u << NA) - 1u;
         any_lt = Z != (1u << NA) - 1u;
         if (Z) {
-          const uint32_t qpos = a.sorted[q];
-          const uint32_t qid = a.ids ? a.ids[qpos] : qpos;
+          const uint32_t qid = a.sorted_id[q];
           for (uint32_t z = Z; z && live; z &= z - 1) {
             const int t = __ffs(z) - 1;
             const uint64_t row = ((a.attrs >> (4 * t)) & 15u) * a.n_pad;
@@ -542,68 +576,82 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a)
     }
     uint32_t acc = 0;       // q's of the partitions before this step's
     uint32_t next_blk = 0;  // blocks below this one were listed already
-    for (uint32_t si = s0; si < s1 && done != kAll && acc < s_hi; si += 32) {
+    // Every slice but the first starts with the list's first block (the
+    // strongest points; partition 0 lies under every mask): on correlated
+    // and tied data it settles the group, which would else walk its slice to
+    // the end for points that the first slice settles at once.
+    bool probe = sp > 0;
+    for (uint32_t si = s0;;) {
       uint32_t beg = 0, end = 0;
-      if (si + lane < s1) {
-        const uint32_t qb = a.sub_list[si + lane];
-        beg = a.boff[qb];
-        end = a.boff[qb + 1];
-      }
-      if (splits > 1) {  // cut to the slice
-        const uint32_t sz = end - beg;
-        uint32_t incl = sz;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(kAll, incl, o);
-          if (lane >= o) incl += y;
+      if (probe) {
+        if (lane == 0) end = min(32u, m);
+      } else {
+        if (si + lane < s1) {
+          const uint32_t qb = a.sub_list[si + lane];
+          beg = a.boff[qb];
+          end = a.boff[qb + 1];
         }
-        const uint32_t start = acc + incl - sz;
-        const uint32_t c0 = max(s_lo, start), c1 = min(s_hi, start + sz);
-        acc += __shfl_sync(kAll, incl, 31);
-        end = c0 < c1 ? beg + (c1 - start) : 0u;
-        beg = c0 < c1 ? beg + (c0 - start) : 0u;
+        si += 32;
+        if (splits > 1) {  // cut to the slice
+          const uint32_t sz = end - beg;
+          uint32_t incl = sz;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kAll, incl, o);
+            if (lane >= o) incl += y;
+          }
+          const uint32_t start = acc + incl - sz;
+          const uint32_t c0 = max(s_lo, start), c1 = min(s_hi, start + sz);
+          acc += __shfl_sync(kAll, incl, 31);
+          end = c0 < c1 ? beg + (c1 - start) : 0u;
+          beg = c0 < c1 ? beg + (c0 - start) : 0u;
+        }
       }
       // The partitions' blocks laid end to end; a block shared with the
       // partition before is listed once (ranks, and so offsets, ascend).
       const bool sel = beg < end;
       const uint32_t be = (end + 31) / 32;
       const uint32_t parts = __ballot_sync(kAll, sel);
-      if (!parts) continue;
-      const uint32_t lower = parts & lt_mask;
-      const uint32_t prev_be = __shfl_sync(kAll, be, lower ? 31 - __clz(lower) : 0);
-      const uint32_t bf = max(beg / 32, lower ? prev_be : next_blk);
-      const uint32_t cnt = (sel && be > bf) ? be - bf : 0u;
-      uint32_t incl = cnt;
+      if (parts) {
+        const uint32_t lower = parts & lt_mask;
+        const uint32_t prev_be = __shfl_sync(kAll, be, lower ? 31 - __clz(lower) : 0);
+        const uint32_t bf = max(beg / 32, lower ? prev_be : next_blk);
+        const uint32_t cnt = (sel && be > bf) ? be - bf : 0u;
+        uint32_t incl = cnt;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kAll, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const uint32_t total = __shfl_sync(kAll, incl, 31);
-      next_blk = max(next_blk, __shfl_sync(kAll, be, 31 - __clz(parts)));
-      const uint32_t base = bf - (incl - cnt);  // list entry g of this lane is block g + base
-      for (uint32_t t0 = 0; t0 < total && done != kAll; t0 += 32) {
-        const uint32_t g = t0 + lane;
-        int j = 0;  // owner of list entry g: the first lane whose inclusive sum is > g
-#pragma unroll
-        for (int step = 16; step; step >>= 1) {
-          const uint32_t v = __shfl_sync(kAll, incl, j + step - 1);
-          if (v <= g) j += step;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(kAll, incl, o);
+          if (lane >= o) incl += y;
         }
-        const uint32_t kb = g + __shfl_sync(kAll, base, j);
-        bool open = false;
-        if (g < total) open = cells_le<NW>(gH, a.bmin[kb]);
-        const uint32_t om = __ballot_sync(kAll, open);
-        if (open) bq[bq_n + __popc(om & lt_mask)] = kb;
-        bq_n += __popc(om);
-        __syncwarp();
-        while (bq_n >= 8) quarter_step(8);
+        const uint32_t total = __shfl_sync(kAll, incl, 31);
+        if (!probe) next_blk = max(next_blk, __shfl_sync(kAll, be, 31 - __clz(parts)));
+        const uint32_t base = bf - (incl - cnt);  // list entry g of this lane is block g + base
+        for (uint32_t t0 = 0; t0 < total && done != kAll; t0 += 32) {
+          const uint32_t g = t0 + lane;
+          int j = 0;  // owner of list entry g: the first lane whose inclusive sum is > g
+#pragma unroll
+          for (int step = 16; step; step >>= 1) {
+            const uint32_t v = __shfl_sync(kAll, incl, j + step - 1);
+            if (v <= g) j += step;
+          }
+          const uint32_t kb = g + __shfl_sync(kAll, base, j);
+          bool open = false;
+          if (g < total) open = cells_le<NW>(gH, a.bmin[kb]);
+          const uint32_t om = __ballot_sync(kAll, open);
+          if (open) bq[bq_n + __popc(om & lt_mask)] = kb;
+          bq_n += __popc(om);
+          __syncwarp();
+          while (bq_n >= 8) quarter_step(8);
+        }
       }
-    }
-    if (done != kAll) {  // what still waits: one short step of each kind
-      if (bq_n) quarter_step(bq_n);
-      if (sq_n) half_step(sq_n);
-      if (hq_n) walk(hq_n);
+      const bool last = !probe && (si >= s1 || acc >= s_hi);
+      if ((probe || last) && done != kAll) {  // what still waits: one short step of each kind
+        if (bq_n) quarter_step(bq_n);
+        if (sq_n) half_step(sq_n);
+        if (hq_n) walk(hq_n);
+      }
+      if (last || done == kAll) break;
+      probe = false;
     }
     const uint32_t st = ((dom >> lane) & 1u) | (((strict >> lane) & 1u) << 1);
     if (valid && st) {
@@ -615,12 +663,21 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a)
   }
 }
 
+int launch_q_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* mq_ptr, uint64_t m_max,
+                     uint32_t* cursor, const uint32_t* qpos, const uint4* pcells, const float* px,
+                     uint64_t pitch, int d, uint4* qcells, float* qx) {
+  k_q_scatter<<<blocks_for(m_max, 256, 152 * 8), 256, 0, s>>>(keys, mq_ptr, cursor, qpos, pcells,
+                                                               px, pitch, d, qcells, qx);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
 int launch_mask_keys(cudaStream_t s, const uint4* cells, const uint32_t* ids,
                      const uint32_t* m_ptr, uint64_t m_max, uint32_t S, int d,
                      int B, int depth, int sub_bits, const uint32_t* rank,
                      uint32_t* keys, uint32_t* counts) {
-  k_mask_keys<<<blocks_for(m_max, 256, 152 * 8), 256, 0, s>>>(cells, ids, m_ptr, S, d, B, depth,
-                                                               sub_bits, rank, keys, counts,
+  k_mask_keys<<<blocks_for(m_max, 256, 152 * 8), 256, 0, s>>>(cells, nullptr, ids, m_ptr, S, d, B,
+                                                               depth, sub_bits, rank, keys, counts,
                                                                nullptr);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
@@ -657,12 +714,12 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, cons
   uint32_t* work = ps.fine + KB;  // the skyline kernel's work counter, behind the buckets
   SKC_CUDA(cudaMemsetAsync(ps.fine, 0, (KB + 1) * sizeof(uint32_t), s));
   const unsigned grid = blocks_for(a.m_max, 256, 152 * 8);
-  k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits, T.rank,
-                                   ps.keys, ps.fine, a.status);
+  k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.sub, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits,
+                                   T.rank, ps.keys, ps.fine, a.sub ? nullptr : a.status);
   SKC_LAUNCH_CHECK();
   SKC_TRY(launch_bucket_scan(s, ps.fine, KB, ps.sums, sub_bits, ps.counts));
-  k_part_scatter<<<grid, 256, 0, s>>>(ps.keys, a.m_ptr, ps.fine, a.cells, a.ids, a.S, d,
-                                      ps.sorted, ps.ccells);
+  k_part_scatter<<<grid, 256, 0, s>>>(ps.keys, a.m_ptr, ps.fine, a.cells, a.sub, a.ids, a.S, d,
+                                      ps.sorted, ps.sorted_id, ps.ccells);
   SKC_LAUNCH_CHECK();
   // Items: enough slices that a warp takes several and the last ones are
   // short (kItemsPerSm per SM, 48 warps resident).
@@ -673,7 +730,7 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, cons
   unsigned long long attrs = 0;
   for (int k = 0, t = 0; k < d; ++k)
     if (a.S & (1u << k)) attrs |= (unsigned long long)k << (4 * t++);
-  const TreeArgs k{ps.sorted, a.ids, ps.ccells, ps.bmin, ps.smin, ps.hmin, a.x, a.n_pad, attrs,
+  const TreeArgs k{ps.sorted, ps.sorted_id, ps.ccells, ps.bmin, ps.smin, ps.hmin, a.x, a.n_pad, attrs,
                    a.amin, ps.counts, T.unrank, T.sub_off, T.sub_list, K, ps.splits, ps.item_off,
                    work, a.status};
 #define SKC_TREE_CASE(N) \

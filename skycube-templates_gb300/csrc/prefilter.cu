@@ -9,13 +9,18 @@
 // is dropped as well. So every point that dominates or strictly dominates a
 // survivor is a survivor, and the skyline / extended-skyline status of each
 // survivor over the survivors equals its status over all points; dropped
-// points are strictly dominated, status 2.
+// points are strictly dominated, status 2. A point that no other can strictly
+// dominate (it holds an attribute's minimum) and that a pruner dominates has
+// status 1; what it dominates, strictly or not, a skyline point below it
+// dominates as well, so it is not needed as a dominator either and leaves
+// the list too.
 //
 // GB300 form. The norm is the cell sum over S (rank space, so attributes of
 // different scales weigh alike; the suite sums raw values). The K smallest
-// are picked without a sort: a 2048-bin histogram of cell sums (127 * 16 <
-// 2048), a one-block scan for the threshold bin, a collection pass, and a
-// one-block rank by (sum, id) so the strongest pruners are tried first.
+// are picked without a sort: a 2048-bin histogram of cell sums (for the full
+// space the cells kernel makes it), a collection pass that finds the
+// threshold bin first, and a one-block rank by (sum, id) so the strongest
+// pruners are tried first.
 // The filter holds the ranked pruners (cells + floats) in shared memory;
 // one thread per point walks them until one strictly dominates it: a SWAR
 // cell test decides most pairs, floats are read only on equal cells.
@@ -24,8 +29,6 @@
 #include "kernels.cuh"
 
 namespace skc {
-
-constexpr uint32_t kSumBins = 2048;
 
 __device__ __forceinline__ uint32_t cell_sum(const uint4& c, uint32_t S, int d) {
   uint32_t s = 0;
@@ -52,64 +55,53 @@ __global__ void __launch_bounds__(256) k_pruner_hist(const uint4* __restrict__ c
     if (h[b]) atomicAdd(&hist[b], h[b]);
 }
 
-// sel[0] = threshold sum, sel[1] = points below it, sel[2] = pruner count
-// Kp = min(K, m), sel[3] / sel[4] = collection cursors (zeroed here).
-__global__ void __launch_bounds__(1024) k_pruner_select(const uint32_t* __restrict__ hist,
-                                                        const uint32_t* __restrict__ m_ptr,
-                                                        uint32_t K, uint32_t* __restrict__ sel) {
-  __shared__ uint32_t wsum[32];
-  const uint32_t m = *m_ptr;
-  const uint32_t Kp = min(K, m);
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  if (t == 0) {
-    sel[0] = 0;
-    sel[1] = 0;
-    sel[2] = Kp;
-    sel[3] = 0;
-    sel[4] = 0;
-  }
-  const uint32_t h0 = hist[2 * t], h1 = hist[2 * t + 1];
-  const uint32_t c = h0 + h1;
-  uint32_t inc = c;  // inclusive scan over the warp
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
-  }
-  if (lane == 31) wsum[wid] = inc;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t v = wsum[lane], vi = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, vi, o);
-      if (lane >= o) vi += u;
-    }
-    wsum[lane] = vi - v;  // exclusive prefix of the warps
-  }
-  __syncthreads();
-  const uint32_t e0 = wsum[wid] + inc - c;  // points with sum < 2t
-  const uint32_t e1 = e0 + h0;              // points with sum < 2t + 1
-  // The threshold bin is the first whose inclusive count reaches Kp.
-  if (Kp > 0) {
-    if (e0 < Kp && e0 + h0 >= Kp) {
-      sel[0] = 2 * t;
-      sel[1] = e0;
-    } else if (e1 < Kp && e1 + h1 >= Kp) {
-      sel[0] = 2 * t + 1;
-      sel[1] = e1;
-    }
-  }
-}
-
+// Collects the K points of smallest cell sum. The threshold bin (the first
+// whose inclusive count reaches Kp = min(K, m)) comes from the histogram, and
+// every CTA finds it for itself (a launch less than a select kernel). sel[2]
+// = Kp; sel[3] and sel[4] are the collection cursors, zero before the launch.
 __global__ void __launch_bounds__(256) k_pruner_collect(const uint4* __restrict__ cells,
                                                         const uint32_t* __restrict__ ids,
                                                         const uint32_t* __restrict__ m_ptr,
-                                                        uint32_t S, int d,
+                                                        uint32_t S, int d, uint32_t K,
+                                                        const uint32_t* __restrict__ hist,
                                                         uint32_t* __restrict__ sel,
                                                         uint32_t* __restrict__ pr_ids,
                                                         uint32_t* __restrict__ pr_key) {
+  __shared__ uint32_t wsum[8];
+  __shared__ uint32_t s_thr, s_below;
   const uint32_t m = *m_ptr;
-  const uint32_t thr = sel[0], below = sel[1], Kp = sel[2];
+  const uint32_t Kp = min(K, m);
+  if (blockIdx.x == 0 && threadIdx.x == 0) sel[2] = Kp;
   if (Kp == 0) return;
+  {
+    const int t = threadIdx.x, ln = t & 31, wid = t >> 5;
+    uint32_t h[8], c = 0;  // this thread's bins 8t .. 8t + 7
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      h[j] = hist[8 * t + j];
+      c += h[j];
+    }
+    uint32_t inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (ln >= o) inc += u;
+    }
+    if (ln == 31) wsum[wid] = inc;
+    __syncthreads();
+    uint32_t e = inc - c;  // points in the bins before this thread's
+    for (int j = 0; j < wid; ++j) e += wsum[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (e < Kp && e + h[j] >= Kp) {
+        s_thr = 8 * t + j;
+        s_below = e;
+      }
+      e += h[j];
+    }
+    __syncthreads();
+  }
+  const uint32_t thr = s_thr, below = s_below;
   const int lane = threadIdx.x & 31;
   const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -145,37 +137,75 @@ __global__ void __launch_bounds__(256) k_pruner_collect(const uint4* __restrict_
   }
 }
 
-// Ranks the Kp pruners by (sum, id) and stores their cells and floats in
-// rank order: out_x[k * K + r] for attribute k.
+// Ranks the Kp pruners by (sum, id) and stores their cells and floats in rank
+// order: out_x[k * K + r] for attribute k. The ranks from K1 on (the second
+// pass) are then reordered by the Gray rank of their median bits over S, so
+// that the eight pruners of a group lie on the same side of most medians and
+// a point skips the group by its minimum cells. Zeroes the passes' counts.
 __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restrict__ pr_ids,
                                                        const uint32_t* __restrict__ pr_key,
                                                        const uint32_t* __restrict__ sel,
                                                        const uint4* __restrict__ cells,
                                                        const float* __restrict__ x,
-                                                       uint64_t n_pad, int d, uint32_t K,
+                                                       uint64_t n_pad, uint32_t S, int d, int sh,
+                                                       uint32_t K, uint32_t K1,
                                                        uint4* __restrict__ out_cells,
-                                                       float* __restrict__ out_x) {
+                                                       float* __restrict__ out_x,
+                                                       uint32_t* __restrict__ blk0,
+                                                       uint32_t* __restrict__ blk1,
+                                                       uint32_t nblk) {
+  static_assert(kMaxPruners <= 1024, "one pruner per thread");
   __shared__ unsigned long long key[kMaxPruners];
+  for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x) blk0[b] = blk1[b] = 0;
   const uint32_t Kp = sel[2];
-  for (uint32_t t = threadIdx.x; t < Kp; t += blockDim.x)
-    key[t] = ((unsigned long long)pr_key[t] << 32) | pr_ids[t];
+  const uint32_t t = threadIdx.x;
+  unsigned long long me = ~0ull;
+  if (t < Kp) me = ((unsigned long long)pr_key[t] << 32) | pr_ids[t];
+  key[t] = me;
   __syncthreads();
-  for (uint32_t t = threadIdx.x; t < Kp; t += blockDim.x) {
-    const unsigned long long me = key[t];
-    uint32_t r = 0;
+  uint32_t r = 0;
+  if (t < Kp) {
+#pragma unroll 8
     for (uint32_t j = 0; j < Kp; ++j) r += key[j] < me;
-    const uint32_t id = (uint32_t)me;
-    out_cells[r] = cells[id];
-    for (int k = 0; k < d; ++k) out_x[(uint64_t)k * K + r] = x[(uint64_t)k * n_pad + id];
   }
+  __syncthreads();
+  uint4 c = make_uint4(0, 0, 0, 0);
+  if (t < Kp) {
+    c = cells[(uint32_t)me];
+    uint32_t g = 0;
+    for (int k = 0; k < d; ++k)
+      if ((S >> k) & 1u) g = 2 * g | ((word_of(c, k >> 2) >> (8 * (k & 3) + sh)) & 1u);
+    for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;
+    key[t] = r < K1 ? r : ((unsigned long long)(1 + g) << 32) | r;  // distinct
+  }
+  __syncthreads();
+  if (t >= Kp) return;
+  if (r >= K1) {
+    const unsigned long long mk = key[t];
+    r = 0;
+#pragma unroll 8
+    for (uint32_t j = 0; j < Kp; ++j) r += key[j] < mk;
+  }
+  const uint32_t id = (uint32_t)me;
+  out_cells[r] = c;
+  for (int k = 0; k < d; ++k) out_x[(uint64_t)k * K + r] = x[(uint64_t)k * n_pad + id];
 }
 
-// st[i] = 2 when one of the pruners of rank [r0, r1) strictly dominates
-// list entry i on S, else 0. With gate_m set, the pass runs only when the
-// list holds at least *gate_m / 4 entries (otherwise every entry is kept).
+// Tests the list positions sub[i] (sub nullptr: i) against the pruners of rank
+// [r0, r1): status 2 when one strictly dominates the point on S; status 1
+// when the point holds the minimum of an attribute of S (amin: nothing can
+// strictly dominate it) and one dominates it; else 0. blk[b] = the entries i
+// of [1024 b, 1024 b + 1024) left at 0 (the count pass of their compaction;
+// zero before). With gate_m set, the pass runs only when it has at least
+// *gate_m / 4 entries (otherwise all are left). On tied data nearly every
+// point that the pruners do not strictly dominate holds a minimum and is
+// settled here: 581k x 10 ties 24,600 of 24,600, where the skyline kernel
+// would search each one's dominator. Groups of eight pruners are skipped by
+// their minimum cells; a point's floats are read only where cells tie.
 template <int D>
 __global__ void __launch_bounds__(256) k_prefilter(const uint4* __restrict__ cells,
                                                    const float* __restrict__ x, uint64_t n_pad,
+                                                   const uint32_t* __restrict__ sub,
                                                    const uint32_t* __restrict__ ids,
                                                    const uint32_t* __restrict__ m_ptr, uint32_t S,
                                                    const uint32_t* __restrict__ sel,
@@ -183,85 +213,125 @@ __global__ void __launch_bounds__(256) k_prefilter(const uint4* __restrict__ cel
                                                    const float* __restrict__ pr_x, uint32_t K,
                                                    uint32_t r0, uint32_t r1,
                                                    const uint32_t* __restrict__ gate_m,
-                                                   uint8_t* __restrict__ st) {
+                                                   const uint32_t* __restrict__ amin,
+                                                   uint8_t* __restrict__ status,
+                                                   uint32_t* __restrict__ blk) {
   constexpr int NW = (D + 3) / 4;
   extern __shared__ uint4 sm4[];
   const uint32_t R = r1 - r0;                      // smem rows
   uint4* s_cells = sm4;                            // [R]
-  float* s_x = reinterpret_cast<float*>(sm4 + R);  // [D][R]
+  uint4* s_min = sm4 + R;                          // [ceil(R / 8)] groups' minimum cells
+  float* s_x = reinterpret_cast<float*>(s_min + (R + 7) / 8);  // [D][R]
   const uint32_t m = *m_ptr;
-  if (gate_m && 4ull * m < *gate_m) {  // few survivors: this pass would not pay
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-      st[i] = 0;
-    return;
-  }
-  const uint32_t Kp = min(sel[2], r1) > r0 ? min(sel[2], r1) - r0 : 0u;
+  // few survivors: this pass would not pay
+  const bool skip = gate_m && 4ull * m < *gate_m;
+  const uint32_t Kp = skip ? 0u : (min(sel[2], r1) > r0 ? min(sel[2], r1) - r0 : 0u);
   for (uint32_t t = threadIdx.x; t < Kp; t += blockDim.x) {
     s_cells[t] = pr_cells[r0 + t];
 #pragma unroll
     for (int k = 0; k < D; ++k) s_x[k * R + t] = pr_x[(uint64_t)k * K + r0 + t];
   }
   __syncthreads();
+  for (uint32_t g = threadIdx.x; g * 8 < Kp; g += blockDim.x) {
+    uint4 mn = s_cells[g * 8];
+    for (uint32_t t = g * 8 + 1; t < min(Kp, g * 8 + 8); ++t) {
+      const uint4 c = s_cells[t];
+      mn.x = __vminu4(mn.x, c.x);
+      mn.y = __vminu4(mn.y, c.y);
+      mn.z = __vminu4(mn.z, c.z);
+      mn.w = __vminu4(mn.w, c.w);
+    }
+    s_min[g] = mn;
+  }
+  __syncthreads();
   uint32_t hS[NW];
 #pragma unroll
   for (int w = 0; w < NW; ++w) hS[w] = guard_mask(S, w);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    const uint32_t id = ids ? ids[i] : i;
-    const uint4 c4 = cells[id];
-    uint32_t pc[NW], pH[NW];
+  // 256 entries a round; their kept count goes to their block of 1024.
+  for (uint64_t base = blockIdx.x * 256ull; base < m; base += gridDim.x * 256ull) {
+    const uint32_t i = (uint32_t)base + threadIdx.x;
+    bool keep = false;
+    if (i < m) {
+      const uint32_t at = sub ? sub[i] : i;
+      const uint32_t id = ids ? ids[at] : at;
+      const uint4 c4 = cells[id];
+      uint32_t pc[NW], pH[NW];
+      uint32_t zero = 0;  // attributes of S whose cell is 0
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      pc[w] = word_of(c4, w);
-      pH[w] = pc[w] | kGuard;
+      for (int w = 0; w < NW; ++w) {
+        pc[w] = word_of(c4, w);
+        pH[w] = pc[w] | kGuard;
+        zero |= pack_guards((kGuard - pc[w]) & hS[w]) << (4 * w);
+      }
+      bool at_min = false;
+      for (uint32_t z = zero; z && !at_min; z &= z - 1) {
+        const int k = __ffs(z) - 1;
+        at_min = ordered_u32(x[(uint64_t)k * n_pad + id]) == amin[k];
+      }
+      uint32_t found = 0;  // the status a pruner gives
+      for (uint32_t t = 0; t < Kp && !found; ++t) {
+        if ((t & 7u) == 0u) {  // a group none of whose pruners is <= p is skipped
+          const uint4 q = s_min[t >> 3];
+          uint32_t worse = 0;  // guard bits where the minimum cell is above p's
+#pragma unroll
+          for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
+          if (worse) {
+            t += 7;
+            continue;
+          }
+        }
+        const uint4 q = s_cells[t];
+        uint32_t worse = 0;  // guard bits where cell(q) > cell(p)
+#pragma unroll
+        for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
+        if (worse) continue;
+        uint32_t Z = 0;  // attributes of S with equal cells
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+          Z |= pack_guards(ge_bytes(word_of(q, w) | kGuard, pc[w]) & hS[w]) << (4 * w);
+        bool le = true, all_lt = true, any_lt = Z != S;
+        for (; Z && le && (all_lt || at_min); Z &= Z - 1) {
+          const int k = __ffs(Z) - 1;
+          const float a = s_x[k * R + t], b = x[(uint64_t)k * n_pad + id];
+          le = a <= b;
+          if (a < b) any_lt = true; else all_lt = false;
+        }
+        if (at_min) found = (le && any_lt) ? 1u : 0u;
+        else found = (le && all_lt) ? 2u : 0u;
+      }
+      keep = !found;
+      status[at] = (uint8_t)found;
     }
-    float pv[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) pv[k] = ((S >> k) & 1u) ? x[(uint64_t)k * n_pad + id] : 0.f;
-    bool pruned = false;
-    for (uint32_t t = 0; t < Kp && !pruned; ++t) {
-      const uint4 q = s_cells[t];
-      uint32_t worse = 0;  // guard bits where cell(q) > cell(p)
-#pragma unroll
-      for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
-      if (worse) continue;
-      uint32_t Z = 0;  // attributes of S with equal cells
-#pragma unroll
-      for (int w = 0; w < NW; ++w)
-        Z |= pack_guards(ge_bytes(word_of(q, w) | kGuard, pc[w]) & hS[w]) << (4 * w);
-      bool strict = true;
-#pragma unroll
-      for (int k = 0; k < D; ++k)
-        if ((Z >> k) & 1u) strict &= s_x[k * R + t] < pv[k];
-      pruned = strict;
-    }
-    st[i] = pruned ? 2 : 0;
+    const int kept = __syncthreads_count(keep);
+    if (threadIdx.x == 0 && kept) atomicAdd(&blk[base >> 10], (uint32_t)kept);
   }
 }
 
 size_t prefilter_smem(int d, uint32_t K) {
-  return (size_t)K * sizeof(uint4) + (size_t)d * K * sizeof(float);
+  return ((size_t)K + (K + 7) / 8) * sizeof(uint4) + (size_t)d * K * sizeof(float);
 }
 
 template <int D>
 static int launch_prefilter_d(cudaStream_t s, const PrefilterArgs& a, unsigned grid,
-                              const uint32_t* ids, const uint32_t* m_ptr, uint32_t r0,
-                              uint32_t r1, const uint32_t* gate_m) {
+                              const uint32_t* sub, const uint32_t* m_ptr, uint32_t r0,
+                              uint32_t r1, const uint32_t* gate_m, uint32_t* blk) {
   const size_t smem = prefilter_smem(D, r1 - r0);
   if (smem > 48 * 1024)
     SKC_CUDA(cudaFuncSetAttribute(k_prefilter<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
-  k_prefilter<D><<<grid, 256, smem, s>>>(a.cells, a.x, a.n_pad, ids, m_ptr, a.S, a.ps.sel,
-                                         a.ps.pr_cells, a.ps.pr_x, a.K, r0, r1, gate_m, a.ps.st);
+  k_prefilter<D><<<grid, 256, smem, s>>>(a.cells, a.x, a.n_pad, sub, a.ids, m_ptr, a.S, a.ps.hist + kSumBins,
+                                         a.ps.pr_cells, a.ps.pr_x, a.K, r0, r1, gate_m, a.amin,
+                                         a.status, blk);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
 static int launch_prefilter_pass(cudaStream_t s, int d, const PrefilterArgs& a, unsigned grid,
-                                 const uint32_t* ids, const uint32_t* m_ptr, uint32_t r0,
-                                 uint32_t r1, const uint32_t* gate_m) {
+                                 const uint32_t* sub, const uint32_t* m_ptr, uint32_t r0,
+                                 uint32_t r1, const uint32_t* gate_m, uint32_t* blk) {
   switch (d) {
 #define SKC_PF_CASE(D) \
-  case D: return launch_prefilter_d<D>(s, a, grid, ids, m_ptr, r0, r1, gate_m);
+  case D: return launch_prefilter_d<D>(s, a, grid, sub, m_ptr, r0, r1, gate_m, blk);
     SKC_PF_CASE(2) SKC_PF_CASE(3) SKC_PF_CASE(4) SKC_PF_CASE(5) SKC_PF_CASE(6)
     SKC_PF_CASE(7) SKC_PF_CASE(8) SKC_PF_CASE(9) SKC_PF_CASE(10) SKC_PF_CASE(11)
     SKC_PF_CASE(12) SKC_PF_CASE(13) SKC_PF_CASE(14) SKC_PF_CASE(15) SKC_PF_CASE(16)
@@ -272,23 +342,26 @@ static int launch_prefilter_pass(cudaStream_t s, int d, const PrefilterArgs& a, 
 }
 
 int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
-                     uint32_t* out_ids, uint32_t* out_count) {
+                     uint32_t* out, uint32_t* out_count) {
   if (a.K < 1 || a.K > (uint32_t)kMaxPruners)
     return set_error(SKC_ERR_INVALID, "pruner count %u outside [1, %d]", a.K, kMaxPruners);
   const PrefilterScratch& p = a.ps;
   const uint64_t want = (a.m_max + 255) / 256;
   const unsigned grid =
       (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)num_sms * 8));
-  SKC_CUDA(cudaMemsetAsync(p.hist, 0, kSumBins * sizeof(uint32_t), s));
-  k_pruner_hist<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, p.hist);
+  if (!a.hist_ready) {
+    SKC_CUDA(cudaMemsetAsync(p.hist, 0, (kSumBins + 8) * sizeof(uint32_t), s));
+    k_pruner_hist<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, p.hist);
+    SKC_LAUNCH_CHECK();
+  }
+  uint32_t* sel = p.hist + kSumBins;
+  k_pruner_collect<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, a.K, p.hist, sel,
+                                        p.pr_ids, p.pr_key);
   SKC_LAUNCH_CHECK();
-  k_pruner_select<<<1, 1024, 0, s>>>(p.hist, a.m_ptr, a.K, p.sel);
-  SKC_LAUNCH_CHECK();
-  k_pruner_collect<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, p.sel, p.pr_ids,
-                                        p.pr_key);
-  SKC_LAUNCH_CHECK();
-  k_pruner_order<<<1, 1024, 0, s>>>(p.pr_ids, p.pr_key, p.sel, a.cells, a.x, a.n_pad, d, a.K,
-                                    p.pr_cells, p.pr_x);
+  const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);  // pruners of the first pass
+  k_pruner_order<<<1, 1024, 0, s>>>(p.pr_ids, p.pr_key, sel, a.cells, a.x, a.n_pad, a.S, d,
+                                    a.depth - 1, a.K, K1, p.pr_cells, p.pr_x, p.blk0, p.blk1,
+                                    (uint32_t)((a.m_max + 1023) / 1024));
   SKC_LAUNCH_CHECK();
   // Two passes: the strongest K1 = K / 16 pruners on every entry, then, only
   // when at least a quarter of the entries survived, the other pruners on
@@ -296,20 +369,12 @@ int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
   // the first pass (more pruners only cost there: survivors that nothing can
   // strictly dominate walk every pruner); anticorrelated data keeps most
   // points, and the second pass removes a good part of them.
-  const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);
-  SKC_TRY(launch_prefilter_pass(s, d, a, grid, a.ids, a.m_ptr, 0, K1, nullptr));
-  if (K1 >= a.K) {
-    return launch_status_compact(s, p.st, a.ids, a.m_ptr, a.m_max, 1, p.blk0, p.blk1, out_ids,
-                                 nullptr, out_count, nullptr);
-  }
-  SKC_TRY(launch_status_compact(s, p.st, a.ids, a.m_ptr, a.m_max, 1, p.blk0, p.blk1, p.mid_ids,
-                                nullptr, p.mid_count, nullptr));
-  SKC_TRY(launch_prefilter_pass(s, d, a, grid, p.mid_ids, p.mid_count, K1, a.K, a.m_ptr));
-  // Survivors (status 0) in list order, as point ids.
-  return launch_status_compact(s, p.st, p.mid_ids, p.mid_count, a.m_max, 1, p.blk0, p.blk1,
-                               out_ids, nullptr, out_count, nullptr);
+  SKC_TRY(launch_prefilter_pass(s, d, a, grid, nullptr, a.m_ptr, 0, K1, nullptr, p.blk0));
+  if (K1 >= a.K)
+    return launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, out, out_count);
+  SKC_TRY(launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, p.mid, p.mid_count));
+  SKC_TRY(launch_prefilter_pass(s, d, a, grid, p.mid, p.mid_count, K1, a.K, a.m_ptr, p.blk1));
+  return launch_status_keep(s, a.status, p.mid, p.mid_count, a.m_max, p.blk1, out, out_count);
 }
-
-uint32_t prefilter_sum_bins() { return kSumBins; }
 
 }  // namespace skc

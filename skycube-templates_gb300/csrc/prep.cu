@@ -5,6 +5,7 @@
 // Every kernel that works on a point list reads the list length from device
 // memory (m_ptr), so a whole pipeline can be enqueued, or captured in a CUDA
 // graph, before any length is known on the host.
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 
@@ -29,12 +30,6 @@ __global__ void k_rows_to_soa(const float* __restrict__ rows, uint64_t n, int d,
     x[(uint64_t)k * n_pad + i] = v;
   }
   if (nbad) atomicAdd(bad, nbad);
-}
-
-__global__ void k_iota(uint32_t* __restrict__ out, uint64_t n) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = (uint32_t)i;
 }
 
 __device__ __forceinline__ float u2f_ordered(uint32_t u) {
@@ -170,16 +165,6 @@ __global__ void k_scatter(const uint32_t* __restrict__ keys,
   }
 }
 
-__global__ void k_scatter_cursor(const uint32_t* __restrict__ keys,
-                                 const uint32_t* __restrict__ m_ptr,
-                                 uint32_t* __restrict__ cursor,
-                                 uint32_t* __restrict__ sorted) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += gridDim.x * blockDim.x)
-    sorted[atomicAdd(&cursor[keys[i]], 1u)] = i;
-}
-
 // --------------------------------------------------------------------------
 // Pivots: one CTA per attribute samples up to kPivotSample values of the
 // list (evenly strided), sorts them in shared memory and keeps
@@ -257,10 +242,12 @@ __device__ __forceinline__ void sort_sample(float* s, uint32_t cnt) {
 __global__ void __launch_bounds__(1024) k_pivots(
     const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, int depth, float* __restrict__ pivots,
-    uint32_t* __restrict__ amin) {
+    uint32_t* __restrict__ amin, uint32_t* __restrict__ hist) {
   __shared__ __align__(16) float s[kPivotSample];
   const int k = blockIdx.x;
   if (amin && threadIdx.x == 0) amin[k] = 0xffffffffu;  // k_cells lowers it
+  if (hist && k == 0)
+    for (uint32_t t = threadIdx.x; t < kSumBins + 8; t += blockDim.x) hist[t] = 0;
   const uint32_t m = *m_ptr;
   const uint32_t cnt = m < kPivotSample ? m : kPivotSample;
   for (int t = threadIdx.x; t < kPivotSample; t += blockDim.x) {
@@ -283,18 +270,33 @@ __global__ void __launch_bounds__(1024) k_pivots(
 }
 
 // cells[i] = grid cells of point ids[i] (see common.cuh). With `amin`, also
-// lowers amin[k] to the ordered-uint minimum of attribute k over the list.
+// lowers amin[k] to the ordered-uint minimum of attribute k over the list;
+// with `hist` (and amin), the histogram of the points' cell sums for the
+// prefilter; with `xout`, the list's floats in list order (xout[k * out_pad
+// + i]). What a later kernel would read the points again for is written here.
 // The D values are loaded before any search, and a search is `depth`
-// branch-free steps, so a thread has D independent chains in flight (the
-// runtime-d loop with a data-dependent search took 46 us on 1M x 10).
+// branch-free steps, so a thread has D independent chains in flight. The
+// pivots lie in shared memory level by level: up to 32 nodes of one level
+// are 32 consecutive words, so a step has no bank conflicts until the last
+// level (in sorted order a level's nodes share a few banks).
 template <int D>
 __global__ void __launch_bounds__(256) k_cells(
     const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, int depth, const float* __restrict__ pivots,
-    uint4* __restrict__ cells, uint32_t* __restrict__ amin) {
-  __shared__ float piv[D * kMaxPivots];
+    uint4* __restrict__ cells, uint32_t* __restrict__ amin, uint32_t* __restrict__ hist,
+    float* __restrict__ xout, uint64_t out_pad) {
+  __shared__ float piv[D * (kMaxPivots + 1)];
   __shared__ uint32_t s_min[D];
-  for (int t = threadIdx.x; t < D * kMaxPivots; t += blockDim.x) piv[t] = pivots[t];
+  __shared__ uint32_t s_hist[kSumBins];
+  if (hist)
+    for (uint32_t t = threadIdx.x; t < kSumBins; t += blockDim.x) s_hist[t] = 0;
+  // Node i of the search tree (its levels one after the other).
+  for (int t = threadIdx.x; t < D * (kMaxPivots + 1); t += blockDim.x) {
+    const int k = t / (kMaxPivots + 1), i = t % (kMaxPivots + 1);
+    const int l = 31 - __clz(i + 1);
+    if (l < depth)
+      piv[t] = pivots[k * kMaxPivots + ((2 * (i + 1 - (1 << l)) + 1) << (depth - 1 - l)) - 1];
+  }
   if (threadIdx.x < D) s_min[threadIdx.x] = 0xffffffffu;
   __syncthreads();
   const uint32_t m = *m_ptr;
@@ -313,16 +315,27 @@ __global__ void __launch_bounds__(256) k_cells(
       lo[k] = 0;
       mn[k] = fminf(mn[k], v[k]);
     }
-    // The number of pivots below v, its bits from the highest down.
-    for (uint32_t step = 1u << (depth - 1); step; step >>= 1) {
+    for (int l = 0; l < depth; ++l) {
 #pragma unroll
       for (int k = 0; k < D; ++k)
-        if (piv[k * kMaxPivots + lo[k] + step - 1] < v[k]) lo[k] += step;
+        lo[k] = 2 * lo[k] + 1 + (piv[k * (kMaxPivots + 1) + lo[k]] < v[k] ? 1u : 0u);
     }
+#pragma unroll
+    for (int k = 0; k < D; ++k) lo[k] -= (1u << depth) - 1u;  // pivots below v
     uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int k = 0; k < D; ++k) w[k >> 2] |= lo[k] << (8 * (k & 3));
     cells[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    if (xout) {
+#pragma unroll
+      for (int k = 0; k < D; ++k) xout[(uint64_t)k * out_pad + i] = v[k];
+    }
+    if (hist) {
+      uint32_t sum = 0;
+#pragma unroll
+      for (int k = 0; k < D; ++k) sum += lo[k];
+      atomicAdd(&s_hist[sum], 1u);
+    }
   }
   if (!amin) return;
 #pragma unroll
@@ -332,79 +345,128 @@ __global__ void __launch_bounds__(256) k_cells(
   }
   __syncthreads();
   if (threadIdx.x < D) atomicMin(&amin[threadIdx.x], s_min[threadIdx.x]);
+  if (hist)
+    for (uint32_t t = threadIdx.x; t < kSumBins; t += blockDim.x)
+      if (s_hist[t]) atomicAdd(&hist[t], s_hist[t]);
 }
 
 // --------------------------------------------------------------------------
-// Order-preserving two-way compaction of a status array: ids of entries
-// with status 0 go to out0, with status 1 to out1 (status 2 is dropped).
-// Works in blocks of 1024 items: count, scan of block counts, write.
+// Order-preserving compaction of a status array in blocks of 1024 entries:
+// entries with status 0 go to out0, with status 1 to out1, both together to
+// both_out (status 2 and above is dropped). k_status_count counts a block's
+// entries per status; k_status_write places them. A block adds up the counts
+// of the blocks before it itself: at most kSelfScanBlocks of them, four loads
+// a thread, instead of a scan launch per output (a compaction took four
+// launches, and the union of two outputs four more). Longer lists scan first.
+constexpr uint32_t kSelfScanBlocks = 4096;
+
 __global__ void __launch_bounds__(1024) k_status_count(
     const uint8_t* __restrict__ st, const uint32_t* __restrict__ m_ptr,
-    int merge01, uint32_t* __restrict__ c0, uint32_t* __restrict__ c1) {
+    uint32_t* __restrict__ c0, uint32_t* __restrict__ c1) {
   __shared__ uint32_t s0[32], s1[32];
   const uint32_t m = *m_ptr;
   const uint32_t nblk = (m + 1023) / 1024;
-  if (blockIdx.x >= nblk) {
-    if (threadIdx.x == 0 && blockIdx.x < gridDim.x) { c0[blockIdx.x] = 0; c1[blockIdx.x] = 0; }
+  if (blockIdx.x >= nblk) {  // the scan of a longer list reads these
+    if (threadIdx.x == 0) { c0[blockIdx.x] = 0; c1[blockIdx.x] = 0; }
     return;
   }
   const uint32_t i = blockIdx.x * 1024 + threadIdx.x;
-  uint8_t v = i < m ? st[i] : 2;
-  if (merge01 && v == 1) v = 0;
+  const uint8_t v = i < m ? st[i] : 2;
   const uint32_t b0 = __ballot_sync(0xffffffffu, v == 0);
   const uint32_t b1 = __ballot_sync(0xffffffffu, v == 1);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) { s0[wid] = __popc(b0); s1[wid] = __popc(b1); }
   __syncthreads();
   if (wid == 0) {
-    uint32_t a = s0[lane], b = s1[lane];
-    for (int o = 16; o; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
+    const uint32_t a = __reduce_add_sync(0xffffffffu, s0[lane]);
+    const uint32_t b = __reduce_add_sync(0xffffffffu, s1[lane]);
     if (lane == 0) { c0[blockIdx.x] = a; c1[blockIdx.x] = b; }
   }
 }
 
+struct StatusOut {
+  uint32_t* out0;      // ids with status 0
+  uint32_t* out1;      // ids with status 1, or nullptr
+  uint32_t* both;      // ids with status 0 or 1, or nullptr
+  uint8_t* both_st;    // per entry of `both`: 0 for status 0, else 2
+  uint32_t* pos0;      // per entry of out0: its position in `both`
+  uint32_t* n;         // [0] entries of out0, and with out1 [1] of out1, [2] of both
+};
+
 __global__ void __launch_bounds__(1024) k_status_write(
-    const uint8_t* __restrict__ st, const uint32_t* __restrict__ ids,
-    const uint32_t* __restrict__ m_ptr, int merge01,
-    const uint32_t* __restrict__ o0, const uint32_t* __restrict__ o1,
-    uint32_t nblk_alloc,
-    uint32_t* __restrict__ out0, uint32_t* __restrict__ out1,
-    uint32_t* __restrict__ n0, uint32_t* __restrict__ n1) {
-  __shared__ uint32_t s0[32], s1[32];
+    const uint8_t* __restrict__ st, const uint32_t* __restrict__ sub,
+    const uint32_t* __restrict__ ids,
+    const uint32_t* __restrict__ m_ptr, const uint32_t* __restrict__ c0,
+    const uint32_t* __restrict__ c1, int scanned, StatusOut o) {
+  __shared__ uint32_t s0[32], s1[32], p0[32], p1[32];
   const uint32_t m = *m_ptr;
   const uint32_t nblk = (m + 1023) / 1024;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (n0) *n0 = o0[nblk_alloc];
-    if (n1) *n1 = o1[nblk_alloc];
+  const uint32_t b = blockIdx.x;
+  if (nblk == 0) {
+    if (b == 0 && threadIdx.x == 0) {
+      o.n[0] = 0;
+      if (o.out1) o.n[1] = o.n[2] = 0;
+    }
+    return;
   }
-  if (blockIdx.x >= nblk) return;
-  const uint32_t i = blockIdx.x * 1024 + threadIdx.x;
-  uint8_t v = i < m ? st[i] : 2;
-  if (merge01 && v == 1) v = 0;
+  if (b >= nblk) return;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t i = b * 1024 + threadIdx.x;
+  const uint32_t at = i < m ? (sub ? sub[i] : i) : 0u;
+  const uint8_t v = i < m ? st[at] : 2;
   const uint32_t b0 = __ballot_sync(0xffffffffu, v == 0);
   const uint32_t b1 = __ballot_sync(0xffffffffu, v == 1);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { s0[wid] = __popc(b0); s1[wid] = __popc(b1); }
+  uint32_t f0 = 0, f1 = 0;  // entries of the blocks before this one
+  if (scanned) {
+    if (threadIdx.x == 0) { f0 = c0[b]; if (o.out1) f1 = c1[b]; }
+  } else {
+    for (uint32_t j = threadIdx.x; j < b; j += 1024) {
+      f0 += c0[j];
+      if (o.out1) f1 += c1[j];
+    }
+  }
+  f0 = __reduce_add_sync(0xffffffffu, f0);
+  f1 = __reduce_add_sync(0xffffffffu, f1);
+  if (lane == 0) {
+    s0[wid] = __popc(b0);
+    s1[wid] = __popc(b1);
+    p0[wid] = f0;
+    p1[wid] = f1;
+  }
   __syncthreads();
   if (wid == 0) {
-    uint32_t a = s0[lane], b = s1[lane];
-    uint32_t ia = a, ib = b;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t u = __shfl_up_sync(0xffffffffu, ia, o);
-      uint32_t w = __shfl_up_sync(0xffffffffu, ib, o);
-      if (lane >= o) { ia += u; ib += w; }
+    const uint32_t a = s0[lane], c = s1[lane];
+    uint32_t ia = a, ic = c;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, ia, k);
+      const uint32_t w = __shfl_up_sync(0xffffffffu, ic, k);
+      if (lane >= k) { ia += u; ic += w; }
     }
-    s0[lane] = ia - a;
-    s1[lane] = ib - b;
+    const uint32_t q0 = __reduce_add_sync(0xffffffffu, p0[lane]);
+    const uint32_t q1 = __reduce_add_sync(0xffffffffu, p1[lane]);
+    s0[lane] = q0 + ia - a;
+    s1[lane] = q1 + ic - c;
+    if (lane == 31 && b == nblk - 1) {
+      o.n[0] = q0 + ia;
+      if (o.out1) {
+        o.n[1] = q1 + ic;
+        o.n[2] = q0 + ia + q1 + ic;
+      }
+    }
   }
   __syncthreads();
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t id = i < m ? (ids ? ids[i] : i) : 0;
-  if (v == 0) out0[o0[blockIdx.x] + s0[wid] + __popc(b0 & lt)] = id;
-  else if (v == 1 && out1) out1[o1[blockIdx.x] + s1[wid] + __popc(b1 & lt)] = id;
+  if (v > 1) return;
+  const uint32_t id = ids ? ids[at] : at;
+  const uint32_t k0 = s0[wid] + __popc(b0 & lt), k1 = s1[wid] + __popc(b1 & lt);
+  if (v == 0) o.out0[k0] = id;
+  else if (o.out1) o.out1[k1] = id;
+  if (o.both) {  // statuses 0 and 1 in list order
+    o.both[k0 + k1] = id;
+    o.both_st[k0 + k1] = v == 0 ? 0 : 2;
+    if (v == 0) o.pos0[k0] = k0 + k1;
+  }
 }
 
 // --------------------------------------------------------------------------
@@ -471,29 +533,6 @@ __global__ void __launch_bounds__(1024) k_scan_apply(
 }
 
 // --------------------------------------------------------------------------
-// Gathers.
-__global__ void k_gather_soa(const float* __restrict__ x, uint64_t n_pad, int d,
-                             const uint32_t* __restrict__ ids,
-                             const uint32_t* __restrict__ m_ptr,
-                             uint64_t out_pad, float* __restrict__ out) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += gridDim.x * blockDim.x) {
-    const uint32_t id = ids[i];
-    for (int k = 0; k < d; ++k) out[(uint64_t)k * out_pad + i] = x[(uint64_t)k * n_pad + id];
-  }
-}
-
-__global__ void k_gather_u4(const uint4* __restrict__ in,
-                            const uint32_t* __restrict__ perm,
-                            const uint32_t* __restrict__ m_ptr,
-                            uint4* __restrict__ out) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += gridDim.x * blockDim.x)
-    out[i] = in[perm[i]];
-}
-
 // Per block of 32 consecutive q's, per 8-q quarter and per 4-q half of a
 // quarter: byte-wise
 // minimum of their cells. Padding entries (index >= m) get cell 127 so they
@@ -519,18 +558,6 @@ __global__ void k_block_min(const uint4* __restrict__ cells,
     }
     if (lane == 0) bmin[b] = c;
   }
-}
-
-// Copies one cuboid's list into a CSR slot: used to assemble per-cuboid
-// outputs of the per-cuboid form into one cuboid-indexed CSR.
-__global__ void k_csr_assemble(const uint32_t* __restrict__ src,
-                               const uint64_t* __restrict__ src_off,
-                               const uint64_t* __restrict__ dst_off,
-                               uint32_t* __restrict__ dst) {
-  const uint32_t c = blockIdx.x;
-  const uint64_t n = dst_off[c + 1] - dst_off[c];
-  const uint64_t s = src_off[c], o = dst_off[c];
-  for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) dst[o + i] = src[s + i];
 }
 
 // Gathers per-cuboid lists held in separate buffers into one CSR:
@@ -569,16 +596,6 @@ __global__ void k_merge_disjoint(const uint32_t* __restrict__ a, uint32_t na,
   }
 }
 
-__global__ void k_gather_u32(const uint32_t* __restrict__ in,
-                             const uint32_t* __restrict__ perm,
-                             const uint32_t* __restrict__ m_ptr,
-                             uint32_t* __restrict__ out) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += gridDim.x * blockDim.x)
-    out[i] = in[perm[i]];
-}
-
 // ==========================================================================
 // Host-side launch helpers.
 static inline unsigned grid_for(uint64_t items, int threads, int max_blocks) {
@@ -591,12 +608,6 @@ static inline unsigned grid_for(uint64_t items, int threads, int max_blocks) {
 int launch_rows_to_soa(cudaStream_t s, const float* rows, uint64_t n, int d,
                        uint64_t n_pad, float* x, uint32_t* bad) {
   k_rows_to_soa<<<grid_for(n * d, 256, 152 * 32), 256, 0, s>>>(rows, n, d, n_pad, x, bad);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-int launch_iota(cudaStream_t s, uint32_t* out, uint64_t n) {
-  k_iota<<<grid_for(n, 256, 152 * 16), 256, 0, s>>>(out, n);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
@@ -633,29 +644,25 @@ int launch_counting_sort(cudaStream_t s, const uint32_t* keys,
 template <int D>
 static int launch_cells(cudaStream_t s, const float* x, uint64_t n_pad, const uint32_t* ids,
                         const uint32_t* m_ptr, uint64_t m_max, int depth, const float* pivots,
-                        uint4* cells, uint32_t* amin) {
-  k_cells<D><<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots,
-                                                            cells, amin);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-// Scatter whose scanned offsets are the cursors themselves (launch_bucket_scan).
-int launch_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* m_ptr, uint64_t m_max,
-                   uint32_t* cursor, uint32_t* sorted) {
-  k_scatter_cursor<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(keys, m_ptr, cursor, sorted);
+                        uint4* cells, uint32_t* amin, uint32_t* hist, float* xout,
+                        uint64_t out_pad) {
+  k_cells<D><<<grid_for(m_max, 256, 152 * 6), 256, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots,
+                                                            cells, amin, hist, xout, out_pad);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
 int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
-                        uint64_t m_max, int depth, float* pivots, uint4* cells, uint32_t* amin) {
-  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, amin);
+                        uint64_t m_max, int depth, float* pivots, uint4* cells, uint32_t* amin,
+                        uint32_t* hist, float* xout, uint64_t out_pad) {
+  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, amin, hist);
   SKC_LAUNCH_CHECK();
   switch (d) {
 #define SKC_CELLS_CASE(D) \
-  case D: return launch_cells<D>(s, x, n_pad, ids, m_ptr, m_max, depth, pivots, cells, amin);
+  case D:                                                                               \
+    return launch_cells<D>(s, x, n_pad, ids, m_ptr, m_max, depth, pivots, cells, amin, hist, \
+                           xout, out_pad);
     SKC_CELLS_CASE(2) SKC_CELLS_CASE(3) SKC_CELLS_CASE(4) SKC_CELLS_CASE(5) SKC_CELLS_CASE(6)
     SKC_CELLS_CASE(7) SKC_CELLS_CASE(8) SKC_CELLS_CASE(9) SKC_CELLS_CASE(10) SKC_CELLS_CASE(11)
     SKC_CELLS_CASE(12) SKC_CELLS_CASE(13) SKC_CELLS_CASE(14) SKC_CELLS_CASE(15)
@@ -666,21 +673,43 @@ int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
   }
 }
 
-int launch_status_compact(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
-                          const uint32_t* m_ptr, uint64_t m_max, int merge01,
-                          uint32_t* blk0, uint32_t* blk1, uint32_t* out0,
-                          uint32_t* out1, uint32_t* n0, uint32_t* n1) {
-  const uint32_t nblk = (uint32_t)((m_max + 1023) / 1024);
-  const uint32_t g = nblk ? nblk : 1;
-  k_status_count<<<g, 1024, 0, s>>>(st, m_ptr, merge01, blk0, blk1);
-  SKC_LAUNCH_CHECK();
-  k_scan_single<uint32_t><<<1, 1024, 0, s>>>(blk0, g);
-  SKC_LAUNCH_CHECK();
-  k_scan_single<uint32_t><<<1, 1024, 0, s>>>(blk1, g);
-  SKC_LAUNCH_CHECK();
-  k_status_write<<<g, 1024, 0, s>>>(st, ids, m_ptr, merge01, blk0, blk1, g, out0, out1, n0, n1);
+// Statuses whose block counts c0 / c1 are already there (c1 unused without
+// out1) into the outputs.
+static int status_write(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
+                        const uint32_t* ids,
+                        const uint32_t* m_ptr, uint64_t m_max, uint32_t* c0, uint32_t* c1,
+                        const StatusOut& o) {
+  const uint32_t g = (uint32_t)std::max<uint64_t>(1, (m_max + 1023) / 1024);
+  const int scan = g > kSelfScanBlocks;
+  if (scan) {
+    k_scan_single<uint32_t><<<1, 1024, 0, s>>>(c0, g);
+    SKC_LAUNCH_CHECK();
+    if (o.out1) {
+      k_scan_single<uint32_t><<<1, 1024, 0, s>>>(c1, g);
+      SKC_LAUNCH_CHECK();
+    }
+  }
+  k_status_write<<<g, 1024, 0, s>>>(st, sub, ids, m_ptr, c0, c1, scan, o);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
+}
+
+int launch_status_split(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
+                        const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* blk1,
+                        uint32_t* sky, uint32_t* ext, uint32_t* n, uint32_t* both,
+                        uint8_t* both_st, uint32_t* pos0) {
+  const uint32_t g = (uint32_t)std::max<uint64_t>(1, (m_max + 1023) / 1024);
+  k_status_count<<<g, 1024, 0, s>>>(st, m_ptr, blk0, blk1);
+  SKC_LAUNCH_CHECK();
+  return status_write(s, st, nullptr, ids, m_ptr, m_max, blk0, blk1,
+                      StatusOut{sky, ext, both, both_st, pos0, n});
+}
+
+int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
+                       const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* out,
+                       uint32_t* n) {
+  return status_write(s, st, sub, nullptr, m_ptr, m_max, blk0, nullptr,
+                      StatusOut{out, nullptr, nullptr, nullptr, nullptr, n});
 }
 
 int launch_scan_u32_to_u64(cudaStream_t s, const uint32_t* in, uint64_t len,
@@ -696,43 +725,13 @@ int launch_scan_u32_to_u64(cudaStream_t s, const uint32_t* in, uint64_t len,
   return SKC_OK;
 }
 
-int launch_scan_single_u32(cudaStream_t s, uint32_t* a, uint32_t len) {
-  k_scan_single<uint32_t><<<1, 1024, 0, s>>>(a, len);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
 uint64_t scan_bsum_entries(uint64_t len) {
   return (len + kScanBlock - 1) / kScanBlock + 1;
-}
-
-int launch_gather_soa(cudaStream_t s, const float* x, uint64_t n_pad, int d,
-                      const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max,
-                      uint64_t out_pad, float* out) {
-  k_gather_soa<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(x, n_pad, d, ids, m_ptr, out_pad, out);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-int launch_gather_u4(cudaStream_t s, const uint4* in, const uint32_t* perm,
-                     const uint32_t* m_ptr, uint64_t m_max, uint4* out) {
-  k_gather_u4<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(in, perm, m_ptr, out);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
 }
 
 int launch_block_min(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr,
                      uint64_t m_max, uint4* bmin, uint4* smin, uint4* hmin) {
   k_block_min<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(cells, m_ptr, bmin, smin, hmin);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-int launch_csr_assemble(cudaStream_t s, const uint32_t* src,
-                        const uint64_t* src_off, const uint64_t* dst_off,
-                        uint32_t ncub, uint32_t* dst) {
-  if (ncub == 0) return SKC_OK;
-  k_csr_assemble<<<ncub, 256, 0, s>>>(src, src_off, dst_off, dst);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
@@ -755,13 +754,6 @@ int launch_merge_disjoint(cudaStream_t s, const uint32_t* a, uint32_t na,
 
 int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v) {
   k_set_u32<<<1, 1, 0, s>>>(p, v);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-int launch_gather_u32(cudaStream_t s, const uint32_t* in, const uint32_t* perm,
-                      const uint32_t* m_ptr, uint64_t m_max, uint32_t* out) {
-  k_gather_u32<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(in, perm, m_ptr, out);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
@@ -820,76 +812,33 @@ int launch_sample_signature(cudaStream_t s, const float* x, uint64_t n_pad, uint
 }
 
 // Plan helpers (graph-captured launch sequences, api.cu). k_cap_count
-// records the true list length in stats[slot] and clamps the device count to
-// the plan's capacity, so every later kernel stays inside the buffers; the
-// host sees the overflow and re-plans. k_stat_u64 copies one device total.
-__global__ void k_cap_count(uint32_t* m_ptr, uint32_t cap, uint64_t* stats, int slot) {
+// records the true candidate count in stats[slot]; when it is over the plan's
+// capacity the device counts become 0 (candidates and skyline points), so
+// every later kernel stays inside the buffers; the host sees the overflow and
+// re-plans. k_stat_u64 copies one device total.
+__global__ void k_cap_count(uint32_t* m_ptr, uint32_t* nsky_ptr, uint32_t cap, uint64_t* stats,
+                            int slot) {
   const uint32_t m = *m_ptr;
   stats[slot] = m;
-  if (m > cap) *m_ptr = cap;
+  if (m > cap) {
+    *m_ptr = 0;
+    *nsky_ptr = 0;
+  }
 }
 
 __global__ void k_stat_u64(const uint64_t* src, uint64_t* stats, int slot) {
   stats[slot] = *src;
 }
 
-int launch_cap_count(cudaStream_t s, uint32_t* m_ptr, uint32_t cap, uint64_t* stats, int slot) {
-  k_cap_count<<<1, 1, 0, s>>>(m_ptr, cap, stats, slot);
+int launch_cap_count(cudaStream_t s, uint32_t* m_ptr, uint32_t* nsky_ptr, uint32_t cap,
+                     uint64_t* stats, int slot) {
+  k_cap_count<<<1, 1, 0, s>>>(m_ptr, nsky_ptr, cap, stats, slot);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
 int launch_stat_u64(cudaStream_t s, const uint64_t* src, uint64_t* stats, int slot) {
   k_stat_u64<<<1, 1, 0, s>>>(src, stats, slot);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-// st[i] = 0 when list[i] occurs in sorted_set[0 .. *nset_ptr) (ascending),
-// else 2: status-compaction input that keeps the members.
-__global__ void k_member_flags(const uint32_t* __restrict__ list,
-                               const uint32_t* __restrict__ m_ptr,
-                               const uint32_t* __restrict__ sorted_set,
-                               const uint32_t* __restrict__ nset_ptr,
-                               uint8_t* __restrict__ st) {
-  const uint32_t m = *m_ptr, ns = *nset_ptr;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    const uint32_t v = list[i];
-    uint32_t lo = 0, hi = ns;  // first position with sorted_set[pos] >= v
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (sorted_set[mid] < v) lo = mid + 1; else hi = mid;
-    }
-    st[i] = (lo < ns && sorted_set[lo] == v) ? 0 : 2;
-  }
-}
-
-int launch_member_flags(cudaStream_t s, const uint32_t* list, const uint32_t* m_ptr,
-                        uint64_t m_max, const uint32_t* sorted_set, const uint32_t* nset_ptr,
-                        uint8_t* st) {
-  k_member_flags<<<grid_for(m_max, 256, 152 * 8), 256, 0, s>>>(list, m_ptr, sorted_set, nset_ptr, st);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
-}
-
-// Pads the q list to a whole number of 32-q blocks with entries that add
-// nothing, so the bitmap kernel can test every lane of a block without a
-// bounds check: cells 127 (the top cell) and floats +inf. Such a q is worse
-// than p on every attribute where p's cell is below 127, and where p's cell
-// is 127 too the float test +inf <= p fails (inputs are finite), so LE = LT
-// = {} for every p: no strict update and no tie pair.
-__global__ void k_pad_q(const uint32_t* __restrict__ mq_ptr, int d, uint4* __restrict__ qc,
-                        float* __restrict__ qx, uint64_t pitch) {
-  const uint32_t mq = *mq_ptr;
-  const uint32_t i = mq + threadIdx.x;
-  if (i >= ((mq + 31) & ~31u)) return;
-  qc[i] = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
-  for (int k = 0; k < d; ++k) qx[(uint64_t)k * pitch + i] = __int_as_float(0x7f800000);
-}
-
-int launch_pad_q(cudaStream_t s, const uint32_t* mq_ptr, int d, uint4* qc, float* qx,
-                 uint64_t pitch) {
-  k_pad_q<<<1, 32, 0, s>>>(mq_ptr, d, qc, qx, pitch);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
