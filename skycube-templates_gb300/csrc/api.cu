@@ -498,7 +498,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   T.mark("bitmap kernel");
 
   // Compaction of skylines (bit clear) and extended skylines (bit set).
-  const uint32_t tiles = compact_tiles(m);
+  const uint32_t tiles = compact_tiles(m, W);
   const uint64_t C = 32ull * W;
   for (int pass = 0; pass < (want_ext ? 2 : 1); ++pass) {
     CompactArgs ca{};

@@ -46,8 +46,10 @@ int launch_status_split(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
 int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
                        const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* out,
                        uint32_t* n);
-int launch_scan_u32_to_u64(cudaStream_t s, const uint32_t* in, uint64_t len,
-                           uint64_t* bsum, uint64_t* out);
+// Exclusive scan of in[0 .. len) into out[0 .. len]; csr_off[c] = out[c * T]
+// for c <= nsub (nsub * T <= len).
+int launch_scan_counts(cudaStream_t s, const uint32_t* in, uint64_t len, uint64_t* bsum,
+                       uint64_t* out, uint32_t T, uint32_t nsub, uint64_t* csr_off);
 uint64_t scan_bsum_entries(uint64_t len);
 int launch_block_min(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr,
                      uint64_t m_max, uint4* bmin, uint4* smin, uint4* hmin);
@@ -223,7 +225,7 @@ struct CompactArgs {
   uint32_t* out;         // ids (sized by the caller after the count pass)
   uint64_t out_cap;      // entries of `out`; ids past it are not written
 };
-uint32_t compact_tiles(uint64_t m_max);
+uint32_t compact_tiles(uint64_t m_max, uint32_t words);
 int launch_bits_count(cudaStream_t s, const CompactArgs& a);
 int launch_bits_write(cudaStream_t s, const CompactArgs& a);
 

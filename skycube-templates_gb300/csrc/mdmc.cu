@@ -992,168 +992,213 @@ int bitmap_tie_slab_words(int d, int num_sms, uint64_t* words) {
 }
 
 // --------------------------------------------------------------------------
-// Compaction of bitmaps into per-cuboid id lists. Rows are cut in tiles of
-// kTileRows; a CTA handles one (tile, word) pair with 8 warps, warp k owning
-// rows [k*256, k*256+256) of the tile, so ids come out ascending per cuboid.
-constexpr uint32_t kTileRows = 2048;
+// Compaction of bitmaps into per-cuboid id lists: a count pass per (column,
+// row tile), a scan, and a write pass, each reading the matrix once in whole
+// row segments. (A CTA per bitmap word read 4 bytes of every 32-byte sector
+// and walked its 32 columns one ballot at a time: 500k x 16 -m 6, 4 GB of
+// bits, 12.6 ms; 1M x 10 0.66 ms; now 5.7 and 0.33.)
+//
+// Rows per tile: as many as 2,048, fewer while the write pass would have
+// under about four warps per scheduler.
+static uint32_t compact_tile_rows(uint64_t m_max, uint32_t W) {
+  uint32_t r = 2048;
+  while (r > 256 && ((m_max + r - 1) / r) * W < 152 * 16) r >>= 1;
+  return r;
+}
 
-uint32_t compact_tiles(uint64_t m_max) {
-  uint64_t t = (m_max + kTileRows - 1) / kTileRows;
+uint32_t compact_tiles(uint64_t m_max, uint32_t W) {
+  const uint32_t r = compact_tile_rows(m_max, W);
+  const uint64_t t = (m_max + r - 1) / r;
   return (uint32_t)(t ? t : 1);
 }
 
-// Cuboids within max_d, plus the full space, which is always computed (the
-// suite computes it first in both algorithms).
-__device__ __forceinline__ bool cuboid_wanted(uint32_t c, uint32_t nsub, int max_d) {
-  return c >= 1 && c < nsub && (__popc(c) <= max_d || c == nsub - 1);
+// Columns of bitmap word w that are output: cuboids within max_d, plus the
+// full space, which is always computed (the suite computes it first in both
+// algorithms).
+__device__ __forceinline__ uint32_t wanted_columns(uint32_t w, uint32_t nsub, int max_d) {
+  uint32_t v = ~pop_above(max_d - __popc(w));
+  const uint32_t full = nsub - 1;
+  if (w == full / 32) v |= 1u << (full & 31u);
+  if (w == 0) v &= ~1u;
+  if (nsub < 32) v &= (1u << nsub) - 1u;
+  return v;
 }
 
-// Bits of row r's word w that count (1 = counted).
-__device__ __forceinline__ uint32_t counted_bits(const uint32_t* bits, uint32_t W,
-                                                 uint32_t r, uint32_t m, uint32_t w,
-                                                 int count_set) {
-  if (r >= m) return 0u;
-  const uint32_t v = bits[(uint64_t)r * W + w];
-  return count_set ? v : ~v;
+// Full adder on 32 columns at once: l = sum, h = carry.
+__device__ __forceinline__ void csa(uint32_t& h, uint32_t& l, uint32_t a, uint32_t b, uint32_t c) {
+  h = (a & b) | (a & c) | (b & c);
+  l = a ^ b ^ c;
 }
 
+// counts[c * T + t] = rows of tile t that belong to column c's list. A lane
+// owns one word of the row (with under 32 words per row, one word of every
+// 32 / W-th row) and adds its rows into bit-sliced counters: 32 columns per
+// lane at 3 to 4 instructions a row, so the pass runs at the speed of its
+// loads.
 __global__ void __launch_bounds__(256) k_bits_count(
-    const uint32_t* __restrict__ bits, uint32_t W,
-    const uint32_t* __restrict__ m_ptr, uint32_t T, int count_set,
-    uint32_t nsub, int max_d, uint32_t* __restrict__ counts) {
-  __shared__ uint32_t wc[8][32];
-  const uint32_t t = blockIdx.x, w = blockIdx.y;
-  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    const uint32_t* __restrict__ bits, uint32_t W, const uint32_t* __restrict__ m_ptr,
+    uint32_t T, uint32_t tile_rows, int count_set, uint32_t nsub, int max_d,
+    uint32_t* __restrict__ counts) {
+  __shared__ uint32_t s_cnt[1024];  // [column of the word][word of the chunk]
+  const uint32_t t = blockIdx.x, w0 = blockIdx.y * 32;
+  const uint32_t Wc = min(W, 32u);  // words of this chunk (W is a power of two)
+  const uint32_t lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const uint32_t wl = lane & (Wc - 1), rp = 32 / Wc, sub = lane / Wc;
   const uint32_t m = *m_ptr;
-  // Cuboids of this word that are computed (all but the empty one without a
-  // cap; under -m a word may hold none): only their bit columns are counted.
-  const uint32_t wanted = __ballot_sync(kFull, cuboid_wanted(w * 32 + lane, nsub, max_d));
-  uint32_t cnt = 0;
-  const uint32_t row0 = t * kTileRows + k * 256;
-  if (t * kTileRows < m && wanted) {
-    const bool dense = __popc(wanted) > 16;  // then all 32 columns, unrolled
-    for (int s = 0; s < 8; ++s) {
-      const uint32_t v = counted_bits(bits, W, row0 + s * 32 + lane, m, w, count_set) & wanted;
-      if (dense) {
+  for (uint32_t i = threadIdx.x; i < 1024; i += 256) s_cnt[i] = 0;
+  __syncthreads();
+  const uint32_t wanted = wanted_columns(w0 + wl, nsub, max_d);
+  const uint32_t per_warp = tile_rows / 8;
+  const uint32_t row0 = t * tile_rows + k * per_warp;
+  const uint32_t row1 = min(m, row0 + per_warp);
+  if (row0 < row1 && __any_sync(kFull, wanted)) {
+    const uint32_t inv = count_set ? 0u : kFull;
+    uint32_t p[9] = {};  // bit j of each column's count (at most 256 rows a lane)
+    for (uint32_t base = row0; base < row1; base += 8 * rp) {
+      uint32_t v[8];
 #pragma unroll
-        for (int b = 0; b < 32; ++b) {  // one warp reduction per bit column
-          const uint32_t tot = __reduce_add_sync(kFull, (v >> b) & 1u);
-          if (lane == b) cnt += tot;
-        }
-      } else {
-        for (uint32_t mm = wanted; mm; mm &= mm - 1) {
-          const int b = __ffs(mm) - 1;
-          const uint32_t tot = __reduce_add_sync(kFull, (v >> b) & 1u);
-          if (lane == b) cnt += tot;
-        }
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t r = base + j * rp + sub;
+        v[j] = (r < row1 && wanted) ? (bits[(uint64_t)r * W + w0 + wl] ^ inv) & wanted : 0u;
       }
-    }
-  }
-  wc[k][lane] = cnt;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t sum = 0;
-    for (int j = 0; j < 8; ++j) sum += wc[j][threadIdx.x];
-    const uint32_t c = w * 32 + threadIdx.x;
-    counts[(uint64_t)c * T + t] = cuboid_wanted(c, nsub, max_d) ? sum : 0u;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_bits_write(
-    const uint32_t* __restrict__ bits, uint32_t W,
-    const uint32_t* __restrict__ m_ptr, uint32_t T, int count_set,
-    uint32_t nsub, int max_d, const uint64_t* __restrict__ offs,
-    const uint32_t* __restrict__ cand, uint32_t* __restrict__ out, uint64_t out_cap) {
-  __shared__ uint32_t wc[8][32];
-  __shared__ uint32_t run[8][32];
-  const uint32_t t = blockIdx.x, w = blockIdx.y;
-  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
-  const uint32_t m = *m_ptr;
-  const uint32_t wanted = __ballot_sync(kFull, cuboid_wanted(w * 32 + lane, nsub, max_d));
-  if (t * kTileRows >= m || !wanted) return;  // uniform over the CTA
-  const uint32_t row0 = t * kTileRows + k * 256;
-  const bool dense = __popc(wanted) > 16;  // then all 32 columns, unrolled
-  // pass 1: per-warp counts
-  uint32_t cnt = 0;
-  for (int s = 0; s < 8; ++s) {
-    const uint32_t v = counted_bits(bits, W, row0 + s * 32 + lane, m, w, count_set) & wanted;
-    if (dense) {
+      uint32_t t1, t2, f1, f2, e;
+      csa(t1, p[0], p[0], v[0], v[1]);
+      csa(t2, p[0], p[0], v[2], v[3]);
+      csa(f1, p[1], p[1], t1, t2);
+      csa(t1, p[0], p[0], v[4], v[5]);
+      csa(t2, p[0], p[0], v[6], v[7]);
+      csa(f2, p[1], p[1], t1, t2);
+      csa(e, p[2], p[2], f1, f2);
 #pragma unroll
-      for (int b = 0; b < 32; ++b) {
-        const uint32_t bal = __ballot_sync(kFull, (v >> b) & 1u);
-        if (lane == b) cnt += __popc(bal);
-      }
-    } else {
-      for (uint32_t mm = wanted; mm; mm &= mm - 1) {
-        const int b = __ffs(mm) - 1;
-        const uint32_t bal = __ballot_sync(kFull, (v >> b) & 1u);
-        if (lane == b) cnt += __popc(bal);
+      for (int j = 3; j < 9; ++j) {
+        const uint32_t c = p[j] & e;
+        p[j] ^= e;
+        e = c;
       }
     }
-  }
-  wc[k][lane] = cnt;
-  __syncthreads();
-  // exclusive prefix over warps, per bit
-  if (threadIdx.x < 32) {
-    uint32_t acc = 0;
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t v = wc[j][threadIdx.x];
-      run[j][threadIdx.x] = acc;
-      acc += v;
-    }
-  }
-  __syncthreads();
-  // pass 2: write ids
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  for (int s = 0; s < 8; ++s) {
-    const uint32_t r = row0 + s * 32 + lane;
-    const uint32_t v = counted_bits(bits, W, r, m, w, count_set) & wanted;
-    const uint32_t id = r < m ? cand[r] : 0u;
-    // Dense words walk all 32 columns (unwanted ones are masked to zero).
-    const uint32_t cols = dense ? kFull : wanted;
 #pragma unroll 4
-    for (uint32_t mm = cols; mm; mm &= mm - 1) {
-      const int b = __ffs(mm) - 1;
-      const uint32_t bal = __ballot_sync(kFull, (v >> b) & 1u);
-      if (!bal) continue;
-      const uint32_t c = w * 32 + b;
-      const uint32_t base = run[k][b];
-      if ((v >> b) & 1u) {
-        const uint64_t pos = offs[(uint64_t)c * T + t] + base + __popc(bal & lt_mask);
-        if (pos < out_cap) out[pos] = id;
-      }
-      __syncwarp();
-      if (lane == 0) run[k][b] = base + __popc(bal);
-      __syncwarp();
+    for (uint32_t b = 0; b < 32; ++b) {
+      uint32_t c = 0;
+#pragma unroll
+      for (int j = 0; j < 9; ++j) c |= ((p[j] >> b) & 1u) << j;
+      if (c) atomicAdd(&s_cnt[b * 32 + wl], c);
     }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < Wc * 32; i += 256) {
+    const uint32_t b = i & 31, w = i >> 5;
+    counts[(uint64_t)((w0 + w) * 32 + b) * T + t] = s_cnt[b * 32 + w];
   }
 }
 
-// csr_off[c] = offs[c * T] for c in [0, nsub]; offs[32*W*T] is the total.
-__global__ void k_extract_csr(const uint64_t* __restrict__ offs, uint32_t T,
-                              uint32_t nsub, uint64_t* __restrict__ csr_off) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nsub;
-       c += gridDim.x * blockDim.x)
-    csr_off[c] = offs[(uint64_t)c * T];
+// Bit matrix transpose over a warp: bit r of lane c's result is bit c of
+// lane r's x. Five exchanges, each a shuffle, a rotate and a select.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
+#pragma unroll
+  for (int j = 16; j; j >>= 1) {
+    const uint32_t lo = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
+                        : j == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(kFull, x, j);
+    const bool up = lane & j;
+    const uint32_t rot = __funnelshift_l(y, y, up ? 32 - j : j);
+    const uint32_t keep = up ? ~lo : lo;
+    x = (x & keep) | (rot & ~keep);
+  }
+  return x;
+}
+
+constexpr uint32_t kWriteWords = 8;   // words (warps) of a write CTA: one 32-byte sector of a row
+constexpr uint32_t kWriteRows = 128;  // rows staged per step
+
+// Ids of tile t's rows into the lists of eight words' columns, ascending per
+// list. The CTA stages 128 rows at a time (whole 32-byte sectors), a warp
+// owns one word, and after a 32 x 32 bit transpose a lane holds one column's
+// 32 rows and appends their ids to its own list; where more than 96 rows
+// belong to the lists (dense columns), a step per column writes its ids from
+// the row lanes instead, next to each other (its steps do not wait for one
+// another, a lane's appends do). The pass waits for its loads and stores and
+// wants all 64 warps: 16 words per CTA, 64 rows per step, the next step's
+// rows prefetched into registers, 64 rows per transpose or ids gathered to
+// 16-byte stores were each slower (count, scan and write of 1M x 10, 0.33 ms
+// as it is: 0.36, 0.34, 0.48, 0.42, 0.64).
+__global__ void __launch_bounds__(32 * kWriteWords, 64 / kWriteWords) k_bits_write(
+    const uint32_t* __restrict__ bits, uint32_t W, const uint32_t* __restrict__ m_ptr,
+    uint32_t T, uint32_t tile_rows, int count_set, uint32_t nsub, int max_d,
+    const uint64_t* __restrict__ offs, const uint32_t* __restrict__ cand,
+    uint32_t* __restrict__ out, uint64_t out_cap) {
+  __shared__ uint32_t s_bits[kWriteRows * (kWriteWords + 1)];
+  __shared__ uint32_t s_id[kWriteRows];
+  const uint32_t t = blockIdx.x, w0 = blockIdx.y * kWriteWords;
+  const uint32_t Wb = min(W, kWriteWords);  // words of this CTA, one warp each
+  const uint32_t lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const uint32_t m = *m_ptr;
+  const uint32_t row0 = t * tile_rows, row1 = min(m, row0 + tile_rows);
+  const uint32_t wanted = wanted_columns(w0 + k, nsub, max_d);
+  if (!__syncthreads_or(wanted != 0u && row0 < row1)) return;
+  const uint32_t c = (w0 + k) * 32 + lane;  // this lane's column
+  uint64_t pos = (wanted >> lane) & 1u ? offs[(uint64_t)c * T + t] : 0u;
+  const uint32_t inv = count_set ? 0u : kFull;
+  for (uint32_t base = row0; base < row1; base += kWriteRows) {
+    for (uint32_t i = threadIdx.x; i < kWriteRows * Wb; i += blockDim.x) {
+      const uint32_t r = i / Wb, w = i & (Wb - 1);
+      s_bits[r * (kWriteWords + 1) + w] =
+          base + r < row1 ? bits[(uint64_t)(base + r) * W + w0 + w] ^ inv : 0u;
+    }
+    for (uint32_t i = threadIdx.x; i < kWriteRows; i += blockDim.x)
+      s_id[i] = base + i < row1 ? cand[base + i] : 0u;
+    __syncthreads();
+    if (wanted) {
+      for (uint32_t g = 0; g < kWriteRows; g += 32) {
+        const uint32_t x = s_bits[(g + lane) * (kWriteWords + 1) + k] & wanted;
+        if (!__any_sync(kFull, x)) continue;
+        uint32_t rows = transpose32(x, lane);
+        const uint32_t cnt = __popc(rows);
+        if (__reduce_add_sync(kFull, cnt) > 96u) {
+          const uint32_t id = s_id[g + lane];
+          const uint32_t lo = (uint32_t)pos, hi = (uint32_t)(pos >> 32);
+#pragma unroll 4
+          for (int j = 0; j < 32; ++j) {
+            const uint32_t col = __shfl_sync(kFull, rows, j);
+            const uint64_t p = ((uint64_t)__shfl_sync(kFull, hi, j) << 32 |
+                                __shfl_sync(kFull, lo, j)) + __popc(col & lt_mask);
+            if (((col >> lane) & 1u) && p < out_cap) out[p] = id;
+          }
+          pos += cnt;
+        } else {
+          const uint32_t n = __reduce_max_sync(kFull, cnt);
+          for (uint32_t i = 0; i < n; ++i) {
+            if (rows) {
+              const uint32_t id = s_id[g + __ffs(rows) - 1];
+              rows &= rows - 1;
+              if (pos < out_cap) out[pos] = id;
+              ++pos;
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
 }
 
 int launch_bits_count(cudaStream_t s, const CompactArgs& a) {
-  const uint32_t T = compact_tiles(a.m_max);
-  const uint64_t C = 32ull * a.words;
-  k_bits_count<<<dim3(T, a.words), 256, 0, s>>>(a.bits, a.words, a.m_ptr, T, a.count_set,
-                                                 a.nsub, a.max_d, a.counts);
+  const uint32_t T = compact_tiles(a.m_max, a.words);
+  const uint32_t rows = compact_tile_rows(a.m_max, a.words);
+  k_bits_count<<<dim3(T, (a.words + 31) / 32), 256, 0, s>>>(
+      a.bits, a.words, a.m_ptr, T, rows, a.count_set, a.nsub, a.max_d, a.counts);
   SKC_LAUNCH_CHECK();
-  SKC_TRY(launch_scan_u32_to_u64(s, a.counts, C * T, a.bsum, a.offs));
-  k_extract_csr<<<(a.nsub + 256) / 256, 256, 0, s>>>(a.offs, T, a.nsub, a.csr_off);
-  SKC_LAUNCH_CHECK();
-  return SKC_OK;
+  return launch_scan_counts(s, a.counts, 32ull * a.words * T, a.bsum, a.offs, T, a.nsub,
+                            a.csr_off);
 }
 
 int launch_bits_write(cudaStream_t s, const CompactArgs& a) {
-  const uint32_t T = compact_tiles(a.m_max);
-  k_bits_write<<<dim3(T, a.words), 256, 0, s>>>(a.bits, a.words, a.m_ptr, T, a.count_set,
-                                                 a.nsub, a.max_d, a.offs, a.cand, a.out,
-                                                 a.out_cap);
+  const uint32_t T = compact_tiles(a.m_max, a.words);
+  const uint32_t rows = compact_tile_rows(a.m_max, a.words);
+  const uint32_t wb = a.words < kWriteWords ? a.words : kWriteWords;
+  k_bits_write<<<dim3(T, a.words / wb), 32 * wb, 0, s>>>(
+      a.bits, a.words, a.m_ptr, T, rows, a.count_set, a.nsub, a.max_d, a.offs, a.cand, a.out,
+      a.out_cap);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }

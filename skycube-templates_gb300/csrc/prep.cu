@@ -493,43 +493,71 @@ __global__ void __launch_bounds__(1024) k_scan_partials(
   }
 }
 
+// A CTA adds up the block sums before its own itself (`scanned` 0; at most
+// kSelfScanBlocks of them), or reads their scan. With csr_off, out[c * T] goes
+// to csr_off[c] for c <= nsub as well.
 __global__ void __launch_bounds__(1024) k_scan_apply(
-    const uint32_t* __restrict__ in, uint64_t len,
-    const uint64_t* __restrict__ bsum_scanned, uint64_t* __restrict__ out) {
-  __shared__ uint64_t wt[32];
+    const uint32_t* __restrict__ in, uint64_t len, const uint64_t* __restrict__ bsum,
+    int scanned, uint64_t* __restrict__ out, uint32_t T, uint32_t nsub,
+    uint64_t* __restrict__ csr_off) {
+  __shared__ uint64_t wt[32], pre[32];
   const uint64_t beg = (uint64_t)blockIdx.x * kScanBlock;
   constexpr int per = kScanBlock / 1024;  // 4 consecutive items per thread
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint64_t before = 0;
+  if (scanned) {
+    if (threadIdx.x == 0) before = bsum[blockIdx.x];
+  } else {
+    for (uint32_t j = threadIdx.x; j < blockIdx.x; j += 1024) before += bsum[j];
+  }
   uint32_t v[per];
   uint64_t local = 0;
+  const uint64_t at = beg + threadIdx.x * per;
+#pragma unroll
   for (int j = 0; j < per; ++j) {
-    const uint64_t i = beg + threadIdx.x * per + j;
-    v[j] = i < len ? in[i] : 0;
+    v[j] = at + j < len ? in[at + j] : 0;
     local += v[j];
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint64_t incl = local;
   for (int o = 1; o < 32; o <<= 1) {
     uint64_t u = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += u;
+    before += __shfl_xor_sync(0xffffffffu, before, o);
   }
-  if (lane == 31) wt[wid] = incl;
+  if (lane == 31) {
+    wt[wid] = incl;
+    pre[wid] = before;
+  }
   __syncthreads();
   if (wid == 0) {
-    uint64_t a = wt[lane], s = a;
+    uint64_t a = wt[lane], s = a, p = pre[lane];
     for (int o = 1; o < 32; o <<= 1) {
       uint64_t u = __shfl_up_sync(0xffffffffu, s, o);
       if (lane >= o) s += u;
+      p += __shfl_xor_sync(0xffffffffu, p, o);
     }
-    wt[lane] = s - a;
+    wt[lane] = p + s - a;
   }
   __syncthreads();
-  uint64_t run = bsum_scanned[blockIdx.x] + wt[wid] + incl - local;
+  uint64_t run = wt[wid] + incl - local;
+  uint64_t c = at / T;  // column of the next item that starts one
+  if (c * T < at) ++c;
+#pragma unroll
   for (int j = 0; j < per; ++j) {
-    const uint64_t i = beg + threadIdx.x * per + j;
-    if (i < len) out[i] = run;
-    run += v[j];
+    const uint64_t i = at + j;
+    if (i < len) {
+      out[i] = run;
+      if (i == c * T) {
+        if (c <= nsub) csr_off[c] = run;
+        ++c;
+      }
+      run += v[j];
+      if (i == len - 1) {
+        out[len] = run;
+        if (len == (uint64_t)nsub * T) csr_off[nsub] = run;
+      }
+    }
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 1023) out[len] = run;
 }
 
 // --------------------------------------------------------------------------
@@ -712,15 +740,19 @@ int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
                       StatusOut{out, nullptr, nullptr, nullptr, nullptr, n});
 }
 
-int launch_scan_u32_to_u64(cudaStream_t s, const uint32_t* in, uint64_t len,
-                           uint64_t* bsum, uint64_t* out) {
-  const uint32_t nb = (uint32_t)((len + kScanBlock - 1) / kScanBlock);
-  const uint32_t g = nb ? nb : 1;
-  k_scan_partials<<<g, 1024, 0, s>>>(in, len, bsum);
-  SKC_LAUNCH_CHECK();
-  k_scan_single<uint64_t><<<1, 1024, 0, s>>>(bsum, g);
-  SKC_LAUNCH_CHECK();
-  k_scan_apply<<<g, 1024, 0, s>>>(in, len, bsum, out);
+int launch_scan_counts(cudaStream_t s, const uint32_t* in, uint64_t len, uint64_t* bsum,
+                       uint64_t* out, uint32_t T, uint32_t nsub, uint64_t* csr_off) {
+  const uint32_t g = (uint32_t)((len + kScanBlock - 1) / kScanBlock);  // len >= 32
+  const int scan = g > kSelfScanBlocks;
+  if (g > 1) {
+    k_scan_partials<<<g, 1024, 0, s>>>(in, len, bsum);
+    SKC_LAUNCH_CHECK();
+  }
+  if (scan) {
+    k_scan_single<uint64_t><<<1, 1024, 0, s>>>(bsum, g);
+    SKC_LAUNCH_CHECK();
+  }
+  k_scan_apply<<<g, 1024, 0, s>>>(in, len, bsum, scan, out, T, nsub, csr_off);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
