@@ -114,10 +114,8 @@ struct BitState {
   static constexpr bool REG = (W <= 32);   // STRICT in registers
   static constexpr uint32_t AW = NSUB / 2;  // tie-map words (2 entries each)
   static constexpr bool A_SMEM = (D <= 12);  // tie map in shared memory
-  // Above, the map lives in a global slab and is closed chunk by chunk
-  // through a 512-word shared scratch (tie_global_output).
-  static constexpr uint32_t CHUNK_WORDS = A_SMEM ? 0 : 512;
-  // Also above: the first LIST_WORDS tie pairs of a candidate are kept as a
+  // Above, the map lives in a global slab and is closed chunk by chunk in
+  // registers (tie_global_output), and the first LIST_WORDS tie pairs of a candidate are kept as a
   // list (E | L << 16) and applied directly when no more come; the global
   // map is used only when a candidate has more.
   static constexpr uint32_t LIST_WORDS = A_SMEM ? 0 : 32;
@@ -128,7 +126,7 @@ struct BitState {
   static constexpr uint32_t WALK_WORDS = BQ_WORDS + WQ_WORDS + HQ_WORDS;
   // shared memory per warp, in words
   static constexpr uint32_t SMEM_WORDS =
-      (REG ? 0 : W) + (A_SMEM ? AW : 0) + CHUNK_WORDS + LIST_WORDS + WALK_WORDS;
+      (REG ? 0 : W) + (A_SMEM ? AW : 0) + LIST_WORDS + WALK_WORDS;
 };
 
 // Splits the subsets of h over 32 lanes: `low` = the lowest five set bits of
@@ -234,14 +232,17 @@ struct FullFix {
   }
 };
 
-// Phase 2, per chunk: load it into the scratch Cs, close its ten low entry
-// bits there, and turn it straight into the chunk's 32 output words (entry
-// S is tie-dominated iff S meets T[S]): word j of the chunk gives the bits
-// of entries 2j and 2j+1, two ballots over j = 32i + lane give output words
-// 2i (lanes 0..15) and 2i+1 (lanes 16..31) after an even/odd interleave.
-// Lane l ends with output word 32c + l and writes dom and ext for it.
+// Phase 2, per chunk: a lane takes its words 32k + lane (k < 16), closes the
+// chunk's ten low entry bits (bit 0 inside a word, bits 1..5 across lanes by
+// shuffles, bits 6..9 across its registers) and turns it straight into the
+// chunk's 32 output words (entry S is tie-dominated iff S meets T[S]): word j
+// of the chunk gives the bits of entries 2j and 2j+1, two ballots over j =
+// 32k + lane give output words 2k (lanes 0..15) and 2k+1 (lanes 16..31) after
+// an even/odd interleave. Lane l ends with output word 32c + l and writes dom
+// and ext for it. (Shared memory holds STRICT only: a 2 KB scratch per warp
+// here cost d = 16 a third of its warps per SM.)
 template <int D>
-__device__ void tie_global_output(uint32_t* A, uint32_t* Cs, const uint32_t* sat_s, int lane,
+__device__ void tie_global_output(uint32_t* A, const uint32_t* sat_s, int lane,
                                   uint32_t p, uint32_t* __restrict__ out_dom,
                                   uint32_t* __restrict__ out_ext, const FullFix& fix) {
   constexpr int HB = D - 10;
@@ -251,29 +252,32 @@ __device__ void tie_global_output(uint32_t* A, uint32_t* Cs, const uint32_t* sat
   if constexpr (HB > 4) closure_chunk_bits<HB - 4>(A, lane, 4, NC);
   __syncwarp();
   for (uint32_t c = 0; c < NC; ++c) {
+    uint32_t v[16];
 #pragma unroll
     for (uint32_t k = 0; k < 16; ++k) {
-      const uint32_t x = A[(c << 9) + 32 * k + lane];
-      Cs[32 * k + lane] = x | (x >> 16);  // entry bit 0 (inside the word)
+      v[k] = A[(c << 9) + 32 * k + lane];
+      v[k] |= v[k] >> 16;  // entry bit 0 (inside the word)
     }
-    __syncwarp();
-    for (int j = 1; j <= 9; ++j) {  // entry bit j: words w and w + 2^(j-1)
-      const uint32_t st = 1u << (j - 1);
 #pragma unroll
-      for (uint32_t t = lane; t < 256; t += 32) {
-        const uint32_t w = ((t >> (j - 1)) << j) | (t & (st - 1));
-        Cs[w] |= Cs[w + st];
+    for (int j = 0; j < 5; ++j) {  // entry bit j + 1: lanes l and l + 2^j
+#pragma unroll
+      for (uint32_t k = 0; k < 16; ++k) {
+        const uint32_t y = __shfl_xor_sync(kFull, v[k], 1 << j);
+        if (!(lane & (1 << j))) v[k] |= y;
       }
-      __syncwarp();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {  // entry bit j + 6: registers k and k + 2^j
+#pragma unroll
+      for (uint32_t k = 0; k < 16; ++k)
+        if (!(k & (1u << j))) v[k] |= v[k | (1u << j)];
     }
     uint32_t mine = 0;
 #pragma unroll
     for (uint32_t i = 0; i < 16; ++i) {
-      const uint32_t j = 32 * i + lane;
-      const uint32_t x = Cs[j];
-      const uint32_t e0 = (c << 10) + 2 * j;
-      const uint32_t ev = __ballot_sync(kFull, (e0 & x & 0xffffu) != 0u);
-      const uint32_t od = __ballot_sync(kFull, ((e0 + 1) & (x >> 16)) != 0u);
+      const uint32_t e0 = (c << 10) + 2 * (32 * i + lane);
+      const uint32_t ev = __ballot_sync(kFull, (e0 & v[i] & 0xffffu) != 0u);
+      const uint32_t od = __ballot_sync(kFull, ((e0 + 1) & (v[i] >> 16)) != 0u);
       const uint32_t lo = spread_even(ev & 0xffffu) | (spread_even(od & 0xffffu) << 1);
       const uint32_t hi = spread_even(ev >> 16) | (spread_even(od >> 16) << 1);
       if ((uint32_t)lane == 2 * i) mine = lo;
@@ -289,7 +293,6 @@ __device__ void tie_global_output(uint32_t* A, uint32_t* Cs, const uint32_t* sat
     fix.apply(t, dom, ext);
     out_dom[(uint64_t)p * W + t] = dom;
     if (out_ext) out_ext[(uint64_t)p * W + t] = ext;
-    __syncwarp();  // Cs is reused by the next chunk
   }
 }
 
@@ -346,25 +349,44 @@ __device__ __forceinline__ uint32_t nr_close_reg(uint32_t x, uint32_t wi, int ca
 }
 
 // Shared memory (d >= 11): lane owns words 32i + lane. Word bits 0..4 are
-// exchanged by shuffles, the row bits i stay inside the lane's column.
+// exchanged by shuffles, the row bits i stay inside the lane's column. Rows
+// go eight at a time through registers (independent chains; one row after
+// the other, the closures of 500k x 16 -m 6 were a third of the kernel's
+// cycles): a block's three low row bits are closed on the way, the others
+// row by row across blocks.
 template <int D>
 __device__ void nr_close_smem(uint32_t* sat_s, int lane, int cap) {
-  constexpr uint32_t R = BitState<D>::W / 32;
+  constexpr uint32_t R = BitState<D>::W / 32;  // rows, a power of two
+  constexpr uint32_t RB = R < 8 ? R : 8;
   __syncwarp();
-  for (uint32_t i = 0; i < R; ++i) {
-    const uint32_t w = 32 * i + lane;
-    uint32_t x = subset_and_in_word(sat_s[w] | pop_above(cap - __popc(w)));
+  for (uint32_t i0 = 0; i0 < R; i0 += RB) {
+    uint32_t x[RB];
+#pragma unroll
+    for (uint32_t r = 0; r < RB; ++r) {
+      const uint32_t w = 32 * (i0 + r) + lane;
+      x[r] = subset_and_in_word(sat_s[w] | pop_above(cap - __popc(w)));
+    }
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
-      const uint32_t y = __shfl_xor_sync(kFull, x, 1 << j);
-      if (lane & (1 << j)) x &= y;
+#pragma unroll
+      for (uint32_t r = 0; r < RB; ++r) {
+        const uint32_t y = __shfl_xor_sync(kFull, x[r], 1 << j);
+        if (lane & (1 << j)) x[r] &= y;
+      }
     }
-    sat_s[w] = x;
+#pragma unroll
+    for (uint32_t st = 1; st < RB; st <<= 1) {
+#pragma unroll
+      for (uint32_t r = 0; r < RB; ++r)
+        if (r & st) x[r] &= x[r ^ st];
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < RB; ++r) sat_s[32 * (i0 + r) + lane] = x[r];
   }
-  for (uint32_t j = 0; (1u << j) < R; ++j) {
-    const uint32_t st = 1u << j;
+  for (uint32_t st = RB; st < R; st <<= 1) {
+#pragma unroll 8
     for (uint32_t t = 0; t < R / 2; ++t) {
-      const uint32_t i = ((t >> j) << (j + 1)) | st | (t & (st - 1));
+      const uint32_t i = ((t & ~(st - 1)) << 1) | st | (t & (st - 1));
       sat_s[32 * i + lane] &= sat_s[32 * (i ^ st) + lane];
     }
   }
@@ -557,7 +579,7 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
           }
           if (tie_lane) atomicOr(&A[le >> 1], lt << (16 * (le & 1)));
         } else {
-          uint32_t* tlist = wsm + W + BS::CHUNK_WORDS;
+          uint32_t* tlist = wsm + W;
           const uint32_t nt = __popc(tb);
           if (tmode != 2 && tcount + nt <= BS::LIST_WORDS) {
             if (tie_lane) tlist[tcount + __popc(tb & ((1u << lane) - 1u))] = le | (lt << 16);
@@ -808,7 +830,7 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
     if constexpr (!BS::A_SMEM) {
       if (tmode == 2) {
         __syncwarp();
-        tie_global_output<D>(A, wsm + W, sat_s, lane, p, out_dom, out_ext, fix);
+        tie_global_output<D>(A, sat_s, lane, p, out_dom, out_ext, fix);
         __syncwarp();
         continue;
       }
@@ -816,7 +838,7 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
         // Few pairs: word w of each pair's tie set down(E) \ down(E \ L)
         // is submask(E & 31) when w is a subset of E >> 5, minus
         // submask(F & 31) when w is also a subset of F >> 5, F = E \ L.
-        const uint32_t* tlist = wsm + W + BS::CHUNK_WORDS;
+        const uint32_t* tlist = wsm + W;
         for (uint32_t w = lane; w < W; w += 32) {
           uint32_t t_ = 0;
           for (uint32_t j = 0; j < tcount; ++j) {
