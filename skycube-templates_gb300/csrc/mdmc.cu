@@ -113,11 +113,13 @@ struct BitState {
   static constexpr uint32_t W = NSUB >= 32 ? NSUB / 32 : 1;  // bitmap words
   static constexpr bool REG = (W <= 32);   // STRICT in registers
   static constexpr uint32_t AW = NSUB / 2;  // tie-map words (2 entries each)
-  static constexpr bool A_SMEM = (D <= 12);  // tie map in shared memory
+  static constexpr bool A_SMEM = (D <= 11);  // tie map in shared memory
   // Above, the map lives in a global slab and is closed chunk by chunk in
-  // registers (tie_global_output), and the first LIST_WORDS tie pairs of a candidate are kept as a
-  // list (E | L << 16) and applied directly when no more come; the global
-  // map is used only when a candidate has more.
+  // registers (tie_global_output), and the first LIST_WORDS tie pairs of a
+  // candidate are kept as a list (E | L << 16) and applied directly when no
+  // more come; the global map is used only when a candidate has more. At 12
+  // attributes the map would take 8 KB of shared memory per warp, 24 warps
+  // per SM: 400k x 12 -m 4 9.4 ms with it, 7.7 without.
   static constexpr uint32_t LIST_WORDS = A_SMEM ? 0 : 32;
   // The walk's queues, last: open blocks (up to 7 waiting + 32 from a
   // box-test step), open 8-q quarters (up to 15 + 32 from a quarter step)
@@ -181,7 +183,7 @@ __device__ void tie_closure(uint32_t* A, int lane) {
   }
 }
 
-// The same closure for a map in the global slab (d >= 13), blocked so that
+// The same closure for a map in the global slab (d >= 12), blocked so that
 // a warp makes tens of memory round trips per candidate instead of one per
 // pass and word. Entries are grouped in chunks of 1024 (512 words): entry
 // bits 0..9 lie inside a chunk, bits 10..d-1 index the chunk.
@@ -357,22 +359,24 @@ __device__ __forceinline__ uint32_t nr_close_reg(uint32_t x, uint32_t wi, int ca
 template <int D>
 __device__ void nr_close_smem(uint32_t* sat_s, int lane, int cap) {
   constexpr uint32_t R = BitState<D>::W / 32;  // rows, a power of two
-  constexpr uint32_t RB = R < 8 ? R : 8;
+  constexpr uint32_t RB = R < 8u ? R : 8u;
   __syncwarp();
+  const uint32_t above = pop_above(lane - 16);  // lane l: pop_above(l - 16)
+  const int cl = cap - __popc(lane) + 16;
   for (uint32_t i0 = 0; i0 < R; i0 += RB) {
     uint32_t x[RB];
+    const int ci = cl - __popc(i0);
+    uint32_t pa[5];  // pop_above(cap - popc(word)) for 0 .. 4 more row bits
 #pragma unroll
-    for (uint32_t r = 0; r < RB; ++r) {
-      const uint32_t w = 32 * (i0 + r) + lane;
-      x[r] = subset_and_in_word(sat_s[w] | pop_above(cap - __popc(w)));
-    }
+    for (int j = 0; j < 5; ++j) pa[j] = __shfl_sync(kFull, above, max(0, min(31, ci - j)));
+#pragma unroll
+    for (uint32_t r = 0; r < RB; ++r)
+      x[r] = subset_and_in_word(sat_s[32 * (i0 + r) + lane] | pa[(r & 1) + ((r >> 1) & 1) + ((r >> 2) & 1) + ((r >> 3) & 1)]);
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
+      const uint32_t keep = lane & (1 << j) ? 0u : kFull;
 #pragma unroll
-      for (uint32_t r = 0; r < RB; ++r) {
-        const uint32_t y = __shfl_xor_sync(kFull, x[r], 1 << j);
-        if (lane & (1 << j)) x[r] &= y;
-      }
+      for (uint32_t r = 0; r < RB; ++r) x[r] &= __shfl_xor_sync(kFull, x[r], 1 << j) | keep;
     }
 #pragma unroll
     for (uint32_t st = 1; st < RB; st <<= 1) {
@@ -383,6 +387,7 @@ __device__ void nr_close_smem(uint32_t* sat_s, int lane, int cap) {
 #pragma unroll
     for (uint32_t r = 0; r < RB; ++r) sat_s[32 * (i0 + r) + lane] = x[r];
   }
+#pragma unroll
   for (uint32_t st = RB; st < R; st <<= 1) {
 #pragma unroll 8
     for (uint32_t t = 0; t < R / 2; ++t) {
@@ -394,11 +399,11 @@ __device__ void nr_close_smem(uint32_t* sat_s, int lane, int cap) {
 }
 
 // Register budgets: d <= 10 (STRICT in registers) 8 CTAs per SM uncapped
-// (32 registers, no spill), 6 capped; d >= 11, 4 CTAs (64 registers).
-// Unbounded, the allocator took 48 registers at d = 10 (40 warps per SM
-// instead of 64) and up to 136 at d = 16.
+// (32 registers, no spill), 6 capped; 11 to 15 attributes 5 CTAs (48
+// registers; 4 CTAs at 64: 300k x 14 -m 5 17.6 ms, 16.9 with 5); 16
+// attributes 3, by shared memory (70 KB per CTA).
 template <int D, bool CAP>
-__global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
+__global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : (D <= 15 ? 5 : 4))) k_bitmaps(
     const uint4* __restrict__ pcells, const float* __restrict__ px,
     uint64_t p_pad, const uint4* __restrict__ qcells,
     const float* __restrict__ qx, const uint4* __restrict__ bmin,
@@ -432,9 +437,11 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
   const uint32_t pend = min(m, p_end_cap);
   const uint32_t wi = REG ? (uint32_t)lane % W : 0;
   const int sh = depth - 1;
-  // Capped mode, d >= 11: blocks walked between closures (a closure costs
-  // about as much as walking W / 32 blocks).
-  constexpr uint32_t kCloseBlocks = W / 32;
+  // Capped mode, d >= 11: steps between closures. A closure costs about as
+  // much as 40 steps at d = 16; 500k x 16 -m 6 with W / 32, W / 20, W / 16 and
+  // W / 10 steps between two: 115.8, 112.4, 112.2, 114.0 ms; 200k x 13 -m 4:
+  // 5.44, 5.44, 5.52, 5.63.
+  constexpr uint32_t kCloseBlocks = W / 20;
 
 #if SKC_BITMAP_COUNTERS
   unsigned long long cnt_[kBitmapCounters] = {};
@@ -496,7 +503,7 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
       }
     };
     bool touched = false;  // tie map in use for this p
-    // d >= 13: 0 no tie pair, 1 pairs in the list, 2 pairs in the global map
+    // d >= 12: 0 no tie pair, 1 pairs in the list, 2 pairs in the global map
     int tmode = 0;
     uint32_t tcount = 0;  // pairs in the list (same in every lane)
     auto in_strict = [&](uint32_t S) -> bool {
@@ -534,33 +541,18 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : 4)) k_bitmaps(
         const uint32_t Z = U & G;   // equal cells: compare the floats
         le = Y;
         lt = Y;
-        // The warp runs the union of its lanes' work: the unrolled form
-        // costs all D predicated steps whenever any lane has a cell tie, the
-        // loop only as many as the lane with the most ties. Measured on one
-        // box (bitmap kernel, identical outputs): 1M x 10 13.53 -> 11.65 ms,
-        // 400k x 12 33.7 -> 31.9 ms, 400k x 12 -m 6 23.06 -> 21.73 ms, 300k x
-        // 14 51.2 -> 49.0 ms; capped above 12 attributes the loop lost
-        // (500k x 16 -m 6 242.7 -> 249.0 ms, -m 8 434 -> 450 ms), and those
-        // keep the unrolled form.
-        if constexpr (!CAP || D <= 12) {
-          for (uint32_t z = Z; z; z &= z - 1) {
-            const int k = __ffs(z) - 1;
-            const float a = qx[(uint64_t)k * p_pad + qi];
-            const float b = pxp[(uint64_t)k * p_pad];
-            const uint32_t bit = 1u << k;
-            if (a <= b) le |= bit;
-            if (a < b) lt |= bit;
-          }
-        } else if (Z) {
-#pragma unroll
-          for (int k = 0; k < D; ++k) {
-            if (Z & (1u << k)) {
-              const float a = qx[(uint64_t)k * p_pad + qi];
-              const float b = pxp[(uint64_t)k * p_pad];
-              if (a <= b) le |= 1u << k;
-              if (a < b) lt |= 1u << k;
-            }
-          }
+        // The warp runs the union of its lanes' work: a loop over the tied
+        // attributes takes as many rounds as the lane with the most ties,
+        // an unrolled pass D predicated steps whenever any lane has one.
+        // Measured (bitmap kernel): 1M x 10 13.53 -> 11.65 ms, 500k x 16
+        // -m 6 136 -> 125 ms, 300k x 14 -m 5 20.0 -> 18.3.
+        for (uint32_t z = Z; z; z &= z - 1) {
+          const int k = __ffs(z) - 1;
+          const float a = qx[(uint64_t)k * p_pad + qi];
+          const float b = pxp[(uint64_t)k * p_pad];
+          const uint32_t bit = 1u << k;
+          if (a <= b) le |= bit;
+          if (a < b) lt |= bit;
         }
       }
       const bool t_lt = in_strict(lt);
@@ -911,7 +903,7 @@ static int bitmap_grid_dc(int num_sms, int* grid, size_t* smem) {
   int per_sm = 0;
   SKC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bitmaps<D, CAP>, threads, *smem));
   if (per_sm < 1) per_sm = 1;
-  if (!BS::A_SMEM && per_sm > 4) per_sm = 4;  // bounds the global tie-map slab
+  if (!BS::A_SMEM && per_sm > 5) per_sm = 5;  // bounds the global tie-map slab
   *grid = per_sm * num_sms;
   return SKC_OK;
 }
