@@ -280,7 +280,32 @@ struct FullSpace {
   uint32_t* sky_pos = nullptr;  // positions of the skyline points among the candidates
   uint32_t* counts = nullptr;  // device [0]=|sky| [1]=|ext| [2]=|cand|
   uint32_t h_counts[3] = {0, 0, 0};
+  // Short input (small.cu): no grid cells were made; every later list is a
+  // part of it and takes the short-list kernel too. With `deferred` the
+  // counts were not read back: h_counts holds n, their upper bound.
+  bool small = false, deferred = false;
+  uint32_t* masks = nullptr;    // small.cu's scratch
+  uint32_t* tickets = nullptr;  // two zeroed words for it
 };
+
+// Lists for which one launch over all pairs replaces the partition pipeline.
+static bool small_list(uint64_t m) { return m <= kSmallList; }
+
+// The full-space counts on the host (or, in plan mode, their capacity).
+static int full_space_counts(Exec& E, uint64_t n, FullSpace& F, Tracer& T) {
+  cudaStream_t s = E.stream;
+  if (E.plan) {
+    // Plan mode: candidates sized by the plan's capacity (no read-back).
+    const uint64_t cap = std::min<uint64_t>(E.plan->m_cap, n);
+    SKC_TRY(launch_cap_count(s, F.counts + 2, F.counts, (uint32_t)cap, E.plan->stats, 0));
+    F.h_counts[0] = F.h_counts[1] = 0;
+    F.h_counts[2] = (uint32_t)cap;
+    return SKC_OK;
+  }
+  SKC_TRY(copy_d2h(F.h_counts, F.counts, 3 * sizeof(uint32_t), s));
+  T.mark("full: compaction");
+  return SKC_OK;
+}
 
 // Scratch of launch_prefilter for lists of up to mmax entries and Kq pruners.
 static int prefilter_scratch(Arena& A, int d, uint64_t mmax, uint32_t Kq, PrefilterScratch* pf) {
@@ -314,16 +339,36 @@ static int part_scratch(Arena& A, uint64_t mmax, PartScratch* ps) {
 }
 
 static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A,
-                          FullSpace& F, Tracer& T) {
+                          FullSpace& F, Tracer& T, bool defer = false) {
   skc_context* ctx = E.ctx;
   cudaStream_t s = E.stream;
   const uint64_t n = ds->n;
   const int d = ds->d;
   const int depth = P.depth;
   const uint32_t full = (1u << d) - 1;
-  uint32_t* d_n;
-  SKC_TRY(A.alloc(&d_n, 1));
-  SKC_TRY(launch_set_u32(s, d_n, (uint32_t)n));
+  uint32_t* d_n;  // n, then the short-list kernel's tickets
+  SKC_TRY(A.alloc(&d_n, 3));
+  SKC_TRY(launch_set_u32(s, d_n, (uint32_t)n, 2));
+  F.tickets = d_n + 1;
+  if (small_list(n) && P.pq_size == 0) {
+    F.small = true;
+    SKC_TRY(A.alloc(&F.counts, 6));
+    SKC_TRY(A.alloc(&F.masks, 2 * (kSmallList / 32)));
+    SKC_TRY(A.alloc(&F.sky, n));
+    SKC_TRY(A.alloc(&F.ext, n));
+    SKC_TRY(A.alloc(&F.cand, n));
+    SKC_TRY(A.alloc(&F.cand_st, n));
+    SKC_TRY(A.alloc(&F.sky_pos, n));
+    SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, d, nullptr, d_n, n, full, F.masks,
+                                 F.tickets, {F.sky, F.ext, F.cand, F.cand_st, F.sky_pos, F.counts}));
+    T.mark("full: skyline kernel");
+    if (defer) {
+      F.deferred = true;
+      for (uint32_t& c : F.h_counts) c = (uint32_t)n;
+      return SKC_OK;
+    }
+    return full_space_counts(E, n, F, T);
+  }
   float* pivots;
   SKC_TRY(A.alloc(&pivots, (uint64_t)kMaxDims * kMaxPivots));
   SKC_TRY(A.alloc(&F.cells, n));
@@ -366,7 +411,7 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   uint32_t *blk0, *blk1;
   SKC_TRY(A.alloc(&blk0, nblk));
   SKC_TRY(A.alloc(&blk1, nblk));
-  SKC_TRY(A.alloc(&F.counts, 3));
+  SKC_TRY(A.alloc(&F.counts, 6));
   SKC_TRY(A.alloc(&F.sky, n));
   SKC_TRY(A.alloc(&F.ext, n));
   SKC_TRY(A.alloc(&F.cand, n));
@@ -374,17 +419,7 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(A.alloc(&F.sky_pos, n));
   SKC_TRY(launch_status_split(s, status, nullptr, d_n, n, blk0, blk1, F.sky, F.ext, F.counts,
                               F.cand, F.cand_st, F.sky_pos));
-  if (E.plan) {
-    // Plan mode: candidates sized by the plan's capacity (no read-back).
-    const uint64_t cap = std::min<uint64_t>(E.plan->m_cap, n);
-    SKC_TRY(launch_cap_count(s, F.counts + 2, F.counts, (uint32_t)cap, E.plan->stats, 0));
-    F.h_counts[0] = F.h_counts[1] = 0;
-    F.h_counts[2] = (uint32_t)cap;
-    return SKC_OK;
-  }
-  SKC_TRY(copy_d2h(F.h_counts, F.counts, 3 * sizeof(uint32_t), s));
-  T.mark("full: compaction");
-  return SKC_OK;
+  return full_space_counts(E, n, F, T);
 }
 
 // Bitmaps of every candidate, then CSR compaction (BATCHED and PLAIN/MDMC).
@@ -559,6 +594,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
 struct CuboidScratch {
   PartScratch ps;
   uint32_t *cand = nullptr, *d_m = nullptr, *blk0 = nullptr, *blk1 = nullptr, *cnt = nullptr;
+  uint32_t* masks = nullptr;  // short lists (small.cu)
   uint8_t* status = nullptr;
   // Counts read back per cuboid. Pageable on purpose: freeing pinned host
   // memory (cudaFreeHost) waits for the whole device, which stalled a
@@ -566,35 +602,42 @@ struct CuboidScratch {
   uint32_t h_cnt[2] = {0, 0};
 };
 
-static int cuboid_scratch(Arena& A, int d, uint64_t mmax, CuboidScratch* cs) {
-  (void)d;
-  SKC_TRY(part_scratch(A, mmax, &cs->ps));
+static int cuboid_scratch(Arena& A, uint64_t mmax, CuboidScratch* cs) {
   SKC_TRY(A.alloc(&cs->cand, mmax));
+  SKC_TRY(A.alloc(&cs->d_m, 2));
+  SKC_TRY(A.alloc(&cs->cnt, 3));
+  SKC_TRY(A.alloc(&cs->masks, 2 * (kSmallList / 32)));
+  if (small_list(mmax)) return SKC_OK;
+  SKC_TRY(part_scratch(A, mmax, &cs->ps));
   SKC_TRY(A.alloc(&cs->status, round_up(mmax, 4)));
-  SKC_TRY(A.alloc(&cs->d_m, 1));
   const uint64_t nblk = (mmax + 1023) / 1024 + 2;
   SKC_TRY(A.alloc(&cs->blk0, nblk));
   SKC_TRY(A.alloc(&cs->blk1, nblk));
-  SKC_TRY(A.alloc(&cs->cnt, 3));
   return SKC_OK;
 }
 
 // Skyline and extended skyline of cuboid c over an ascending candidate list
-// (both outputs ascending), with the median-partition pipeline; one host
-// round trip for the counts.
+// of mc entries (both outputs ascending), with the short-list kernel or the
+// median-partition pipeline; cs.d_m holds mc and 0. One host round trip for
+// the counts.
 static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Arena& A,
                         CuboidScratch& cs, uint32_t c, const uint32_t* cand, uint64_t mc,
                         uint32_t** osky, uint32_t** oext, uint64_t* nsky, uint64_t* next) {
   cudaStream_t s = E.stream;
-  SKC_TRY(launch_set_u32(s, cs.d_m, (uint32_t)mc));
-  LevelTables LT;
-  SKC_TRY(level_tables(E.ctx, partition_dims(c), &LT));
-  PartitionSkylineArgs pa{nullptr, cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status, F.amin};
-  SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, depth, LT, pa, cs.ps));
   SKC_TRY(A.alloc(osky, mc));
   SKC_TRY(A.alloc(oext, mc));
-  SKC_TRY(launch_status_split(s, cs.status, cand, cs.d_m, mc, cs.blk0, cs.blk1, *osky, *oext,
-                              cs.cnt));
+  if (small_list(mc)) {
+    SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, ds->d, cand, cs.d_m, mc, c, cs.masks,
+                                 cs.d_m + 1, {*osky, *oext, nullptr, nullptr, nullptr, cs.cnt}));
+  } else {
+    LevelTables LT;
+    SKC_TRY(level_tables(E.ctx, partition_dims(c), &LT));
+    PartitionSkylineArgs pa{nullptr, cand, F.cells, ds->x, ds->n_pad, cs.d_m, mc, c, cs.status,
+                            F.amin};
+    SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, depth, LT, pa, cs.ps));
+    SKC_TRY(launch_status_split(s, cs.status, cand, cs.d_m, mc, cs.blk0, cs.blk1, *osky, *oext,
+                                cs.cnt));
+  }
   SKC_TRY(copy_d2h(cs.h_cnt, cs.cnt, 2 * sizeof(uint32_t), s));
   *nsky = cs.h_cnt[0];
   *next = cs.h_cnt[1];
@@ -681,7 +724,7 @@ static int run_sdsc_plain(Exec& E, skc_dataset* ds, int max_d,
   done[full] = 1;
 
   CuboidScratch cs;
-  SKC_TRY(cuboid_scratch(A, d, nsky[full] + next[full], &cs));
+  SKC_TRY(cuboid_scratch(A, nsky[full] + next[full], &cs));
   for (int lev = d - 1; lev >= 1; --lev) {
     if (lev > max_d) continue;
     for (uint32_t c = 1; c < full; ++c) {
@@ -693,7 +736,7 @@ static int run_sdsc_plain(Exec& E, skc_dataset* ds, int max_d,
       // Candidates = parent skyline + extended skyline, merged ascending so
       // every output list stays ascending (compaction keeps list order).
       SKC_TRY(launch_merge_disjoint(E.stream, sky[src], (uint32_t)nsky[src], ext[src],
-                                    (uint32_t)next[src], cs.cand));
+                                    (uint32_t)next[src], cs.cand, cs.d_m));
       SKC_TRY(cuboid_lists(E, ds, F, depth_of_call, A, cs, c, cs.cand, mc, &sky[c], &ext[c],
                            &nsky[c], &next[c]));
     }
@@ -947,10 +990,11 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
       // Over a capacity: the single-cuboid pipeline on the full-space
       // candidates (ascending, a superset of every cuboid's lists).
       if (!cs_ready) {
-        SKC_TRY(cuboid_scratch(A, d, F.h_counts[2], &cs));
+        SKC_TRY(cuboid_scratch(A, F.h_counts[2], &cs));
         cs_ready = true;
       }
       ++fallbacks;
+      SKC_TRY(launch_set_u32(s, cs.d_m, F.h_counts[2], 1));
       SKC_TRY(cuboid_lists(E, ds, F, J.depth, A, cs, c, F.cand, F.h_counts[2], &sky[c], &ext[c],
                            &nsky[c], &next[c]));
     }
@@ -1424,20 +1468,28 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
   const int d = ds->d;
   const uint32_t nsub = 1u << d, full = nsub - 1;
   uint32_t *sky = F.sky, *ext = F.ext;
-  uint64_t nsky = F.h_counts[0], next = F.h_counts[1];
-  if (S != full) {
-    const uint64_t m = F.h_counts[2];
+  uint32_t* cnt = F.counts;  // counts of the two lists, on the device
+  uint32_t h[6] = {F.h_counts[0], F.h_counts[1], F.h_counts[2], 0, 0, 0};
+  const uint64_t m = F.h_counts[2];
+  if (S != full && small_list(m)) {
+    cnt = F.counts + 3;
+    if (!F.masks) SKC_TRY(A.alloc(&F.masks, 2 * (kSmallList / 32)));
+    SKC_TRY(A.alloc(&sky, m));
+    SKC_TRY(A.alloc(&ext, m));
+    SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, d, F.cand, F.counts + 2, m, S, F.masks,
+                                 F.tickets + 1, {sky, ext, nullptr, nullptr, nullptr, cnt}));
+  } else if (S != full) {
+    cnt = F.counts + 3;
     LevelTables LT;
     SKC_TRY(level_tables(E.ctx, partition_dims(S), &LT));
     PartScratch ps;
     SKC_TRY(part_scratch(A, m, &ps));
     uint8_t* status;
-    uint32_t *blk0, *blk1, *cnt;
+    uint32_t *blk0, *blk1;
     SKC_TRY(A.alloc(&status, round_up(m, 4)));
     const uint64_t nblk = (m + 1023) / 1024 + 2;
     SKC_TRY(A.alloc(&blk0, nblk));
     SKC_TRY(A.alloc(&blk1, nblk));
-    SKC_TRY(A.alloc(&cnt, 3));
     SKC_TRY(A.alloc(&sky, m));
     SKC_TRY(A.alloc(&ext, m));
     const uint32_t* open = nullptr;
@@ -1461,33 +1513,25 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
     PartitionSkylineArgs pa{open, F.cand, F.cells, ds->x, ds->n_pad, m_open, m, S, status, F.amin};
     SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, d, depth, LT, pa, ps));
     SKC_TRY(launch_status_split(s, status, F.cand, m_ptr, m, blk0, blk1, sky, ext, cnt));
-    uint32_t h[2] = {0, 0};
-    SKC_TRY(copy_d2h(h, cnt, sizeof(h), s));
-    nsky = h[0];
-    next = h[1];
-    T.mark("subspace skyline");
   }
-  for (int pass = 0; pass < 2; ++pass) {
-    std::vector<uint64_t> off(nsub + 1, 0);
-    const uint64_t cntc = pass == 0 ? nsky : next;
-    for (uint32_t c = 0; c < nsub; ++c) off[c + 1] = off[c] + (c == S ? cntc : 0);
-    uint64_t* d_off;
-    SKC_TRY(A.alloc(&d_off, nsub + 1));
-    SKC_TRY(copy_h2d(d_off, off.data(), (nsub + 1) * sizeof(uint64_t), s));
-    SKC_CUDA(cudaStreamSynchronize(s));  // `off` is a host temporary
-    uint32_t* ids = pass == 0 ? sky : ext;
-    A.release(d_off);
-    A.release(ids);
-    if (pass == 0) {
-      R->d_off = d_off;
-      R->d_ids = ids;
-      R->total_ids = cntc;
-    } else {
-      R->d_eoff = d_off;
-      R->d_eids = ids;
-      R->total_ext = cntc;
-    }
-  }
+  uint64_t* off[2];
+  SKC_TRY(A.alloc(&off[0], nsub + 1));
+  SKC_TRY(A.alloc(&off[1], nsub + 1));
+  SKC_TRY(launch_single_offsets(s, cnt, S, nsub, off[0], off[1]));
+  if (S != full || F.deferred) SKC_TRY(copy_d2h(h, F.counts, sizeof(h), s));
+  if (S != full) T.mark("subspace skyline");
+  for (int i = 0; i < 3; ++i) F.h_counts[i] = h[i];
+  const uint32_t* hc = S != full ? h + 3 : h;
+  for (uint64_t* p : off) A.release(p);
+  A.release(sky);
+  A.release(ext);
+  R->d_off = off[0];
+  R->d_ids = sky;
+  R->total_ids = hc[0];
+  R->d_eoff = off[1];
+  R->d_eids = ext;
+  R->total_ext = hc[1];
+  R->n_cand = h[2];
   return SKC_OK;
 }
 
@@ -1520,7 +1564,7 @@ static int skycube_exec(Exec& E, skc_dataset* ds, const skc_options* opt, skc_re
     Arena A(s);
     FullSpace F;
     Tracer T(E);
-    st = run_full_space(E, ds, P, A, F, T);
+    st = run_full_space(E, ds, P, A, F, T, o.subspace != 0);
     if (st == SKC_OK) {
       R->n_cand = F.h_counts[2];
       if (o.subspace) {

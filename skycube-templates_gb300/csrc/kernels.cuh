@@ -55,9 +55,11 @@ int launch_block_min(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr,
                      uint64_t m_max, uint4* bmin, uint4* smin, uint4* hmin);
 int launch_csr_gather(cudaStream_t s, const uint32_t* const* srcs,
                       const uint64_t* dst_off, uint32_t ncub, uint32_t* dst);
-int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v);
+// p[0] = v, p[1 .. zeros] = 0.
+int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v, uint32_t zeros = 0);
+// Also n[0] = na + nb, n[1] = 0.
 int launch_merge_disjoint(cudaStream_t s, const uint32_t* a, uint32_t na,
-                          const uint32_t* b, uint32_t nb, uint32_t* out);
+                          const uint32_t* b, uint32_t nb, uint32_t* out, uint32_t* n);
 int launch_sample_signature(cudaStream_t s, const float* x, uint64_t n_pad, uint64_t n, int d,
                             uint32_t* out);
 int launch_cap_count(cudaStream_t s, uint32_t* m_ptr, uint32_t* nsky_ptr, uint32_t cap,
@@ -140,6 +142,23 @@ int launch_q_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* mq_pt
 int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth,
                              const LevelTables& T, const PartitionSkylineArgs& a,
                              const PartScratch& ps);
+
+// small.cu: skyline of a list of at most kSmallList points on subspace S,
+// compaction included, in one launch. masks: [2 * kSmallList / 32], ticket: 0.
+constexpr uint32_t kSmallList = 6144;
+struct SplitOut {
+  uint32_t* sky;      // skyline ids, list order
+  uint32_t* ext;      // extended skyline ids
+  uint32_t* both;     // their union in list order, or nullptr
+  uint8_t* both_st;   // per entry of `both`: 0 skyline, else 2
+  uint32_t* pos0;     // per skyline id: its position in `both`
+  uint32_t* n;        // [3] counts: sky, ext, both
+};
+int launch_small_skyline(cudaStream_t s, const float* x, uint64_t n_pad, int d,
+                         const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max, uint32_t S,
+                         uint32_t* masks, uint32_t* ticket, const SplitOut& out);
+int launch_single_offsets(cudaStream_t s, const uint32_t* n, uint32_t S, uint32_t nsub,
+                          uint64_t* sky_off, uint64_t* ext_off);
 
 // prefilter.cu: pruner prefilter of a list on subspace S. Every list position
 // gets a status: 2 strictly dominated by a pruner, 1 dominated by one and

@@ -601,15 +601,22 @@ __global__ void k_csr_gather(const uint32_t* const* __restrict__ srcs,
   for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) dst[o + i] = src[i];
 }
 
-__global__ void k_set_u32(uint32_t* p, uint32_t v) { *p = v; }
+__global__ void k_set_u32(uint32_t* p, uint32_t v, uint32_t zeros) {
+  p[0] = v;
+  for (uint32_t i = 1; i <= zeros; ++i) p[i] = 0;
+}
 
 // Merges two ascending, disjoint id lists a[0..na) and b[0..nb) into
 // out[0..na+nb) (ascending): every element finds its rank in the other list
 // by binary search.
 __global__ void k_merge_disjoint(const uint32_t* __restrict__ a, uint32_t na,
                                  const uint32_t* __restrict__ b, uint32_t nb,
-                                 uint32_t* __restrict__ out) {
+                                 uint32_t* __restrict__ out, uint32_t* __restrict__ n) {
   const uint32_t total = na + nb;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    n[0] = total;
+    n[1] = 0;
+  }
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += gridDim.x * blockDim.x) {
     const bool from_a = i < na;
@@ -777,15 +784,14 @@ int launch_csr_gather(cudaStream_t s, const uint32_t* const* srcs,
 }
 
 int launch_merge_disjoint(cudaStream_t s, const uint32_t* a, uint32_t na,
-                          const uint32_t* b, uint32_t nb, uint32_t* out) {
-  if (na + nb == 0) return SKC_OK;
-  k_merge_disjoint<<<grid_for((uint64_t)na + nb, 256, 152 * 8), 256, 0, s>>>(a, na, b, nb, out);
+                          const uint32_t* b, uint32_t nb, uint32_t* out, uint32_t* n) {
+  k_merge_disjoint<<<grid_for((uint64_t)na + nb, 256, 152 * 8), 256, 0, s>>>(a, na, b, nb, out, n);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
 
-int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v) {
-  k_set_u32<<<1, 1, 0, s>>>(p, v);
+int launch_set_u32(cudaStream_t s, uint32_t* p, uint32_t v, uint32_t zeros) {
+  k_set_u32<<<1, 1, 0, s>>>(p, v, zeros);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }

@@ -1,0 +1,261 @@
+// Skyline of a short list (at most kSmallList points) on one subspace, in one
+// launch: statuses by comparing every pair's floats, then the compaction into
+// id lists by the last CTA to finish.
+//
+// The median-partition pipeline (partition.cu) takes eight launches and a
+// grid of cells before it compares anything, 60 to 90 us on one GB300 however
+// short the list. Up to a few thousand points all pairs are less work than
+// that: the full space of 1,000 x 4 uniform 20 us against 71, 5,003 x 8
+// correlated 45 against 95, 4,000 x 16 anticorrelated 47 against 110. At
+// 8,192 points it is even (ties x 10 110 against 105, anticorrelated x 16 143
+// against 150), so the limit lies below. Bound by the shared-memory broadcasts
+// and compares of the pairs. The suite has no counterpart (SkyAlign runs on
+// every list, src/sdsc/skyAlign.cu:9-53).
+#include "kernels.cuh"
+
+namespace skc {
+
+constexpr uint32_t kAllLanes = 0xffffffffu;
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr uint32_t kSmallUnroll = 4;  // q's tested side by side: a warp's chain of compares is its latency
+static_assert(kSmallList % 32 == 0 && kSmallList / 32 <= kSmallThreads,
+              "the last CTA scans one 32-point mask per thread");
+
+struct SmallArgs {
+  const float* x;            // attribute-major points
+  uint64_t n_pad;
+  unsigned long long attrs;  // attribute t of S in bits 4t .. 4t + 3
+  const uint32_t* ids;       // list position -> point id (nullptr: identity)
+  const uint32_t* m_ptr;     // list length, at most kSmallList
+  uint32_t* masks;           // [2 * kSmallList / 32] skyline, extended skyline bits
+  uint32_t* ticket;          // CTAs done, 0 before the launch
+  SplitOut out;
+};
+
+// The largest float below v (finite): q < v exactly when q <= float_below(v).
+__device__ __forceinline__ float float_below(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return __uint_as_float(v > 0.f ? u - 1u : v < 0.f ? u + 1u : 0x80000001u);
+}
+
+// A CTA owns 32 list entries (a lane each, in every warp); its warps share the
+// q's, staged a tile at a time, and read them by broadcast. Once a point is dominated
+// only strict domination matters, so its values become their predecessors and
+// the same <= test decides it (tied points else pass it again and again).
+template <int NA>
+__global__ void __launch_bounds__(kSmallThreads) k_small_skyline(SmallArgs a) {
+  constexpr int NV = (NA + 3) / 4;
+  constexpr uint32_t TQ = NV <= 2 ? 1024 : 512;  // q's per tile (at most 32 KB)
+  __shared__ float4 s_q[TQ * NV];  // [q][its NA values]
+  __shared__ uint32_t s_dom, s_strict, s_last;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t m = *a.m_ptr;
+  const uint32_t i = blockIdx.x * 32 + lane;
+  if (blockIdx.x * 32 < m) {
+    float pv[NA];
+    uint32_t id = 0;
+    if (i < m) id = a.ids ? a.ids[i] : i;
+#pragma unroll
+    for (int t = 0; t < NA; ++t)
+      pv[t] = i < m ? a.x[((a.attrs >> (4 * t)) & 15u) * a.n_pad + id] : 0.f;
+    const uint32_t none = __ballot_sync(kAllLanes, i >= m);
+    if (threadIdx.x == 0) {
+      s_dom = 0;
+      s_strict = none;  // lanes without a point count as settled
+    }
+    bool dom = false, strict = i >= m;
+    for (uint32_t base = 0; base < m; base += TQ) {
+      const uint32_t j = base + threadIdx.x;
+      if (threadIdx.x < TQ && j < m) {
+        const uint32_t qid = a.ids ? a.ids[j] : j;
+        float v[4 * NV];
+#pragma unroll
+        for (int t = 0; t < 4 * NV; ++t)
+          v[t] = t < NA ? a.x[((a.attrs >> (4 * t)) & 15u) * a.n_pad + qid] : 0.f;
+#pragma unroll
+        for (int t = 0; t < NV; ++t)
+          s_q[threadIdx.x * NV + t] = make_float4(v[4 * t], v[4 * t + 1], v[4 * t + 2], v[4 * t + 3]);
+      }
+      __syncthreads();
+      constexpr uint32_t QW = TQ / kSmallWarps;  // q's of a warp
+      const uint32_t end = min(QW, m - min(m, base + wid * QW));
+      for (uint32_t t0 = 0; t0 < end; t0 += kSmallUnroll) {
+        bool le[kSmallUnroll];
+        bool some = false;
+#pragma unroll
+        for (uint32_t u = 0; u < kSmallUnroll; ++u) {
+          // past the end the last q again: a q tested twice changes nothing
+          const float4* q = s_q + (wid * QW + min(t0 + u, end - 1)) * NV;
+          le[u] = !strict;
+#pragma unroll
+          for (int g = 0; g < NV; ++g) {
+            const float4 v = q[g];
+            le[u] &= v.x <= pv[4 * g];
+            if (4 * g + 1 < NA) le[u] &= v.y <= pv[4 * g + 1 < NA ? 4 * g + 1 : 0];
+            if (4 * g + 2 < NA) le[u] &= v.z <= pv[4 * g + 2 < NA ? 4 * g + 2 : 0];
+            if (4 * g + 3 < NA) le[u] &= v.w <= pv[4 * g + 3 < NA ? 4 * g + 3 : 0];
+          }
+          some |= le[u];
+        }
+        if (!__any_sync(kAllLanes, some)) continue;
+        for (uint32_t u = 0; u < kSmallUnroll; ++u) {
+          const float* qf = reinterpret_cast<const float*>(
+              s_q + (wid * QW + min(t0 + u, end - 1)) * NV);
+          // pv may have changed since the test above: compare again
+          bool lt_all = !strict, le_all = !strict, any = false;
+#pragma unroll
+          for (int k = 0; k < NA; ++k) {
+            const bool lt = qf[k] < pv[k];
+            le_all &= qf[k] <= pv[k];
+            lt_all &= lt;
+            any |= lt;
+          }
+          if (!le_all) continue;
+          if (dom || lt_all) {  // with dom, pv holds the predecessors
+            dom = true;
+            strict = true;
+          } else if (any) {
+            dom = true;
+#pragma unroll
+            for (int k = 0; k < NA; ++k) pv[k] = float_below(pv[k]);
+          }
+        }
+        if (__all_sync(kAllLanes, strict)) break;
+      }
+      const uint32_t sm = __ballot_sync(kAllLanes, strict);
+      if (lane == 0) atomicOr(&s_strict, sm);
+      __syncthreads();
+      const uint32_t settled = s_strict;
+      strict = strict || ((settled >> lane) & 1u);
+      if (settled == kAllLanes) break;  // the same for every warp
+    }
+    const uint32_t dm = __ballot_sync(kAllLanes, dom);
+    if (lane == 0) atomicOr(&s_dom, dm);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const uint32_t st = s_strict;
+      a.masks[blockIdx.x] = ~s_dom & ~st;
+      a.masks[kSmallList / 32 + blockIdx.x] = s_dom & ~st;
+    }
+  }
+  // The last CTA compacts; the masks are read past L1.
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  __shared__ uint32_t s_m0[kSmallList / 32], s_m1[kSmallList / 32];
+  __shared__ uint32_t s_o0[kSmallList / 32], s_o1[kSmallList / 32];
+  __shared__ uint32_t s_w0[kSmallWarps], s_w1[kSmallWarps];
+  const uint32_t nw = (m + 31) / 32;
+  const uint32_t t = threadIdx.x;
+  uint32_t m0 = 0, m1 = 0;
+  if (t < nw) {
+    m0 = __ldcg(a.masks + t);
+    m1 = __ldcg(a.masks + kSmallList / 32 + t);
+  }
+  uint32_t i0 = __popc(m0), i1 = __popc(m1);
+  const uint32_t c0 = i0, c1 = i1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(kAllLanes, i0, o), v = __shfl_up_sync(kAllLanes, i1, o);
+    if (lane >= (uint32_t)o) {
+      i0 += u;
+      i1 += v;
+    }
+  }
+  if (lane == 31) {
+    s_w0[wid] = i0;
+    s_w1[wid] = i1;
+  }
+  __syncthreads();
+  for (uint32_t w = 0; w < wid; ++w) {
+    i0 += s_w0[w];
+    i1 += s_w1[w];
+  }
+  if (t < kSmallList / 32) {
+    s_m0[t] = m0;
+    s_m1[t] = m1;
+    s_o0[t] = i0 - c0;
+    s_o1[t] = i1 - c1;
+  }
+  if (t == kSmallThreads - 1) {
+    a.out.n[0] = i0;
+    a.out.n[1] = i1;
+    a.out.n[2] = i0 + i1;
+  }
+  __syncthreads();
+  const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll 4
+  for (uint32_t w = wid; w < nw; w += kSmallWarps) {
+    const uint32_t b0 = s_m0[w], b1 = s_m1[w];
+    const bool sky = (b0 >> lane) & 1u, ext = (b1 >> lane) & 1u;
+    if (!sky && !ext) continue;
+    const uint32_t at = w * 32 + lane;
+    const uint32_t pid = a.ids ? a.ids[at] : at;
+    const uint32_t k0 = s_o0[w] + __popc(b0 & lt), k1 = s_o1[w] + __popc(b1 & lt);
+    if (sky) a.out.sky[k0] = pid;
+    else a.out.ext[k1] = pid;
+    if (a.out.both) {
+      a.out.both[k0 + k1] = pid;
+      a.out.both_st[k0 + k1] = sky ? 0 : 2;
+      if (sky) a.out.pos0[k0] = k0 + k1;
+    }
+  }
+}
+
+template <int NA>
+static int launch_small_na(cudaStream_t s, unsigned grid, const SmallArgs& a) {
+  k_small_skyline<NA><<<grid, kSmallThreads, 0, s>>>(a);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
+int launch_small_skyline(cudaStream_t s, const float* x, uint64_t n_pad, int d,
+                         const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max, uint32_t S,
+                         uint32_t* masks, uint32_t* ticket, const SplitOut& out) {
+  if (m_max > kSmallList)
+    return set_error(SKC_ERR_INVALID, "list of %llu points for the short-list skyline",
+                     (unsigned long long)m_max);
+  unsigned long long attrs = 0;
+  int na = 0;
+  for (int k = 0; k < d; ++k)
+    if (S & (1u << k)) attrs |= (unsigned long long)k << (4 * na++);
+  const unsigned grid = (unsigned)(m_max ? (m_max + 31) / 32 : 1);
+  const SmallArgs a{x, n_pad, attrs, ids, m_ptr, masks, ticket, out};
+  switch (na) {
+#define SKC_SMALL_CASE(N) \
+  case N: return launch_small_na<N>(s, grid, a);
+    SKC_SMALL_CASE(1) SKC_SMALL_CASE(2) SKC_SMALL_CASE(3) SKC_SMALL_CASE(4)
+    SKC_SMALL_CASE(5) SKC_SMALL_CASE(6) SKC_SMALL_CASE(7) SKC_SMALL_CASE(8)
+    SKC_SMALL_CASE(9) SKC_SMALL_CASE(10) SKC_SMALL_CASE(11) SKC_SMALL_CASE(12)
+    SKC_SMALL_CASE(13) SKC_SMALL_CASE(14) SKC_SMALL_CASE(15) SKC_SMALL_CASE(16)
+#undef SKC_SMALL_CASE
+    default:
+      return set_error(SKC_ERR_INVALID, "subspace with %d attributes", na);
+  }
+}
+
+// Offsets of a result that holds one cuboid, S, for both of its lists:
+// off[c] = 0 up to S and the list's count above.
+__global__ void k_single_offsets(const uint32_t* __restrict__ n, uint32_t S, uint32_t nsub,
+                                 uint64_t* __restrict__ sky_off, uint64_t* __restrict__ ext_off) {
+  const uint64_t n0 = n[0], n1 = n[1];
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nsub;
+       c += gridDim.x * blockDim.x) {
+    sky_off[c] = c > S ? n0 : 0;
+    ext_off[c] = c > S ? n1 : 0;
+  }
+}
+
+int launch_single_offsets(cudaStream_t s, const uint32_t* n, uint32_t S, uint32_t nsub,
+                          uint64_t* sky_off, uint64_t* ext_off) {
+  k_single_offsets<<<(nsub + 256) / 256, 256, 0, s>>>(n, S, nsub, sky_off, ext_off);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
+}  // namespace skc

@@ -1,0 +1,52 @@
+"""Short lists (small.cu, k_small_skyline): one launch that compares all pairs
+and compacts in the last CTA, against brute-force statuses, as a subspace
+query, a skycube and the per-cuboid form, around its edges (groups of 32
+points, tiles of 512 and 1,024 q's, the longest list it takes and one more)."""
+import numpy as np
+import pytest
+
+import skycube_gb300 as sk
+from skycube_gb300 import datagen
+from test_gpu_skyline_tree import brute
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 511, 513, 1023, 1025, 2047])
+@pytest.mark.parametrize("kind,d", [("uniform", 2), ("ties", 5), ("anticorrelated", 9),
+                                    ("correlated_q", 16)])
+def test_queries(gpu_ctx, n, kind, d):
+    x = datagen.generate(kind, n, d, 31 * n + d)
+    if n > 4:
+        x[n // 2] = x[0]      # an equal point
+        x[n // 3, 0] = -0.0   # a signed zero
+    ds = sk.Dataset(gpu_ctx, x)
+    full = (1 << d) - 1
+    for S in (full, full & 0b1010101010101010, 1):
+        if not S:
+            continue
+        sky, ext = brute(x[:, [k for k in range(d) if S >> k & 1]])
+        r = sk.skycube(gpu_ctx, ds, subspace=S)
+        assert np.array_equal(r.cuboid(S), sky) and np.array_equal(r.extended(S), ext), (n, S)
+        info = r.info()
+        fsky, fext = brute(x)
+        assert info["n_candidates"] == len(fsky) + len(fext)
+        assert info["total_skyline_ids"] == len(sky)
+        r.close()
+    ds.close()
+
+
+@pytest.mark.parametrize("kind,d", [("ties", 6), ("anticorrelated", 6)])
+@pytest.mark.parametrize("n", [6143, 6144, 6145])
+def test_longest_list_and_the_pipeline_agree(gpu_ctx, kind, d, n):
+    x = datagen.generate(kind, n, d, 5)
+    ds = sk.Dataset(gpu_ctx, x)
+    a = sk.skycube(gpu_ctx, ds, want_extended=True)
+    b = sk.skycube(gpu_ctx, ds, want_extended=True, pq_size=16)  # the pipeline
+    c = sk.skycube(gpu_ctx, ds, "sdsc", "plain", want_extended=True)
+    for S in range(1, 1 << d):
+        for o in (b, c):
+            assert np.array_equal(a.cuboid(S), o.cuboid(S)), S
+            assert np.array_equal(a.extended(S), o.extended(S)), S
+    for o in (a, b, c, ds):
+        o.close()
