@@ -103,6 +103,10 @@ struct Exec {
   const PlanCaps* plan = nullptr;  // plan mode (no host synchronisation)
 };
 
+// Events are kept by the context between runs (creating and destroying eight
+// of them is a tenth of a small query's host time).
+constexpr size_t kMaxPooledEvents = 64;
+
 // Records phase marks on the Exec's stream; fills Exec::phases when it goes
 // out of scope and prints them to stderr when SKC_TRACE=1.
 struct Tracer {
@@ -116,8 +120,15 @@ struct Tracer {
   }
   void mark(const char* name) {
     if (E.plan) return;  // plan mode: the graph is timed as a whole
-    cudaEvent_t ev;
-    if (cudaEventCreate(&ev) != cudaSuccess) return;
+    cudaEvent_t ev = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(E.ctx->mu);
+      if (!E.ctx->event_pool.empty()) {
+        ev = E.ctx->event_pool.back();
+        E.ctx->event_pool.pop_back();
+      }
+    }
+    if (!ev && cudaEventCreate(&ev) != cudaSuccess) return;
     cudaEventRecord(ev, E.stream);
     marks.push_back({name, ev});
   }
@@ -133,15 +144,25 @@ struct Tracer {
       }
       cudaEventElapsedTime(&E.ms, marks.front().second, marks.back().second);
     }
-    for (auto& m : marks) cudaEventDestroy(m.second);
+    std::lock_guard<std::mutex> lock(E.ctx->mu);
+    for (auto& m : marks) {
+      if (E.ctx->event_pool.size() < kMaxPooledEvents) E.ctx->event_pool.push_back(m.second);
+      else cudaEventDestroy(m.second);
+    }
   }
 };
 
 // Owns the temporary device buffers of one call; frees them stream-ordered.
+// Buffers of up to kArenaSmall bytes are cut from blocks of kArenaBlock (a
+// call takes some thirty of them, an allocation and a free each); a buffer
+// that a result will own is allocated by itself (`own`) and released from the
+// arena.
 // For a plan (skc_plan) it runs in one of two other modes: RECORD allocates
 // with cudaMalloc and keeps every buffer in *bufs (the plan owns them);
 // REPLAY hands the recorded buffers out again in the same order, so the
 // launch sequence captured into the graph allocates nothing.
+constexpr size_t kArenaSmall = 128 << 10, kArenaBlock = 1 << 20;
+
 struct Arena {
   enum Mode { STREAM, RECORD, REPLAY };
   cudaStream_t s;
@@ -149,6 +170,8 @@ struct Arena {
   Mode mode = STREAM;
   std::vector<std::pair<void*, size_t>>* bufs = nullptr;
   size_t next = 0;
+  char* block = nullptr;  // rest of the current block
+  size_t block_left = 0;
   explicit Arena(cudaStream_t st) : s(st) {}
   Arena(cudaStream_t st, Mode m, std::vector<std::pair<void*, size_t>>* b)
       : s(st), mode(m), bufs(b) {}
@@ -157,7 +180,11 @@ struct Arena {
       for (void* p : ptrs) cudaFreeAsync(p, s);
   }
   template <typename T>
-  int alloc(T** p, uint64_t count) {
+  int own(T** p, uint64_t count) {
+    return alloc(p, count, true);
+  }
+  template <typename T>
+  int alloc(T** p, uint64_t count, bool own = false) {
     const size_t bytes = (size_t)std::max<uint64_t>(count, 1) * sizeof(T);
     if (mode == REPLAY) {
       if (next >= bufs->size() || (*bufs)[next].second != bytes)
@@ -173,15 +200,30 @@ struct Arena {
       bufs->push_back({(void*)*p, bytes});
       return SKC_OK;
     }
-    cudaError_t e = cudaMallocAsync((void**)p, bytes, s);
+    const size_t padded = (bytes + 255) & ~size_t(255);
+    const bool cut = !own && padded <= kArenaSmall;
+    if (cut && padded <= block_left) {
+      *p = (T*)block;
+      block += padded;
+      block_left -= padded;
+      return SKC_OK;
+    }
+    const size_t want = cut ? kArenaBlock : bytes;
+    void* m = nullptr;
+    cudaError_t e = cudaMallocAsync(&m, want, s);
     if (e != cudaSuccess)
       return set_error(e == cudaErrorMemoryAllocation ? SKC_ERR_OOM : SKC_ERR_CUDA,
-                       "device allocation of %zu bytes failed: %s", bytes,
+                       "device allocation of %zu bytes failed: %s", want,
                        cudaGetErrorString(e));
-    ptrs.push_back((void*)*p);
+    ptrs.push_back(m);
+    *p = (T*)m;
+    if (cut) {
+      block = (char*)m + padded;
+      block_left = kArenaBlock - padded;
+    }
     return SKC_OK;
   }
-  // Hands a buffer over to the caller (it is no longer freed here).
+  // Hands a buffer of its own over to the caller (it is no longer freed here).
   void release(void* p) {
     auto it = std::find(ptrs.begin(), ptrs.end(), p);
     if (it != ptrs.end()) ptrs.erase(it);
@@ -354,9 +396,9 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
     F.small = true;
     SKC_TRY(A.alloc(&F.counts, 6));
     SKC_TRY(A.alloc(&F.masks, 2 * (kSmallList / 32)));
-    SKC_TRY(A.alloc(&F.sky, n));
-    SKC_TRY(A.alloc(&F.ext, n));
-    SKC_TRY(A.alloc(&F.cand, n));
+    SKC_TRY(A.own(&F.sky, n));
+    SKC_TRY(A.own(&F.ext, n));
+    SKC_TRY(A.own(&F.cand, n));
     SKC_TRY(A.alloc(&F.cand_st, n));
     SKC_TRY(A.alloc(&F.sky_pos, n));
     SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, d, nullptr, d_n, n, full, F.masks,
@@ -412,9 +454,9 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(A.alloc(&blk0, nblk));
   SKC_TRY(A.alloc(&blk1, nblk));
   SKC_TRY(A.alloc(&F.counts, 6));
-  SKC_TRY(A.alloc(&F.sky, n));
-  SKC_TRY(A.alloc(&F.ext, n));
-  SKC_TRY(A.alloc(&F.cand, n));
+  SKC_TRY(A.own(&F.sky, n));
+  SKC_TRY(A.own(&F.ext, n));
+  SKC_TRY(A.own(&F.cand, n));
   SKC_TRY(A.alloc(&F.cand_st, n));
   SKC_TRY(A.alloc(&F.sky_pos, n));
   SKC_TRY(launch_status_split(s, status, nullptr, d_n, n, blk0, blk1, F.sky, F.ext, F.counts,
@@ -492,7 +534,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
 
   T.mark("cand: cells+q order");
   uint32_t *dom, *ext = nullptr, *work = buckets + KB;
-  SKC_TRY(A.alloc(&dom, m * W));
+  SKC_TRY(A.own(&dom, m * W));
   if (want_ext) SKC_TRY(A.alloc(&ext, m * W));
 
   uint64_t slab_words = 0;
@@ -549,7 +591,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
     SKC_TRY(A.alloc(&ca.offs, C * tiles + 1));
     SKC_TRY(A.alloc(&ca.bsum, scan_bsum_entries(C * tiles)));
     uint64_t* csr;
-    SKC_TRY(A.alloc(&csr, nsub + 1));
+    SKC_TRY(A.own(&csr, nsub + 1));
     ca.csr_off = csr;
     SKC_TRY(launch_bits_count(s, ca));
     uint64_t total = 0;
@@ -562,7 +604,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
       SKC_TRY(copy_d2h(&total, csr + nsub, sizeof(uint64_t), s));
     }
     uint32_t* ids;
-    SKC_TRY(A.alloc(&ids, total));
+    SKC_TRY(A.own(&ids, total));
     ca.out = ids;
     ca.out_cap = total;
     SKC_TRY(launch_bits_write(s, ca));
@@ -664,8 +706,8 @@ static int assemble_csr(Exec& E, Arena& A, int d, int max_d, bool want_ext,
     uint64_t* d_off;
     uint32_t* ids;
     const uint32_t** d_srcs;
-    SKC_TRY(A.alloc(&d_off, nsub + 1));
-    SKC_TRY(A.alloc(&ids, off[nsub]));
+    SKC_TRY(A.own(&d_off, nsub + 1));
+    SKC_TRY(A.own(&ids, off[nsub]));
     SKC_TRY(A.alloc(&d_srcs, nsub));
     std::vector<const uint32_t*> srcs(nsub, nullptr);
     for (uint32_t c = 0; c < nsub; ++c)
@@ -1338,6 +1380,7 @@ int skc_context_destroy(skc_context* ctx) {
     if (p) cudaFree(p);
   cudaEventDestroy(ctx->ev_start);
   cudaEventDestroy(ctx->ev_stop);
+  for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return SKC_OK;
@@ -1474,8 +1517,8 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
   if (S != full && small_list(m)) {
     cnt = F.counts + 3;
     if (!F.masks) SKC_TRY(A.alloc(&F.masks, 2 * (kSmallList / 32)));
-    SKC_TRY(A.alloc(&sky, m));
-    SKC_TRY(A.alloc(&ext, m));
+    SKC_TRY(A.own(&sky, m));
+    SKC_TRY(A.own(&ext, m));
     SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, d, F.cand, F.counts + 2, m, S, F.masks,
                                  F.tickets + 1, {sky, ext, nullptr, nullptr, nullptr, cnt}));
   } else if (S != full) {
@@ -1490,8 +1533,8 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
     const uint64_t nblk = (m + 1023) / 1024 + 2;
     SKC_TRY(A.alloc(&blk0, nblk));
     SKC_TRY(A.alloc(&blk1, nblk));
-    SKC_TRY(A.alloc(&sky, m));
-    SKC_TRY(A.alloc(&ext, m));
+    SKC_TRY(A.own(&sky, m));
+    SKC_TRY(A.own(&ext, m));
     const uint32_t* open = nullptr;
     const uint32_t* m_ptr = F.counts + 2;
     const uint32_t* m_open = m_ptr;
@@ -1515,8 +1558,8 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
     SKC_TRY(launch_status_split(s, status, F.cand, m_ptr, m, blk0, blk1, sky, ext, cnt));
   }
   uint64_t* off[2];
-  SKC_TRY(A.alloc(&off[0], nsub + 1));
-  SKC_TRY(A.alloc(&off[1], nsub + 1));
+  SKC_TRY(A.own(&off[0], nsub + 1));
+  SKC_TRY(A.own(&off[1], nsub + 1));
   SKC_TRY(launch_single_offsets(s, cnt, S, nsub, off[0], off[1]));
   if (S != full || F.deferred) SKC_TRY(copy_d2h(h, F.counts, sizeof(h), s));
   if (S != full) T.mark("subspace skyline");

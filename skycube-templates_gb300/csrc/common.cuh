@@ -115,6 +115,8 @@ struct skc_context {
   // buffer costs its zero fill and first-touch page faults (about 3 ms for
   // the 65 MB of a 1M x 10 skycube, eight times the copy itself).
   std::vector<std::vector<uint32_t>> host_id_pool;
+  // Timing events between runs (Tracer), at most kMaxPooledEvents.
+  std::vector<cudaEvent_t> event_pool;
   // Work parameters chosen by skc_autotune, by signature key (api.cu).
   struct Tuned {
     int depth, pq_size, tile_points, chunk, blocks_per_sm;
