@@ -102,9 +102,10 @@ typedef struct skc_options {
   int blocks_per_sm; /* bitmap kernel: persistent CTAs per SM, 1..32 (capped
                         by occupancy); 0 auto (the occupancy limit) */
   int form;          /* computation of a batched skycube (SKC_FORM_*): 0 auto
-                        (the level form from 65,536 candidates at caps under
-                        4, at 16 attributes, or at 14-15 attributes from
-                        600,000 candidates; else the bitmaps);
+                        (the level form from 8,192 to 65,536 candidates,
+                        by cap and attributes, at caps up to 3 and from 12
+                        attributes at cap 4, unless over an eighth of the
+                        candidates are extended skyline; else the bitmaps);
                         SKC_FORM_BITMAPS; SKC_FORM_LEVELS where it applies
                         (max_d <= 4 and <= d - 2, no per-point bitmaps; it
                         hands over to the bitmaps when too many cuboids
@@ -194,8 +195,9 @@ int skc_result_free(skc_result* res);
  * as a slot is free and its estimated device-memory footprint fits what the
  * requests in flight leave of `budget` (bytes; 0: 80% of the free device
  * memory). A capped skycube request that the level form takes (batched
- * form, max_d <= 4 and <= d - 2, no bitmaps; SKC_FORM_LEVELS, or the
- * automatic rule of skc_options.form with n for the candidate count) takes
+ * form, max_d <= 4 and <= d - 2, no bitmaps; SKC_FORM_LEVELS, or at least
+ * 65,536 points and a cap under 4, 16 attributes, or 14-15 attributes and
+ * 600,000 points) takes
  * such requests right behind it in the queue (up to 8, within the budget)
  * into the same pass (skc_skycube_batch), where those the level form takes
  * share one persistent lattice launch. Requests whose estimate exceeds the

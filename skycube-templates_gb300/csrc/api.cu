@@ -846,8 +846,12 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
     SKC_TRY(A.alloc(&cc, std::max<uint64_t>(1, m)));
     SKC_TRY(A.alloc(&J.lv_cells, ds->n));
     SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, J.F->cand, J.F->counts + 2, m, J.depth,
-                                pivots, cc));
+                                pivots, cc, nullptr, nullptr, nullptr, 0, 1));
     SKC_TRY(launch_scatter_u4(s, cc, J.F->cand, J.F->counts + 2, m, J.lv_cells));
+    const uint64_t cpitch = round_up(std::max<uint64_t>(1, m), 128);
+    uint8_t* cbytes;
+    SKC_TRY(A.alloc(&cbytes, (uint64_t)d * cpitch));
+    SKC_TRY(launch_cells_bytes(s, cc, J.F->counts + 2, m, d, cpitch, cbytes));
     J.cub0 = (uint32_t)c_mask.size();
     const uint32_t full = (1u << d) - 1;
     index[j].assign(1u << d, 0xffffffffu);
@@ -862,7 +866,8 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
     J.masks.assign(c_mask.begin() + J.cub0, c_mask.end());
     SKC_TRY(A.alloc(&J.d_index, 1u << d));
     SKC_TRY(copy_h2d(J.d_index, index[j].data(), sizeof(uint32_t) << d, s));
-    hjobs[j] = LtJob{ds->x, ds->n_pad, J.lv_cells, J.F->cand, (uint32_t)m, J.d_index, d, J.max_d};
+    hjobs[j] = LtJob{ds->x, ds->n_pad, J.lv_cells, J.F->cand, (uint32_t)m, cbytes, cpitch,
+                     J.d_index, d, J.max_d};
     max_cand = std::max<uint64_t>(max_cand, m);
     top = std::max(top, J.max_d);
   }
@@ -936,10 +941,11 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
   SKC_TRY(A.alloc(&d_scr, ncub));
   SKC_TRY(A.alloc(&d_list, ncub));
   SKC_TRY(A.alloc(&d_list_n, ncub));
-  SKC_TRY(A.alloc(&d_nsky, ncub));
-  SKC_TRY(A.alloc(&d_next, ncub));
-  SKC_TRY(A.alloc(&d_flag, ncub));
+  SKC_TRY(A.alloc(&d_nsky, 3ull * ncub));  // skyline and extended counts, flags: one read-back
+  d_next = d_nsky + ncub;
+  d_flag = d_next + ncub;
   SKC_TRY(A.alloc(&d_slot, (uint64_t)ncub * kLvSlot));
+  SKC_TRY(A.alloc(&a.tab, (uint64_t)g_used * 128 * kLvMaxDims));
   SKC_TRY(A.alloc(&a.pr_c, (uint64_t)g_used * kLvPruners));
   SKC_TRY(A.alloc(&a.pr_v, (uint64_t)g_used * kLvMaxDims * kLvPruners));
   SKC_TRY(A.alloc(&a.pr_n, g_used));
@@ -992,11 +998,10 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
   a.max_fallbacks = kLvMaxFallbacks;
   SKC_TRY(launch_lattice(s, ctx->num_sms, a));
 
-  std::vector<uint32_t> h_nsky(ncub), h_next(ncub), h_flag(ncub), h_tail(2 + nj);
-  SKC_TRY(copy_d2h(h_nsky.data(), d_nsky, ncub * 4, s));
-  SKC_TRY(copy_d2h(h_next.data(), d_next, ncub * 4, s));
-  SKC_TRY(copy_d2h(h_flag.data(), d_flag, ncub * 4, s));
+  std::vector<uint32_t> h_out(3ull * ncub), h_tail(2 + nj);
+  SKC_CUDA(cudaMemcpyAsync(h_out.data(), d_nsky, 3ull * ncub * 4, cudaMemcpyDeviceToHost, s));
   SKC_TRY(copy_d2h(h_tail.data(), d_counters + n_ph, (2 + nj) * 4, s));
+  const uint32_t *h_nsky = h_out.data(), *h_next = h_nsky + ncub, *h_flag = h_next + ncub;
   if (h_tail[1]) return set_error(SKC_ERR_TIMEOUT, "lattice kernel: a phase wait ran out");
   T.mark("lattice kernel");
 
@@ -1011,6 +1016,39 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
     const int d = ds->d;
     const uint32_t nsub = 1u << d, full = nsub - 1;
     FullSpace& F = *J.F;
+    const uint32_t jcub = (uint32_t)J.masks.size();
+    bool within = true;
+    uint64_t total[2] = {F.h_counts[0], F.h_counts[1]};
+    for (uint32_t t = J.cub0; t < J.cub0 + jcub; ++t) {
+      within = within && h_flag[t] == 0;
+      total[0] += h_nsky[t];
+      total[1] += h_next[t];
+    }
+    if (within) {  // every list lies in its slot: the device assembles the result
+      J.R->level_fallbacks = 0;
+      uint32_t* counts;
+      uint64_t *tmp, *bsum;
+      SKC_TRY(A.alloc(&counts, nsub));
+      SKC_TRY(A.alloc(&tmp, nsub + 1));
+      SKC_TRY(A.alloc(&bsum, scan_bsum_entries(nsub)));
+      for (int pass = 0; pass < (J.want_ext ? 2 : 1); ++pass) {
+        const uint32_t* n_of = pass ? d_next : d_nsky;
+        uint64_t* off;
+        uint32_t* ids;
+        SKC_TRY(A.own(&off, nsub + 1));
+        SKC_TRY(A.own(&ids, total[pass]));
+        SKC_TRY(launch_lv_counts(s, J.d_index, nsub, F.h_counts[pass], n_of, counts));
+        SKC_TRY(launch_scan_counts(s, counts, nsub, bsum, tmp, 1, nsub, off));
+        SKC_TRY(launch_lv_lists(s, d_mask, J.cub0, jcub, d_slot, pass ? d_nsky : nullptr, n_of, off,
+                                pass ? F.ext : F.sky, full, F.h_counts[pass], ids));
+        A.release(off);
+        A.release(ids);
+        (pass ? J.R->d_eoff : J.R->d_off) = off;
+        (pass ? J.R->d_eids : J.R->d_ids) = ids;
+        (pass ? J.R->total_ext : J.R->total_ids) = total[pass];
+      }
+      continue;
+    }
     std::vector<uint32_t*> sky(nsub, nullptr), ext(nsub, nullptr);
     std::vector<uint64_t> nsky(nsub, 0), next(nsub, 0);
     sky[full] = F.sky;
@@ -1063,31 +1101,31 @@ static int run_levels(Exec& E, skc_dataset* ds, const skc_options& o, int max_d,
 // The level form can replace the bitmaps for batched capped skycubes of
 // small caps, when no per-point bitmaps are wanted and no plan is being
 // recorded (the level form syncs per level). Auto takes it where it was
-// faster on one GB300 (device ms, level / bitmap form, cap 4 unless noted):
-//   16 attributes: anticorrelated 500k 48.3 / 83.5, 396k 36.7 / 64.1;
-//     uniform 937k 69.4 / 84.8, 200k 16.0 / 17.2
-//   14-15 attributes: anticorrelated 799k x 14 (737k candidates) 51.9 /
-//     58.8; but anticorrelated 150k x 14 9.7 / 9.1 and uniform 951k x 15
-//     (503k candidates) 49.2 / 39.9
-//   12 attributes and fewer, cap 4: anticorrelated 500k x 12 17.7 / 17.7,
-//     1M x 10 15.3 / 11.5
-//   caps under 4: anticorrelated 1M x 8 cap 3 4.55 / 4.69, uniform
-//     400k x 11 cap 2 2.3 / 2.8
-// Below 65,536 candidates the bitmap kernel is as fast or faster, and
-// tie-heavy data (whose small cuboids have skylines over the level kernels'
-// capacities) has few candidates.
-constexpr uint64_t kLvMinCandidates = 65536;
-constexpr uint64_t kLvMinCandidatesMidD = 600000;  // 14 and 15 attributes
-static bool levels_by_default(int d, int max_d, uint64_t candidates) {
-  if (candidates < kLvMinCandidates) return false;
-  return max_d <= 3 || d >= 16 || (d >= 14 && candidates >= kLvMinCandidatesMidD);
+// faster on one GB300; device ms of the whole call, level / bitmap form,
+// anticorrelated:
+//   cap 4: 16 attributes 198k candidates 5.3 / 19.4, 20k 2.25 / 2.32; 14:
+//     59k 2.0 / 2.9, 20k 1.41 / 1.26; 12: 57k 1.30 / 1.81, 20k 0.94 / 0.84
+//   cap 3: 16: 20k 1.1 / 2.0; 12: 20k 0.56 / 0.70, 8k 0.49 / 0.44; 10: 50k
+//     0.63 / 0.74, 18k 0.48 / 0.44; 8: 85k 0.77 / 0.88, 36k 0.54 / 0.53
+//   caps 1, 2: 16: 8k 0.75 / 1.21; 12: 8k 0.39 / 0.43; 10: 50k 0.54 / 0.65,
+//     18k 0.41 / 0.40; 8: 36k 0.44 / 0.49
+// Cap 4 under 12 attributes keeps the bitmaps. Tied data does too (its
+// candidates are mostly extended skyline, and its small cuboids' lists over
+// the level kernel's capacities): 400k x 16 ties, cap 4, 8.8 / 4.6, correlated
+// 6.2 / 0.7.
+static bool levels_by_default(int d, int max_d, const FullSpace& F) {
+  const uint64_t cand = F.h_counts[2], ext = F.h_counts[1];
+  if (8 * ext > cand) return false;
+  if (max_d <= 2) return cand >= (d >= 12 ? 8192u : d >= 8 ? 24576u : 65536u);
+  if (max_d == 3) return cand >= (d >= 12 ? 16384u : d >= 9 ? 32768u : 65536u);
+  return d >= 12 && cand >= 32768u;
 }
 static bool use_levels(const Exec& E, const skc_dataset* ds, const skc_options& o, int max_d,
                        const FullSpace& F) {
   if (o.form == SKC_FORM_BITMAPS) return false;
   const bool can = !E.plan && o.mode == SKC_MODE_BATCHED && !o.want_bitmaps &&
                    max_d <= kLvMaxDims && max_d <= ds->d - 2 && ds->n < (1ull << 31);
-  return can && (o.form == SKC_FORM_LEVELS || levels_by_default(ds->d, max_d, F.h_counts[2]));
+  return can && (o.form == SKC_FORM_LEVELS || levels_by_default(ds->d, max_d, F));
 }
 
 static int auto_depth(uint64_t n, int d) {
@@ -2374,17 +2412,23 @@ struct skc_server {
 };
 
 // Requests that may share one lattice launch: batched capped skycubes the
-// lattice form takes (max_d <= kLvMaxDims and <= d - 2, no bitmaps; forced,
-// or by the automatic rule with n for the candidate count, its upper
-// bound). A request bound for the bitmap form keeps a slot of its own, as
-// it would run alone inside a batch's pass anyway.
+// lattice form takes (max_d <= kLvMaxDims and <= d - 2, no bitmaps), forced or
+// long enough that they likely take it: their candidates are not known yet,
+// and a request that ends in the bitmap form runs alone inside the batch's
+// pass, where a slot of its own would overlap it.
+constexpr uint64_t kBatchMinPoints = 65536;
+constexpr uint64_t kBatchMinPointsMidD = 600000;  // 14 and 15 attributes, cap 4
+static bool batch_by_default(int d, int max_d, uint64_t n) {
+  if (n < kBatchMinPoints) return false;
+  return max_d <= 3 || d >= 16 || (d >= 14 && n >= kBatchMinPointsMidD);
+}
 static bool batchable(const Request& q) {
   const skc_options& o = q.opt;
   const int md = (o.max_d <= 0 || o.max_d > q.d) ? q.d : o.max_d;
   if (o.subspace || o.mode != SKC_MODE_BATCHED || o.want_bitmaps ||
       o.form == SKC_FORM_BITMAPS || md > kLvMaxDims || md > q.d - 2)
     return false;
-  return o.form == SKC_FORM_LEVELS || levels_by_default(q.d, md, q.n);
+  return o.form == SKC_FORM_LEVELS || batch_by_default(q.d, md, q.n);
 }
 constexpr size_t kMaxServerBatch = 8;
 

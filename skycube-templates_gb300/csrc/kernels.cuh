@@ -32,7 +32,7 @@ int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
                         uint64_t m_max, int depth, float* pivots, uint4* cells,
                         uint32_t* amin = nullptr, uint32_t* hist = nullptr,
-                        float* xout = nullptr, uint64_t out_pad = 0);
+                        float* xout = nullptr, uint64_t out_pad = 0, int low = 0);
 // Entries of status 0 / 1 into sky / ext (ids in list order), n[0] / n[1]
 // their counts, n[2] the sum; with `both`, also their union in list order,
 // its entries' flags (0 for status 0, else 2) and the union positions of the
@@ -267,6 +267,8 @@ struct LtJob {
   const uint4* cells;        // point id -> cells on the candidates' quantile grid
   const uint32_t* cand;      // full-space skyline + extended skyline ids
   uint32_t n_cand;
+  const uint8_t* cand_cells; // the candidates' cells: [d][cell_pitch] bytes in candidate order
+  uint64_t cell_pitch;       // a multiple of 16
   const uint32_t* cub_index; // [2^d] mask -> cuboid table index (0xffffffff: none)
   int d, max_d;
 };
@@ -283,6 +285,7 @@ struct LtArgs {
   uint32_t* c_next;          // [ncub]
   uint32_t* c_flag;          // [ncub] 1: over a capacity; 2: skipped (job handed over)
   uint32_t* slot;            // [ncub * kLvSlot]: skyline ids, then extended
+  unsigned long long* tab;   // [G * 128 * kLvMaxDims] first-level pruner tables
   uint32_t* pr_c;            // [G * kLvPruners] per scratch index
   float* pr_v;               // [G * kLvMaxDims * kLvPruners]
   uint32_t* pr_n;            // [G]
@@ -303,9 +306,17 @@ struct LtArgs {
   uint32_t max_fallbacks;    // more than this on a job's first level: job handed over
   uint32_t* status;          // 0, or 1 when a wait ran out (zeroed)
 };
+int launch_lv_counts(cudaStream_t s, const uint32_t* index, uint32_t nsub, uint32_t full_n,
+                     const uint32_t* n_of, uint32_t* counts);
+int launch_lv_lists(cudaStream_t s, const uint32_t* mask, uint32_t cub0, uint32_t ncub,
+                    const uint32_t* slot, const uint32_t* skip, const uint32_t* n_of,
+                    const uint64_t* off, const uint32_t* full, uint32_t full_c, uint32_t full_n,
+                    uint32_t* out);
 // One cooperative launch of the lattice kernel on `num_sms` SMs.
 int launch_lattice(cudaStream_t s, int num_sms, const LtArgs& a);
 int lattice_grid(int num_sms, int* grid);
+int launch_cells_bytes(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr, uint64_t m_max,
+                       int d, uint64_t pitch, uint8_t* out);
 int launch_scatter_u4(cudaStream_t s, const uint4* in, const uint32_t* idx, const uint32_t* m_ptr,
                       uint64_t m_max, uint4* out);
 

@@ -28,6 +28,8 @@
 // passes them by point id). A cuboid whose survivors, skyline or extended
 // skyline exceed the capacities is flagged; the host then computes it with
 // the single-cuboid pipeline.
+#include <initializer_list>
+
 #include "kernels.cuh"
 
 namespace skc {
@@ -203,6 +205,221 @@ __device__ void lv_pruners_cta(const CubAttrs& A, const uint32_t* L, uint32_t n,
   if (tid == 0) pr_n_g[g] = min(s_np, kLvPruners);
 }
 
+// ---------------------------------------------------------------------------
+// A job's first level runs over its whole candidate list, the bulk of the
+// work: every (candidate, cuboid) pair meets the cuboid's pruners. There the
+// pruner test is a table lookup: T[a][v] holds, one bit per pruner, the
+// pruners whose cell on the cuboid's a-th attribute is below v, so the AND of
+// T[a][p's cell a] over the attributes is nonzero exactly when a pruner is
+// strictly below p in every cell. 64 pruners cost four 8-byte loads from
+// shared memory and the cells come as bytes, attribute-major in candidate
+// order, eight candidates per load; equal cells count as not below (such a
+// candidate survives to the sort-filter skyline, which compares floats). The
+// grid is finer towards the minimum (k_pivots, low): a candidate in the
+// lowest cell of an attribute can never be dropped, and on an even grid
+// those were 15,300 of the 17,500 survivors.
+// Before, each pair was packed from its 16-byte cells and walked 4 to 32
+// pruners, the best of a sample of 1,024: 500k x 16 -m 4, 1,820 first-level
+// cuboids over 491k candidates, filter 19.5 ms of SM time, 48,600 survivors
+// per cuboid and 18.2 ms for their sort-filter; now 3.1 ms, 5,100 and 3.1.
+// The filter is bound by the table loads' bank conflicts; a second table from
+// what the first leaves of the sample cost in pruner selection what it saved
+// in the sort-filter (3,700 survivors).
+constexpr uint32_t kLvFullPruners = 64;  // per table
+constexpr uint32_t kLvFullSample = 16384;  // sampled packs of four candidates
+constexpr uint32_t kLvFullStep = 8 * kLvThreads;   // candidates per filter step
+constexpr uint32_t kLvFullStage = 2 * kLvFullStep;  // survivors staged at most
+
+// Four candidates' cells on attribute k, from candidate 4 * pk.
+__device__ __forceinline__ uint32_t lv_pack4(const LtJob& J, int k, uint32_t pk) {
+  return __ldg(reinterpret_cast<const uint32_t*>(J.cand_cells + (uint64_t)k * J.cell_pitch) + pk);
+}
+
+// Cell byte e (0 .. 3) of each attribute's pack: the candidate's packed cells.
+__device__ __forceinline__ uint32_t lv_pick(const uint32_t* w, int e) {
+  uint32_t pc = 0;
+#pragma unroll
+  for (int a = 0; a < kLvMaxDims; ++a) pc |= ((w[a] >> (8 * e)) & 0x7fu) << (8 * a);
+  return pc;
+}
+
+// Pruners strictly below packed cells pc in every attribute (bit mask).
+__device__ __forceinline__ unsigned long long lv_below(const unsigned long long* T, uint32_t pc) {
+  unsigned long long t = T[pc & 0x7fu];
+#pragma unroll
+  for (int a = 1; a < kLvMaxDims; ++a) t &= T[128 * a + ((pc >> (8 * a)) & 0x7fu)];
+  return t;
+}
+
+// First bin whose inclusive count reaches kLvFullPruners, or the last count:
+// thr, the count below it, and the pruners to take. One warp.
+__device__ __forceinline__ void lv_threshold(const uint32_t* hist, int lane, uint32_t* thr,
+                                             uint32_t* below, uint32_t* take) {
+  constexpr uint32_t per = (kLvKeyBins + 31) / 32;
+  uint32_t c = 0;
+  for (uint32_t j = 0; j < per; ++j) {
+    const uint32_t b = lane * per + j;
+    if (b < kLvKeyBins) c += hist[b];
+  }
+  uint32_t inc = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(kWarpAll, inc, o);
+    if (lane >= o) inc += u;
+  }
+  const uint32_t want = min(kLvFullPruners, __shfl_sync(kWarpAll, inc, 31));
+  if (lane == 0) {
+    *take = want;
+    *thr = 0;
+    *below = 0;
+  }
+  __syncwarp();
+  uint32_t e = inc - c;
+  for (uint32_t j = 0; j < per; ++j) {
+    const uint32_t b = lane * per + j;
+    const uint32_t h = b < kLvKeyBins ? hist[b] : 0u;
+    if (e < want && e + h >= want) {
+      *thr = b;
+      *below = e;
+    }
+    e += h;
+  }
+}
+
+// Pruner table of a cuboid over the job's candidates, into tab[g * 512 ..):
+// the lowest cell sums of a sample.
+__device__ void lv_full_pruners_cta(const CubAttrs& A, const LtJob& J, uint32_t g,
+                                    unsigned long long* tab, uint32_t* hist) {
+  __shared__ uint32_t s_thr, s_below, s_take, s_c0, s_c1;
+  __shared__ uint32_t s_pr[kLvFullPruners];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t n = J.n_cand, packs = (n + 3) / 4;
+  const uint32_t ns = min(packs, kLvFullSample);
+  // Runs f(packed cells) for the sample's candidates.
+  auto sample = [&](auto f) {
+    for (uint32_t t = tid; t < ns; t += blockDim.x) {
+      const uint32_t pk = (uint32_t)((uint64_t)t * packs / ns);
+      uint32_t w[kLvMaxDims];
+#pragma unroll
+      for (int a = 0; a < kLvMaxDims; ++a) w[a] = a < A.na ? lv_pack4(J, A.att[a], pk) : 0u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (4 * pk + e < n) f(lv_pick(w, e));
+    }
+  };
+  for (uint32_t i = tid; i < kLvKeyBins; i += blockDim.x) hist[i] = 0;
+  if (tid == 0) s_c0 = s_c1 = 0;
+  __syncthreads();
+  sample([&](uint32_t pc) { atomicAdd(&hist[lv_key(pc)], 1u); });
+  __syncthreads();
+  if (tid < 32) lv_threshold(hist, lane, &s_thr, &s_below, &s_take);
+  __syncthreads();
+  const uint32_t thr = s_thr, below = s_below, take = s_take;
+  sample([&](uint32_t pc) {
+    const uint32_t key = lv_key(pc);
+    if (key > thr) return;
+    const uint32_t k = key < thr ? atomicAdd(&s_c0, 1u) : below + atomicAdd(&s_c1, 1u);
+    if (k < take) s_pr[k] = pc;
+  });
+  __syncthreads();
+  if (tid < 128 * kLvMaxDims) {
+    const int a = tid >> 7;
+    const uint32_t v = tid & 127;
+    unsigned long long t = 0;
+    for (uint32_t j = 0; j < take; ++j)
+      if (a >= A.na || ((s_pr[j] >> (8 * a)) & 0x7fu) < v) t |= 1ull << j;
+    tab[(uint64_t)g * (128 * kLvMaxDims) + tid] = t;
+  }
+}
+
+// Shared memory of the first-level filter, in bytes: table, staged survivors.
+static constexpr size_t kLvFullSmem = 128 * kLvMaxDims * 8 + (size_t)kLvFullStage * (4 + 2);
+
+// The candidates [beg, end) of the job against cuboid g's pruner table;
+// survivors are appended to g's scratch. beg is a multiple of 8.
+__device__ void lv_filter_full(const CubAttrs& A, const LtJob& J, uint32_t beg, uint32_t end,
+                               uint32_t g, const unsigned long long* tab, uint32_t cap,
+                               uint32_t* cnt, uint32_t* surv_id, uint16_t* surv_key,
+                               unsigned char* sm) {
+  __shared__ uint32_t s_n, s_base;
+  constexpr uint32_t kTab = 128 * kLvMaxDims;
+  unsigned long long* T = reinterpret_cast<unsigned long long*>(sm);  // [kLvMaxDims][128]
+  uint32_t* st_id = reinterpret_cast<uint32_t*>(T + kTab);
+  uint16_t* st_key = reinterpret_cast<uint16_t*>(st_id + kLvFullStage);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  if (tid < (int)kTab) T[tid] = __ldcg(tab + (uint64_t)g * kTab + tid);
+  if (tid == 0) s_n = 0;
+  __syncthreads();
+  for (uint32_t base = beg; base < end; base += kLvFullStep) {
+    const uint32_t i = base + 8 * tid;
+    uint2 w[kLvMaxDims];
+#pragma unroll
+    for (int a = 0; a < kLvMaxDims; ++a) {
+      w[a] = make_uint2(0, 0);
+      if (a < A.na && i < end)
+        w[a] = __ldg(reinterpret_cast<const uint2*>(
+            J.cand_cells + (uint64_t)A.att[a] * J.cell_pitch + i));
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      uint32_t pc = 0;
+#pragma unroll
+      for (int a = 0; a < kLvMaxDims; ++a)
+        pc |= (((e < 4 ? w[a].x : w[a].y) >> (8 * (e & 3))) & 0x7fu) << (8 * a);
+      const bool keep = i + e < end && lv_below(T, pc) == 0;
+      const uint32_t live = __ballot_sync(kWarpAll, keep);
+      if (!live) continue;
+      uint32_t pos = 0;
+      if (lane == 0) pos = atomicAdd(&s_n, (uint32_t)__popc(live));
+      pos = __shfl_sync(kWarpAll, pos, 0) + __popc(live & lt_mask);
+      if (keep) {  // at most kLvFullStep staged before this step, so pos < kLvFullStage
+        st_id[pos] = J.cand[i + e];
+        st_key[pos] = (uint16_t)lv_key(pc);
+      }
+    }
+    __syncthreads();
+    const uint32_t n = s_n;
+    if (n <= kLvFullStage - kLvFullStep && base + kLvFullStep < end) {
+      __syncthreads();  // every thread has read s_n
+      continue;
+    }
+    if (tid == 0) s_base = n ? atomicAdd(&cnt[g], n) : 0u;
+    __syncthreads();
+    const uint32_t b0 = s_base;
+    for (uint32_t k = tid; k < n; k += blockDim.x) {
+      const uint32_t pos = b0 + k;
+      if (pos < cap) {
+        surv_id[(uint64_t)g * cap + pos] = st_id[k];
+        surv_key[(uint64_t)g * cap + pos] = st_key[k];
+      }
+    }
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+  }
+}
+
+// out[k * pitch + i] = cell of attribute k of list entry i.
+__global__ void k_cells_bytes(const uint4* __restrict__ cells, const uint32_t* __restrict__ m_ptr,
+                              int d, uint64_t pitch, uint8_t* __restrict__ out) {
+  const uint32_t m = *m_ptr;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    const uint4 c = cells[i];
+    for (int k = 0; k < d; ++k)
+      out[(uint64_t)k * pitch + i] = (uint8_t)((word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu);
+  }
+}
+
+int launch_cells_bytes(cudaStream_t s, const uint4* cells, const uint32_t* m_ptr, uint64_t m_max,
+                       int d, uint64_t pitch, uint8_t* out) {
+  uint64_t b = (m_max + 255) / 256;
+  if (b < 1) b = 1;
+  if (b > 152 * 8) b = 152 * 8;
+  k_cells_bytes<<<(unsigned)b, 256, 0, s>>>(cells, m_ptr, d, pitch, out);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
 // Shared memory of one filter chunk, in bytes.
 static constexpr size_t kLvFilterSmem = (size_t)kLvChunk * (4 + 4 + 4 + 2);
 
@@ -370,7 +587,9 @@ __device__ uint32_t lv_sfs_cta(const CubAttrs& A, uint32_t c, uint32_t g,
   constexpr uint32_t kWarps = kLvThreads / 32;
   for (uint32_t base = 0, bend = 0; base < n; base = bend) {
     if (tid == 0) {
-      const uint32_t target = base + kLvThreads;
+      // Short first batches: a batch's entries meet each other in pairs, and
+      // a window of the strongest entries settles most of the next batch.
+      const uint32_t target = base + (base < 256 ? 256 : base < 1024 ? 512 : kLvThreads);
       uint32_t e = n;
       if (target < n) {
         uint32_t lo = 0, hi = kLvKeyBins;  // largest k with kb[k] <= target
@@ -606,6 +825,53 @@ int launch_scatter_u4(cudaStream_t s, const uint4* in, const uint32_t* idx, cons
   return SKC_OK;
 }
 
+// Result lists of a job whose cuboids all stayed within the capacities.
+// counts[c] = the length of cuboid c's list (0 for cuboids not output).
+__global__ void k_lv_counts(const uint32_t* __restrict__ index, uint32_t nsub, uint32_t full_n,
+                            const uint32_t* __restrict__ n_of, uint32_t* __restrict__ counts) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nsub;
+       c += gridDim.x * blockDim.x) {
+    const uint32_t i = index[c];
+    counts[c] = c == nsub - 1 ? full_n : i == 0xffffffffu ? 0u : n_of[i];
+  }
+}
+
+// A warp per cuboid copies its list from its slot (table entries cub0 ..
+// cub0 + ncub), the last CTAs copy the full space's.
+__global__ void __launch_bounds__(256) k_lv_lists(
+    const uint32_t* __restrict__ mask, uint32_t cub0, uint32_t ncub, const uint32_t* __restrict__ slot,
+    const uint32_t* __restrict__ skip, const uint32_t* __restrict__ n_of,
+    const uint64_t* __restrict__ off, const uint32_t* __restrict__ full, uint32_t full_c,
+    uint32_t full_n, uint32_t* __restrict__ out) {
+  const uint32_t warps = gridDim.x * 8, w = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  for (uint32_t t = cub0 + w; t < cub0 + ncub; t += warps) {
+    const uint32_t* src = slot + (uint64_t)t * kLvSlot + (skip ? skip[t] : 0u);
+    uint32_t* dst = out + off[mask[t]];
+    const uint32_t n = n_of[t];
+    for (uint32_t i = lane; i < n; i += 32) dst[i] = src[i];
+  }
+  uint32_t* dst = out + off[full_c];
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < full_n; i += gridDim.x * 256) dst[i] = full[i];
+}
+
+int launch_lv_counts(cudaStream_t s, const uint32_t* index, uint32_t nsub, uint32_t full_n,
+                     const uint32_t* n_of, uint32_t* counts) {
+  k_lv_counts<<<(nsub + 255) / 256, 256, 0, s>>>(index, nsub, full_n, n_of, counts);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
+int launch_lv_lists(cudaStream_t s, const uint32_t* mask, uint32_t cub0, uint32_t ncub,
+                    const uint32_t* slot, const uint32_t* skip, const uint32_t* n_of,
+                    const uint64_t* off, const uint32_t* full, uint32_t full_c, uint32_t full_n,
+                    uint32_t* out) {
+  k_lv_lists<<<152 * 4, 256, 0, s>>>(mask, cub0, ncub, slot, skip, n_of, off, full, full_c, full_n,
+                                     out);
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
 // ---------------------------------------------------------------------------
 // The lattice work queue: one persistent launch computes every wanted cuboid
 // of every job (dataset). Items sit in lattice-level order: for each level,
@@ -723,13 +989,23 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_lattice(LtArgs a) {
           s_n = n;
         }
         __syncthreads();
-        lv_pruners_cta(A, s_list, s_n, J.cells, J.x, J.n_pad, g, a.pr_c, a.pr_v, a.pr_n,
-                       reinterpret_cast<uint32_t*>(lt_smem));
+        if (s_list == J.cand)
+          lv_full_pruners_cta(A, J, g, a.tab, reinterpret_cast<uint32_t*>(lt_smem));
+        else
+          lv_pruners_cta(A, s_list, s_n, J.cells, J.x, J.n_pad, g, a.pr_c, a.pr_v, a.pr_n,
+                         reinterpret_cast<uint32_t*>(lt_smem));
       } else if (kind == 1) {  // F: chunks slice, slice + nslices, ... of the list
         const uint32_t slice = a.it_arg[it] & 0xffffu, nsl = a.it_arg[it] >> 16;
         const uint32_t* L = reinterpret_cast<const uint32_t*>(
             __ldcg(reinterpret_cast<const unsigned long long*>(a.c_list + c)));
         const uint32_t n = ld_l2(a.c_list_n + c);
+        if (L == J.cand) {  // slice of the candidates, whole filter steps
+          const uint32_t per = ((n + nsl - 1) / nsl + kLvFullStep - 1) / kLvFullStep * kLvFullStep;
+          const uint64_t beg = (uint64_t)slice * per;
+          if (beg < n)
+            lv_filter_full(A, J, (uint32_t)beg, (uint32_t)min((uint64_t)n, beg + per), g, a.tab,
+                           a.cap, a.cnt, a.surv_id, a.surv_key, lt_smem);
+        } else
         for (uint32_t k = slice; (uint64_t)k * kLvChunk < n; k += nsl)
           lv_filter_chunk(A, L, k * kLvChunk, min(n, (k + 1) * kLvChunk), J.cells, J.x, J.n_pad,
                           g, a.pr_c, a.pr_v, a.pr_n, a.cap, a.cnt, a.surv_id, a.surv_key, lt_smem);
@@ -754,7 +1030,9 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_lattice(LtArgs a) {
 }
 
 static size_t lattice_smem() {
-  return kLvSfsSmem > kLvFilterSmem ? kLvSfsSmem : kLvFilterSmem;
+  size_t b = kLvSfsSmem;
+  for (size_t o : {kLvFilterSmem, kLvFullSmem}) b = o > b ? o : b;
+  return b;
 }
 
 // Persistent CTAs of the lattice kernel on `num_sms` SMs (one per SM).

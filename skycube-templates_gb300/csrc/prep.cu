@@ -242,7 +242,7 @@ __device__ __forceinline__ void sort_sample(float* s, uint32_t cnt) {
 __global__ void __launch_bounds__(1024) k_pivots(
     const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, int depth, float* __restrict__ pivots,
-    uint32_t* __restrict__ amin, uint32_t* __restrict__ hist) {
+    uint32_t* __restrict__ amin, uint32_t* __restrict__ hist, int low) {
   __shared__ __align__(16) float s[kPivotSample];
   const int k = blockIdx.x;
   if (amin && threadIdx.x == 0) amin[k] = 0xffffffffu;  // k_cells lowers it
@@ -261,10 +261,14 @@ __global__ void __launch_bounds__(1024) k_pivots(
   }
   __syncthreads();
   sort_sample(s, cnt);
+  // `low`: quadratic ranks, cells finer towards the minimum.
   const int P = (1 << depth) - 1;
   for (int r = threadIdx.x; r < kMaxPivots; r += blockDim.x) {
     float v = FLT_MAX;
-    if (r < P && cnt > 0) v = s[((uint64_t)(r + 1) * cnt) / (P + 1)];
+    if (r < P && cnt > 0) {
+      const uint64_t at = (uint64_t)(r + 1) * cnt;
+      v = s[low ? at * (r + 1) / ((uint64_t)(P + 1) * (P + 1)) : at / (P + 1)];
+    }
     pivots[k * kMaxPivots + r] = v;
   }
 }
@@ -690,8 +694,8 @@ static int launch_cells(cudaStream_t s, const float* x, uint64_t n_pad, const ui
 int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                         const uint32_t* ids, const uint32_t* m_ptr,
                         uint64_t m_max, int depth, float* pivots, uint4* cells, uint32_t* amin,
-                        uint32_t* hist, float* xout, uint64_t out_pad) {
-  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, amin, hist);
+                        uint32_t* hist, float* xout, uint64_t out_pad, int low) {
+  k_pivots<<<d, 1024, 0, s>>>(x, n_pad, ids, m_ptr, depth, pivots, amin, hist, low);
   SKC_LAUNCH_CHECK();
   switch (d) {
 #define SKC_CELLS_CASE(D) \
