@@ -123,7 +123,7 @@ struct PartitionSkylineArgs {
   const uint32_t* amin; // [d] ordered-uint minima over a superset of the list
 };
 constexpr uint32_t kMaxScanSums = 64;  // kMaxSortBuckets / 4096
-// Skyline kernel: work items per SM the plan aims at (48 warps are resident).
+// Skyline kernel: work items per SM the plan aims at (32 warps are resident).
 constexpr uint32_t kItemsPerSm = 256;
 constexpr int kMaxSubBits = 15;  // sub-key bits inside a partition
 int sort_sub_bits(uint64_t m_max, uint32_t K, int most);

@@ -385,8 +385,8 @@ __device__ __forceinline__ bool cells_le(const uint32_t (&pH)[NW], const uint4& 
 // 561 blocks lie under its mask, 75 of their quarters are open, 34 halves,
 // and 2 q's pass the cell test. Bound by instruction issue. Full skyline
 // step (sort, boxes, kernel) on one GB300, before -> after: 1M x 10
-// anticorrelated 5.62 -> 1.25 ms, 500k x 16 anticorrelated 8.07 -> 1.52,
-// 1M x 12 uniform 4.08 -> 0.91, 581k x 10 ties 2.10 -> 0.27.
+// anticorrelated 5.62 -> 1.15 ms, 500k x 16 anticorrelated 8.07 -> 1.33,
+// 1M x 12 uniform 4.08 -> 0.82.
 //
 // A point that holds the list's minimum on some attribute of S cannot be
 // strictly dominated, so its first dominator settles it (status 1); one that
@@ -399,8 +399,11 @@ __device__ __forceinline__ bool cells_le(const uint32_t (&pH)[NW], const uint4& 
 //
 // Slices of one item combine their statuses with a byte-wise atomic OR of
 // flags (1 dominated, 2 strictly dominated; 3 reads as strictly dominated).
+//
+// Four CTAs per SM (64 registers, no spill): the step at 1M x 10 1.15 ms; five
+// (48 registers, 50 bytes spilled) 1.26, six 1.23.
 template <int NA>
-__global__ void __launch_bounds__(32 * kTreeWarps, 5) k_skyline_tree(TreeArgs a) {
+__global__ void __launch_bounds__(32 * kTreeWarps, 4) k_skyline_tree(TreeArgs a) {
   constexpr int NW = (NA + 3) / 4;
   __shared__ uint4 s_p[kTreeWarps][32];
   __shared__ uint32_t s_bq[kTreeWarps][kBlkQ];
@@ -722,7 +725,7 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, cons
                                       ps.sorted, ps.sorted_id, ps.ccells);
   SKC_LAUNCH_CHECK();
   // Items: enough slices that a warp takes several and the last ones are
-  // short (kItemsPerSm per SM, 48 warps resident).
+  // short (kItemsPerSm per SM, 32 warps resident).
   k_boxes_and_plan<<<1 + blocks_for(a.m_max, 1024, 152 * 2), 1024, 0, s>>>(
       ps.ccells, a.m_ptr, ps.bmin, ps.smin, ps.hmin, ps.counts, T.rank, T.unrank, K, T.B,
       (uint32_t)num_sms * kItemsPerSm, ps.splits, ps.item_off);
