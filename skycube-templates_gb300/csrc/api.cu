@@ -464,6 +464,8 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   return full_space_counts(E, n, F, T);
 }
 
+constexpr uint64_t kIdBound = 1u << 19;  // ids (2 MB)
+
 // Bitmaps of every candidate, then CSR compaction (BATCHED and PLAIN/MDMC).
 static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
                        const RunParams& P, int max_d, Arena& A, FullSpace& F,
@@ -574,9 +576,21 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   }
   T.mark("bitmap kernel");
 
-  // Compaction of skylines (bit clear) and extended skylines (bit set).
+  // Compaction of skylines (bit clear) and extended skylines (bit set). The
+  // id lists are sized by their total, read back between the passes, or,
+  // where even every candidate on every cuboid is little, by that bound, and
+  // the totals are read at the end.
   const uint32_t tiles = compact_tiles(m, W);
   const uint64_t C = 32ull * W;
+  uint64_t bound = 0;
+  {
+    uint64_t cuboids = 1, choose = 1;
+    for (int k = 1; k <= std::min(max_d, d); ++k) cuboids += choose = choose * (d - k + 1) / k;
+    bound = m * cuboids;
+  }
+  const bool bounded = !E.plan && bound <= kIdBound;
+  uint64_t totals[2] = {0, 0};
+  const uint64_t* d_total[2] = {nullptr, nullptr};
   for (int pass = 0; pass < (want_ext ? 2 : 1); ++pass) {
     CompactArgs ca{};
     ca.bits = pass == 0 ? dom : ext;
@@ -600,6 +614,9 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
       // the stats and writes past the capacity are skipped.
       total = E.plan->ids_cap[pass];
       SKC_TRY(launch_stat_u64(s, csr + nsub, E.plan->stats, 1 + pass));
+    } else if (bounded) {
+      total = bound;
+      d_total[pass] = csr + nsub;
     } else {
       SKC_TRY(copy_d2h(&total, csr + nsub, sizeof(uint64_t), s));
     }
@@ -620,6 +637,15 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
       R->d_eids = ids;
       R->total_ext = total;
     }
+  }
+  if (bounded) {
+    for (int pass = 0; pass < 2; ++pass)
+      if (d_total[pass])
+        SKC_CUDA(cudaMemcpyAsync(&totals[pass], d_total[pass], sizeof(uint64_t),
+                                 cudaMemcpyDeviceToHost, s));
+    SKC_CUDA(cudaStreamSynchronize(s));
+    R->total_ids = totals[0];
+    if (want_ext) R->total_ext = totals[1];
   }
   if (o.want_bitmaps) {
     A.release(dom);
