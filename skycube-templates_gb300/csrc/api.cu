@@ -492,8 +492,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   SKC_TRY(A.alloc(&bmin, (m + 31) / 32));
   SKC_TRY(A.alloc(&smin, (m + 31) / 32 * 4));
   SKC_TRY(A.alloc(&hmin, (m + 31) / 32 * 8));
-  SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, F.cand, m_ptr, m, depth, pivots, cc,
-                              nullptr, nullptr, xc, m_pad));
+  const bool few = !E.plan && m <= kSmallCandidates;
 
   // q list: the full-space skyline only. If a point q' weakly dominates q
   // (q' <= q on every attribute), then for every p, LT(q, p) and LE(q, p)
@@ -511,7 +510,7 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   // q order: partitions by median mask over the first B attributes, in
   // lattice-level order (strongest partitions first).
   LevelTables LT;
-  SKC_TRY(level_tables(ctx, bitmap_partition_dims(d, mq_host, P.tile_points), &LT));
+  SKC_TRY(level_tables(ctx, few ? 0 : bitmap_partition_dims(d, mq_host, P.tile_points), &LT));
   // Inside a partition, q's are ordered by the quartile-cell bits of the
   // first 8 attributes in Gray-code order, so consecutive q's share their
   // quartile on most attributes and the 32-q blocks' minimum-cell boxes stay
@@ -527,12 +526,19 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   SKC_TRY(A.alloc(&buckets, KB + 1));
   SKC_TRY(A.alloc(&sums, kMaxScanSums));
   SKC_TRY(A.alloc(&boff, K + 1));
-  SKC_CUDA(cudaMemsetAsync(buckets, 0, (KB + 1) * sizeof(uint32_t), s));
-  SKC_TRY(launch_mask_keys(s, cc, qpos, mq_ptr, m, nsub - 1, d, LT.B, depth, sub_bits, LT.rank,
-                           keys, buckets));
-  SKC_TRY(launch_bucket_scan(s, buckets, KB, sums, sub_bits, boff));
-  SKC_TRY(launch_q_scatter(s, keys, mq_ptr, m, buckets, qpos, cc, xc, m_pad, d, qc, xq));
-  SKC_TRY(launch_block_min(s, qc, mq_ptr, m, bmin, smin, hmin));
+  if (few) {
+    SKC_TRY(launch_small_prep(s, d, ds->x, ds->n_pad, F.cand, F.cand_st, m_ptr, m, depth, m_pad, cc,
+                              xc, qc, xq, bmin, smin, hmin, boff, buckets + KB));
+  } else {
+    SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, F.cand, m_ptr, m, depth, pivots, cc,
+                                nullptr, nullptr, xc, m_pad));
+    SKC_CUDA(cudaMemsetAsync(buckets, 0, (KB + 1) * sizeof(uint32_t), s));
+    SKC_TRY(launch_mask_keys(s, cc, qpos, mq_ptr, m, nsub - 1, d, LT.B, depth, sub_bits, LT.rank,
+                             keys, buckets));
+    SKC_TRY(launch_bucket_scan(s, buckets, KB, sums, sub_bits, boff));
+    SKC_TRY(launch_q_scatter(s, keys, mq_ptr, m, buckets, qpos, cc, xc, m_pad, d, qc, xq));
+    SKC_TRY(launch_block_min(s, qc, mq_ptr, m, bmin, smin, hmin));
+  }
 
   T.mark("cand: cells+q order");
   uint32_t *dom, *ext = nullptr, *work = buckets + KB;

@@ -157,6 +157,12 @@ struct SplitOut {
 int launch_small_skyline(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                          const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max, uint32_t S,
                          uint32_t* masks, uint32_t* ticket, const SplitOut& out);
+// The bitmap kernel's inputs for few candidates in one launch (one partition).
+constexpr uint32_t kSmallCandidates = 1024;
+int launch_small_prep(cudaStream_t s, int d, const float* x, uint64_t n_pad, const uint32_t* cand,
+                      const uint8_t* cand_st, const uint32_t* m_ptr, uint64_t m_max, int depth,
+                      uint64_t pitch, uint4* cells, float* px, uint4* qcells, float* qx,
+                      uint4* bmin, uint4* smin, uint4* hmin, uint32_t* boff, uint32_t* work);
 int launch_single_offsets(cudaStream_t s, const uint32_t* n, uint32_t S, uint32_t nsub,
                           uint64_t* sky_off, uint64_t* ext_off);
 

@@ -239,6 +239,125 @@ int launch_small_skyline(cudaStream_t s, const float* x, uint64_t n_pad, int d,
   }
 }
 
+// The bitmap kernel's inputs for at most kSmallCandidates candidates, one per
+// thread of one CTA: cells, floats in candidate order, and the skyline points
+// as q's in candidate order with their box minima, one partition. The cells
+// come from an even grid between the attribute's least and greatest value
+// (any monotone cells are exact). Quantile pivots, the sort by partition and
+// the box pass are seven launches, some 35 us on one GB300, where the q's fill
+// 32 blocks at most; this one takes 7.
+template <int D>
+__global__ void __launch_bounds__(kSmallCandidates) k_small_prep(
+    const float* __restrict__ x, uint64_t n_pad, const uint32_t* __restrict__ cand,
+    const uint8_t* __restrict__ cand_st, const uint32_t* __restrict__ m_ptr, int depth,
+    uint64_t pitch, uint4* __restrict__ cells, float* __restrict__ px, uint4* __restrict__ qcells,
+    float* __restrict__ qx, uint4* __restrict__ bmin, uint4* __restrict__ smin,
+    uint4* __restrict__ hmin, uint32_t* __restrict__ boff, uint32_t* __restrict__ work) {
+  __shared__ uint32_t s_lo[D], s_hi[D], s_w[32];
+  const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const uint32_t m = *m_ptr;
+  if (t < D) {
+    s_lo[t] = 0xffffffffu;
+    s_hi[t] = 0;
+  }
+  __syncthreads();
+  float v[D];
+  const bool in = t < m;
+  const uint32_t id = in ? cand[t] : 0u;
+#pragma unroll
+  for (int k = 0; k < D; ++k) v[k] = in ? x[(uint64_t)k * n_pad + id] : 0.f;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const uint32_t u = ordered_u32(v[k]);
+    const uint32_t lo = __reduce_min_sync(kAllLanes, in ? u : 0xffffffffu);
+    const uint32_t hi = __reduce_max_sync(kAllLanes, in ? u : 0u);
+    if (lane == 0) {
+      atomicMin(&s_lo[k], lo);
+      atomicMax(&s_hi[k], hi);
+    }
+  }
+  const bool sky = in && cand_st[t] == 0;
+  const uint32_t ball = __ballot_sync(kAllLanes, sky);
+  if (lane == 0) s_w[wid] = __popc(ball);
+  __syncthreads();
+  uint32_t j = __popc(ball & ((1u << lane) - 1u)), mq = 0;
+  for (uint32_t w = 0; w < 32; ++w) {
+    if (w < wid) j += s_w[w];
+    mq += s_w[w];
+  }
+  if (in) {
+    uint32_t w[4] = {0, 0, 0, 0};
+    const float top = (float)((1u << depth) - 1u);
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const uint32_t a = s_lo[k], b = s_hi[k];
+      const float lo = __uint_as_float((a & 0x80000000u) ? (a & 0x7fffffffu) : ~a);
+      const float hi = __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
+      const float scale = (top + 1.0f) / (hi - lo);
+      // a degenerate range (one value, overflow) has one cell
+      const float c = scale < 3.0e38f && hi - lo < 3.0e38f ? (v[k] - lo) * scale : 0.f;
+      w[k >> 2] |= (uint32_t)fminf(c, top) << (8 * (k & 3));
+      px[(uint64_t)k * pitch + t] = v[k];
+    }
+    const uint4 c4 = make_uint4(w[0], w[1], w[2], w[3]);
+    cells[t] = c4;
+    if (sky) {
+      qcells[j] = c4;
+#pragma unroll
+      for (int k = 0; k < D; ++k) qx[(uint64_t)k * pitch + j] = v[k];
+    }
+  }
+  const uint32_t pad = (mq + 31) & ~31u;
+  if (t >= mq && t < pad) {  // entries that add nothing (k_q_scatter)
+    qcells[t] = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
+#pragma unroll
+    for (int k = 0; k < D; ++k) qx[(uint64_t)k * pitch + t] = __int_as_float(0x7f800000);
+  }
+  if (t == 0) {
+    boff[0] = 0;
+    boff[1] = mq;
+    *work = 0;
+  }
+  __syncthreads();
+  if (wid * 32 >= pad) return;
+  uint4 c = qcells[t];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    c.x = __vminu4(c.x, __shfl_xor_sync(kAllLanes, c.x, o));
+    c.y = __vminu4(c.y, __shfl_xor_sync(kAllLanes, c.y, o));
+    c.z = __vminu4(c.z, __shfl_xor_sync(kAllLanes, c.z, o));
+    c.w = __vminu4(c.w, __shfl_xor_sync(kAllLanes, c.w, o));
+    if (o == 2 && (lane & 3) == 0) hmin[wid * 8 + (lane >> 2)] = c;
+    if (o == 4 && (lane & 7) == 0) smin[wid * 4 + (lane >> 3)] = c;
+  }
+  if (lane == 0) bmin[wid] = c;
+}
+
+int launch_small_prep(cudaStream_t s, int d, const float* x, uint64_t n_pad, const uint32_t* cand,
+                      const uint8_t* cand_st, const uint32_t* m_ptr, uint64_t m_max, int depth,
+                      uint64_t pitch, uint4* cells, float* px, uint4* qcells, float* qx,
+                      uint4* bmin, uint4* smin, uint4* hmin, uint32_t* boff, uint32_t* work) {
+  if (m_max > kSmallCandidates)
+    return set_error(SKC_ERR_INVALID, "%llu candidates for the one-CTA preparation",
+                     (unsigned long long)m_max);
+  switch (d) {
+#define SKC_PREP_CASE(D)                                                                        \
+  case D:                                                                                       \
+    k_small_prep<D><<<1, kSmallCandidates, 0, s>>>(x, n_pad, cand, cand_st, m_ptr, depth, pitch, \
+                                                   cells, px, qcells, qx, bmin, smin, hmin, boff, \
+                                                   work);                                       \
+    break;
+    SKC_PREP_CASE(2) SKC_PREP_CASE(3) SKC_PREP_CASE(4) SKC_PREP_CASE(5) SKC_PREP_CASE(6)
+    SKC_PREP_CASE(7) SKC_PREP_CASE(8) SKC_PREP_CASE(9) SKC_PREP_CASE(10) SKC_PREP_CASE(11)
+    SKC_PREP_CASE(12) SKC_PREP_CASE(13) SKC_PREP_CASE(14) SKC_PREP_CASE(15) SKC_PREP_CASE(16)
+#undef SKC_PREP_CASE
+    default:
+      return set_error(SKC_ERR_INVALID, "unsupported d=%d", d);
+  }
+  SKC_LAUNCH_CHECK();
+  return SKC_OK;
+}
+
 // Offsets of a result that holds one cuboid, S, for both of its lists:
 // off[c] = 0 up to S and the list's count above.
 __global__ void k_single_offsets(const uint32_t* __restrict__ n, uint32_t S, uint32_t nsub,
