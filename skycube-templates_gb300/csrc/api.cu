@@ -356,6 +356,7 @@ static int prefilter_scratch(Arena& A, int d, uint64_t mmax, uint32_t Kq, Prefil
   SKC_TRY(A.alloc(&pf->pr_key, Kq));
   SKC_TRY(A.alloc(&pf->pr_cells, Kq));
   SKC_TRY(A.alloc(&pf->pr_x, (uint64_t)d * Kq));
+  SKC_TRY(A.alloc(&pf->tab, prefilter_table_bytes(d, Kq) / sizeof(unsigned long long)));
   SKC_TRY(A.alloc(&pf->blk0, (mmax + 1023) / 1024 + 2));
   SKC_TRY(A.alloc(&pf->blk1, (mmax + 1023) / 1024 + 2));
   SKC_TRY(A.alloc(&pf->mid, mmax));
@@ -433,7 +434,7 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
     uint32_t *surv, *d_ns;
     SKC_TRY(A.alloc(&surv, n));
     SKC_TRY(A.alloc(&d_ns, 1));
-    PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, nullptr, d_n, n, full, Kq, depth, F.amin, pf, status, true};
+    PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, nullptr, d_n, n, full, Kq, F.amin, pf, status, true};
     SKC_TRY(launch_prefilter(s, d, ctx->num_sms, pfa, surv, d_ns));
     open = surv;
     m_open = d_ns;
@@ -1172,10 +1173,10 @@ static int auto_depth(uint64_t n, int d) {
 // points left open when those are at least a quarter; prefilter.cu): 128, the
 // suite's -q default, up to 700,000 points, 512 above, where each further
 // pruner meets more dominated points. Prefilter + skyline kernel with 128 /
-// 512 pruners, ms on one GB300: 1M points: anticorrelated x 10 1.71 / 1.66, x
-// 6 0.52 / 0.47, uniform x 12 1.33 / 1.19; below: ties 581k x 10 0.09 / 0.11,
-// anticorrelated 500k x 16 1.67 / 1.81, uniform 200k x 9 0.20 / 0.24, 100k x 6
-// 0.12 / 0.15.
+// 512 pruners, ms on one GB300: 1M points: anticorrelated x 10 1.44 / 1.27, x
+// 6 0.44 / 0.35, uniform x 12 1.14 / 0.94; below: ties 581k x 10 0.097 / 0.109,
+// anticorrelated 500k x 16 1.40 / 1.43, uniform 200k x 9 0.177 / 0.182, 100k x
+// 6 0.119 / 0.135.
 constexpr uint64_t kManyPrunersMinPoints = 700000;
 static int default_pruners(uint64_t n) { return n >= kManyPrunersMinPoints ? 512 : 128; }
 constexpr uint64_t kPrefilterMinPoints = 32768;  // below: launch-bound anyway
@@ -1618,7 +1619,7 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
       uint32_t *surv, *d_ns;
       SKC_TRY(A.alloc(&surv, m));
       SKC_TRY(A.alloc(&d_ns, 1));
-      PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, F.cand, m_ptr, m, S, Kq, depth, F.amin, pf, status, false};
+      PrefilterArgs pfa{F.cells, ds->x, ds->n_pad, F.cand, m_ptr, m, S, Kq, F.amin, pf, status, false};
       SKC_TRY(launch_prefilter(s, d, E.ctx->num_sms, pfa, surv, d_ns));
       open = surv;
       m_open = d_ns;

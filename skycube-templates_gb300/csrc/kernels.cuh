@@ -177,6 +177,7 @@ struct PrefilterScratch {
   uint32_t* pr_key;    // [K]
   uint4* pr_cells;     // [K] pruner cells, rank order
   float* pr_x;         // [d * K] pruner floats, rank order
+  unsigned long long* tab;  // [prefilter_table_bytes(d, K)] pruner tables
   uint32_t* blk0;      // [m_max / 1024 + 2] kept entries per 1024, first pass
   uint32_t* blk1;      // [m_max / 1024 + 2] and second pass
   uint32_t* mid;       // [m_max] open positions after the first pass
@@ -191,7 +192,6 @@ struct PrefilterArgs {
   uint64_t m_max;
   uint32_t S;
   uint32_t K;            // pruners, 1 .. kMaxPruners
-  int depth;             // grid depth of the cells
   const uint32_t* amin;  // [d] ordered-uint minima over a superset of the list
   PrefilterScratch ps;
   uint8_t* status;       // [m_max] by list position
@@ -199,7 +199,7 @@ struct PrefilterArgs {
 };
 int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
                      uint32_t* out, uint32_t* out_count);
-size_t prefilter_smem(int d, uint32_t K);
+size_t prefilter_table_bytes(int d, uint32_t K);
 
 // mdmc.cu: per-point dominated-subspace bitmaps over the candidate set.
 struct BitmapArgs {

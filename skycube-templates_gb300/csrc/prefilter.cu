@@ -21,9 +21,8 @@
 // space the cells kernel makes it), a collection pass that finds the
 // threshold bin first, and a one-block rank by (sum, id) so the strongest
 // pruners are tried first.
-// The filter holds the ranked pruners (cells + floats) in shared memory;
-// one thread per point walks them until one strictly dominates it: a SWAR
-// cell test decides most pairs, floats are read only on equal cells.
+// The filter looks a point's cells up in bit tables of the ranked pruners
+// (k_prefilter); floats are read only where cells tie.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -138,17 +137,13 @@ __global__ void __launch_bounds__(256) k_pruner_collect(const uint4* __restrict_
 }
 
 // Ranks the Kp pruners by (sum, id) and stores their cells and floats in rank
-// order: out_x[k * K + r] for attribute k. The ranks from K1 on (the second
-// pass) are then reordered by the Gray rank of their median bits over S, so
-// that the eight pruners of a group lie on the same side of most medians and
-// a point skips the group by its minimum cells. Zeroes the passes' counts.
+// order: out_x[k * K + r] for attribute k. Zeroes the passes' counts.
 __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restrict__ pr_ids,
                                                        const uint32_t* __restrict__ pr_key,
                                                        const uint32_t* __restrict__ sel,
                                                        const uint4* __restrict__ cells,
                                                        const float* __restrict__ x,
-                                                       uint64_t n_pad, uint32_t S, int d, int sh,
-                                                       uint32_t K, uint32_t K1,
+                                                       uint64_t n_pad, int d, uint32_t K,
                                                        uint4* __restrict__ out_cells,
                                                        float* __restrict__ out_x,
                                                        uint32_t* __restrict__ blk0,
@@ -163,175 +158,180 @@ __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restric
   if (t < Kp) me = ((unsigned long long)pr_key[t] << 32) | pr_ids[t];
   key[t] = me;
   __syncthreads();
-  uint32_t r = 0;
-  if (t < Kp) {
-#pragma unroll 8
-    for (uint32_t j = 0; j < Kp; ++j) r += key[j] < me;
-  }
-  __syncthreads();
-  uint4 c = make_uint4(0, 0, 0, 0);
-  if (t < Kp) {
-    c = cells[(uint32_t)me];
-    uint32_t g = 0;
-    for (int k = 0; k < d; ++k)
-      if ((S >> k) & 1u) g = 2 * g | ((word_of(c, k >> 2) >> (8 * (k & 3) + sh)) & 1u);
-    for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;
-    key[t] = r < K1 ? r : ((unsigned long long)(1 + g) << 32) | r;  // distinct
-  }
-  __syncthreads();
   if (t >= Kp) return;
-  if (r >= K1) {
-    const unsigned long long mk = key[t];
-    r = 0;
+  uint32_t r = 0;
 #pragma unroll 8
-    for (uint32_t j = 0; j < Kp; ++j) r += key[j] < mk;
-  }
+  for (uint32_t j = 0; j < Kp; ++j) r += key[j] < me;
   const uint32_t id = (uint32_t)me;
-  out_cells[r] = c;
+  out_cells[r] = cells[id];
   for (int k = 0; k < d; ++k) out_x[(uint64_t)k * K + r] = x[(uint64_t)k * n_pad + id];
 }
 
-// Tests the list positions sub[i] (sub nullptr: i) against the pruners of rank
-// [r0, r1): status 2 when one strictly dominates the point on S; status 1
-// when the point holds the minimum of an attribute of S (amin: nothing can
-// strictly dominate it) and one dominates it; else 0. blk[b] = the entries i
-// of [1024 b, 1024 b + 1024) left at 0 (the count pass of their compaction;
-// zero before). With gate_m set, the pass runs only when it has at least
-// *gate_m / 4 entries (otherwise all are left). On tied data nearly every
-// point that the pruners do not strictly dominate holds a minimum and is
-// settled here: 581k x 10 ties 24,600 of 24,600, where the skyline kernel
-// would search each one's dominator. Groups of eight pruners are skipped by
-// their minimum cells; a point's floats are read only where cells tie.
-template <int D>
-__global__ void __launch_bounds__(256) k_prefilter(const uint4* __restrict__ cells,
-                                                   const float* __restrict__ x, uint64_t n_pad,
-                                                   const uint32_t* __restrict__ sub,
-                                                   const uint32_t* __restrict__ ids,
-                                                   const uint32_t* __restrict__ m_ptr, uint32_t S,
-                                                   const uint32_t* __restrict__ sel,
-                                                   const uint4* __restrict__ pr_cells,
-                                                   const float* __restrict__ pr_x, uint32_t K,
-                                                   uint32_t r0, uint32_t r1,
-                                                   const uint32_t* __restrict__ gate_m,
-                                                   const uint32_t* __restrict__ amin,
-                                                   uint8_t* __restrict__ status,
-                                                   uint32_t* __restrict__ blk) {
-  constexpr int NW = (D + 3) / 4;
-  extern __shared__ uint4 sm4[];
-  const uint32_t R = r1 - r0;                      // smem rows
-  uint4* s_cells = sm4;                            // [R]
-  uint4* s_min = sm4 + R;                          // [ceil(R / 8)] groups' minimum cells
-  float* s_x = reinterpret_cast<float*>(s_min + (R + 7) / 8);  // [D][R]
-  const uint32_t m = *m_ptr;
-  // few survivors: this pass would not pay
-  const bool skip = gate_m && 4ull * m < *gate_m;
-  const uint32_t Kp = skip ? 0u : (min(sel[2], r1) > r0 ? min(sel[2], r1) - r0 : 0u);
-  for (uint32_t t = threadIdx.x; t < Kp; t += blockDim.x) {
-    s_cells[t] = pr_cells[r0 + t];
-#pragma unroll
-    for (int k = 0; k < D; ++k) s_x[k * R + t] = pr_x[(uint64_t)k * K + r0 + t];
-  }
+// Pruner tables. A group is up to 64 consecutive ranks (group 0 the first
+// pass's K1); T[g][k][v] holds, one bit per pruner, those whose cell on
+// attribute k is at most v (all of the group's for k outside S). The AND over
+// a point's attributes is the group's pruners that may dominate it.
+constexpr uint32_t kGroupPruners = 64;
+
+static uint32_t pruner_groups(uint32_t K, uint32_t K1) {
+  return 1 + (K - K1 + kGroupPruners - 1) / kGroupPruners;
+}
+
+__device__ __forceinline__ uint32_t group_begin(uint32_t g, uint32_t K1) {
+  return g ? K1 + (g - 1) * kGroupPruners : 0u;
+}
+
+__global__ void __launch_bounds__(128) k_pruner_tables(const uint4* __restrict__ pr_cells,
+                                                       const uint32_t* __restrict__ sel,
+                                                       uint32_t S, uint32_t K1,
+                                                       unsigned long long* __restrict__ tab) {
+  const uint32_t g = blockIdx.x, k = blockIdx.y, v = threadIdx.x;
+  const uint32_t beg = group_begin(g, K1), end = min(sel[2], group_begin(g + 1, K1));
+  __shared__ uint8_t c[kGroupPruners];
+  if (beg + v < end && v < kGroupPruners)
+    c[v] = (uint8_t)(word_of(pr_cells[beg + v], k >> 2) >> (8 * (k & 3)));
   __syncthreads();
-  for (uint32_t g = threadIdx.x; g * 8 < Kp; g += blockDim.x) {
-    uint4 mn = s_cells[g * 8];
-    for (uint32_t t = g * 8 + 1; t < min(Kp, g * 8 + 8); ++t) {
-      const uint4 c = s_cells[t];
-      mn.x = __vminu4(mn.x, c.x);
-      mn.y = __vminu4(mn.y, c.y);
-      mn.z = __vminu4(mn.z, c.z);
-      mn.w = __vminu4(mn.w, c.w);
-    }
-    s_min[g] = mn;
-  }
+  unsigned long long b = 0;
+  for (uint32_t j = 0; beg + j < end; ++j)
+    if (!((S >> k) & 1u) || c[j] <= v) b |= 1ull << j;
+  tab[((uint64_t)g * gridDim.y + k) * 128 + v] = b;
+}
+
+// Tests the list positions sub[i] (sub nullptr: i) against the pruner groups
+// [g0, g1): status 2 when one strictly dominates the point on S; status 1
+// when the point holds the minimum of an attribute of S (amin: nothing can
+// strictly dominate it) and one dominates it; else 0. A further launch on the
+// same positions (`again`) leaves the settled ones. With blk, blk[b] = the
+// entries i of [1024 b, 1024 b + 1024) left at 0 (the count pass of their
+// compaction; zero before). With gate_m set, the pass runs only when it has
+// at least *gate_m / 4 entries (otherwise all are left).
+//
+// The tables give the pruners whose cells are all at most the point's with D
+// 8-byte loads from shared memory per 64 pruners; only those few are compared
+// in the exact floats where cells tie. A walk over the pruners one by one (a
+// warp as many as its last open lane), groups of eight skipped by their
+// minimum cells, took 0.40 ms for the 512 pruners of 1M x 10 anticorrelated
+// points and 0.29 for 1M x 12 uniform; now 0.12 and 0.12. Settling the
+// points with a minimum matters on tied data: nearly every point left holds
+// one there (581k x 10 ties: 24,600 of 24,600), and the skyline kernel would
+// search each one's dominator.
+template <int D>
+__global__ void __launch_bounds__(1024) k_prefilter(
+    const uint4* __restrict__ cells, const float* __restrict__ x, uint64_t n_pad,
+    const uint32_t* __restrict__ sub, const uint32_t* __restrict__ ids,
+    const uint32_t* __restrict__ m_ptr, uint32_t S, const uint4* __restrict__ pr_cells,
+    const float* __restrict__ pr_x, uint32_t K, uint32_t K1,
+    const unsigned long long* __restrict__ tab, uint32_t g0, uint32_t g1,
+    const uint32_t* __restrict__ gate_m, const uint32_t* __restrict__ amin, int again,
+    uint8_t* __restrict__ status, uint32_t* __restrict__ blk) {
+  constexpr int NW = (D + 3) / 4;
+  extern __shared__ uint4 s_tab4[];  // [groups][D][128] eight-byte masks
+  const unsigned long long* s_tab = reinterpret_cast<const unsigned long long*>(s_tab4);
+  const uint32_t m = *m_ptr;
+  // few entries left: this pass would not pay
+  const uint32_t groups = gate_m && 4ull * m < *gate_m ? 0u : g1 - g0;
+  if ((uint64_t)blockIdx.x * 1024 >= m) return;
+  const uint4* src = reinterpret_cast<const uint4*>(tab + (uint64_t)g0 * (D * 128));
+  for (uint32_t t = threadIdx.x; t < groups * (D * 64); t += 1024) s_tab4[t] = src[t];
   __syncthreads();
   uint32_t hS[NW];
 #pragma unroll
   for (int w = 0; w < NW; ++w) hS[w] = guard_mask(S, w);
-  // 256 entries a round; their kept count goes to their block of 1024.
-  for (uint64_t base = blockIdx.x * 256ull; base < m; base += gridDim.x * 256ull) {
+  for (uint64_t base = (uint64_t)blockIdx.x * 1024; base < m; base += (uint64_t)gridDim.x * 1024) {
     const uint32_t i = (uint32_t)base + threadIdx.x;
     bool keep = false;
     if (i < m) {
       const uint32_t at = sub ? sub[i] : i;
-      const uint32_t id = ids ? ids[at] : at;
-      const uint4 c4 = cells[id];
-      uint32_t pc[NW], pH[NW];
-      uint32_t zero = 0;  // attributes of S whose cell is 0
+      if (again && status[at]) {
+        keep = false;
+      } else {
+        const uint32_t id = ids ? ids[at] : at;
+        const uint4 c4 = cells[id];
+        uint32_t found = 0;  // the status a pruner gives
+        bool at_min = false, min_known = false;
+        for (uint32_t g = 0; g < groups && !found; ++g) {
+          const unsigned long long* T = s_tab + g * (D * 128);
+          unsigned long long b = ~0ull;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        pc[w] = word_of(c4, w);
-        pH[w] = pc[w] | kGuard;
-        zero |= pack_guards((kGuard - pc[w]) & hS[w]) << (4 * w);
-      }
-      bool at_min = false;
-      for (uint32_t z = zero; z && !at_min; z &= z - 1) {
-        const int k = __ffs(z) - 1;
-        at_min = ordered_u32(x[(uint64_t)k * n_pad + id]) == amin[k];
-      }
-      uint32_t found = 0;  // the status a pruner gives
-      for (uint32_t t = 0; t < Kp && !found; ++t) {
-        if ((t & 7u) == 0u) {  // a group none of whose pruners is <= p is skipped
-          const uint4 q = s_min[t >> 3];
-          uint32_t worse = 0;  // guard bits where the minimum cell is above p's
+          for (int k = 0; k < D; ++k)
+            b &= T[128 * k + ((word_of(c4, k >> 2) >> (8 * (k & 3))) & 0x7fu)];
+          for (; b && !found; b &= b - 1) {
+            const uint32_t t = group_begin(g0 + g, K1) + __ffsll(b) - 1;
+            const uint4 q = pr_cells[t];
+            uint32_t Z = 0;  // attributes of S with equal cells
 #pragma unroll
-          for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
-          if (worse) {
-            t += 7;
-            continue;
+            for (int w = 0; w < NW; ++w)
+              Z |= pack_guards(ge_bytes(word_of(q, w) | kGuard, word_of(c4, w)) & hS[w]) << (4 * w);
+            if (!min_known) {  // a minimum's cell is 0, and so is the pruner's there
+              uint32_t zero = 0;
+#pragma unroll
+              for (int w = 0; w < NW; ++w)
+                zero |= pack_guards((kGuard - word_of(c4, w)) & hS[w]) << (4 * w);
+              for (; zero && !at_min; zero &= zero - 1) {
+                const int k = __ffs(zero) - 1;
+                at_min = ordered_u32(x[(uint64_t)k * n_pad + id]) == amin[k];
+              }
+              min_known = true;
+            }
+            bool le = true, all_lt = true, any_lt = Z != S;
+            for (; Z && le && (all_lt || at_min); Z &= Z - 1) {
+              const int k = __ffs(Z) - 1;
+              const float a = pr_x[(uint64_t)k * K + t], p = x[(uint64_t)k * n_pad + id];
+              le = a <= p;
+              if (a < p) any_lt = true; else all_lt = false;
+            }
+            if (at_min) found = (le && any_lt) ? 1u : 0u;
+            else found = (le && all_lt) ? 2u : 0u;
           }
         }
-        const uint4 q = s_cells[t];
-        uint32_t worse = 0;  // guard bits where cell(q) > cell(p)
-#pragma unroll
-        for (int w = 0; w < NW; ++w) worse |= ~(pH[w] - word_of(q, w)) & hS[w];
-        if (worse) continue;
-        uint32_t Z = 0;  // attributes of S with equal cells
-#pragma unroll
-        for (int w = 0; w < NW; ++w)
-          Z |= pack_guards(ge_bytes(word_of(q, w) | kGuard, pc[w]) & hS[w]) << (4 * w);
-        bool le = true, all_lt = true, any_lt = Z != S;
-        for (; Z && le && (all_lt || at_min); Z &= Z - 1) {
-          const int k = __ffs(Z) - 1;
-          const float a = s_x[k * R + t], b = x[(uint64_t)k * n_pad + id];
-          le = a <= b;
-          if (a < b) any_lt = true; else all_lt = false;
-        }
-        if (at_min) found = (le && any_lt) ? 1u : 0u;
-        else found = (le && all_lt) ? 2u : 0u;
+        keep = !found;
+        status[at] = (uint8_t)found;
       }
-      keep = !found;
-      status[at] = (uint8_t)found;
     }
     const int kept = __syncthreads_count(keep);
-    if (threadIdx.x == 0 && kept) atomicAdd(&blk[base >> 10], (uint32_t)kept);
+    if (blk && threadIdx.x == 0) blk[base >> 10] = kept;
   }
 }
 
-size_t prefilter_smem(int d, uint32_t K) {
-  return ((size_t)K + (K + 7) / 8) * sizeof(uint4) + (size_t)d * K * sizeof(float);
+size_t prefilter_table_bytes(int d, uint32_t K) {
+  const uint32_t K1 = std::max<uint32_t>(1, K / 16);
+  return (size_t)pruner_groups(K, K1) * d * 128 * sizeof(unsigned long long);
 }
 
+// Groups of one launch: their tables have to fit the shared memory.
+constexpr size_t kMaxTableSmem = 200 * 1024;
+
 template <int D>
-static int launch_prefilter_d(cudaStream_t s, const PrefilterArgs& a, unsigned grid,
-                              const uint32_t* sub, const uint32_t* m_ptr, uint32_t r0,
-                              uint32_t r1, const uint32_t* gate_m, uint32_t* blk) {
-  const size_t smem = prefilter_smem(D, r1 - r0);
-  if (smem > 48 * 1024)
-    SKC_CUDA(cudaFuncSetAttribute(k_prefilter<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-  k_prefilter<D><<<grid, 256, smem, s>>>(a.cells, a.x, a.n_pad, sub, a.ids, m_ptr, a.S, a.ps.hist + kSumBins,
-                                         a.ps.pr_cells, a.ps.pr_x, a.K, r0, r1, gate_m, a.amin,
-                                         a.status, blk);
-  SKC_LAUNCH_CHECK();
+static int launch_prefilter_d(cudaStream_t s, int num_sms, const PrefilterArgs& a,
+                              const uint32_t* sub, const uint32_t* m_ptr, uint32_t g0, uint32_t g1,
+                              const uint32_t* gate_m, uint32_t* blk) {
+  constexpr size_t kGroupBytes = D * 128 * sizeof(unsigned long long);
+  constexpr uint32_t kMost = (uint32_t)(kMaxTableSmem / kGroupBytes);
+  const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);
+  SKC_CUDA(cudaFuncSetAttribute(k_prefilter<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(kMost * kGroupBytes)));
+  const uint64_t want = (a.m_max + 1023) / 1024;
+  for (uint32_t g = g0; g < g1; g += kMost) {
+    const uint32_t e = std::min(g1, g + kMost);
+    const size_t smem = (e - g) * kGroupBytes;
+    const uint64_t per_sm = smem > 110 * 1024 ? 1 : 2;
+    const unsigned grid =
+        (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)num_sms * per_sm));
+    k_prefilter<D><<<grid, 1024, smem, s>>>(a.cells, a.x, a.n_pad, sub, a.ids, m_ptr, a.S,
+                                            a.ps.pr_cells, a.ps.pr_x, a.K, K1, a.ps.tab, g, e,
+                                            gate_m, a.amin, g > g0, a.status,
+                                            e == g1 ? blk : nullptr);
+    SKC_LAUNCH_CHECK();
+  }
   return SKC_OK;
 }
 
-static int launch_prefilter_pass(cudaStream_t s, int d, const PrefilterArgs& a, unsigned grid,
-                                 const uint32_t* sub, const uint32_t* m_ptr, uint32_t r0,
-                                 uint32_t r1, const uint32_t* gate_m, uint32_t* blk) {
+static int launch_prefilter_pass(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
+                                 const uint32_t* sub, const uint32_t* m_ptr, uint32_t g0,
+                                 uint32_t g1, const uint32_t* gate_m, uint32_t* blk) {
   switch (d) {
 #define SKC_PF_CASE(D) \
-  case D: return launch_prefilter_d<D>(s, a, grid, sub, m_ptr, r0, r1, gate_m, blk);
+  case D: return launch_prefilter_d<D>(s, num_sms, a, sub, m_ptr, g0, g1, gate_m, blk);
     SKC_PF_CASE(2) SKC_PF_CASE(3) SKC_PF_CASE(4) SKC_PF_CASE(5) SKC_PF_CASE(6)
     SKC_PF_CASE(7) SKC_PF_CASE(8) SKC_PF_CASE(9) SKC_PF_CASE(10) SKC_PF_CASE(11)
     SKC_PF_CASE(12) SKC_PF_CASE(13) SKC_PF_CASE(14) SKC_PF_CASE(15) SKC_PF_CASE(16)
@@ -359,9 +359,12 @@ int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
                                         p.pr_ids, p.pr_key);
   SKC_LAUNCH_CHECK();
   const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);  // pruners of the first pass
-  k_pruner_order<<<1, 1024, 0, s>>>(p.pr_ids, p.pr_key, sel, a.cells, a.x, a.n_pad, a.S, d,
-                                    a.depth - 1, a.K, K1, p.pr_cells, p.pr_x, p.blk0, p.blk1,
+  k_pruner_order<<<1, 1024, 0, s>>>(p.pr_ids, p.pr_key, sel, a.cells, a.x, a.n_pad, d, a.K,
+                                    p.pr_cells, p.pr_x, p.blk0, p.blk1,
                                     (uint32_t)((a.m_max + 1023) / 1024));
+  SKC_LAUNCH_CHECK();
+  const uint32_t G = pruner_groups(a.K, K1);
+  k_pruner_tables<<<dim3(G, d), 128, 0, s>>>(p.pr_cells, sel, a.S, K1, p.tab);
   SKC_LAUNCH_CHECK();
   // Two passes: the strongest K1 = K / 16 pruners on every entry, then, only
   // when at least a quarter of the entries survived, the other pruners on
@@ -369,11 +372,11 @@ int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
   // the first pass (more pruners only cost there: survivors that nothing can
   // strictly dominate walk every pruner); anticorrelated data keeps most
   // points, and the second pass removes a good part of them.
-  SKC_TRY(launch_prefilter_pass(s, d, a, grid, nullptr, a.m_ptr, 0, K1, nullptr, p.blk0));
-  if (K1 >= a.K)
+  SKC_TRY(launch_prefilter_pass(s, d, num_sms, a, nullptr, a.m_ptr, 0, 1, nullptr, p.blk0));
+  if (G == 1)
     return launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, out, out_count);
   SKC_TRY(launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, p.mid, p.mid_count));
-  SKC_TRY(launch_prefilter_pass(s, d, a, grid, p.mid, p.mid_count, K1, a.K, a.m_ptr, p.blk1));
+  SKC_TRY(launch_prefilter_pass(s, d, num_sms, a, p.mid, p.mid_count, 1, G, a.m_ptr, p.blk1));
   return launch_status_keep(s, a.status, p.mid, p.mid_count, a.m_max, p.blk1, out, out_count);
 }
 
