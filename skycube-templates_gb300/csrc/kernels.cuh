@@ -148,15 +148,29 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth,
 constexpr uint32_t kSmallList = 6144;
 struct SplitOut {
   uint32_t* sky;      // skyline ids, list order
-  uint32_t* ext;      // extended skyline ids
+  uint32_t* ext;      // extended skyline ids (nullptr: behind the skyline's in `sky`)
   uint32_t* both;     // their union in list order, or nullptr
-  uint8_t* both_st;   // per entry of `both`: 0 skyline, else 2
+  uint8_t* both_st;   // per entry of `both`: 0 skyline, else 2 (nullptr: neither it nor pos0)
   uint32_t* pos0;     // per skyline id: its position in `both`
   uint32_t* n;        // [3] counts: sky, ext, both
 };
 int launch_small_skyline(cudaStream_t s, const float* x, uint64_t n_pad, int d,
                          const uint32_t* ids, const uint32_t* m_ptr, uint64_t m_max, uint32_t S,
                          uint32_t* masks, uint32_t* ticket, const SplitOut& out);
+// The same for several lists and subspaces with one attribute count (below
+// 16) in one launch; fills in `attrs` and `first`.
+constexpr uint32_t kSmallJobs = 64;
+struct SmallJob {
+  const uint32_t* ids;
+  uint32_t* lists;  // [m] skyline ids, then extended skyline ids
+  uint32_t* both;   // [m] their union in list order, or nullptr
+  uint32_t* n;      // [3] counts: sky, ext, both
+  uint32_t m, S;    // list length (1 to kSmallList), subspace
+  unsigned long long attrs;
+  uint32_t first;   // first CTA
+};
+int launch_small_batch(cudaStream_t s, const float* x, uint64_t n_pad, int d, SmallJob* jobs,
+                       uint32_t nj, uint32_t* masks, uint32_t* tickets);
 // The bitmap kernel's inputs for few candidates in one launch (one partition).
 constexpr uint32_t kSmallCandidates = 1024;
 int launch_small_prep(cudaStream_t s, int d, const float* x, uint64_t n_pad, const uint32_t* cand,

@@ -50,3 +50,23 @@ def test_longest_list_and_the_pipeline_agree(gpu_ctx, kind, d, n):
             assert np.array_equal(a.extended(S), o.extended(S)), S
     for o in (a, b, c, ds):
         o.close()
+
+
+@pytest.mark.parametrize("kind,n,d,max_d", [
+    ("uniform", 33, 4, 0), ("ties", 3000, 9, 0), ("anticorrelated", 1500, 9, 0),
+    ("anticorrelated", 30000, 6, 0), ("correlated_q", 40000, 10, 3), ("uniform", 60000, 8, 5),
+])
+def test_levels_of_the_per_cuboid_form(gpu_ctx, kind, n, d, max_d):
+    """k_small_batch: a lattice level's short lists in one launch, more than 64
+    of them in several (9 attributes: 126 on two levels), beside longer lists
+    of the same level, with parents from either, against the bitmap form."""
+    ds = sk.Dataset(gpu_ctx, datagen.generate(kind, n, d, 3 * n + d))
+    a = sk.skycube(gpu_ctx, ds, max_d=max_d, want_extended=True, form="bitmaps")
+    b = sk.skycube(gpu_ctx, ds, "sdsc", "plain", max_d=max_d, want_extended=True)
+    top = max_d or d
+    for S in range(1, 1 << d):
+        if bin(S).count("1") <= top or S == (1 << d) - 1:
+            assert np.array_equal(a.cuboid(S), b.cuboid(S)), S
+            assert np.array_equal(a.extended(S), b.extended(S)), S
+    for o in (a, b, ds):
+        o.close()
