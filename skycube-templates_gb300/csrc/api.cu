@@ -357,10 +357,7 @@ static int prefilter_scratch(Arena& A, int d, uint64_t mmax, uint32_t Kq, Prefil
   SKC_TRY(A.alloc(&pf->pr_cells, Kq));
   SKC_TRY(A.alloc(&pf->pr_x, (uint64_t)d * Kq));
   SKC_TRY(A.alloc(&pf->tab, prefilter_table_bytes(d, Kq) / sizeof(unsigned long long)));
-  SKC_TRY(A.alloc(&pf->blk0, (mmax + 1023) / 1024 + 2));
-  SKC_TRY(A.alloc(&pf->blk1, (mmax + 1023) / 1024 + 2));
-  SKC_TRY(A.alloc(&pf->mid, mmax));
-  return A.alloc(&pf->mid_count, 1);
+  return A.alloc(&pf->blk, (mmax + 1023) / 1024 + 2);
 }
 
 // Scratch of launch_partition_skyline for lists of up to mmax entries.
@@ -378,6 +375,7 @@ static int part_scratch(Arena& A, uint64_t mmax, PartScratch* ps) {
   SKC_TRY(A.alloc(&ps->fine, kMaxSortBuckets + 1));
   SKC_TRY(A.alloc(&ps->sums, kMaxScanSums));
   SKC_TRY(A.alloc(&ps->splits, Kmax));
+  SKC_TRY(A.alloc(&ps->rest, 1));
   return A.alloc(&ps->item_off, Kmax + 1);
 }
 
@@ -1229,14 +1227,12 @@ static int auto_depth(uint64_t n, int d) {
 
 // Defaults of the work parameters (used when neither the options nor a
 // stored tuning set them).
-// Pruners, in two passes (a 16th of them on every point, the rest on the
-// points left open when those are at least a quarter; prefilter.cu): 128, the
-// suite's -q default, up to 700,000 points, 512 above, where each further
-// pruner meets more dominated points. Prefilter + skyline kernel with 128 /
-// 512 pruners, ms on one GB300: 1M points: anticorrelated x 10 1.44 / 1.27, x
-// 6 0.44 / 0.35, uniform x 12 1.14 / 0.94; below: ties 581k x 10 0.097 / 0.109,
-// anticorrelated 500k x 16 1.40 / 1.43, uniform 200k x 9 0.177 / 0.182, 100k x
-// 6 0.119 / 0.135.
+// Pruners (prefilter.cu): 128, the suite's -q default, up to 700,000 points,
+// 512 above, where each further pruner meets more dominated points. Prefilter
+// + skyline kernel with 128 / 512 pruners, ms on one GB300: 1M points:
+// anticorrelated x 10 1.39 / 1.23, x 6 0.43 / 0.35, uniform x 12 1.10 / 0.91;
+// below: ties 581k x 10 0.084 / 0.094, anticorrelated 500k x 16 1.35 / 1.38,
+// uniform 200k x 9 0.153 / 0.161, 100k x 6 0.090 / 0.102.
 constexpr uint64_t kManyPrunersMinPoints = 700000;
 static int default_pruners(uint64_t n) { return n >= kManyPrunersMinPoints ? 512 : 128; }
 constexpr uint64_t kPrefilterMinPoints = 32768;  // below: launch-bound anyway

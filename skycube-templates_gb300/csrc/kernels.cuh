@@ -41,11 +41,10 @@ int launch_status_split(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
                         const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* blk1,
                         uint32_t* sky, uint32_t* ext, uint32_t* n, uint32_t* both = nullptr,
                         uint8_t* both_st = nullptr, uint32_t* pos0 = nullptr);
-// List entries sub[i] (sub nullptr: i) of status 0 into out, *n their count;
+// List positions of status 0 into out, *n their count;
 // blk0[b] holds the count over i in [1024 b, 1024 b + 1024) (zero past the list).
-int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
-                       const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* out,
-                       uint32_t* n);
+int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* m_ptr, uint64_t m_max,
+                       uint32_t* blk0, uint32_t* out, uint32_t* n);
 // Exclusive scan of in[0 .. len) into out[0 .. len]; csr_off[c] = out[c * T]
 // for c <= nsub (nsub * T <= len).
 int launch_scan_counts(cudaStream_t s, const uint32_t* in, uint64_t len, uint64_t* bsum,
@@ -107,6 +106,7 @@ struct PartScratch {
   uint32_t* fine;      // [kMaxSortBuckets + 1] counting-sort offsets, work counter
   uint32_t* sums;      // [kMaxScanSums]
   uint32_t* splits;    // [2^B]
+  uint32_t* rest;      // points left by launch_small_status
   uint32_t* item_off;  // [2^B + 1]
 };
 struct PartitionSkylineArgs {
@@ -135,7 +135,7 @@ int launch_mask_keys(cudaStream_t s, const uint4* cells, const uint32_t* ids,
 // kMaxSortBuckets); boff[b] = offset of bucket b << sub_bits, boff[len >>
 // sub_bits] = the total.
 int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t* sums,
-                       int sub_bits, uint32_t* boff);
+                       int sub_bits, uint32_t* boff, const uint32_t* m_ptr = nullptr);
 int launch_q_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* mq_ptr, uint64_t m_max,
                      uint32_t* cursor, const uint32_t* qpos, const uint4* pcells, const float* px,
                      uint64_t pitch, int d, uint4* qcells, float* qx);
@@ -171,6 +171,9 @@ struct SmallJob {
 };
 int launch_small_batch(cudaStream_t s, const float* x, uint64_t n_pad, int d, SmallJob* jobs,
                        uint32_t nj, uint32_t* masks, uint32_t* tickets);
+// Statuses of a prefilter's open points by all pairs when there are few enough
+// of them (small.cu); *rest = those left to the partition pipeline (all or 0).
+int launch_small_status(cudaStream_t s, int d, const PartitionSkylineArgs& a, uint32_t* rest);
 // The bitmap kernel's inputs for few candidates in one launch (one partition).
 constexpr uint32_t kSmallCandidates = 1024;
 int launch_small_prep(cudaStream_t s, int d, const float* x, uint64_t n_pad, const uint32_t* cand,
@@ -192,10 +195,7 @@ struct PrefilterScratch {
   uint4* pr_cells;     // [K] pruner cells, rank order
   float* pr_x;         // [d * K] pruner floats, rank order
   unsigned long long* tab;  // [prefilter_table_bytes(d, K)] pruner tables
-  uint32_t* blk0;      // [m_max / 1024 + 2] kept entries per 1024, first pass
-  uint32_t* blk1;      // [m_max / 1024 + 2] and second pass
-  uint32_t* mid;       // [m_max] open positions after the first pass
-  uint32_t* mid_count; // [1]
+  uint32_t* blk;       // [m_max / 1024 + 2] kept entries per 1024
 };
 struct PrefilterArgs {
   const uint4* cells;    // point id -> grid cells

@@ -85,11 +85,14 @@ __global__ void k_mask_keys(const uint4* __restrict__ cells,
 // buckets adds them up, then every CTA adds the sums before it (at most 64)
 // and scans its own 4,096 in place. The former single-CTA scan walked 2^18
 // buckets in 64 dependent tiles: 115 us on one GB300; these two: 5.
-// boff[b] = offset of bucket b << sub_bits, boff[K] = the total.
+// boff[b] = offset of bucket b << sub_bits, boff[K] = the total. With m_ptr, a
+// list of length 0 is left alone (nothing reads its offsets).
 constexpr uint32_t kScanTile = 4096;
 
 __global__ void __launch_bounds__(1024) k_bucket_sums(const uint32_t* __restrict__ counts,
-                                                      uint32_t* __restrict__ sums) {
+                                                      uint32_t* __restrict__ sums,
+                                                      const uint32_t* __restrict__ m_ptr) {
+  if (m_ptr && *m_ptr == 0) return;
   __shared__ uint32_t red[32];
   const uint4 v = reinterpret_cast<const uint4*>(counts)[(size_t)blockIdx.x * 1024 + threadIdx.x];
   const uint32_t s = __reduce_add_sync(0xffffffffu, v.x + v.y + v.z + v.w);
@@ -103,7 +106,9 @@ __global__ void __launch_bounds__(1024) k_bucket_sums(const uint32_t* __restrict
 
 __global__ void __launch_bounds__(1024) k_bucket_scan(uint32_t* __restrict__ counts, uint32_t len,
                                                       const uint32_t* __restrict__ sums,
-                                                      int sub_bits, uint32_t* __restrict__ boff) {
+                                                      int sub_bits, uint32_t* __restrict__ boff,
+                                                      const uint32_t* __restrict__ m_ptr) {
+  if (m_ptr && *m_ptr == 0) return;
   __shared__ uint32_t wsum[32];
   __shared__ uint32_t s_base;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -154,13 +159,13 @@ __global__ void __launch_bounds__(1024) k_bucket_scan(uint32_t* __restrict__ cou
 }
 
 int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t* sums,
-                       int sub_bits, uint32_t* boff) {
+                       int sub_bits, uint32_t* boff, const uint32_t* m_ptr) {
   const uint32_t g = (len + kScanTile - 1) / kScanTile;
   if (g > 1) {  // then len is a multiple of the tile (both are powers of two)
-    k_bucket_sums<<<g, 1024, 0, s>>>(counts, sums);
+    k_bucket_sums<<<g, 1024, 0, s>>>(counts, sums, m_ptr);
     SKC_LAUNCH_CHECK();
   }
-  k_bucket_scan<<<g, 1024, 0, s>>>(counts, len, sums, sub_bits, boff);
+  k_bucket_scan<<<g, 1024, 0, s>>>(counts, len, sums, sub_bits, boff, m_ptr);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
@@ -254,6 +259,10 @@ __global__ void __launch_bounds__(1024) k_boxes_and_plan(
     const uint32_t* __restrict__ unrank, uint32_t K, int B, uint32_t target,
     uint32_t* __restrict__ splits, uint32_t* __restrict__ item_off) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (*m_ptr == 0) {  // an empty list has no items
+    if (blockIdx.x == 0 && threadIdx.x == 0) item_off[K] = 0;
+    return;
+  }
   if (blockIdx.x > 0) {
     const uint32_t nblk = (*m_ptr + 31) / 32;
     for (uint32_t b = (blockIdx.x - 1) * 32 + wid; b < nblk; b += (gridDim.x - 1) * 32) {
@@ -421,6 +430,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps, 4) k_skyline_tree(TreeArgs a)
   uint2* sq = s_sq[wid];
   uint2* hq = s_hq[wid];
   const uint32_t n_items = a.item_off[a.K];
+  if (n_items == 0) return;
   const uint32_t m = a.boff[a.K];
 
   for (;;) {
@@ -714,7 +724,12 @@ static int launch_tree(cudaStream_t s, int num_sms, const TreeArgs& a) {
 }
 
 int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, const LevelTables& T,
-                             const PartitionSkylineArgs& a, const PartScratch& ps) {
+                             const PartitionSkylineArgs& args, const PartScratch& ps) {
+  PartitionSkylineArgs a = args;
+  if (a.sub) {  // a prefilter ran: few points may be left
+    SKC_TRY(launch_small_status(s, d, args, ps.rest));
+    a.m_ptr = ps.rest;
+  }
   const uint32_t K = 1u << T.B;
   const int na = __builtin_popcount(a.S);
   const int sub_bits = sort_sub_bits(a.m_max, K, std::min(kMaxSubBits, na * (depth - 1)));
@@ -725,7 +740,7 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, cons
   k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.sub, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits,
                                    T.rank, ps.keys, ps.fine, a.sub ? nullptr : a.status);
   SKC_LAUNCH_CHECK();
-  SKC_TRY(launch_bucket_scan(s, ps.fine, KB, ps.sums, sub_bits, ps.counts));
+  SKC_TRY(launch_bucket_scan(s, ps.fine, KB, ps.sums, sub_bits, ps.counts, a.m_ptr));
   k_part_scatter<<<grid, 256, 0, s>>>(ps.keys, a.m_ptr, ps.fine, a.cells, a.sub, a.ids, a.S, d,
                                       ps.sorted, ps.sorted_id, ps.ccells);
   SKC_LAUNCH_CHECK();

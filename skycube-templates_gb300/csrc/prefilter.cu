@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) k_pruner_collect(const uint4* __restrict_
 }
 
 // Ranks the Kp pruners by (sum, id) and stores their cells and floats in rank
-// order: out_x[k * K + r] for attribute k. Zeroes the passes' counts.
+// order: out_x[k * K + r] for attribute k. Zeroes the filter's counts.
 __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restrict__ pr_ids,
                                                        const uint32_t* __restrict__ pr_key,
                                                        const uint32_t* __restrict__ sel,
@@ -146,12 +146,10 @@ __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restric
                                                        uint64_t n_pad, int d, uint32_t K,
                                                        uint4* __restrict__ out_cells,
                                                        float* __restrict__ out_x,
-                                                       uint32_t* __restrict__ blk0,
-                                                       uint32_t* __restrict__ blk1,
-                                                       uint32_t nblk) {
+                                                       uint32_t* __restrict__ blk, uint32_t nblk) {
   static_assert(kMaxPruners <= 1024, "one pruner per thread");
   __shared__ unsigned long long key[kMaxPruners];
-  for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x) blk0[b] = blk1[b] = 0;
+  for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x) blk[b] = 0;
   const uint32_t Kp = sel[2];
   const uint32_t t = threadIdx.x;
   unsigned long long me = ~0ull;
@@ -167,26 +165,20 @@ __global__ void __launch_bounds__(1024) k_pruner_order(const uint32_t* __restric
   for (int k = 0; k < d; ++k) out_x[(uint64_t)k * K + r] = x[(uint64_t)k * n_pad + id];
 }
 
-// Pruner tables. A group is up to 64 consecutive ranks (group 0 the first
-// pass's K1); T[g][k][v] holds, one bit per pruner, those whose cell on
-// attribute k is at most v (all of the group's for k outside S). The AND over
-// a point's attributes is the group's pruners that may dominate it.
+// Pruner tables. A group is 64 consecutive ranks; T[g][k][v] holds, one bit
+// per pruner, those whose cell on attribute k is at most v (all of the group's
+// for k outside S). The AND over a point's attributes is the group's pruners
+// that may dominate it.
 constexpr uint32_t kGroupPruners = 64;
 
-static uint32_t pruner_groups(uint32_t K, uint32_t K1) {
-  return 1 + (K - K1 + kGroupPruners - 1) / kGroupPruners;
-}
-
-__device__ __forceinline__ uint32_t group_begin(uint32_t g, uint32_t K1) {
-  return g ? K1 + (g - 1) * kGroupPruners : 0u;
-}
+static uint32_t pruner_groups(uint32_t K) { return (K + kGroupPruners - 1) / kGroupPruners; }
 
 __global__ void __launch_bounds__(128) k_pruner_tables(const uint4* __restrict__ pr_cells,
                                                        const uint32_t* __restrict__ sel,
-                                                       uint32_t S, uint32_t K1,
+                                                       uint32_t S,
                                                        unsigned long long* __restrict__ tab) {
   const uint32_t g = blockIdx.x, k = blockIdx.y, v = threadIdx.x;
-  const uint32_t beg = group_begin(g, K1), end = min(sel[2], group_begin(g + 1, K1));
+  const uint32_t beg = g * kGroupPruners, end = min(sel[2], beg + kGroupPruners);
   __shared__ uint8_t c[kGroupPruners];
   if (beg + v < end && v < kGroupPruners)
     c[v] = (uint8_t)(word_of(pr_cells[beg + v], k >> 2) >> (8 * (k & 3)));
@@ -197,14 +189,12 @@ __global__ void __launch_bounds__(128) k_pruner_tables(const uint4* __restrict__
   tab[((uint64_t)g * gridDim.y + k) * 128 + v] = b;
 }
 
-// Tests the list positions sub[i] (sub nullptr: i) against the pruner groups
-// [g0, g1): status 2 when one strictly dominates the point on S; status 1
-// when the point holds the minimum of an attribute of S (amin: nothing can
-// strictly dominate it) and one dominates it; else 0. A further launch on the
-// same positions (`again`) leaves the settled ones. With blk, blk[b] = the
-// entries i of [1024 b, 1024 b + 1024) left at 0 (the count pass of their
-// compaction; zero before). With gate_m set, the pass runs only when it has
-// at least *gate_m / 4 entries (otherwise all are left).
+// Tests the list's points against the pruner groups [g0, g1): status 2 when
+// one strictly dominates the point on S; status 1 when the point holds the
+// minimum of an attribute of S (amin: nothing can strictly dominate it) and
+// one dominates it; else 0. A further launch (`again`) leaves the settled
+// ones. With blk, blk[b] = the entries of [1024 b, 1024 b + 1024) left at 0
+// (the count pass of their compaction; zero before).
 //
 // The tables give the pruners whose cells are all at most the point's with D
 // 8-byte loads from shared memory per 64 pruners; only those few are compared
@@ -214,22 +204,28 @@ __global__ void __launch_bounds__(128) k_pruner_tables(const uint4* __restrict__
 // points and 0.29 for 1M x 12 uniform; now 0.12 and 0.12. Settling the
 // points with a minimum matters on tied data: nearly every point left holds
 // one there (581k x 10 ties: 24,600 of 24,600), and the skyline kernel would
-// search each one's dominator.
+// search each one's dominator. A point with every minimum is equal to the
+// pruners it passes: it is left at once (500k x 8 correlated: a walk over all pruners,
+// 0.090 -> 0.046 ms for the step).
+//
+// One pass over the list with all pruners. Two, the second over what a 16th
+// of the pruners left and only when that was a quarter, take a compaction
+// and two launches more, and the skyline kernel then got 20,200 points of
+// 250k x 5 uniform where 2,600 are left now: prefilter and skyline kernel
+// 0.130 -> 0.096 ms there, 100k x 6 0.118 -> 0.091, 1M x 10 1.25 -> 1.23.
 template <int D>
 __global__ void __launch_bounds__(1024) k_prefilter(
     const uint4* __restrict__ cells, const float* __restrict__ x, uint64_t n_pad,
-    const uint32_t* __restrict__ sub, const uint32_t* __restrict__ ids,
-    const uint32_t* __restrict__ m_ptr, uint32_t S, const uint4* __restrict__ pr_cells,
-    const float* __restrict__ pr_x, uint32_t K, uint32_t K1,
+    const uint32_t* __restrict__ ids, const uint32_t* __restrict__ m_ptr, uint32_t S,
+    const uint4* __restrict__ pr_cells, const float* __restrict__ pr_x, uint32_t K,
     const unsigned long long* __restrict__ tab, uint32_t g0, uint32_t g1,
-    const uint32_t* __restrict__ gate_m, const uint32_t* __restrict__ amin, int again,
+    const uint32_t* __restrict__ amin, int again,
     uint8_t* __restrict__ status, uint32_t* __restrict__ blk) {
   constexpr int NW = (D + 3) / 4;
   extern __shared__ uint4 s_tab4[];  // [groups][D][128] eight-byte masks
   const unsigned long long* s_tab = reinterpret_cast<const unsigned long long*>(s_tab4);
   const uint32_t m = *m_ptr;
-  // few entries left: this pass would not pay
-  const uint32_t groups = gate_m && 4ull * m < *gate_m ? 0u : g1 - g0;
+  const uint32_t groups = g1 - g0;
   if ((uint64_t)blockIdx.x * 1024 >= m) return;
   const uint4* src = reinterpret_cast<const uint4*>(tab + (uint64_t)g0 * (D * 128));
   for (uint32_t t = threadIdx.x; t < groups * (D * 64); t += 1024) s_tab4[t] = src[t];
@@ -237,42 +233,44 @@ __global__ void __launch_bounds__(1024) k_prefilter(
   uint32_t hS[NW];
 #pragma unroll
   for (int w = 0; w < NW; ++w) hS[w] = guard_mask(S, w);
+  const int na = __popc(S);
   for (uint64_t base = (uint64_t)blockIdx.x * 1024; base < m; base += (uint64_t)gridDim.x * 1024) {
     const uint32_t i = (uint32_t)base + threadIdx.x;
     bool keep = false;
     if (i < m) {
-      const uint32_t at = sub ? sub[i] : i;
-      if (again && status[at]) {
+      if (again && status[i]) {
         keep = false;
       } else {
-        const uint32_t id = ids ? ids[at] : at;
+        const uint32_t id = ids ? ids[i] : i;
         const uint4 c4 = cells[id];
         uint32_t found = 0;  // the status a pruner gives
-        bool at_min = false, min_known = false;
-        for (uint32_t g = 0; g < groups && !found; ++g) {
+        int n_min = -1;  // attributes of S on which the point holds the minimum (-1: not counted)
+        for (uint32_t g = 0; g < groups && !found && n_min != na; ++g) {
           const unsigned long long* T = s_tab + g * (D * 128);
           unsigned long long b = ~0ull;
 #pragma unroll
           for (int k = 0; k < D; ++k)
             b &= T[128 * k + ((word_of(c4, k >> 2) >> (8 * (k & 3))) & 0x7fu)];
           for (; b && !found; b &= b - 1) {
-            const uint32_t t = group_begin(g0 + g, K1) + __ffsll(b) - 1;
+            const uint32_t t = (g0 + g) * kGroupPruners + __ffsll(b) - 1;
             const uint4 q = pr_cells[t];
             uint32_t Z = 0;  // attributes of S with equal cells
 #pragma unroll
             for (int w = 0; w < NW; ++w)
               Z |= pack_guards(ge_bytes(word_of(q, w) | kGuard, word_of(c4, w)) & hS[w]) << (4 * w);
-            if (!min_known) {  // a minimum's cell is 0, and so is the pruner's there
+            if (n_min < 0) {  // a minimum's cell is 0, and so is the pruner's there
               uint32_t zero = 0;
 #pragma unroll
               for (int w = 0; w < NW; ++w)
                 zero |= pack_guards((kGuard - word_of(c4, w)) & hS[w]) << (4 * w);
-              for (; zero && !at_min; zero &= zero - 1) {
+              n_min = 0;
+              for (; zero; zero &= zero - 1) {
                 const int k = __ffs(zero) - 1;
-                at_min = ordered_u32(x[(uint64_t)k * n_pad + id]) == amin[k];
+                n_min += ordered_u32(x[(uint64_t)k * n_pad + id]) == amin[k];
               }
-              min_known = true;
+              if (n_min == na) break;  // nothing dominates it
             }
+            const bool at_min = n_min > 0;
             bool le = true, all_lt = true, any_lt = Z != S;
             for (; Z && le && (all_lt || at_min); Z &= Z - 1) {
               const int k = __ffs(Z) - 1;
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(1024) k_prefilter(
           }
         }
         keep = !found;
-        status[at] = (uint8_t)found;
+        status[i] = (uint8_t)found;
       }
     }
     const int kept = __syncthreads_count(keep);
@@ -294,51 +292,32 @@ __global__ void __launch_bounds__(1024) k_prefilter(
 }
 
 size_t prefilter_table_bytes(int d, uint32_t K) {
-  const uint32_t K1 = std::max<uint32_t>(1, K / 16);
-  return (size_t)pruner_groups(K, K1) * d * 128 * sizeof(unsigned long long);
+  return (size_t)pruner_groups(K) * d * 128 * sizeof(unsigned long long);
 }
 
 // Groups of one launch: their tables have to fit the shared memory.
 constexpr size_t kMaxTableSmem = 200 * 1024;
 
 template <int D>
-static int launch_prefilter_d(cudaStream_t s, int num_sms, const PrefilterArgs& a,
-                              const uint32_t* sub, const uint32_t* m_ptr, uint32_t g0, uint32_t g1,
-                              const uint32_t* gate_m, uint32_t* blk) {
+static int launch_prefilter_d(cudaStream_t s, int num_sms, const PrefilterArgs& a) {
   constexpr size_t kGroupBytes = D * 128 * sizeof(unsigned long long);
   constexpr uint32_t kMost = (uint32_t)(kMaxTableSmem / kGroupBytes);
-  const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);
+  const uint32_t G = pruner_groups(a.K);
   SKC_CUDA(cudaFuncSetAttribute(k_prefilter<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(kMost * kGroupBytes)));
   const uint64_t want = (a.m_max + 1023) / 1024;
-  for (uint32_t g = g0; g < g1; g += kMost) {
-    const uint32_t e = std::min(g1, g + kMost);
+  for (uint32_t g = 0; g < G; g += kMost) {
+    const uint32_t e = std::min(G, g + kMost);
     const size_t smem = (e - g) * kGroupBytes;
     const uint64_t per_sm = smem > 110 * 1024 ? 1 : 2;
     const unsigned grid =
         (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)num_sms * per_sm));
-    k_prefilter<D><<<grid, 1024, smem, s>>>(a.cells, a.x, a.n_pad, sub, a.ids, m_ptr, a.S,
-                                            a.ps.pr_cells, a.ps.pr_x, a.K, K1, a.ps.tab, g, e,
-                                            gate_m, a.amin, g > g0, a.status,
-                                            e == g1 ? blk : nullptr);
+    k_prefilter<D><<<grid, 1024, smem, s>>>(a.cells, a.x, a.n_pad, a.ids, a.m_ptr, a.S,
+                                            a.ps.pr_cells, a.ps.pr_x, a.K, a.ps.tab, g, e, a.amin,
+                                            g > 0, a.status, e == G ? a.ps.blk : nullptr);
     SKC_LAUNCH_CHECK();
   }
   return SKC_OK;
-}
-
-static int launch_prefilter_pass(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
-                                 const uint32_t* sub, const uint32_t* m_ptr, uint32_t g0,
-                                 uint32_t g1, const uint32_t* gate_m, uint32_t* blk) {
-  switch (d) {
-#define SKC_PF_CASE(D) \
-  case D: return launch_prefilter_d<D>(s, num_sms, a, sub, m_ptr, g0, g1, gate_m, blk);
-    SKC_PF_CASE(2) SKC_PF_CASE(3) SKC_PF_CASE(4) SKC_PF_CASE(5) SKC_PF_CASE(6)
-    SKC_PF_CASE(7) SKC_PF_CASE(8) SKC_PF_CASE(9) SKC_PF_CASE(10) SKC_PF_CASE(11)
-    SKC_PF_CASE(12) SKC_PF_CASE(13) SKC_PF_CASE(14) SKC_PF_CASE(15) SKC_PF_CASE(16)
-#undef SKC_PF_CASE
-    default:
-      return set_error(SKC_ERR_INVALID, "unsupported d=%d", d);
-  }
 }
 
 int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
@@ -358,26 +337,23 @@ int launch_prefilter(cudaStream_t s, int d, int num_sms, const PrefilterArgs& a,
   k_pruner_collect<<<grid, 256, 0, s>>>(a.cells, a.ids, a.m_ptr, a.S, d, a.K, p.hist, sel,
                                         p.pr_ids, p.pr_key);
   SKC_LAUNCH_CHECK();
-  const uint32_t K1 = std::max<uint32_t>(1, a.K / 16);  // pruners of the first pass
   k_pruner_order<<<1, 1024, 0, s>>>(p.pr_ids, p.pr_key, sel, a.cells, a.x, a.n_pad, d, a.K,
-                                    p.pr_cells, p.pr_x, p.blk0, p.blk1,
+                                    p.pr_cells, p.pr_x, p.blk,
                                     (uint32_t)((a.m_max + 1023) / 1024));
   SKC_LAUNCH_CHECK();
-  const uint32_t G = pruner_groups(a.K, K1);
-  k_pruner_tables<<<dim3(G, d), 128, 0, s>>>(p.pr_cells, sel, a.S, K1, p.tab);
+  k_pruner_tables<<<dim3(pruner_groups(a.K), d), 128, 0, s>>>(p.pr_cells, sel, a.S, p.tab);
   SKC_LAUNCH_CHECK();
-  // Two passes: the strongest K1 = K / 16 pruners on every entry, then, only
-  // when at least a quarter of the entries survived, the other pruners on
-  // the survivors. Tie-heavy and correlated data lose nearly everything to
-  // the first pass (more pruners only cost there: survivors that nothing can
-  // strictly dominate walk every pruner); anticorrelated data keeps most
-  // points, and the second pass removes a good part of them.
-  SKC_TRY(launch_prefilter_pass(s, d, num_sms, a, nullptr, a.m_ptr, 0, 1, nullptr, p.blk0));
-  if (G == 1)
-    return launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, out, out_count);
-  SKC_TRY(launch_status_keep(s, a.status, nullptr, a.m_ptr, a.m_max, p.blk0, p.mid, p.mid_count));
-  SKC_TRY(launch_prefilter_pass(s, d, num_sms, a, p.mid, p.mid_count, 1, G, a.m_ptr, p.blk1));
-  return launch_status_keep(s, a.status, p.mid, p.mid_count, a.m_max, p.blk1, out, out_count);
+  switch (d) {
+#define SKC_PF_CASE(D) \
+  case D: SKC_TRY(launch_prefilter_d<D>(s, num_sms, a)); break;
+    SKC_PF_CASE(2) SKC_PF_CASE(3) SKC_PF_CASE(4) SKC_PF_CASE(5) SKC_PF_CASE(6)
+    SKC_PF_CASE(7) SKC_PF_CASE(8) SKC_PF_CASE(9) SKC_PF_CASE(10) SKC_PF_CASE(11)
+    SKC_PF_CASE(12) SKC_PF_CASE(13) SKC_PF_CASE(14) SKC_PF_CASE(15) SKC_PF_CASE(16)
+#undef SKC_PF_CASE
+    default:
+      return set_error(SKC_ERR_INVALID, "unsupported d=%d", d);
+  }
+  return launch_status_keep(s, a.status, a.m_ptr, a.m_max, p.blk, out, out_count);
 }
 
 }  // namespace skc

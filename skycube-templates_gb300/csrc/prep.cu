@@ -398,8 +398,7 @@ struct StatusOut {
 };
 
 __global__ void __launch_bounds__(1024) k_status_write(
-    const uint8_t* __restrict__ st, const uint32_t* __restrict__ sub,
-    const uint32_t* __restrict__ ids,
+    const uint8_t* __restrict__ st, const uint32_t* __restrict__ ids,
     const uint32_t* __restrict__ m_ptr, const uint32_t* __restrict__ c0,
     const uint32_t* __restrict__ c1, int scanned, StatusOut o) {
   __shared__ uint32_t s0[32], s1[32], p0[32], p1[32];
@@ -416,8 +415,7 @@ __global__ void __launch_bounds__(1024) k_status_write(
   if (b >= nblk) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t i = b * 1024 + threadIdx.x;
-  const uint32_t at = i < m ? (sub ? sub[i] : i) : 0u;
-  const uint8_t v = i < m ? st[at] : 2;
+  const uint8_t v = i < m ? st[i] : 2;
   const uint32_t b0 = __ballot_sync(0xffffffffu, v == 0);
   const uint32_t b1 = __ballot_sync(0xffffffffu, v == 1);
   uint32_t f0 = 0, f1 = 0;  // entries of the blocks before this one
@@ -462,7 +460,7 @@ __global__ void __launch_bounds__(1024) k_status_write(
   __syncthreads();
   const uint32_t lt = (1u << lane) - 1u;
   if (v > 1) return;
-  const uint32_t id = ids ? ids[at] : at;
+  const uint32_t id = ids ? ids[i] : i;
   const uint32_t k0 = s0[wid] + __popc(b0 & lt), k1 = s1[wid] + __popc(b1 & lt);
   if (v == 0) o.out0[k0] = id;
   else if (o.out1) o.out1[k1] = id;
@@ -714,8 +712,7 @@ int launch_pivots_cells(cudaStream_t s, const float* x, uint64_t n_pad, int d,
 
 // Statuses whose block counts c0 / c1 are already there (c1 unused without
 // out1) into the outputs.
-static int status_write(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
-                        const uint32_t* ids,
+static int status_write(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
                         const uint32_t* m_ptr, uint64_t m_max, uint32_t* c0, uint32_t* c1,
                         const StatusOut& o) {
   const uint32_t g = (uint32_t)std::max<uint64_t>(1, (m_max + 1023) / 1024);
@@ -728,7 +725,7 @@ static int status_write(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
       SKC_LAUNCH_CHECK();
     }
   }
-  k_status_write<<<g, 1024, 0, s>>>(st, sub, ids, m_ptr, c0, c1, scan, o);
+  k_status_write<<<g, 1024, 0, s>>>(st, ids, m_ptr, c0, c1, scan, o);
   SKC_LAUNCH_CHECK();
   return SKC_OK;
 }
@@ -740,14 +737,13 @@ int launch_status_split(cudaStream_t s, const uint8_t* st, const uint32_t* ids,
   const uint32_t g = (uint32_t)std::max<uint64_t>(1, (m_max + 1023) / 1024);
   k_status_count<<<g, 1024, 0, s>>>(st, m_ptr, blk0, blk1);
   SKC_LAUNCH_CHECK();
-  return status_write(s, st, nullptr, ids, m_ptr, m_max, blk0, blk1,
+  return status_write(s, st, ids, m_ptr, m_max, blk0, blk1,
                       StatusOut{sky, ext, both, both_st, pos0, n});
 }
 
-int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* sub,
-                       const uint32_t* m_ptr, uint64_t m_max, uint32_t* blk0, uint32_t* out,
-                       uint32_t* n) {
-  return status_write(s, st, sub, nullptr, m_ptr, m_max, blk0, nullptr,
+int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* m_ptr, uint64_t m_max,
+                       uint32_t* blk0, uint32_t* out, uint32_t* n) {
+  return status_write(s, st, nullptr, m_ptr, m_max, blk0, nullptr,
                       StatusOut{out, nullptr, nullptr, nullptr, nullptr, n});
 }
 

@@ -70,3 +70,38 @@ def test_levels_of_the_per_cuboid_form(gpu_ctx, kind, n, d, max_d):
             assert np.array_equal(a.extended(S), b.extended(S)), S
     for o in (a, b, ds):
         o.close()
+
+
+@pytest.mark.parametrize("open_points", [1, 33, 2049, 4095, 4096, 4097, 6143, 6144, 6145])
+@pytest.mark.parametrize("d", [3, 8, 13])
+def test_few_points_left_by_the_prefilter(gpu_ctx, open_points, d):
+    """k_small_status and the emptied pipeline, around the longest list it
+    takes: `open_points` points of a plane, a tenth of them repeated with one
+    attribute raised (dominated, not strictly), and 40,000 points that all of
+    them strictly dominate; then with three equal points below everything."""
+    rng = np.random.default_rng(open_points + d)
+    e = rng.exponential(size=(open_points, d))
+    a = (e / e.sum(axis=1, keepdims=True)).astype(np.float32)
+    t = open_points // 10
+    if t:
+        a[-t:] = a[:t]
+        a[-t:, rng.integers(0, d, t)] += np.float32(0.125)
+    x = np.concatenate([a, (2 + rng.random((40000, d))).astype(np.float32)])
+    at = rng.permutation(len(x))
+    x = np.ascontiguousarray(x[at])
+    back = np.flatnonzero(at < open_points)  # where the plane's points went
+    sky, ext = brute(x[back])
+    sky, ext = back[sky], back[ext]
+    ds = sk.Dataset(gpu_ctx, x)
+    full = (1 << d) - 1
+    for pq in (0, 64, 512):
+        r = sk.skycube(gpu_ctx, ds, subspace=full, pq_size=pq)
+        assert np.array_equal(r.cuboid(full), sky) and np.array_equal(r.extended(full), ext), pq
+        r.close()
+    ds.close()
+    x[7] = x[4099] = x[30000] = -1.0
+    ds = sk.Dataset(gpu_ctx, x)
+    r = sk.skycube(gpu_ctx, ds, subspace=full)
+    assert np.array_equal(r.cuboid(full), [7, 4099, 30000]) and len(r.extended(full)) == 0
+    r.close()
+    ds.close()
