@@ -1006,10 +1006,14 @@ int bitmap_tie_slab_words(int d, int num_sms, uint64_t* words) {
 // bits, 12.6 ms; 1M x 10 0.66 ms; now 5.7 and 0.33.)
 //
 // Rows per tile: as many as 2,048, fewer while the write pass would have
-// under about four warps per scheduler.
+// under about four warps per scheduler, but 64 at least (a warp walks its
+// tile's rows 32 at a time). Compaction with at least 256 / 128 / 64 / 32 rows,
+// us on one GB300: 250k x 5 uniform (2,000 candidates) 37 / 27 / 22 / 20,
+// 234k x 6 33 / 25 / 22 / 25, 200k x 9 57 / 55 / 49 / 53, ties 581k x 10 57 / 57
+// / 56 / 58.
 static uint32_t compact_tile_rows(uint64_t m_max, uint32_t W) {
   uint32_t r = 2048;
-  while (r > 256 && ((m_max + r - 1) / r) * W < 152 * 16) r >>= 1;
+  while (r > 64 && ((m_max + r - 1) / r) * W < 152 * 16) r >>= 1;
   return r;
 }
 

@@ -1,6 +1,6 @@
 """The compaction of bitmaps into per-cuboid id lists (mdmc.cu, k_bits_count
 and k_bits_write) against the per-point bitmaps themselves: candidate counts
-around the edges of its 32-row groups, staged 128-row steps and 256-row tiles,
+around the edges of its 32-row groups, its tiles (64 rows and more) and staged 128-row steps,
 one word per row up to 1,024, sparse and dense columns, skylines and extended
 skylines, and caps (words with no wanted column)."""
 import numpy as np
