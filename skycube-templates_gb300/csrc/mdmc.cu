@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : (D <= 15 ? 5 :
     // half t / 4) or, with `quarters`, quarters (c <= 4: lane t on q t % 8
     // of quarter t / 8); lanes past the last one repeat it (a q tested twice
     // changes nothing). The q arrays are padded to whole blocks with
-    // entries that add nothing (k_pad_q). One call site of test_q: a second
+    // entries that add nothing (k_q_scatter). One call site of test_q: a second
     // one spilled the capped 15-attribute kernel.
     auto walk = [&](bool quarters, uint32_t c) {
       SKC_T0(t_walk);
