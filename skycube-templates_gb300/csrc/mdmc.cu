@@ -115,9 +115,13 @@ struct BitState {
   static constexpr uint32_t AW = NSUB / 2;  // tie-map words (2 entries each)
   static constexpr bool A_SMEM = (D <= 11);  // tie map in shared memory
   // Above, the map lives in a global slab and is closed chunk by chunk in
-  // registers (tie_global_output), and the first LIST_WORDS tie pairs of a
-  // candidate are kept as a list (E | L << 16) and applied directly when no
-  // more come; the global map is used only when a candidate has more. At 12
+  // registers (tie_global_output), and a candidate's maximal tie pairs, up to
+  // LIST_WORDS, are kept as a list (E | L << 16) and applied directly; the
+  // global map is used only when a candidate has more. Few do: on correlated
+  // data clipped at 0 (500k x 16, 1,328 q's) a candidate has 600 useful pairs
+  // but 2 maximal ones, 24 at most. Bitmap kernel with all pairs listed /
+  // maximal ones: there 4.65 / 1.59 ms, 200k x 14 ties -m 5 0.42 / 0.15, 100k
+  // x 16 ties -m 6 1.12 / 0.54, correlated_q 566k x 15 0.16 / 0.10. At 12
   // attributes the map would take 8 KB of shared memory per warp, 24 warps
   // per SM: 400k x 12 -m 4 9.4 ms with it, 7.7 without.
   static constexpr uint32_t LIST_WORDS = A_SMEM ? 0 : 32;
@@ -543,27 +547,41 @@ __global__ void __launch_bounds__(256, (D <= 10 ? (CAP ? 6 : 8) : (D <= 15 ? 5 :
           }
           if (tie_lane) atomicOr(&A[le >> 1], lt << (16 * (le & 1)));
         } else {
+          // The list keeps maximal pairs only: one whose LE and LT lie inside
+          // another's adds no subspace to that one's.
           uint32_t* tlist = wsm + W;
-          const uint32_t nt = __popc(tb);
-          if (tmode != 2 && tcount + nt <= BS::LIST_WORDS) {
-            if (tie_lane) tlist[tcount + __popc(tb & ((1u << lane) - 1u))] = le | (lt << 16);
-            tcount += nt;
-            tmode = 1;
-            __syncwarp();
-          } else {
-            if (tmode != 2) {
-              // Too many pairs: move to the global map (zeroed, then
-              // the listed pairs OR-ed in).
-              for (uint32_t w = lane; w < AW; w += 32) A[w] = 0;
-              __syncwarp();
-              if ((uint32_t)lane < tcount) {
-                const uint32_t e = tlist[lane];
-                atomicOr(&A[(e & 0xffffu) >> 1], (e >> 16) << (16 * (e & 1u)));
+          const uint32_t pair = le | (lt << 16);
+          if (tmode != 2) {
+            bool need = tie_lane && lt;
+            for (uint32_t j = 0; j < tcount; ++j) need = need && (pair & ~tlist[j]);
+            uint32_t add = __ballot_sync(kFull, need);
+            if (add) {
+              uint32_t mine = (uint32_t)lane < tcount ? tlist[lane] : 0u;  // 0: free
+              for (; add; add &= add - 1) {
+                const uint32_t v = __shfl_sync(kFull, pair, __ffs(add) - 1);
+                if (__any_sync(kFull, (v & ~mine) == 0u)) continue;  // v is not 0
+                if ((mine & ~v) == 0u) mine = 0;
+                const uint32_t free = __ballot_sync(kFull, mine == 0u);
+                if (!free) break;
+                if (lane == __ffs(free) - 1) mine = v;
               }
-              tmode = 2;
+              if (add) {
+                // More than 32: move to the global map (zeroed, then the
+                // listed pairs OR-ed in).
+                for (uint32_t w = lane; w < AW; w += 32) A[w] = 0;
+                __syncwarp();
+                atomicOr(&A[(mine & 0xffffu) >> 1], (mine >> 16) << (16 * (mine & 1u)));
+                tmode = 2;
+              } else {
+                const uint32_t held = __ballot_sync(kFull, mine != 0u);
+                if (mine) tlist[__popc(held & ((1u << lane) - 1u))] = mine;
+                tcount = __popc(held);
+                tmode = 1;
+                __syncwarp();
+              }
             }
-            if (tie_lane) atomicOr(&A[le >> 1], lt << (16 * (le & 1)));
           }
+          if (tmode == 2 && tie_lane) atomicOr(&A[le >> 1], lt << (16 * (le & 1)));
         }
       }
       // Strict updates: down(LT) into STRICT, one pair at a time.

@@ -4,9 +4,12 @@ full space, so every point is a q and ties with most others), in shared
 memory (11 attributes), as a list and in the global slab, closed in registers
 (12 and more); per-point bitmaps against their definition, and capped runs
 (the closure over 1 to 64 rows) against the uncapped bits."""
+import itertools
+
 import numpy as np
 import pytest
 
+import oracle
 import skycube_gb300 as sk
 
 pytestmark = pytest.mark.gpu
@@ -53,5 +56,44 @@ def test_bitmaps_with_many_ties(gpu_ctx, d, n, levels):
             else:
                 assert len(ids) == 0
         a.close()
+    r.close()
+    ds.close()
+
+
+def tie_pairs(d, k, covered, seed):
+    """A point p (index 0) that ties with k points on 6 attributes each, below
+    it on one of those and above it on the others: k maximal (LE, LT) pairs,
+    and `covered` points more whose 5 or 4 attributes lie inside one of them."""
+    rng = np.random.default_rng(seed)
+    sets = [c for c in itertools.islice(itertools.combinations(range(d), 6), 4000)]
+    rows = [np.full(d, 5.0)]
+    for i in rng.permutation(len(sets))[:k]:
+        q = np.full(d, 6.0)
+        q[list(sets[i])] = 5.0
+        q[sets[i][rng.integers(6)]] = 4.0
+        rows.append(q)
+    for j in range(covered):
+        q = rows[1 + j % k].copy()
+        same = np.flatnonzero(q == 5.0)
+        q[rng.choice(same, 1 + j % 2, replace=False)] = 6.5 + j
+        rows.append(q)
+    return np.array(rows, np.float32)
+
+
+@pytest.mark.parametrize("d,max_d", [(12, 0), (13, 6), (16, 4)])
+@pytest.mark.parametrize("k,covered", [(1, 40), (31, 30), (32, 0), (32, 90), (33, 0), (300, 50)])
+def test_lists_of_maximal_pairs(gpu_ctx, d, max_d, k, covered):
+    """A candidate's tie pairs above 11 attributes: maximal ones in a list of
+    32, the global map from the 33rd on, pairs inside another dropped in
+    whichever order they come; against the oracle."""
+    x = tie_pairs(d, k, covered, 7 * k + d)
+    order = np.random.default_rng(k).permutation(len(x))
+    x = np.ascontiguousarray(x[order])
+    sky, ext = oracle.stsc(x, max_d or d)
+    ds = sk.Dataset(gpu_ctx, x)
+    r = sk.skycube(gpu_ctx, ds, max_d=max_d, want_extended=True, form="bitmaps")
+    for c in sky:
+        assert np.array_equal(r.cuboid(c), sky[c]), c
+        assert np.array_equal(r.extended(c), ext[c]), c
     r.close()
     ds.close()
