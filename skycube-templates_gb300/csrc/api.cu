@@ -313,7 +313,7 @@ constexpr int kDefaultChunk = 1;
 
 // Device-side result of the full-space step.
 struct FullSpace {
-  uint4* cells = nullptr;    // by point id (depth of the call)
+  uint4* cells = nullptr;    // by point id, kMaxDepth deep at any depth of the call
   uint32_t* amin = nullptr;  // per attribute: ordered-uint minimum over all points
   uint32_t* sky = nullptr;   // full-space skyline ids, ascending
   uint32_t* ext = nullptr;   // full-space extended skyline ids, ascending
@@ -385,7 +385,6 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   cudaStream_t s = E.stream;
   const uint64_t n = ds->n;
   const int d = ds->d;
-  const int depth = P.depth;
   const uint32_t full = (1u << d) - 1;
   uint32_t* d_n;  // n, then the short-list kernel's tickets
   SKC_TRY(A.alloc(&d_n, 3));
@@ -410,13 +409,17 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
     }
     return full_space_counts(E, n, F, T);
   }
+  // The finest grid at any depth of the call: the prefilter and the skyline
+  // kernel read floats by point id where cells tie, on two cells per attribute
+  // nearly everywhere (query on 5 of 10 attributes, 500k uniform points: 16 ms
+  // at depth 1, 3.2 at 2, 0.7 so).
   float* pivots;
   SKC_TRY(A.alloc(&pivots, (uint64_t)kMaxDims * kMaxPivots));
   SKC_TRY(A.alloc(&F.cells, n));
   SKC_TRY(A.alloc(&F.amin, kMaxDims));
   PrefilterScratch pf{};
   if (P.pq_size > 0) SKC_TRY(A.alloc(&pf.hist, kSumBins + 8));
-  SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, nullptr, d_n, n, depth, pivots, F.cells,
+  SKC_TRY(launch_pivots_cells(s, ds->x, ds->n_pad, d, nullptr, d_n, n, kMaxDepth, pivots, F.cells,
                               F.amin, pf.hist));
   T.mark("full: pivots+cells");
 
@@ -445,7 +448,7 @@ static int run_full_space(Exec& E, skc_dataset* ds, const RunParams& P, Arena& A
   SKC_TRY(part_scratch(A, n, &ps));
   PartitionSkylineArgs pa{open, nullptr, F.cells, ds->x, ds->n_pad, m_open, n, full, status,
                           F.amin};
-  SKC_TRY(launch_partition_skyline(s, ctx->num_sms, d, depth, LT, pa, ps));
+  SKC_TRY(launch_partition_skyline(s, ctx->num_sms, d, LT, pa, ps));
   T.mark("full: skyline kernel");
 
   const uint64_t nblk = (n + 1023) / 1024 + 2;
@@ -692,15 +695,15 @@ static int cuboid_scratch(Arena& A, uint64_t mmax, CuboidScratch* cs) {
 // Median-partition pipeline of cuboid c over an ascending candidate list of
 // mc entries (m_ptr holds mc): skyline and extended skyline ids, ascending,
 // and their counts on the device.
-static int cuboid_pipeline(Exec& E, skc_dataset* ds, FullSpace& F, int depth, CuboidScratch& cs,
-                           uint32_t c, const uint32_t* cand, const uint32_t* m_ptr, uint64_t mc,
+static int cuboid_pipeline(Exec& E, skc_dataset* ds, FullSpace& F, CuboidScratch& cs, uint32_t c,
+                           const uint32_t* cand, const uint32_t* m_ptr, uint64_t mc,
                            uint32_t* osky, uint32_t* oext, uint32_t* cnt) {
   cudaStream_t s = E.stream;
   LevelTables LT;
   SKC_TRY(level_tables(E.ctx, partition_dims(c), &LT));
   PartitionSkylineArgs pa{nullptr, cand, F.cells, ds->x, ds->n_pad, m_ptr, mc, c, cs.status,
                           F.amin};
-  SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, depth, LT, pa, cs.ps));
+  SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, ds->d, LT, pa, cs.ps));
   return launch_status_split(s, cs.status, cand, m_ptr, mc, cs.blk0, cs.blk1, osky, oext, cnt);
 }
 
@@ -708,8 +711,8 @@ static int cuboid_pipeline(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Cu
 // of mc entries (both outputs ascending), with the short-list kernel or the
 // median-partition pipeline; cs.d_m holds mc and 0. One host round trip for
 // the counts.
-static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Arena& A,
-                        CuboidScratch& cs, uint32_t c, const uint32_t* cand, uint64_t mc,
+static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, Arena& A, CuboidScratch& cs,
+                        uint32_t c, const uint32_t* cand, uint64_t mc,
                         uint32_t** osky, uint32_t** oext, uint64_t* nsky, uint64_t* next) {
   cudaStream_t s = E.stream;
   SKC_TRY(A.alloc(osky, mc));
@@ -718,7 +721,7 @@ static int cuboid_lists(Exec& E, skc_dataset* ds, FullSpace& F, int depth, Arena
     SKC_TRY(launch_small_skyline(s, ds->x, ds->n_pad, ds->d, cand, cs.d_m, mc, c, cs.masks,
                                  cs.d_m + 1, {*osky, *oext, nullptr, nullptr, nullptr, cs.cnt}));
   } else {
-    SKC_TRY(cuboid_pipeline(E, ds, F, depth, cs, c, cand, cs.d_m, mc, *osky, *oext, cs.cnt));
+    SKC_TRY(cuboid_pipeline(E, ds, F, cs, c, cand, cs.d_m, mc, *osky, *oext, cs.cnt));
   }
   SKC_TRY(copy_d2h(cs.h_cnt, cs.cnt, 2 * sizeof(uint32_t), s));
   *nsky = cs.h_cnt[0];
@@ -796,8 +799,7 @@ static uint32_t min_parent(uint32_t c, int d, const std::vector<uint64_t>& nsky,
 // and those with a short candidate list share a launch: the 62 cuboids below
 // the full space of 100k x 6 uniform took 1.76 ms with a launch and a read
 // each, 0.20 so.
-static int run_sdsc_plain(Exec& E, skc_dataset* ds, int max_d,
-                          int depth_of_call, Arena& A, FullSpace& F,
+static int run_sdsc_plain(Exec& E, skc_dataset* ds, int max_d, Arena& A, FullSpace& F,
                           skc_result* R, Tracer& T) {
   cudaStream_t s = E.stream;
   const int d = ds->d;
@@ -859,7 +861,7 @@ static int run_sdsc_plain(Exec& E, skc_dataset* ds, int max_d,
         }
         SKC_TRY(A.alloc(&sky[c], mc));
         SKC_TRY(A.alloc(&ext[c], mc));
-        SKC_TRY(cuboid_pipeline(E, ds, F, depth_of_call, cs, c, cand, m_ptr, mc, sky[c], ext[c], cnt));
+        SKC_TRY(cuboid_pipeline(E, ds, F, cs, c, cand, m_ptr, mc, sky[c], ext[c], cnt));
       }
     }
     SKC_TRY(flush());
@@ -1166,7 +1168,7 @@ static int run_lattice(Exec& E, std::vector<LatticeJob>& jobs, Arena& A, Tracer&
       }
       ++fallbacks;
       SKC_TRY(launch_set_u32(s, cs.d_m, F.h_counts[2], 1));
-      SKC_TRY(cuboid_lists(E, ds, F, J.depth, A, cs, c, F.cand, F.h_counts[2], &sky[c], &ext[c],
+      SKC_TRY(cuboid_lists(E, ds, F, A, cs, c, F.cand, F.h_counts[2], &sky[c], &ext[c],
                            &nsky[c], &next[c]));
     }
     if (fallbacks) T.mark("lattice fallbacks");
@@ -1633,7 +1635,6 @@ static int check_options(skc_dataset* ds, const skc_options* opt, skc_options* o
 // so S is computed over those candidates.
 static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunParams& P,
                              Arena& A, FullSpace& F, skc_result* R, Tracer& T) {
-  const int depth = P.depth;
   cudaStream_t s = E.stream;
   const int d = ds->d;
   const uint32_t nsub = 1u << d, full = nsub - 1;
@@ -1681,7 +1682,7 @@ static int run_single_cuboid(Exec& E, skc_dataset* ds, uint32_t S, const RunPara
       m_open = d_ns;
     }
     PartitionSkylineArgs pa{open, F.cand, F.cells, ds->x, ds->n_pad, m_open, m, S, status, F.amin};
-    SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, d, depth, LT, pa, ps));
+    SKC_TRY(launch_partition_skyline(s, E.ctx->num_sms, d, LT, pa, ps));
     SKC_TRY(launch_status_split(s, status, F.cand, m_ptr, m, blk0, blk1, sky, ext, cnt));
   }
   uint64_t* off[2];
@@ -1742,7 +1743,7 @@ static int skycube_exec(Exec& E, skc_dataset* ds, const skc_options* opt, skc_re
         st = run_single_cuboid(E, ds, o.subspace, P, A, F, R, T);
       } else if (o.algo == SKC_ALGO_SDSC && o.mode == SKC_MODE_PLAIN) {
         R->form = SKC_FORM_CUBOIDS;
-        st = run_sdsc_plain(E, ds, max_d, depth, A, F, R, T);
+        st = run_sdsc_plain(E, ds, max_d, A, F, R, T);
       } else if (use_levels(E, ds, o, max_d, F)) {
         R->form = SKC_FORM_LEVELS;
         st = run_levels(E, ds, o, max_d, depth, A, F, R, T);
@@ -1822,7 +1823,7 @@ static int skycube_exec_batch(Exec& E, const std::vector<skc_dataset*>& dss,
         st = run_single_cuboid(E, ds, o[i].subspace, P[i], A, F[i], R[i], T);
       } else if (o[i].algo == SKC_ALGO_SDSC && o[i].mode == SKC_MODE_PLAIN) {
         R[i]->form = SKC_FORM_CUBOIDS;
-        st = run_sdsc_plain(E, ds, max_d[i], P[i].depth, A, F[i], R[i], T);
+        st = run_sdsc_plain(E, ds, max_d[i], A, F[i], R[i], T);
       } else if (use_levels(E, ds, o[i], max_d[i], F[i])) {
         LatticeJob J;
         J.ds = ds;

@@ -113,7 +113,7 @@ struct PartitionSkylineArgs {
   const uint32_t* sub;  // the list's positions to settle, ascending (the prefilter's
                         // survivors, whose statuses are 0 already); nullptr: all
   const uint32_t* ids;  // list position -> point id (nullptr: identity)
-  const uint4* cells;   // point id -> grid cells
+  const uint4* cells;   // point id -> grid cells, kMaxDepth deep
   const float* x;
   uint64_t n_pad;
   const uint32_t* m_ptr;  // entries of `sub`, or of the list
@@ -139,9 +139,8 @@ int launch_bucket_scan(cudaStream_t s, uint32_t* counts, uint32_t len, uint32_t*
 int launch_q_scatter(cudaStream_t s, const uint32_t* keys, const uint32_t* mq_ptr, uint64_t m_max,
                      uint32_t* cursor, const uint32_t* qpos, const uint4* pcells, const float* px,
                      uint64_t pitch, int d, uint4* qcells, float* qx);
-int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth,
-                             const LevelTables& T, const PartitionSkylineArgs& a,
-                             const PartScratch& ps);
+int launch_partition_skyline(cudaStream_t s, int num_sms, int d, const LevelTables& T,
+                             const PartitionSkylineArgs& a, const PartScratch& ps);
 
 // small.cu: skyline of a list of at most kSmallList points on subspace S,
 // compaction included, in one launch. masks: [2 * kSmallList / 32], ticket: 0.

@@ -723,7 +723,7 @@ static int launch_tree(cudaStream_t s, int num_sms, const TreeArgs& a) {
   return SKC_OK;
 }
 
-int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, const LevelTables& T,
+int launch_partition_skyline(cudaStream_t s, int num_sms, int d, const LevelTables& T,
                              const PartitionSkylineArgs& args, const PartScratch& ps) {
   PartitionSkylineArgs a = args;
   if (a.sub) {  // a prefilter ran: few points may be left
@@ -732,12 +732,12 @@ int launch_partition_skyline(cudaStream_t s, int num_sms, int d, int depth, cons
   }
   const uint32_t K = 1u << T.B;
   const int na = __builtin_popcount(a.S);
-  const int sub_bits = sort_sub_bits(a.m_max, K, std::min(kMaxSubBits, na * (depth - 1)));
+  const int sub_bits = sort_sub_bits(a.m_max, K, std::min(kMaxSubBits, na * (kMaxDepth - 1)));
   const uint32_t KB = K << sub_bits;
   uint32_t* work = ps.fine + KB;  // the skyline kernel's work counter, behind the buckets
   SKC_CUDA(cudaMemsetAsync(ps.fine, 0, (KB + 1) * sizeof(uint32_t), s));
   const unsigned grid = blocks_for(a.m_max, 256, 152 * 8);
-  k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.sub, a.ids, a.m_ptr, a.S, d, T.B, depth, sub_bits,
+  k_mask_keys<<<grid, 256, 0, s>>>(a.cells, a.sub, a.ids, a.m_ptr, a.S, d, T.B, kMaxDepth, sub_bits,
                                    T.rank, ps.keys, ps.fine, a.sub ? nullptr : a.status);
   SKC_LAUNCH_CHECK();
   SKC_TRY(launch_bucket_scan(s, ps.fine, KB, ps.sums, sub_bits, ps.counts, a.m_ptr));

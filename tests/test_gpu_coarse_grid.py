@@ -1,0 +1,38 @@
+"""Coarse grids asked for by the caller (depth 1 and 2): results never depend
+on the depth, and neither does the cost of the steps whose kernels live on fine
+cells. On two cells per attribute nearly every pair of points ties, so the
+skyline kernel, which reads tied floats by point id, was 20 times as slow as on
+the default grid; it, the prefilter and the subspace skylines use that grid at
+any depth. Bounds are ratios of device times of the same call, far from 1
+before and within noise of it now."""
+import numpy as np
+import pytest
+
+import skycube_gb300 as sk
+from skycube_gb300 import datagen
+
+pytestmark = pytest.mark.gpu
+
+
+def device_ms(ctx, ds, reps=4, **opts):
+    best = float("inf")
+    for _ in range(reps):
+        r = sk.skycube(ctx, ds, **opts)
+        best = min(best, ctx.last_device_ms())
+        r.close()
+    return best
+
+
+@pytest.mark.parametrize("kind,n,d,S", [("uniform", 300000, 10, 0b1010110100),
+                                        ("anticorrelated", 200000, 8, 0b11111111)])
+@pytest.mark.parametrize("depth", [1, 2])
+def test_skyline_queries_cost_the_same(gpu_ctx, kind, n, d, S, depth):
+    ds = sk.Dataset(gpu_ctx, datagen.generate(kind, n, d, 4))
+    a = sk.skycube(gpu_ctx, ds, subspace=S)
+    b = sk.skycube(gpu_ctx, ds, subspace=S, depth=depth)
+    assert np.array_equal(a.cuboid(S), b.cuboid(S))
+    assert np.array_equal(a.extended(S), b.extended(S))
+    for o in (a, b):
+        o.close()
+    assert device_ms(gpu_ctx, ds, subspace=S, depth=depth) < 2 * device_ms(gpu_ctx, ds, subspace=S)
+    ds.close()
