@@ -80,7 +80,8 @@ typedef struct skc_options {
   int max_d;       /* only cuboids with <= max_d attributes (-m); <= 0: all */
   int depth;       /* grid depth of the bitmap kernel: 2^depth cells per
                       attribute, 1..7; 0: auto (7). The full-space and
-                      per-cuboid skylines use 7 at any depth (-d) */
+                      per-cuboid skylines and the level form use 7
+                      at any depth (-d) */
   int want_extended; /* also produce per-cuboid extended skylines */
   int want_bitmaps;  /* keep per-point bitmaps for skc_result_bitmaps */
   uint32_t subspace; /* 0: the skycube; a cuboid mask: only that cuboid's

@@ -36,3 +36,24 @@ def test_skyline_queries_cost_the_same(gpu_ctx, kind, n, d, S, depth):
         o.close()
     assert device_ms(gpu_ctx, ds, subspace=S, depth=depth) < 2 * device_ms(gpu_ctx, ds, subspace=S)
     ds.close()
+
+
+@pytest.mark.parametrize("kind,n,d,max_d", [("anticorrelated", 200000, 12, 3), ("uniform", 300000, 12, 4)])
+@pytest.mark.parametrize("depth", [1, 2])
+def test_level_form_costs_the_same(gpu_ctx, kind, n, d, max_d, depth):
+    """The level form's first-level filter drops by cells alone, so on two
+    cells per attribute it dropped next to nothing (23 ms against 1.0 at 200k x
+    12, and past the survivors' capacity at 500k x 16 the whole launch was
+    thrown away); its grid is its own."""
+    ds = sk.Dataset(gpu_ctx, datagen.generate(kind, n, d, 4))
+    a = sk.skycube(gpu_ctx, ds, max_d=max_d, form="levels")
+    b = sk.skycube(gpu_ctx, ds, max_d=max_d, form="levels", depth=depth)
+    assert a.form() == b.form() == ("levels", 0)
+    for c in range(1, 1 << d):
+        if bin(c).count("1") <= max_d:
+            assert np.array_equal(a.cuboid(c), b.cuboid(c)), c
+    for o in (a, b):
+        o.close()
+    opts = {"max_d": max_d, "form": "levels"}
+    assert device_ms(gpu_ctx, ds, depth=depth, **opts) < 2 * device_ms(gpu_ctx, ds, **opts)
+    ds.close()
