@@ -521,7 +521,8 @@ static int run_bitmaps(Exec& E, skc_dataset* ds, const skc_options& o,
   // anticorrelated, bitmap kernel 29.6 -> 23.2 ms (binary pattern order)
   // -> 21.6 ms (Gray order).
   const uint32_t K = 1u << LT.B;
-  const int sub_bits = sort_sub_bits(m, K, std::min(8, d * (depth - 1)));
+  // On two cells per attribute there are no such bits; their sum stands in.
+  const int sub_bits = sort_sub_bits(m, K, depth == 1 ? 8 : std::min(8, d * (depth - 1)));
   const uint32_t KB = K << sub_bits;
   uint32_t *keys, *buckets, *boff, *sums;  // buckets[KB]: the bitmap kernel's work counter
   SKC_TRY(A.alloc(&keys, m));

@@ -40,7 +40,10 @@ static inline unsigned blocks_for(uint64_t items, int threads, int cap) {
 // first bit most significant, so consecutive patterns differ in one bit and
 // any run of them varies in few). Consecutive points then share their
 // quartile on most attributes, which keeps the minimum-cell boxes of the
-// blocks tight. Only the partition part matters for correctness.
+// blocks tight. A grid of two cells (depth 1) has no such bits: the sub-key is
+// the cell sum over S scaled to sub_bits, strong points first (bitmap kernel,
+// 300k x 10 uniform 8.95 -> 6.97 ms, with one partition attribute 21.8 -> 17.0).
+// Only the partition part matters for correctness.
 // With `counts`, also the histogram of the keys (zeroed by the caller); with
 // `status`, zeroes the list's statuses.
 __global__ void k_mask_keys(const uint4* __restrict__ cells,
@@ -65,6 +68,11 @@ __global__ void k_mask_keys(const uint4* __restrict__ cells,
       cm |= ((cell >> sh) & 1u) << j;
       ++j;
     }
+    if (sh == 0) {
+      for (int k = 0; k < d; ++k)
+        if (S & (1u << k)) g += (word_of(c, k >> 2) >> (8 * (k & 3))) & 0x7fu;
+      g = g * ((1u << sub_bits) - 1u) / (uint32_t)__popc(S);
+    }
     int t = sub_bits;
     for (int lv = sh - 1; lv >= 0 && t > 0; --lv) {
       for (int k = 0; k < d && t > 0; ++k) {
@@ -73,7 +81,8 @@ __global__ void k_mask_keys(const uint4* __restrict__ cells,
         g |= ((word_of(c, k >> 2) >> (8 * (k & 3) + lv)) & 1u) << t;
       }
     }
-    for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;  // rank in the Gray sequence
+    if (sh > 0)
+      for (int s2 = 1; s2 < 32; s2 <<= 1) g ^= g >> s2;  // rank in the Gray sequence
     const uint32_t key = (rank[cm] << sub_bits) | g;
     keys[i] = key;
     if (counts) atomicAdd(&counts[key], 1u);
