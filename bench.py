@@ -8,7 +8,7 @@ form (MDMC bitmaps, one launch for every cuboid). The JSON line reports:
              each skycube call, L2 flushed by a 256 MiB write before each step)
   e2e        points/s through the C ABI with host buffers: pinned-host upload
              (H2D), skycube, download of every cuboid's id list (D2H)
-  plain      the per-cuboid form (one launch sequence per cuboid), for the
+  plain      the per-cuboid form (by lattice level, one host read each), for the
              batched-versus-plain ratio
   roofline   of the dominant kernel (bitmap kernel): algorithmic bytes / its
              event-timed duration against measured HBM bandwidth, plus the
@@ -431,7 +431,7 @@ def run_configs(sk, ctx, flush):
         return round(best, 3)
 
     out = {}
-    # 100k x 6 uniform: the plain form (one launch sequence per cuboid)
+    # 100k x 6 uniform: the plain form (by lattice level)
     kind, n, d, m, seed = datagen.CONFIGS["uniform-100k-6"]
     x = datagen.generate(kind, n, d, seed)
     ds = sk.Dataset(ctx, x)

@@ -61,11 +61,13 @@ extern "C" {
 #define SKC_ALGO_MDMC 0
 #define SKC_ALGO_SDSC 1
 
-/* Execution forms. PLAIN issues one launch sequence per cuboid with a host
- * round trip after each (the suite's SDSC shape; for MDMC, one bitmap launch
- * per batch of points as in tombstoning_hearting_gpu). BATCHED computes all
- * cuboids in one persistent launch with no host synchronisation until the
- * result is read. */
+/* Execution forms. PLAIN computes each cuboid by itself from its smallest
+ * parent (the suite's SDSC shape): a lattice level's short lists (up to 6,144
+ * points) share a launch, longer ones take a launch sequence each, and the
+ * host reads the counts once per level; for MDMC, one bitmap launch per batch
+ * of points with a host round trip after each, as in
+ * tombstoning_hearting_gpu. BATCHED computes all cuboids in one persistent
+ * launch; the host reads the candidate count and the ids' total. */
 #define SKC_MODE_PLAIN 0
 #define SKC_MODE_BATCHED 1
 
@@ -94,10 +96,8 @@ typedef struct skc_options {
                         > 0 that many, applied when n > 2 * pq_size as the
                         suite does (src/mdmc/MDMC.cu:251); < 0 off; 0 auto
                         (default 128 from 32,768 points, 512
-                        from 700,000). Applied in two
-                        passes: the strongest pq_size / 16 on every point,
-                        the rest on the survivors when at least a quarter
-                        of the points survive */
+                        from 700,000). Applied in one pass over the points
+                        with all pruners */
   int tile_points;   /* bitmap kernel: mean q points per median partition
                         (a power of two, 32..65536); 0 auto (256) */
   int chunk;         /* bitmap kernel: candidates a warp takes per work-queue
@@ -157,8 +157,8 @@ int skc_skycube_batch(skc_context* ctx, skc_dataset* const* datasets,
  * counterpart (the suite's algorithm is chosen by -s). */
 enum {
   SKC_FORM_BITMAPS = 1, /* per-point dominated-subspace bitmaps, one launch */
-  SKC_FORM_CUBOIDS = 2, /* per cuboid, one launch sequence each (plain SDSC) */
-  SKC_FORM_LEVELS = 3,  /* per cuboid, one lattice level per launch pair:
+  SKC_FORM_CUBOIDS = 2, /* per cuboid, by lattice level (plain SDSC) */
+  SKC_FORM_LEVELS = 3,  /* per cuboid, all of them in one persistent launch:
                            batched capped skycubes, max_d <= 4 and <= d - 2 */
   SKC_FORM_SKYLINE = 4  /* a single-subspace skyline query */
 };

@@ -4,8 +4,9 @@
 // Pipelines (all on the context's stream, device memory from the stream-
 // ordered pool):
 //
-//  full space   grid pivots + cells of all points, Manhattan-norm bucket
-//               order, skyline kernel on the full space, compaction into the
+//  full space   grid pivots + cells of all points, pruner prefilter,
+//               median-partition order, skyline kernel on the full space (one
+//               launch over all pairs for a short input), compaction into the
 //               full-space skyline, extended skyline and their union, the
 //               candidate set (ascending ids). Replaces gpu_extended_skyline
 //               + run_skyalign (src/mdmc/MDMC.cu:504-522).
@@ -20,8 +21,9 @@
 //               src/sdsc/SDSC.cu:248-335): lattice levels top-down, each
 //               cuboid's candidates are the skyline + extended skyline of its
 //               smallest computed parent (findMinParent, :366-376; full space
-//               when the first parent was skipped by max_d, :84-93); one
-//               launch sequence and one host synchronisation per cuboid.
+//               when the first parent was skipped by max_d, :84-93). A level's
+//               short lists share a launch, longer ones take a launch sequence
+//               each; one host synchronisation per level.
 //
 //  PLAIN/MDMC   the bitmap kernel launched on batches of 5,600 points with a
 //               synchronisation after each batch, the shape of
@@ -1195,7 +1197,7 @@ static int run_levels(Exec& E, skc_dataset* ds, const skc_options& o, int max_d,
 
 // The level form can replace the bitmaps for batched capped skycubes of
 // small caps, when no per-point bitmaps are wanted and no plan is being
-// recorded (the level form syncs per level). Auto takes it where it was
+// recorded (its lists are sized by counts the host reads). Auto takes it where it was
 // faster on one GB300; device ms of the whole call, level / bitmap form,
 // anticorrelated:
 //   cap 4: 16 attributes 198k candidates 5.3 / 19.4, 20k 2.25 / 2.32; 14:
@@ -1232,11 +1234,18 @@ static int auto_depth(uint64_t n, int d) {
 // Defaults of the work parameters (used when neither the options nor a
 // stored tuning set them).
 // Pruners (prefilter.cu): 128, the suite's -q default, up to 700,000 points,
-// 512 above, where each further pruner meets more dominated points. Prefilter
-// + skyline kernel with 128 / 512 pruners, ms on one GB300: 1M points:
-// anticorrelated x 10 1.39 / 1.23, x 6 0.43 / 0.35, uniform x 12 1.10 / 0.91;
-// below: ties 581k x 10 0.084 / 0.094, anticorrelated 500k x 16 1.35 / 1.38,
-// uniform 200k x 9 0.153 / 0.161, 100k x 6 0.090 / 0.102.
+// 512 above. More pruners cost every point more lookups and leave fewer open,
+// by how much depends on the data, which this rule does not see: it takes 512
+// where they save about a tenth of a millisecond on the data that gains.
+// Full-space skyline query with 128 / 512 pruners, device ms on one GB300:
+//   points               100k       300k       500k       710k       1M
+//   anticorrelated x 10  .257/.264  .533/.477  .776/.723  1.07/.97  1.54/1.35
+//   anticorrelated x 6   .194/.191  .288/.251  .346/.305  .41/.36   .53/.43
+//   uniform x 12         .252/.259  .477/.440  .703/.613  .96/.81   1.35/1.09
+//   uniform x 6          .156/.164  .205/.217  .230/.249  .245/.271 .277/.292
+//   ties x 10            .134/.143  .145/.155  .160/.171  .172/.183 .186/.195
+//   correlated x 8       .131/.141  .146/.152  .159/.165  .168/.174 .181/.188
+// and anticorrelated x 16 within 1 % from 600k to 1M.
 constexpr uint64_t kManyPrunersMinPoints = 700000;
 static int default_pruners(uint64_t n) { return n >= kManyPrunersMinPoints ? 512 : 128; }
 constexpr uint64_t kPrefilterMinPoints = 32768;  // below: launch-bound anyway
@@ -2505,7 +2514,13 @@ struct skc_server {
 // lattice form takes (max_d <= kLvMaxDims and <= d - 2, no bitmaps), forced or
 // long enough that they likely take it: their candidates are not known yet,
 // and a request that ends in the bitmap form runs alone inside the batch's
-// pass, where a slot of its own would overlap it.
+// pass, where a slot of its own would overlap it. levels_by_default takes the
+// lattice form from fewer points and at cap 4 from 12 attributes; those keep
+// slots of their own, whose full-space steps, uploads and copies overlap.
+// Eight equal anticorrelated requests through four slots, ms, apart / batched:
+// 100k x 12 cap 4 9.9 / 10.3, 200k x 14 cap 4 22.3 / 23.9, 50k x 13 cap 4 8.8 /
+// 9.4, 50k x 10 cap 3 2.7 / 3.2, 30k x 12 cap 2 1.8 / 2.5, 12k x 12 cap 2 1.6 /
+// 2.2.
 constexpr uint64_t kBatchMinPoints = 65536;
 constexpr uint64_t kBatchMinPointsMidD = 600000;  // 14 and 15 attributes, cap 4
 static bool batch_by_default(int d, int max_d, uint64_t n) {

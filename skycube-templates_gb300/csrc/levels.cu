@@ -1,5 +1,5 @@
-// Capped skycubes by lattice level: the skyline and extended skyline of
-// every cuboid of one level, all cuboids of the level in one launch pair.
+// Capped skycubes by lattice level: the skyline and extended skyline of every
+// wanted cuboid, level by level, in one persistent launch (k_lattice below).
 // This is the per-cuboid computation of the suite's SDSC (each cuboid from
 // its smallest computed parent's skyline + extended skyline, or from the
 // full space's when the parents lie above the cap: findMinParent and
@@ -8,15 +8,15 @@
 // kLvMaxDims attributes.
 //
 // Per cuboid S and candidate list L:
-//  1. k_lv_pruners: 32 pruners = the lowest cell sums over S of a
-//     1,024-entry strided sample of L. k_lv_filter: every entry of L that a
-//     pruner strictly dominates on S is dropped (exact float test on equal
-//     cells). If a dropped q dominated a kept p, the pruner that drops q
-//     would strictly dominate p, so the kept entries (survivors) decide each
-//     other's status alone.
-//  2. k_lv_sfs: the survivors, counting-sorted by cell sum over S (a
+//  1. Pruners = the lowest cell sums over S of a strided sample of L (32 of
+//     1,024 entries; on the first level 64 of 65,536, as bit tables). Every
+//     entry of L that a pruner strictly dominates on S is dropped (exact float
+//     test on equal cells; the tables drop by cells alone). If a dropped q
+//     dominated a kept p, the pruner that drops q would strictly dominate p,
+//     so the kept entries (survivors) decide each other's status alone.
+//  2. The survivors, counting-sorted by cell sum over S (a
 //     dominator's sum is never larger), go through a sort-filter skyline in
-//     batches of 1,024: each entry is tested against the window of skyline
+//     batches of 256, 512 and then 1,024: each entry is tested against the window of skyline
 //     points found so far (strict domination drops it), the batch's
 //     remaining entries against each other, and the batch's new skyline
 //     points join the window. An entry can only be dominated by an entry of
@@ -576,7 +576,7 @@ __device__ uint32_t lv_sfs_cta(const CubAttrs& A, uint32_t c, uint32_t g,
   }
   __syncthreads();
 
-  // 2. Sort-filter skyline in batches of kLvThreads entries. The tests are
+  // 2. Sort-filter skyline in batches of up to kLvThreads entries. The tests are
   // warp-cooperative: a warp takes one entry at a time and its lanes test
   // 32 window (or batch) entries per step, so no warp waits for its slowest
   // lane's scan.

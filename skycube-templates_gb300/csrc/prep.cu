@@ -749,7 +749,7 @@ int launch_status_keep(cudaStream_t s, const uint8_t* st, const uint32_t* m_ptr,
 
 int launch_scan_counts(cudaStream_t s, const uint32_t* in, uint64_t len, uint64_t* bsum,
                        uint64_t* out, uint32_t T, uint32_t nsub, uint64_t* csr_off) {
-  const uint32_t g = (uint32_t)((len + kScanBlock - 1) / kScanBlock);  // len >= 32
+  const uint32_t g = (uint32_t)((len + kScanBlock - 1) / kScanBlock);  // len >= 1
   const int scan = g > kSelfScanBlocks;
   if (g > 1) {
     k_scan_partials<<<g, 1024, 0, s>>>(in, len, bsum);

@@ -9,9 +9,9 @@ Vocabulary follows the skycube suite: a *cuboid* is a non-empty subspace,
 given as a bitmask over the d attributes; its *skyline* holds the point ids
 (row indices) no other point dominates on it, its *extended skyline* the
 dominated points nobody strictly dominates. ``algo`` is "mdmc" or "sdsc"
-(the suite's ``-s``), ``mode`` "plain" (one launch sequence per cuboid) or
-"batched" (one persistent launch for all cuboids), ``max_d`` the suite's
-``-m`` cap and ``depth`` its ``-d`` grid depth.
+(the suite's ``-s``), ``mode`` "plain" (each cuboid by itself, by lattice
+level) or "batched" (one persistent launch for all cuboids), ``max_d`` the
+suite's ``-m`` cap and ``depth`` its ``-d`` grid depth.
 """
 import ctypes
 import os
