@@ -40,11 +40,9 @@ def left_out(x, cells, hashes):
     for i in range(len(x)):
         b = i // 32
         block = range(32 * b, min(len(x), 32 * b + 32))
-        heads = [j for j in block if all(hashes[t] != hashes[j] for t in range(32 * b, j))]
-        if len(heads) == len(block) and len(block) == 32:
-            continue
-        src = next(j for j in block if hashes[j] == hashes[i])
-        if b > 0 and i in heads:
+        same = [j for j in block if hashes[j] == hashes[i]]
+        src = same[0]
+        if b > 0 and i == src and len(same) > 1:
             prev = [j for j in range(32 * b - 32, 32 * b) if hashes[j] == hashes[i]]
             src = prev[0] if prev else src
         out[i] = src != i and (x[i] == x[src]).all()
