@@ -2210,12 +2210,14 @@ int skc_autotune(skc_context* ctx, skc_dataset* ds, const skc_options* base, int
   cur.chunk = o.chunk ? o.chunk : kDefaultChunk;
   cur.blocks_per_sm = o.blocks_per_sm;
 
+  int form = 0;
   auto time_run = [&](const RunParams& P, float* ms) -> int {
     float bestv = 3.0e38f;
     for (int r = 0; r < repeats; ++r) {
       skc_result* R = nullptr;
       SKC_TRY(skycube_exec(E, ds, &o, &R, &P));
       bestv = std::min(bestv, E.ms);
+      form = R->form;
       skc_result_free(R);
     }
     *ms = bestv;
@@ -2225,8 +2227,10 @@ int skc_autotune(skc_context* ctx, skc_dataset* ds, const skc_options* base, int
   SKC_TRY(time_run(cur, &cur_ms));
 
   // One pass of coordinate search over the parameters the options leave
-  // automatic; a change is kept when it is at least 2% faster.
-  const bool bitmap_stage = !o.subspace && !(o.algo == SKC_ALGO_SDSC && o.mode == SKC_MODE_PLAIN);
+  // automatic; a change is kept when it is at least 2% faster. All but the
+  // pruners belong to the bitmap kernel: a call that another form computes
+  // would store what its noise prefers for a dataset that takes the bitmaps.
+  const bool bitmap_stage = form == SKC_FORM_BITMAPS;
   auto try_values = [&](int RunParams::*field, const std::vector<int>& values) -> int {
     for (int v : values) {
       if (cur.*field == v) continue;
@@ -2241,7 +2245,7 @@ int skc_autotune(skc_context* ctx, skc_dataset* ds, const skc_options* base, int
     }
     return SKC_OK;
   };
-  if (!o.depth) SKC_TRY(try_values(&RunParams::depth, {7, 6, 5, 4, 3, 2}));
+  if (bitmap_stage && !o.depth) SKC_TRY(try_values(&RunParams::depth, {7, 6, 5, 4, 3, 2}));
   if (!o.pq_size) {
     std::vector<int> pqs;
     for (int v : {0, 32, 128, 512, kMaxPruners})
